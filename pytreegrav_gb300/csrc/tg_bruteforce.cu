@@ -1,15 +1,18 @@
 // Exact direct summation (pytreegrav bruteforce.py).
 //
-// FP64: one target per thread, sources staged through shared memory tiles, every operation
-// rounded once in pytreegrav's expression order and summed over sources in ascending order -- the
-// same arithmetic as the per-target CPU kernels (bruteforce.py:7-50, 86-116, 164-256, 259-282,
-// 319-386), so results agree bit for bit. This is the FP64 judge the FP32 walk is scored against.
+// FP64: every operation rounded once in pytreegrav's expression order and summed over sources in
+// ascending order -- the same arithmetic as the per-target CPU kernels (bruteforce.py:7-50, 86-116,
+// 164-256, 259-282, 319-386), so results agree bit for bit. This is the FP64 judge the FP32 walk is scored
+// against. Two forms: the pairs' terms formed by several warps and added in order by one (k_bf64_chain),
+// and one target per thread (k_bf64) where such blocks fill the GPU.
 //
 // FP32: the fast path (the numba-cuda CudaPotentialBruteforce/CudaAccelBruteforce of cuda.py:627-796
 // rebuilt): tiles of 256 sources in shared memory, two targets per thread so every broadcast source
 // load feeds two interactions, rsqrt, and tile sums added into Kahan-compensated accumulators. For
 // the potential and acceleration, four lanes share each pair of targets (k_bf32_split) and the two
 // targets are computed with paired f32x2 arithmetic.
+#include <algorithm>
+
 #include "tg_common.cuh"
 
 namespace tg {
@@ -161,6 +164,187 @@ __global__ void __launch_bounds__(BF64_THREADS) k_bf64(const double *pt, const d
     if (FIELDS & BF_TID) {
         double v[9] = {T0, T1, T2, T1, T4, T5, T2, T5, T8};
         for (int q = 0; q < 9; q++) o[k + q] = dmul(G, v[q]);
+    }
+}
+
+// Few targets: k_bf64 gives a target one thread, and its FP64 stream (~33 instructions per source, one
+// issued every ~76 cycles whatever the number of active lanes) is then the kernel's length: 700
+// targets are 22 warps on 608 sub-partitions. Here a block takes T targets and cuts the stream in
+// two: seven warps form the pairs' terms, lane = source, 32 sources of one target at a time, into a
+// ring of tiles in shared memory, and the eighth adds the terms, lane = (target, component), one
+// FP64 add per source. Every sum takes the same terms in the same ascending order as k_bf64's, so the
+// results are the same bits: a pair that k_bf64 skips adds -0.0, the exact identity of a sum.
+// The adder needs one instruction per source and block, the others ~30 T / 32: T is the targets'
+// number over the SMs, at most what fills the adder's lanes. Two items per producer and stage keep the
+// pipeline's fill short against 700 sources. The softening tests run on the integer units, and 1 / x is
+// __drcp_rn, the same correctly rounded value as the division.
+// Acceleration: 700 bodies' own 860 -> 53 us (FP64 pipe 64 % busy; floor ~28 us of pairs); 2000 sources
+// and 100 targets 2499 -> 116 us, 2000 targets 2498 -> 318, 1e4 2499 -> 1402, 2e4 4608 -> 2760.
+constexpr int BFC_PRODUCERS = 7, BFC_THREADS = 32 * (BFC_PRODUCERS + 1);
+constexpr int BFC_UNITS = 2;                                 // (tile, target) items per producer and stage
+constexpr int BFC_STAGE = BFC_PRODUCERS * BFC_UNITS;         // items per stage
+constexpr int BFC_ROW = 33;                                  // doubles per chain and tile (odd: no bank conflicts)
+template <int FIELDS>
+__host__ __device__ constexpr int bfc_comps() {
+    return ((FIELDS & BF_POT) ? 1 : 0) + ((FIELDS & BF_ACC) ? 3 : 0) + ((FIELDS & BF_TID) ? 6 : 0);
+}
+// k_bf64 is the faster form only where its blocks of 128 targets, one per SM, fill their last wave. Its
+// time goes by whole waves (2000 sources, acceleration: 2.31 ms each), this form's by targets and with
+// the adder (60000 targets 7.80 ms, 1.10 times as much per target as a full wave; potential 1.11,
+// tidal tensor 1.06). With every field (ten components, three targets per block) this form is the
+// faster one throughout: 18.0 ms for 60000 targets against 20.5 for three full waves (58368).
+constexpr int64_t BFC_MAX_SOURCES = 1 << 29;  // (tile, target) items are counted in 32 bits
+template <int FIELDS>
+static bool bf64_chain_better(int64_t nt, int64_t ns) {
+    if (ns > BFC_MAX_SOURCES) return false;
+    if (FIELDS == (BF_POT | BF_ACC | BF_TID)) return true;
+    const int64_t wave = (int64_t)num_sms() * BF64_THREADS, waves = (nt + wave - 1) / wave;
+    return 100 * nt < 92 * waves * wave;
+}
+// Tiles of the ring: a stage writes at most BFC_STAGE / T + 2 tiles while as many are summed.
+__host__ __device__ inline int bfc_ring(int T) { return 2 * BFC_STAGE / T + 3; }
+
+// Order key of a softening length: a signed integer of the same order as the value (-0.0 as +0.0), the
+// least for NaN, which no distance is below.
+__device__ __forceinline__ long long soft_key(double h) {
+    const long long b = __double_as_longlong(h);
+    const long long mag = b & 0x7fffffffffffffffll;
+    if (mag > 0x7ff0000000000000ll) return (long long)0x8000000000000000ull;
+    return b < 0 ? -mag : mag;
+}
+// r < pymax(a, b) for a distance r (>= 0 or NaN), decided on the integer units: pymax is NaN when a
+// is, and a when b is.
+__device__ __forceinline__ bool below_max(double r, long long ka, long long kb) {
+    const long long none = (long long)0x8000000000000000ull;
+    const long long k = ka == none ? none : (kb > ka ? kb : ka);
+    return (__double_as_longlong(r) & 0x7fffffffffffffffll) < k;
+}
+
+template <int FIELDS, bool MUTUAL>
+__global__ void __launch_bounds__(BFC_THREADS) k_bf64_chain(const double *pt, const double *ht, int64_t nt,
+                                                            const double *ps, const double *ms, const double *hs,
+                                                            int64_t ns, int T, double G, double *out, int W) {
+    extern __shared__ double bfc_ring_mem[];  // [ring][T * C][BFC_ROW]
+    constexpr int C = bfc_comps<FIELDS>();
+    __shared__ double tx[32], ty[32], tz[32], th[32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int ring = bfc_ring(T);
+    const int64_t t0 = (int64_t)blockIdx.x * T;
+    if (threadIdx.x < T) {
+        const int64_t i = t0 + threadIdx.x < nt ? t0 + threadIdx.x : nt - 1;
+        tx[threadIdx.x] = pt[3 * i];
+        ty[threadIdx.x] = pt[3 * i + 1];
+        tz[threadIdx.x] = pt[3 * i + 2];
+        th[threadIdx.x] = ht[i];
+    }
+    __syncthreads();
+    const int ntiles = (int)((ns + 31) / 32), nitems = ntiles * T;  // ns <= BFC_MAX_SOURCES
+    const int nstages = (nitems + BFC_STAGE - 1) / BFC_STAGE;
+    double sum = 0.0;  // the adder's chain
+    int consumed = 0;  // tiles added so far
+    for (int st = 0; st <= nstages; st++) {
+        if (w < BFC_PRODUCERS) {
+#pragma unroll 1
+            for (int u = 0; u < BFC_UNITS; u++) {
+                const int item = st * BFC_STAGE + w * BFC_UNITS + u;
+                if (item >= nitems) break;
+                const int tile = item / T, t = item - tile * T;
+                const int64_t j = (int64_t)tile * 32 + lane;
+                double term[C];
+#pragma unroll
+                for (int c = 0; c < C; c++) term[c] = -0.0;
+                if (j < ns && !(MUTUAL && j == t0 + t)) {
+                    const double m = ms[j], hj = hs[j], hti = th[t];
+                    const double d0 = dsub(ps[3 * j], tx[t]), d1 = dsub(ps[3 * j + 1], ty[t]);
+                    const double d2 = dsub(ps[3 * j + 2], tz[t]);
+                    const double r2 = dadd(dadd(dmul(d0, d0), dmul(d1, d1)), dmul(d2, d2));
+                    const double r = __dsqrt_rn(r2);
+                    const long long kt = soft_key(hti), kj = soft_key(hj);
+                    if (FIELDS & BF_POT) {  // phi - m / r is phi + (-(m / r))
+                        const bool in = MUTUAL ? below_max(r, kt, kj) : below_max(r, kj, kt);
+                        // mutual: r > 0 outside the softening; else r != 0 (true of NaN too)
+                        const long long rb = __double_as_longlong(r) & 0x7fffffffffffffffll;
+                        if (MUTUAL) {
+                            if (in) term[0] = dmul(m, potential_kernel_x(r, pymax(hti, hj)));
+                            else if (rb > 0 && rb <= 0x7ff0000000000000ll) term[0] = -ddiv(m, r);
+                        } else if (rb != 0) {
+                            if (in) term[0] = dmul(m, potential_kernel_x(r, pymax(hj, hti)));
+                            else term[0] = -ddiv(m, r);
+                        }
+                    }
+                    if ((FIELDS & (BF_ACC | BF_TID)) && (__double_as_longlong(r2) << 1) != 0) {
+                        const bool in = below_max(r, kt, kj);
+                        const double h = in ? pymax(hti, hj) : 0.0;
+                        double *p = term + ((FIELDS & BF_POT) ? 1 : 0);
+                        if (FIELDS & BF_ACC) {
+                            // 1 / x correctly rounded is the same value from __drcp_rn
+                            const double mf = in ? dmul(force_kernel_x(r, h), m) : dmul(m, __drcp_rn(dmul(r2, r)));
+                            p[0] = dmul(mf, d0);
+                            p[1] = dmul(mf, d1);
+                            p[2] = dmul(mf, d2);
+                            p += 3;
+                        }
+                        if (FIELDS & BF_TID) {
+                            double K, Q;
+                            if (in) {
+                                K = dmul(m, force_kernel_x(r, h));
+                                Q = dmul(m, tidal_kernel_x(r, h));
+                            } else {
+                                K = ddiv(m, dmul(r, r2));
+                                Q = ddiv(dmul(3.0, K), r2);
+                            }
+                            const double q0 = dmul(Q, d0), q1 = dmul(Q, d1);
+                            p[0] = dsub(dmul(q0, d0), K);
+                            p[1] = dmul(q0, d1);
+                            p[2] = dmul(q0, d2);
+                            p[3] = dsub(dmul(q1, d1), K);
+                            p[4] = dmul(q1, d2);
+                            p[5] = dsub(dmul(dmul(Q, d2), d2), K);
+                        }
+                    }
+                }
+                double *slot = bfc_ring_mem + ((tile % ring) * T + t) * (C * BFC_ROW) + lane;
+#pragma unroll
+                for (int c = 0; c < C; c++) slot[c * BFC_ROW] = term[c];
+            }
+        } else {
+            // the tiles that the earlier stages completed
+            const int ready = min(st * BFC_STAGE / T, ntiles);
+            if (lane < T * C)
+                for (; consumed < ready; consumed++) {
+                    const double *row = bfc_ring_mem + (consumed % ring) * (T * C * BFC_ROW) + lane * BFC_ROW;
+#pragma unroll 16
+                    for (int k = 0; k < 32; k++) sum = dadd(sum, row[k]);
+                }
+        }
+        __syncthreads();
+    }
+    if (w == BFC_PRODUCERS && lane < T * C) {
+        const int t = lane / C;
+        int c = lane - t * C;
+        if (t0 + t >= nt) return;
+        double *o = out + (t0 + t) * W;
+        const double v = dmul(G, sum);
+        if (FIELDS & BF_POT) {
+            if (c == 0) {
+                o[0] = v;
+                return;
+            }
+            c--;
+            o++;
+        }
+        if (FIELDS & BF_ACC) {
+            if (c < 3) {
+                o[c] = v;
+                return;
+            }
+            c -= 3;
+            o += 3;
+        }
+        // xx xy xz yy yz zz into the symmetric 3x3
+        const int row = c < 3 ? 0 : (c < 5 ? 1 : 2), col = c < 3 ? c : (c < 5 ? c - 2 : 2);
+        o[3 * row + col] = v;
+        o[3 * col + row] = v;
     }
 }
 
@@ -455,9 +639,18 @@ __global__ void __launch_bounds__(BF32S_THREADS) k_bf32_split(const double *pt, 
 }
 
 template <int FIELDS, bool MUTUAL>
-static void launch_bf(int precision, const double *pt, const double *ht, int64_t nt, const double *ps,
+static tg_status launch_bf(int precision, const double *pt, const double *ht, int64_t nt, const double *ps,
                       const double *ms, const double *hs, int64_t ns, double G, double *out, int W, cudaStream_t st) {
-    if (precision == TG_FP64) {
+    if (precision == TG_FP64 && bf64_chain_better<FIELDS>(nt, ns)) {
+        constexpr int C = bfc_comps<FIELDS>(), most = 32 / C;
+        // as many targets per block as let every SM have the same number of blocks
+        const int64_t sms = num_sms();
+        const int T = div_up(nt, sms * div_up(nt, sms * most));
+        const size_t smem = sizeof(double) * (size_t)bfc_ring(T) * T * C * BFC_ROW;
+        auto kern = k_bf64_chain<FIELDS, MUTUAL>;
+        TG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        { kern<<<div_up(nt, T), BFC_THREADS, smem, st>>>(pt, ht, nt, ps, ms, hs, ns, T, G, out, W); tg::note_launch(); }
+    } else if (precision == TG_FP64) {
         { k_bf64<FIELDS, MUTUAL><<<div_up(nt, BF64_THREADS), BF64_THREADS, 0, st>>>(pt, ht, nt, ps, ms, hs, ns, G, out, W); tg::note_launch(); }
     } else if constexpr ((FIELDS & BF_TID) == 0) {
         { k_bf32_split<FIELDS, MUTUAL><<<div_up(nt, BF32S_TARGETS), BF32S_THREADS, 0, st>>>(pt, ht, nt, ps, ms, hs, ns,
@@ -466,19 +659,20 @@ static void launch_bf(int precision, const double *pt, const double *ht, int64_t
         { k_bf32<FIELDS, MUTUAL><<<div_up(nt, BF32_THREADS * BF32_TPT), BF32_THREADS, 0, st>>>(pt, ht, nt, ps, ms, hs, ns,
                                                                                            G, out, W); tg::note_launch(); }
     }
+    return TG_OK;
 }
 
 template <bool MUTUAL>
-static void dispatch_bf(int fields, int precision, const double *pt, const double *ht, int64_t nt, const double *ps,
+static tg_status dispatch_bf(int fields, int precision, const double *pt, const double *ht, int64_t nt, const double *ps,
                         const double *ms, const double *hs, int64_t ns, double G, double *out, int W, cudaStream_t st) {
     switch (fields) {
-        case 1: launch_bf<1, MUTUAL>(precision, pt, ht, nt, ps, ms, hs, ns, G, out, W, st); break;
-        case 2: launch_bf<2, MUTUAL>(precision, pt, ht, nt, ps, ms, hs, ns, G, out, W, st); break;
-        case 3: launch_bf<3, MUTUAL>(precision, pt, ht, nt, ps, ms, hs, ns, G, out, W, st); break;
-        case 4: launch_bf<4, MUTUAL>(precision, pt, ht, nt, ps, ms, hs, ns, G, out, W, st); break;
-        case 5: launch_bf<5, MUTUAL>(precision, pt, ht, nt, ps, ms, hs, ns, G, out, W, st); break;
-        case 6: launch_bf<6, MUTUAL>(precision, pt, ht, nt, ps, ms, hs, ns, G, out, W, st); break;
-        default: launch_bf<7, MUTUAL>(precision, pt, ht, nt, ps, ms, hs, ns, G, out, W, st); break;
+        case 1: return launch_bf<1, MUTUAL>(precision, pt, ht, nt, ps, ms, hs, ns, G, out, W, st);
+        case 2: return launch_bf<2, MUTUAL>(precision, pt, ht, nt, ps, ms, hs, ns, G, out, W, st);
+        case 3: return launch_bf<3, MUTUAL>(precision, pt, ht, nt, ps, ms, hs, ns, G, out, W, st);
+        case 4: return launch_bf<4, MUTUAL>(precision, pt, ht, nt, ps, ms, hs, ns, G, out, W, st);
+        case 5: return launch_bf<5, MUTUAL>(precision, pt, ht, nt, ps, ms, hs, ns, G, out, W, st);
+        case 6: return launch_bf<6, MUTUAL>(precision, pt, ht, nt, ps, ms, hs, ns, G, out, W, st);
+        default: return launch_bf<7, MUTUAL>(precision, pt, ht, nt, ps, ms, hs, ns, G, out, W, st);
     }
 }
 
@@ -487,8 +681,8 @@ tg_status run_bruteforce(const double *pt, const double *ht, int64_t nt, const d
                          cudaStream_t st) {
     int W = ((fields & BF_POT) ? 1 : 0) + ((fields & BF_ACC) ? 3 : 0) + ((fields & BF_TID) ? 9 : 0);
     if (nt <= 0) return TG_OK;
-    if (mutual) dispatch_bf<true>(fields, precision, pt, ht, nt, ps, ms, hs, ns, G, out, W, st);
-    else dispatch_bf<false>(fields, precision, pt, ht, nt, ps, ms, hs, ns, G, out, W, st);
+    if (mutual) TG_TRY(dispatch_bf<true>(fields, precision, pt, ht, nt, ps, ms, hs, ns, G, out, W, st));
+    else TG_TRY(dispatch_bf<false>(fields, precision, pt, ht, nt, ps, ms, hs, ns, G, out, W, st));
     TG_CUDA(cudaGetLastError());
     return TG_OK;
 }
