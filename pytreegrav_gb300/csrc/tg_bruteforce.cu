@@ -9,8 +9,10 @@
 // FP32: the fast path (the numba-cuda CudaPotentialBruteforce/CudaAccelBruteforce of cuda.py:627-796
 // rebuilt): tiles of 256 sources in shared memory, two targets per thread so every broadcast source
 // load feeds two interactions, rsqrt, and tile sums added into Kahan-compensated accumulators. For
-// the potential and acceleration, four lanes share each pair of targets (k_bf32_split) and the two
-// targets are computed with paired f32x2 arithmetic.
+// the potential and acceleration, four lanes share each pair of targets (k_bf32_split), the two
+// targets are computed with paired f32x2 arithmetic, and the sources are narrowed once (k_bf32_prep).
+#include <cuda_pipeline.h>
+
 #include <algorithm>
 
 #include "tg_common.cuh"
@@ -479,14 +481,31 @@ __global__ void __launch_bounds__(BF32_THREADS) k_bf32(const double *pt, const d
 }
 
 // Potential and/or acceleration, the main FP32 form: BF32S_LANES lanes share each pair of targets,
-// lane q of the group taking the sources k = q (mod BF32S_LANES) of every shared-memory tile, so a
-// target set of 1e5 still fills the GPU; the lanes' Kahan-compensated sums are combined at the end
-// by a fixed pattern of shuffles (deterministic). The two targets of a lane are computed together
+// lane q of the group taking the sources k = q (mod BF32S_LANES) of every tile, so a target set of 1e5
+// still fills the GPU; the lanes' Kahan-compensated sums (compensated once per tile) are combined at
+// the end by a fixed pattern of shuffles (deterministic). The two targets are computed together
 // with paired f32x2 arithmetic for every source outside both softening lengths (with a 1e-5 margin)
 // and not coincident; any other source takes bf32_pair for each target.
-constexpr int BF32S_THREADS = 256;
+//
+// Bound by issue slots and the FP32 pipe (12 operations and an rsqrt per pair of particles; 0.75 ms at
+// 5e4 x 5e4), and by the chain of one source's operations where the targets are few. For that:
+//   * BF32S_UNROLL sources at a time, their distances first: the chains overlap (5e4 sources, acceleration:
+//     1000 targets 778 us at 2, 504 at 4, 433 at 8 and 411 at 16, where 1e5 targets lose 30 % to spills);
+//   * one test per distance against a bound beyond which no source of the tile (its largest h^2 comes
+//     from k_bf32_prep) and neither target is softened, instead of the exact test, which only a batch
+//     that fails the bound takes, source by source;
+//   * the sources are narrowed to FP32 once (k_bf32_prep), not by every block for every tile, which kept the
+//     FP64 pipe busy with conversions.
+// 5e4 sources, acceleration, before and after: 1000 targets 1330 -> 433 us, 2e4 1645 -> 761, 50001
+// 2262 -> 1403, 1e5 4271 -> 2461. Measured and dropped: two pairs of targets per lane (50001: 1458;
+// 1e5: 2686; 1000: 761), each staged value duplicated for the paired operands (1e5: 2795; shared-memory
+// reads return 4 words per lane and cycle), scalar subtractions and products (1e5: 2644).
+constexpr int BF32S_THREADS = 128;
+constexpr int BF32S_BLOCKS_PER_SM = 4;  // at most 128 registers
 constexpr int BF32S_LANES = 4;
-constexpr int BF32S_TARGETS = 2 * BF32S_THREADS / BF32S_LANES;  // per block
+constexpr int BF32S_TILE = 256;  // sources per tile
+constexpr int BF32S_UNROLL = 8;
+constexpr int BF32S_PAIRS = BF32S_THREADS / BF32S_LANES;  // pairs of targets per block
 
 typedef unsigned long long bf2;
 __device__ __forceinline__ bf2 bf2_pack(float a, float b) {
@@ -513,58 +532,108 @@ __device__ __forceinline__ bf2 bf2_sub(bf2 a, bf2 b) {
     return d;
 }
 
+__device__ __forceinline__ float bf32_rsqrt_normal(float x) {  // rsqrtf's value for a normal x > 0
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
+// Sources in FP32, (x, y, z, m) and (h, h^2), and each tile's largest h^2 (infinite when one is NaN, so that
+// the tile's sources all take the exact test).
+__global__ void __launch_bounds__(BF32S_TILE) k_bf32_prep(const double *ps, const double *ms, const double *hs,
+                                                          int64_t ns, float4 *src, float2 *soft, float *tile_h2) {
+    __shared__ float wmax[BF32S_TILE / 32];
+    const int64_t j = (int64_t)blockIdx.x * BF32S_TILE + threadIdx.x;
+    float h2 = 0.f;
+    if (j < ns) {
+        const float h = d2f(hs[j]);
+        h2 = h * h;
+        src[j] = make_float4(d2f(ps[3 * j]), d2f(ps[3 * j + 1]), d2f(ps[3 * j + 2]), d2f(ms[j]));
+        soft[j] = make_float2(h, h2);
+        if (!(h2 == h2)) h2 = INFINITY;
+    }
+    for (int o = 16; o; o >>= 1) h2 = fmaxf(h2, __shfl_xor_sync(FULL, h2, o));
+    if ((threadIdx.x & 31) == 0) wmax[threadIdx.x >> 5] = h2;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < BF32S_TILE / 32; w++) h2 = fmaxf(h2, wmax[w]);
+        tile_h2[blockIdx.x] = h2;
+    }
+}
+
 template <int FIELDS, bool MUTUAL>
-__global__ void __launch_bounds__(BF32S_THREADS) k_bf32_split(const double *pt, const double *ht, int64_t nt,
-                                                              const double *ps, const double *ms,
-                                                              const double *hs, int64_t ns, double G,
-                                                              double *out, int W) {
-    __shared__ float4 spos[BF32S_THREADS];
-    __shared__ float sh[BF32S_THREADS], sh2[BF32S_THREADS];
+__global__ void __launch_bounds__(BF32S_THREADS, BF32S_BLOCKS_PER_SM) k_bf32_split(
+    const double *pt, const double *ht, int64_t nt, const float4 *src, const float2 *soft, const float *tile_h2,
+    int64_t ns, double G, double *out, int W) {
+    __shared__ float4 spos[2][BF32S_TILE];
+    __shared__ float2 ssoft[2][BF32S_TILE];
+    constexpr int C0 = (FIELDS & BF_POT) ? 0 : 1, C1 = (FIELDS & BF_ACC) ? 4 : 1;  // components used
     const int q = threadIdx.x % BF32S_LANES;
-    const int64_t pair = (int64_t)blockIdx.x * (BF32S_THREADS / BF32S_LANES) + threadIdx.x / BF32S_LANES;
-    float tx[2], ty[2], tz[2], th[2], th2[2];
-    int64_t ti[2];
+    const int64_t t0 = 2 * ((int64_t)blockIdx.x * BF32S_PAIRS + threadIdx.x / BF32S_LANES);  // targets t0, t0 + 1
+    float tx[2], ty[2], tz[2], th[2], th2[2], th2max = 0.f;
     float S[2][4], C[2][4];
 #pragma unroll
     for (int u = 0; u < 2; u++) {
-        ti[u] = 2 * pair + u;
-        const int64_t i = ti[u] < nt ? ti[u] : 0;
-        tx[u] = (float)pt[3 * i];
-        ty[u] = (float)pt[3 * i + 1];
-        tz[u] = (float)pt[3 * i + 2];
-        th[u] = (float)ht[i];
+        const int64_t i = t0 + u < nt ? t0 + u : 0;
+        tx[u] = d2f(pt[3 * i]);
+        ty[u] = d2f(pt[3 * i + 1]);
+        tz[u] = d2f(pt[3 * i + 2]);
+        th[u] = d2f(ht[i]);
         th2[u] = th[u] * th[u];
+        th2max = fmaxf(th2max, th2[u] == th2[u] ? th2[u] : INFINITY);
 #pragma unroll
         for (int c = 0; c < 4; c++) S[u][c] = C[u][c] = 0.f;
     }
     const bf2 TX = bf2_pack(tx[0], tx[1]), TY = bf2_pack(ty[0], ty[1]), TZ = bf2_pack(tz[0], tz[1]);
-    for (int64_t base = 0; base < ns; base += BF32S_THREADS) {
-        const int64_t j = base + threadIdx.x;
-        if (j < ns) {
-            const float hj = (float)hs[j];
-            spos[threadIdx.x] = make_float4((float)ps[3 * j], (float)ps[3 * j + 1], (float)ps[3 * j + 2], (float)ms[j]);
-            sh[threadIdx.x] = hj;
-            sh2[threadIdx.x] = hj * hj;
+    const int64_t ntiles = (ns + BF32S_TILE - 1) / BF32S_TILE;
+    auto stage = [&](int64_t tile, int buf) {  // the next tile is copied while one is summed
+        for (int i = threadIdx.x; i < BF32S_TILE; i += BF32S_THREADS) {
+            const int64_t j = tile * BF32S_TILE + i;
+            if (j < ns) {
+                __pipeline_memcpy_async(&spos[buf][i], src + j, sizeof(float4));
+                __pipeline_memcpy_async(&ssoft[buf][i], soft + j, sizeof(float2));
+            }
         }
+        __pipeline_commit();
+    };
+    stage(0, 0);
+    for (int64_t tile = 0; tile < ntiles; tile++) {
+        const int buf = (int)(tile & 1);
+        stage(tile + 1, buf ^ 1);  // past the last tile: nothing to copy
+        __pipeline_wait_prior(1);
         __syncthreads();
-        const int lim = (int)((ns - base) < BF32S_THREADS ? (ns - base) : BF32S_THREADS);
+        const int64_t base = tile * BF32S_TILE;
+        const int lim = (int)((ns - base) < BF32S_TILE ? (ns - base) : BF32S_TILE);
+        // beyond this squared distance no pair of the tile is softened, and r2 is a normal number
+        const float far2 = fmaxf(fmaxf(tile_h2[tile], th2max) * 1.00001f, 1.2e-38f);
         bf2 ph = 0, ax = 0, ay = 0, az = 0;  // the two targets' tile sums (bit pattern 0 is +0.0f, +0.0f)
         float P[2][10];
 #pragma unroll
         for (int u = 0; u < 2; u++)
 #pragma unroll
             for (int c = 0; c < 10; c++) P[u][c] = 0.f;
-        for (int k = q; k < lim; k += BF32S_LANES) {
-            const float4 s = spos[k];
+        auto add_far = [&](float m, bf2 dx, bf2 dy, bf2 dz, float ri0, float ri1) {
+            const bf2 rinv = bf2_pack(ri0, ri1);
+            const bf2 mr = bf2_mul(bf2_pack(m, m), rinv);
+            if (FIELDS & BF_POT) ph = bf2_sub(ph, mr);
+            if (FIELDS & BF_ACC) {
+                const bf2 K = bf2_mul(mr, bf2_mul(rinv, rinv));
+                ax = bf2_fma(K, dx, ax);
+                ay = bf2_fma(K, dy, ay);
+                az = bf2_fma(K, dz, az);
+            }
+        };
+        // one source with the exact test
+        auto one = [&](int k) {
+            const float4 s = spos[buf][k];
+            const float2 hk = ssoft[buf][k];
             const bf2 dx = bf2_sub(bf2_pack(s.x, s.x), TX), dy = bf2_sub(bf2_pack(s.y, s.y), TY);
             const bf2 dz = bf2_sub(bf2_pack(s.z, s.z), TZ);
-            const bf2 r2 = bf2_fma(dz, dz, bf2_fma(dy, dy, bf2_mul(dx, dx)));
             float r20, r21;
-            bf2_unpack(r2, r20, r21);
-            const float hs2 = sh2[k];
-            const float lim0 = fmaxf(hs2, th2[0]) * 1.00001f, lim1 = fmaxf(hs2, th2[1]) * 1.00001f;
+            bf2_unpack(bf2_fma(dz, dz, bf2_fma(dy, dy, bf2_mul(dx, dx))), r20, r21);
+            const float lim0 = fmaxf(hk.y, th2[0]) * 1.00001f, lim1 = fmaxf(hk.y, th2[1]) * 1.00001f;
             bool slow = !(r20 > lim0) || !(r21 > lim1) || !(r20 > 0.f) || !(r21 > 0.f);
-            if (MUTUAL) slow = slow || base + k == ti[0] || base + k == ti[1];
+            if (MUTUAL) slow = slow || base + k == t0 || base + k == t0 + 1;
             if (slow) {
                 float d[3][2];
                 bf2_unpack(dx, d[0][0], d[0][1]);
@@ -572,43 +641,51 @@ __global__ void __launch_bounds__(BF32S_THREADS) k_bf32_split(const double *pt, 
                 bf2_unpack(dz, d[2][0], d[2][1]);
 #pragma unroll
                 for (int u = 0; u < 2; u++) {
-                    const bool skip = MUTUAL && (base + k == ti[u]);
-                    bf32_pair<FIELDS>(s.w, sh[k], th[u], d[0][u], d[1][u], d[2][u], skip, P[u]);
+                    const bool skip = MUTUAL && (base + k == t0 + u);
+                    bf32_pair<FIELDS>(s.w, hk.x, th[u], d[0][u], d[1][u], d[2][u], skip, P[u]);
                 }
             } else {
-                const float r0 = rsqrtf(r20), r1 = rsqrtf(r21);
-                const bf2 rinv = bf2_pack(r0, r1);
-                const bf2 mr = bf2_mul(bf2_pack(s.w, s.w), rinv);
-                if (FIELDS & BF_POT) ph = bf2_sub(ph, mr);
-                if (FIELDS & BF_ACC) {
-                    const bf2 K = bf2_mul(mr, bf2_mul(rinv, rinv));
-                    ax = bf2_fma(K, dx, ax);
-                    ay = bf2_fma(K, dy, ay);
-                    az = bf2_fma(K, dz, az);
-                }
+                add_far(s.w, dx, dy, dz, rsqrtf(r20), rsqrtf(r21));
+            }
+        };
+        int k = q;
+        for (; k + (BF32S_UNROLL - 1) * BF32S_LANES < lim; k += BF32S_UNROLL * BF32S_LANES) {
+            bf2 dx[BF32S_UNROLL], dy[BF32S_UNROLL], dz[BF32S_UNROLL];
+            float r2[BF32S_UNROLL][2], m[BF32S_UNROLL];
+            bool far = true;
+#pragma unroll
+            for (int e = 0; e < BF32S_UNROLL; e++) {
+                const float4 s = spos[buf][k + e * BF32S_LANES];
+                m[e] = s.w;
+                dx[e] = bf2_sub(bf2_pack(s.x, s.x), TX);
+                dy[e] = bf2_sub(bf2_pack(s.y, s.y), TY);
+                dz[e] = bf2_sub(bf2_pack(s.z, s.z), TZ);
+                bf2_unpack(bf2_fma(dz[e], dz[e], bf2_fma(dy[e], dy[e], bf2_mul(dx[e], dx[e]))), r2[e][0], r2[e][1]);
+                far = far && r2[e][0] > far2 && r2[e][1] > far2;
+            }
+            if (far) {
+#pragma unroll
+                for (int e = 0; e < BF32S_UNROLL; e++)
+                    add_far(m[e], dx[e], dy[e], dz[e], bf32_rsqrt_normal(r2[e][0]), bf32_rsqrt_normal(r2[e][1]));
+            } else {
+#pragma unroll 1
+                for (int e = 0; e < BF32S_UNROLL; e++) one(k + e * BF32S_LANES);
             }
         }
-        float a0, a1;
-        if (FIELDS & BF_POT) {
-            bf2_unpack(ph, a0, a1);
-            P[0][0] += a0;
-            P[1][0] += a1;
-        }
-        if (FIELDS & BF_ACC) {
-            bf2_unpack(ax, a0, a1);
-            P[0][1] += a0;
-            P[1][1] += a1;
-            bf2_unpack(ay, a0, a1);
-            P[0][2] += a0;
-            P[1][2] += a1;
-            bf2_unpack(az, a0, a1);
-            P[0][3] += a0;
-            P[1][3] += a1;
+#pragma unroll 1
+        for (; k < lim; k += BF32S_LANES) one(k);
+        const bf2 fast[4] = {ph, ax, ay, az};
+#pragma unroll
+        for (int c = C0; c < C1; c++) {
+            float a0, a1;
+            bf2_unpack(fast[c], a0, a1);
+            P[0][c] += a0;
+            P[1][c] += a1;
         }
 #pragma unroll
         for (int u = 0; u < 2; u++)
 #pragma unroll
-            for (int c = 0; c < 4; c++) {
+            for (int c = C0; c < C1; c++) {
                 const float yv = P[u][c] - C[u][c];
                 const float tv = S[u][c] + yv;
                 C[u][c] = (tv - S[u][c]) - yv;
@@ -616,18 +693,19 @@ __global__ void __launch_bounds__(BF32S_THREADS) k_bf32_split(const double *pt, 
             }
         __syncthreads();
     }
+    __pipeline_wait_prior(0);
     // the group's lanes combined in double, the same fixed pattern on every lane
 #pragma unroll
     for (int u = 0; u < 2; u++) {
         double v[4];
 #pragma unroll
-        for (int c = 0; c < 4; c++) {
+        for (int c = C0; c < C1; c++) {
             v[c] = (double)S[u][c] - (double)C[u][c];
 #pragma unroll
             for (int o = 1; o < BF32S_LANES; o <<= 1) v[c] += __shfl_xor_sync(0xffffffffu, v[c], o);
         }
-        if (q != 0 || ti[u] >= nt) continue;
-        double *o = out + ti[u] * W;
+        if (q != 0 || t0 + u >= nt) continue;
+        double *o = out + (t0 + u) * W;
         int k = 0;
         if (FIELDS & BF_POT) o[k++] = G * v[0];
         if (FIELDS & BF_ACC) {
@@ -653,8 +731,16 @@ static tg_status launch_bf(int precision, const double *pt, const double *ht, in
     } else if (precision == TG_FP64) {
         { k_bf64<FIELDS, MUTUAL><<<div_up(nt, BF64_THREADS), BF64_THREADS, 0, st>>>(pt, ht, nt, ps, ms, hs, ns, G, out, W); tg::note_launch(); }
     } else if constexpr ((FIELDS & BF_TID) == 0) {
-        { k_bf32_split<FIELDS, MUTUAL><<<div_up(nt, BF32S_TARGETS), BF32S_THREADS, 0, st>>>(pt, ht, nt, ps, ms, hs, ns,
-                                                                                          G, out, W); tg::note_launch(); }
+        const int64_t ntiles = div_up(ns, BF32S_TILE);
+        DevArray<float4> src(st);
+        DevArray<float2> soft(st);
+        DevArray<float> tile_h2(st);
+        TG_CUDA(src.alloc(ns));
+        TG_CUDA(soft.alloc(ns));
+        TG_CUDA(tile_h2.alloc(ntiles));
+        if (ntiles > 0) { k_bf32_prep<<<(unsigned)ntiles, BF32S_TILE, 0, st>>>(ps, ms, hs, ns, src.p, soft.p, tile_h2.p); tg::note_launch(); }
+        { k_bf32_split<FIELDS, MUTUAL><<<div_up(nt, 2 * BF32S_PAIRS), BF32S_THREADS, 0, st>>>(pt, ht, nt, src.p, soft.p,
+                                                                                         tile_h2.p, ns, G, out, W); tg::note_launch(); }
     } else {
         { k_bf32<FIELDS, MUTUAL><<<div_up(nt, BF32_THREADS * BF32_TPT), BF32_THREADS, 0, st>>>(pt, ht, nt, ps, ms, hs, ns,
                                                                                            G, out, W); tg::note_launch(); }
