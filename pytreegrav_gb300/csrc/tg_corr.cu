@@ -31,21 +31,15 @@ namespace tg {
 namespace {
 
 constexpr int CORR_THREADS = 128;
+// 80 registers. 200000 targets, structure function: 8.91, 6.79, 5.68, 5.43, 5.17, 5.40 and 5.69 ms with 2 to
+// 8 blocks (from 7 the registers spill and the rows outgrow L2)
+constexpr int CORR_BLOCKS_PER_SM = 6;
 constexpr int CORR_RED = 256;
 constexpr int MAX_DEPTH_CLIMB = 4096;
 
 __device__ __forceinline__ double nearest_image(double x, double box) {
     if (fabs(x) > 0.5 * box) return -copysign(box - fabs(x), x);
     return x;
-}
-
-// Uniform double in [0, 1) from (seed, target, draw): splitmix64 finalisation of a Weyl sequence.
-__host__ __device__ __forceinline__ double corr_uniform(uint64_t seed, int64_t target, int64_t draw) {
-    uint64_t z = seed + 0x9E3779B97F4A7C15ull * (uint64_t)(target + 1) + 0xD1B54A32D192ED03ull * (uint64_t)(draw + 1);
-    z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
-    z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
-    z ^= z >> 31;
-    return (double)(z >> 11) * 0x1.0p-53;
 }
 
 // Depth of every node (root 0) by climbing parent links; a climb longer than the bound sets *bad.
@@ -122,11 +116,49 @@ struct CorrArgs {
     uint64_t seed;
     int nrows;
     double *rows;  // nrows x 2 nbins: bin sums, then weight sums
-    // the FP32 screen: per element hi parts of the position and, for nodes, the opening radius
-    // max(s / theta + delta, 0.6 s + delta) rounded to FP32 (-1 for particles); lo parts and the size
-    const float4 *ehi, *elo;
-    float rmin32, rmax32, lmin32, dl32, box32;
+    // the FP32 screen, three words per element: hi parts of the position and, for nodes, the opening
+    // radius max(s / theta + delta, 0.6 s + delta) rounded to FP32 (-1 for particles); lo parts and the
+    // size; the links (next, first; LINK_NONE: none)
+    const float4 *rec;
+    // per bin: order key of max_bin_size_ratio times its width (nodes below it are binned whole), and the
+    // product in FP32 (NaN where the key decides alone)
+    const long long *whole;
+    const float *whole32;
+    float rmin32, rmax32, lmin32, tscale32, box32;
 };
+
+constexpr uint32_t LINK_NONE = 0xffffffffu;  // elements number below 2^32 - 1 (N < 2^31 and fewer nodes)
+__device__ __forceinline__ uint32_t pack_link(int64_t e) { return e < 0 ? LINK_NONE : (uint32_t)e; }
+
+// A signed integer of the same order as the (non-NaN) double, -0.0 as +0.0: comparisons on the integer units.
+__device__ __forceinline__ long long order_of(double x) {
+    const long long b = __double_as_longlong(x);
+    return b < 0 ? -(b & 0x7fffffffffffffffll) : b;
+}
+__device__ __forceinline__ float sqrt_approx(float x) {  // relative error below 2^-22; subnormals as 0
+    float y;
+    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ float log10_approx(float x) {  // error below 1e-6 (1 + |log10 x|), x a normal number
+    return __log2f(x) * 0.301029996f;
+}
+
+// splitmix64 of a Weyl sequence: the jitter's random word for (seed, target, draw).
+__host__ __device__ __forceinline__ uint64_t corr_bits(uint64_t seed, int64_t target, int64_t draw) {
+    uint64_t z = seed + 0x9E3779B97F4A7C15ull * (uint64_t)(target + 1) + 0xD1B54A32D192ED03ull * (uint64_t)(draw + 1);
+    z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
+    z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
+    return z ^ (z >> 31);
+}
+// Uniform double in [0, 1), and the FP32 nearest to it less 1/2 (exactly as (float)(uniform - 0.5), the
+// difference being exact), formed on the integer units.
+__host__ __device__ __forceinline__ double corr_uniform(uint64_t seed, int64_t target, int64_t draw) {
+    return (double)(corr_bits(seed, target, draw) >> 11) * 0x1.0p-53;
+}
+__device__ __forceinline__ float corr_jitter32(uint64_t seed, int64_t target, int64_t draw) {
+    return __ll2float_rn((long long)(corr_bits(seed, target, draw) >> 11) - (1ll << 52)) * 0x1.0p-53f;
+}
 
 // Bin of distance r: int(nbins (log10 r - log10 rbins[0]) / dlogr) as pytreegrav writes it, clamped to
 // [0, nbins).
@@ -173,6 +205,15 @@ __device__ void spread_bins(const CorrArgs &a, double *row, double r, int r_idx,
     }
 }
 
+// Whether node no (FP32 size s32) is smaller than max_bin_size_ratio times the width of bin b: in FP32 where
+// the rounding of both cannot change the answer.
+__device__ __forceinline__ bool node_whole(const CorrArgs &a, uint32_t no, float s32, int b) {
+    const float w32 = a.whole32[b];
+    if (s32 < w32 * 0.999999f) return true;
+    if (s32 > w32 * 1.000001f) return false;
+    return order_of(a.size[no]) < a.whole[b];
+}
+
 // Per-target state of a walk: the target, its velocity and weight, the rows it adds into, the FP64
 // bin constants, and the count of jitter draws so far.
 struct CorrTarget {
@@ -184,47 +225,22 @@ struct CorrTarget {
     int64_t draws;
 };
 
-// A particle's contribution (in bin r_idx): its mass, v . V M, or |v - V|^2 M summed over the
-// components, times the target's weight (w = 1 for the density).
-__device__ __forceinline__ void add_particle(const CorrArgs &a, CorrTarget &t, int64_t no, int r_idx) {
-    const double M = a.mass[no];
-    double amount = M;
-    if (a.kind == TG_CORR_VELOCITY) {
-        amount = 0.0;
-        for (int k = 0; k < 3; k++) amount = dadd(amount, dmul(dmul(t.tv[k], a.vel[3 * no + k]), M));
-    } else if (a.kind == TG_CORR_STRUCTURE) {
-        amount = 0.0;
-        for (int k = 0; k < 3; k++) {
-            const double u = dsub(t.tv[k], a.vel[3 * no + k]);
-            amount = dadd(amount, dmul(dmul(u, u), M));
-        }
-    }
-    bin_add(t.bins, r_idx, dmul(t.w, amount));
-    if (a.kind) bin_add(t.wts, r_idx, dmul(t.w, M));
-}
-
-// A node's quantity per unit mass: 1, v . V, or |v - V|^2 plus its dispersion.
+// An element's quantity per unit mass: 1, v . V, or |v - V|^2 plus its dispersion (a particle's is zero).
 __device__ __forceinline__ double node_q(const CorrArgs &a, const CorrTarget &t, int64_t no) {
-    double q = 1.0;
-    if (a.kind == TG_CORR_VELOCITY) {
-        q = 0.0;
-        for (int k = 0; k < 3; k++) q = dadd(q, dmul(t.tv[k], a.vel[3 * no + k]));
-    } else if (a.kind == TG_CORR_STRUCTURE) {
-        q = 0.0;
-        for (int k = 0; k < 3; k++) {
-            const double u = dsub(t.tv[k], a.vel[3 * no + k]);
-            q = dadd(q, dmul(u, u));
-        }
-        q = dadd(q, a.disp[no]);
-    }
-    return q;
+    if (a.kind == TG_CORR_DENSITY) return 1.0;
+    const double v0 = a.vel[3 * no], v1 = a.vel[3 * no + 1], v2 = a.vel[3 * no + 2];
+    if (a.kind == TG_CORR_VELOCITY) return fma(t.tv[2], v2, fma(t.tv[1], v1, dmul(t.tv[0], v0)));
+    const double u0 = dsub(t.tv[0], v0), u1 = dsub(t.tv[1], v1), u2 = dsub(t.tv[2], v2);
+    const double q = fma(u2, u2, fma(u1, u1, dmul(u0, u0)));
+    return no < a.ntot ? q : dadd(q, a.disp[no]);
 }
 
-// A binned node's contribution at jittered bin j.
-__device__ __forceinline__ void add_node_at(const CorrArgs &a, CorrTarget &t, int64_t no, int j) {
-    const double M = a.mass[no];
-    bin_add(t.bins, j, dmul(t.w, a.kind ? dmul(node_q(a, t, no), M) : M));
-    if (a.kind) bin_add(t.wts, j, dmul(t.w, M));
+// What element no (a particle, or a binned node) adds to bin b: its mass times its quantity per unit mass
+// times the target's weight (w = 1 for the density).
+__device__ __forceinline__ void add_elem(const CorrArgs &a, CorrTarget &t, int64_t no, int b) {
+    const double wm = a.kind ? dmul(t.w, a.mass[no]) : a.mass[no];
+    bin_add(t.bins, b, a.kind ? dmul(wm, node_q(a, t, no)) : wm);
+    if (a.kind) bin_add(t.wts, b, wm);
 }
 
 // The FP64 distance from the target to element no (nearest periodic image when box > 0).
@@ -250,7 +266,7 @@ __device__ int64_t elem_exact(const CorrArgs &a, CorrTarget &t, int64_t no) {
     if (r > a.rbins[0] && r < a.rbins[nb]) {
         const int r_idx = bin_of(r, t.logr_min, t.dlogr, nb);
         if (part) {
-            add_particle(a, t, no, r_idx);
+            add_elem(a, t, no, r_idx);
             return a.next[no];
         }
         if (far && s < dmul(a.mbr, dsub(a.rbins[r_idx + 1], a.rbins[r_idx]))) {
@@ -261,7 +277,7 @@ __device__ int64_t elem_exact(const CorrArgs &a, CorrTarget &t, int64_t no) {
                 if (a.kind) spread_bins(a, t.wts, r, r_idx, dmul(0.5, s), M, 1.0, t.w);
             } else {
                 const double rnew = dadd(r, dmul(dsub(corr_uniform(a.seed, t.i, t.draws++), 0.5), s));
-                add_node_at(a, t, no, rnew > 0.0 ? bin_of(rnew, t.logr_min, t.dlogr, nb) : 0);
+                add_elem(a, t, no, rnew > 0.0 ? bin_of(rnew, t.logr_min, t.dlogr, nb) : 0);
             }
             return a.next[no];
         }
@@ -276,12 +292,14 @@ __device__ __forceinline__ int side(float x, float c, float e) { return x > c + 
 // The bin of distance r (FP32, relative error below er / r) when the FP32 value of pytreegrav's bin
 // formula is farther than its error bound from a bin edge (the clamps included); -1 otherwise.
 __device__ __forceinline__ int bin_screen(const CorrArgs &a, float r, float er) {
-    const float lr = log10f(r);
-    const float tscale = (float)a.nbins / a.dl32;
-    const float t = __fdiv_rn(__fmul_rn((float)a.nbins, __fsub_rn(lr, a.lmin32)), a.dl32);
-    // log10f (a few ulp), the FP32 constants and r's own error, with a factor of 4 to spare
-    const float dt = tscale * (4e-6f * (1.f + fabsf(lr) + fabsf(a.lmin32)) + 2.f * er / r);
-    if (!(r > 0.f) || !(dt < 0.25f)) return -1;
+    const float lr = log10_approx(r);
+    const float tscale = a.tscale32;
+    const float t = (lr - a.lmin32) * tscale;
+    // The logarithm (lg2.approx: 2^-22 absolute or relative, whichever is larger, and its scaling: 7.2e-8 +
+    // 3.3e-7 |lr|), the difference and the FP32 constants (1.8e-7 |lr| + 2.4e-7 |lmin|): twice that; and r's
+    // own error, d log10 r = 0.434 dr / r. An element within dt of an edge costs ~200 FP64 instructions.
+    const float dt = tscale * (1e-6f * (1.f + fabsf(lr) + fabsf(a.lmin32)) + 0.5f * __fdividef(er, r));
+    if (!(r > 1.2e-38f) || !(r < 1e38f) || !(dt < 0.25f)) return -1;
     if (t < -dt) return 0;
     if (t - dt >= (float)a.nbins) return a.nbins - 1;
     const float fl = floorf(t);
@@ -289,53 +307,98 @@ __device__ __forceinline__ int bin_screen(const CorrArgs &a, float r, float er) 
     return -1;
 }
 
-// The walk of target i (treewalk.py:380-818). Every decision -- inside the radial range, the opening
-// test, the bin, a jittered node's bin -- is first taken in FP32 from hi/lo positions when the FP32
-// value lies farther from its threshold than a bound on its error; otherwise (and for weighted
-// binning) the element is evaluated by elem_exact. So the decisions are pytreegrav's FP64 ones, and
-// GB300 (FP64 at 1/73 of the FP32 rate) spends FP64 only on the sums. Contributions add into row
-// (bin sums at row[0..nbins), weight sums at row[nbins..2 nbins), kinds 1 and 2 only), each formed in
-// pytreegrav's order of operations and multiplied by the target's weight (pytreegrav multiplies the
-// target's per-bin sums instead, which differs in rounding only).
-__device__ void corr_walk(const CorrArgs &a, int64_t i, double *row) {
-    const int64_t N = a.ntot;
+// The walks (treewalk.py:380-818), one target per lane, a warp's lanes visiting one element each per step.
+// Every decision -- inside the radial range, the opening test, the bin, a jittered node's bin -- is
+// first taken in FP32 from hi/lo positions when the FP32 value lies farther from its threshold than a
+// bound on its error; otherwise (and for weighted binning) the element is evaluated by elem_exact. So the
+// decisions are pytreegrav's FP64 ones, and GB300 (FP64 at 1/73 of the FP32 rate) spends FP64 only on
+// the sums. Those do not steer the walk: a lane puts (element, bin) in its queue in shared memory, and once a
+// lane's queue is full the warp adds all its queues' entries, each lane its own in its walk's order. A step's
+// additions alone would run with the few lanes that have one, at ~76 cycles for each FP64 instruction
+// whatever their number. A lane whose target is done takes its next one after that.
+// Contributions add into the lane's row (bin sums at row[0..nbins), weight sums at row[nbins..2 nbins),
+// kinds 1 and 2 only), each multiplied by the target's weight (pytreegrav multiplies the target's per-bin
+// sums instead, which differs in rounding only).
+// A visit reads one 48-byte record, links included; the jitter, the whole-node test and the bin come from
+// integer and FP32 arithmetic; a contribution takes 11 FP64 instructions (16 before).
+// VelocityStructFunc's walk, 200000 Plummer particles, 57 bins: 11.1 ms with the additions in the step (FP64
+// pipe 79 % busy), 5.17 ms now; 1e6 particles 51.9 -> 23.8 ms. Bound by the FP64 pipe (70 % busy) and the rows'
+// read-add-write latency.
+constexpr int CORR_QUEUE = 16;  // entries per lane (8 to 32: within 4 %)
+
+__global__ void __launch_bounds__(CORR_THREADS, CORR_BLOCKS_PER_SM) k_corr(CorrArgs a) {
+    __shared__ uint32_t q_elem[CORR_QUEUE][CORR_THREADS];
+    __shared__ uint16_t q_bin[CORR_QUEUE][CORR_THREADS];
+    const int tid = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t N = (uint32_t)a.ntot, ne = (uint32_t)a.nelem;
     const int nb = a.nbins;
+    const bool has_row = tid < a.nrows;
+    double *row = a.rows + (int64_t)(has_row ? tid : 0) * 2 * nb;
+    if (has_row)
+        for (int b = 0; b < 2 * nb; b++) row[b] = 0.0;
+    const float box = a.box32, half = 0.5f * a.box32;
     CorrTarget t;
-    t.i = i;
-    t.px = a.pos[3 * i];
-    t.py = a.pos[3 * i + 1];
-    t.pz = a.pos[3 * i + 2];
-    t.tv[0] = t.tv[1] = t.tv[2] = 0.0;
-    if (a.kind) {
-        t.tv[0] = a.tvel[3 * i];
-        t.tv[1] = a.tvel[3 * i + 1];
-        t.tv[2] = a.tvel[3 * i + 2];
-    }
-    t.w = a.kind ? a.weight[i] : 1.0;
     t.logr_min = log10(a.rbins[0]);
     t.dlogr = dsub(log10(a.rbins[nb]), t.logr_min);
     t.bins = row;
     t.wts = row + nb;
+    t.tv[0] = t.tv[1] = t.tv[2] = 0.0;
+    t.px = t.py = t.pz = 0.0;
+    t.w = 1.0;
     t.draws = 0;
-    float phx, plx, phy, ply, phz, plz;
-    d2f_split(t.px, phx, plx);
-    d2f_split(t.py, phy, ply);
-    d2f_split(t.pz, phz, plz);
-    const float box = a.box32, half = 0.5f * a.box32;
-    // the hi/lo splits keep positions to ~2^-48 of their size: an absolute error term for very close pairs
-    const float eabs = 1e-12f * (fabsf(phx) + fabsf(phy) + fabsf(phz)) + 1e-30f;
-    int64_t no = N;
-    for (int64_t guard = 0; no > -1; guard++) {
-        if (guard > a.nelem || no >= a.nelem) {  // one visit per element always suffices
-            atomicOr(a.runaway, 1);
-            return;
+    t.i = 0;
+    float phx = 0.f, plx = 0.f, phy = 0.f, ply = 0.f, phz = 0.f, plz = 0.f, eabs = 0.f;
+    int64_t next_i = has_row ? tid : a.n;
+    uint32_t no = LINK_NONE;
+    int64_t visits = 0;
+    int queued = 0;
+    auto flush = [&]() {
+        for (int k = 0; __any_sync(FULL, k < queued); k++)
+            if (k < queued) add_elem(a, t, q_elem[k][threadIdx.x], q_bin[k][threadIdx.x]);
+        queued = 0;
+    };
+    for (;;) {
+        // (a lane whose target is done, with entries still queued, waits for the others' next flush)
+        if (__any_sync(FULL, queued == CORR_QUEUE) || !__any_sync(FULL, no != LINK_NONE)) flush();
+        if (no == LINK_NONE && queued == 0 && next_i < a.n) {  // the lane's next target
+            const int64_t i = next_i;
+            next_i += a.nrows;
+            t.i = i;
+            t.px = a.pos[3 * i];
+            t.py = a.pos[3 * i + 1];
+            t.pz = a.pos[3 * i + 2];
+            if (a.kind) {
+                t.tv[0] = a.tvel[3 * i];
+                t.tv[1] = a.tvel[3 * i + 1];
+                t.tv[2] = a.tvel[3 * i + 2];
+                t.w = a.weight[i];
+            }
+            t.draws = 0;
+            d2f_split(t.px, phx, plx);
+            d2f_split(t.py, phy, ply);
+            d2f_split(t.pz, phz, plz);
+            // the hi/lo splits keep positions to ~2^-48 of their size: an absolute error term for very
+            // close pairs (and for distances whose squares underflow)
+            eabs = 1e-12f * (fabsf(phx) + fabsf(phy) + fabsf(phz)) + 1.2e-19f;
+            no = N;
+            visits = 0;
         }
-        const float4 h = a.ehi[no], l = a.elo[no];
+        if (!__any_sync(FULL, no != LINK_NONE)) break;
+        if (no == LINK_NONE) continue;
+        if (visits++ > a.nelem || no >= ne) {  // one visit per element always suffices
+            atomicOr(a.runaway, 1);
+            no = LINK_NONE;
+            next_i = a.n;
+            continue;
+        }
+        const float4 h = a.rec[3 * (int64_t)no], l = a.rec[3 * (int64_t)no + 1];
+        const float2 lk = *reinterpret_cast<const float2 *>(a.rec + 3 * (int64_t)no + 2);
+        const uint32_t next = __float_as_uint(lk.x), first = __float_as_uint(lk.y);
         float d[3] = {__fadd_rn(__fsub_rn(h.x, phx), __fsub_rn(l.x, plx)),
                       __fadd_rn(__fsub_rn(h.y, phy), __fsub_rn(l.y, ply)),
                       __fadd_rn(__fsub_rn(h.z, phz), __fsub_rn(l.z, plz))};
         bool sure = true;
-        if (a.box > 0.0) {
+        if (box > 0.f) {
 #pragma unroll
             for (int k = 0; k < 3; k++) {
                 const float ad = fabsf(d[k]);
@@ -344,52 +407,50 @@ __device__ void corr_walk(const CorrArgs &a, int64_t i, double *row) {
                 else if (sd > 0) d[k] = -copysignf(__fsub_rn(box, ad), d[k]);
             }
         }
-        const float r = sqrtf(__fadd_rn(__fadd_rn(__fmul_rn(d[0], d[0]), __fmul_rn(d[1], d[1])), __fmul_rn(d[2], d[2])));
+        const float r = sqrt_approx(__fadd_rn(__fadd_rn(__fmul_rn(d[0], d[0]), __fmul_rn(d[1], d[1])), __fmul_rn(d[2], d[2])));
         // hi/lo offsets (~1e-7 relative), the nearest image, the squares and the root
         const float er = 2e-6f * (r + box) + 1e-12f * (fabsf(h.x) + fabsf(h.y) + fabsf(h.z)) + eabs;
         const bool part = no < N;
         const int inlo = side(r, a.rmin32, er + 2e-7f * a.rmin32), inhi = side(r, a.rmax32, er + 2e-7f * a.rmax32);
         const int fs = part ? -1 : side(r, h.w, er + 2e-7f * h.w);  // far: r > opening radius
-        if (!sure || inlo == 0 || inhi == 0 || fs == 0 || a.weighted) {
-            no = elem_exact(a, t, no);
-            continue;
-        }
-        if (inlo > 0 && inhi < 0) {  // inside (rbins[0], rbins[-1])
-            const int r_idx = bin_screen(a, r, er);
-            if (r_idx < 0) {
-                no = elem_exact(a, t, no);
-                continue;
-            }
-            if (part) {
-                add_particle(a, t, no, r_idx);
-                no = a.next[no];
-            } else if (fs > 0 && a.size[no] < dmul(a.mbr, dsub(a.rbins[r_idx + 1], a.rbins[r_idx]))) {
-                // jittered distance r + (u - 0.5) s: its bin in FP32 when clear of the edges
-                const double u = corr_uniform(a.seed, i, t.draws);
-                const float rn = __fadd_rn(r, __fmul_rn((float)(u - 0.5), l.w));
-                const int j = rn > 4.f * er ? bin_screen(a, rn, er + 1e-6f * l.w) : -1;
-                if (j >= 0) {
+        bool exact = !sure || inlo == 0 || inhi == 0 || fs == 0 || a.weighted;
+        if (!exact) {
+            if (inlo > 0 && inhi < 0 && (part || fs > 0)) {  // inside (rbins[0], rbins[-1]), not an open node
+                const int r_idx = bin_screen(a, r, er);
+                if (r_idx < 0) {
+                    exact = true;
+                } else if (part) {
+                    q_elem[queued][threadIdx.x] = no;
+                    q_bin[queued++][threadIdx.x] = (uint16_t)r_idx;
+                    no = next;
+                } else if (node_whole(a, no, l.w, r_idx)) {
+                    // jittered distance r + (u - 0.5) s: its bin in FP32 when clear of the edges
+                    const float rn = __fadd_rn(r, __fmul_rn(corr_jitter32(a.seed, t.i, t.draws), l.w));
+                    int j = rn > 4.f * er ? bin_screen(a, rn, er + 1e-6f * l.w) : -1;
+                    if (j < 0) {  // the FP64 distance, then pytreegrav's expression
+                        const double rnew = dadd(dist64(a, t, no),
+                                                 dmul(dsub(corr_uniform(a.seed, t.i, t.draws), 0.5), a.size[no]));
+                        j = rnew > 0.0 ? bin_of(rnew, t.logr_min, t.dlogr, nb) : 0;
+                    }
                     t.draws++;
-                    add_node_at(a, t, no, j);
-                } else {  // the FP64 distance, then pytreegrav's expression
-                    const double r64 = dist64(a, t, no);
-                    const double rnew = dadd(r64, dmul(dsub(corr_uniform(a.seed, i, t.draws++), 0.5), a.size[no]));
-                    add_node_at(a, t, no, rnew > 0.0 ? bin_of(rnew, t.logr_min, t.dlogr, nb) : 0);
+                    q_elem[queued][threadIdx.x] = no;
+                    q_bin[queued++][threadIdx.x] = (uint16_t)j;
+                    no = next;
+                } else {
+                    no = first;
                 }
-                no = a.next[no];
             } else {
-                no = a.first[no];
+                no = (part || fs > 0) ? next : first;
             }
-        } else {
-            no = (part || fs > 0) ? a.next[no] : a.first[no];
         }
+        if (exact) no = pack_link(elem_exact(a, t, no));
     }
 }
 
-// FP32 element records of the screen: hi/lo position, the node's opening radius (pytreegrav's
-// max(s / theta + delta, 0.6 s + delta), formed in FP64 and rounded) or -1, the size.
+// FP32 element records of the screen (see CorrArgs): the opening radius is pytreegrav's
+// max(s / theta + delta, 0.6 s + delta), formed in FP64 and rounded.
 __global__ void k_corr_prep(int64_t ntot, int64_t nelem, const double *coord, const double *size, const double *delta,
-                            double theta, float4 *ehi, float4 *elo) {
+                            const int64_t *next, const int64_t *first, double theta, float4 *rec) {
     const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= nelem) return;
     float hx, lx, hy, ly, hz, lz;
@@ -402,16 +463,18 @@ __global__ void k_corr_prep(int64_t ntot, int64_t nelem, const double *coord, co
         crit = d2f(fmax(dadd(ddiv(s, theta), del), dadd(dmul(s, 0.6), del)));
         s32 = d2f(s);
     }
-    ehi[e] = make_float4(hx, hy, hz, crit);
-    elo[e] = make_float4(lx, ly, lz, s32);
+    rec[3 * e] = make_float4(hx, hy, hz, crit);
+    rec[3 * e + 1] = make_float4(lx, ly, lz, s32);
+    rec[3 * e + 2] = make_float4(__uint_as_float(pack_link(next[e])), __uint_as_float(pack_link(first[e])), 0.f, 0.f);
 }
 
-__global__ void __launch_bounds__(CORR_THREADS) k_corr(CorrArgs a) {
-    const int tid = blockIdx.x * blockDim.x + threadIdx.x;
-    if (tid >= a.nrows) return;
-    double *row = a.rows + (int64_t)tid * 2 * a.nbins;
-    for (int b = 0; b < 2 * a.nbins; b++) row[b] = 0.0;
-    for (int64_t i = tid; i < a.n; i += a.nrows) corr_walk(a, i, row);
+__global__ void k_corr_whole(const double *rbins, int nbins, double mbr, long long *whole, float *whole32) {
+    const int b = blockIdx.x * blockDim.x + threadIdx.x;
+    if (b >= nbins) return;
+    const double w = dmul(mbr, dsub(rbins[b + 1], rbins[b]));
+    whole[b] = w == w ? order_of(w) : (long long)0x8000000000000000ull;  // nothing is below NaN
+    const float f = d2f(w);
+    whole32[b] = f > 1e-30f && f < 1e30f ? f : __int_as_float(0x7fffffff);
 }
 
 // One block per output value (bin sums, then weight sums): thread t adds rows t, t + CORR_RED, ...
@@ -564,19 +627,24 @@ tg_status tg_tree_correlation(tg_tree t, int kind, const double *pos, const doub
     a.seed = seed;
     // a fixed number of rows (threads), bounded so that the rows stay within 512 MB
     const int64_t per_row = 2 * (int64_t)nbins * (int64_t)sizeof(double);
-    int64_t nrows = std::min<int64_t>((int64_t)num_sms() * 4 * CORR_THREADS, ((int64_t)1 << 29) / per_row);
+    int64_t nrows = std::min<int64_t>((int64_t)num_sms() * CORR_BLOCKS_PER_SM * CORR_THREADS, ((int64_t)1 << 29) / per_row);
     nrows = std::max<int64_t>(1, std::min<int64_t>(nrows, std::max<int64_t>(n, 1)));
     a.nrows = (int)nrows;
     TG_CUDA(rows.alloc(nrows * 2 * nbins));
     a.rows = rows.p;
     TG_CUDA(dout.alloc(2 * nbins));
-    DevArray<float4> ehi(st), elo(st);
-    TG_CUDA(ehi.alloc(a.nelem));
-    TG_CUDA(elo.alloc(a.nelem));
-    { k_corr_prep<<<div_up(a.nelem, 256), 256, 0, st>>>(t->ntot, a.nelem, t->coord, t->size, t->delta, theta, ehi.p,
-                                                          elo.p); note_launch(); }
-    a.ehi = ehi.p;
-    a.elo = elo.p;
+    DevArray<float4> rec(st);
+    DevArray<long long> whole(st);
+    DevArray<float> whole32(st);
+    TG_CUDA(rec.alloc(3 * a.nelem));
+    TG_CUDA(whole.alloc(nbins));
+    TG_CUDA(whole32.alloc(nbins));
+    { k_corr_prep<<<div_up(a.nelem, 256), 256, 0, st>>>(t->ntot, a.nelem, t->coord, t->size, t->delta, t->next, t->first,
+                                                          theta, rec.p); note_launch(); }
+    { k_corr_whole<<<div_up(nbins, 256), 256, 0, st>>>(a.rbins, nbins, max_bin_size_ratio, whole.p, whole32.p); note_launch(); }
+    a.rec = rec.p;
+    a.whole = whole.p;
+    a.whole32 = whole32.p;
     {  // FP32 copies of the radial range for the screen (its error bounds cover their rounding)
         double rb0 = 0.0, rbn = 0.0;
         if (host) {
@@ -590,7 +658,7 @@ tg_status tg_tree_correlation(tg_tree t, int kind, const double *pos, const doub
         a.rmin32 = (float)rb0;
         a.rmax32 = (float)rbn;
         a.lmin32 = (float)std::log10(rb0);
-        a.dl32 = (float)(std::log10(rbn) - std::log10(rb0));
+        a.tscale32 = (float)((double)nbins / (std::log10(rbn) - std::log10(rb0)));
         a.box32 = (float)boxsize;
     }
     { k_corr<<<div_up(nrows, CORR_THREADS), CORR_THREADS, 0, st>>>(a); note_launch(); }
