@@ -9,6 +9,9 @@
 // The test runs in FP32 with an error bound; a node inside the bound is re-tested with the exact
 // FP64 expression on the tree's FP64 arrays, so the accepted set is exactly pytreegrav's.
 //
+// A long group of consecutive targets is walked by a whole block (TEAM): its first warp traverses, the others
+// sum the batches, the last one adds their sums in the order a single warp would have.
+//
 // Evaluation: every 32 list entries are staged in shared memory as offsets from a group reference
 // point (hi/lo float pairs keep near-field offsets exact to FP32 rounding) and swept by all lanes:
 // lane = (target, slice): a group of n targets takes P lanes per slice, P the smallest power of two
@@ -363,6 +366,10 @@ struct WalkArgs {
     // (its partial work taken back) and is appended to heavy, for the split walk (walk_heavy).
     int *heavy = nullptr, *heavy_count = nullptr;
     unsigned heavy_budget = 0;
+    // Long groups: with team set, a group whose evaluated list entries exceed stop_budget stops likewise
+    // and is appended to team, for the pass that walks a group with a whole block (TEAM).
+    int *team = nullptr, *team_count = nullptr;
+    unsigned stop_budget = ~0u;  // the smaller budget of the two lists that are set
     // Item mode (the split walk): unit k walks, for group item_group[k], the subtree of item_node[k]
     // (a node; or a particle, ~leaf, taken as one interaction) and writes its unscaled partial sums,
     // 10 components for each of gs target slots, to partial + 10 * gs * k.
@@ -387,6 +394,28 @@ struct WarpSmem {
     vec4<T> sq[QUAD ? 64 : 1];   // quadrupole records of the staged nodes
     double xbox[8];  // the exact test's FP64 group box: min (3), max (3), max softening, theta
 };
+
+// Shared memory of a block that walks one group together (TEAM): the batches that the first warp's traversal
+// emitted, of two rounds, and the sums that the other warps made of them, of two rounds.
+constexpr int TEAM_WARPS = 8;
+constexpr int TEAM_ROUND = 2 * (TEAM_WARPS - 1);  // batches after which a round ends
+// a step lists at most 32 * 8 particles and 32 nodes beside the 31 left over (9 + 1 batches of 32, or 9
+// and 1), and the group's end two short batches
+constexpr int TEAM_SLOTS = TEAM_ROUND - 1 + 11 + 2;
+template <int COMPS>
+struct TeamSmem {
+    int entry[2][TEAM_SLOTS][32];
+    int info[2][TEAM_SLOTS];  // entries of the batch; + 64: quadrupole nodes
+    float sum[2][TEAM_SLOTS][COMPS][32];
+    int nbatch[4], state[4];  // of round k at k & 3: its batches, and whether the group goes on after it
+    int unit;
+};
+enum { TEAM_RUN = 0, TEAM_DONE = 1, TEAM_STOP = 2 };
+
+template <int FIELDS>
+__host__ __device__ constexpr int field_comps() {
+    return ((FIELDS & F_POT) ? 1 : 0) + ((FIELDS & F_ACC) ? 3 : 0) + ((FIELDS & F_TID) ? 6 : 0);
+}
 
 template <typename T>
 struct Acc {
@@ -565,16 +594,21 @@ __device__ __forceinline__ void write_fields(double *o, int out_fields, const do
 // walk with the small stack runs at 72, which with its shared memory lets 7 blocks of 4 warps share
 // an SM (6 at 80); the other small-stack walks at 80 (6 blocks of 4 warps, 3 of 8; 81 would round
 // to 88 and leave 5 or 2); large-stack walks uncapped.
-template <typename T, int FIELDS, bool QUAD, int STACK>
+template <typename T, int FIELDS, bool QUAD, int STACK, bool TEAM = false>
 constexpr int walk_reg_cap() {
+    if (TEAM) return 128;  // two blocks of eight warps per SM
     if (STACK != STACK_SMALL) return 255;
     return (sizeof(T) == 4 && FIELDS == F_ACC && QUAD) ? 72 : 80;
 }
-template <typename T, int FIELDS, bool QUAD, int STACK>
-__global__ void __launch_bounds__(MAX_WALK_WARPS * 32) __maxnreg__((walk_reg_cap<T, FIELDS, QUAD, STACK>()))
+template <typename T, int FIELDS, bool QUAD, int STACK, bool TEAM = false>
+__global__ void __launch_bounds__(MAX_WALK_WARPS * 32) __maxnreg__((walk_reg_cap<T, FIELDS, QUAD, STACK, TEAM>()))
     k_walk(WalkArgs<T> a) {
     extern __shared__ unsigned char smem_raw[];
     WarpSmem<T, QUAD, STACK> &sm = reinterpret_cast<WarpSmem<T, QUAD, STACK> *>(smem_raw)[threadIdx.x >> 5];
+    // a block that walks one group together: its shared part lies behind the warps'
+    typedef TeamSmem<field_comps<FIELDS>()> Team;
+    Team &team = *reinterpret_cast<Team *>(smem_raw + (TEAM ? sizeof(WarpSmem<T, QUAD, STACK>) * TEAM_WARPS : 0));
+    const int warp = threadIdx.x >> 5;
     const int lane = lane_id();
     const unsigned lt = lanemask_lt();
     unsigned long long n_int = 0, n_tests = 0, n_steps = 0, n_qint = 0;
@@ -587,8 +621,14 @@ __global__ void __launch_bounds__(MAX_WALK_WARPS * 32) __maxnreg__((walk_reg_cap
 
     for (;;) {
         int g = 0;
-        if (lane == 0) g = atomicAdd(a.queue, 1);
-        g = __shfl_sync(FULL, g, 0);
+        if constexpr (TEAM) {
+            if (threadIdx.x == 0) team.unit = atomicAdd(a.queue, 1);
+            __syncthreads();
+            g = team.unit;
+        } else {
+            if (lane == 0) g = atomicAdd(a.queue, 1);
+            g = __shfl_sync(FULL, g, 0);
+        }
         if (g >= ngroups) break;
         const int unit = g;
         int start;  // the node the traversal starts from (an item may be a particle: ~leaf)
@@ -679,6 +719,16 @@ __global__ void __launch_bounds__(MAX_WALK_WARPS * 32) __maxnreg__((walk_reg_cap
 #pragma unroll
         for (int c = 0; c < 10; c++) S.v[c] = C.v[c] = T(0);
 
+        // a batch's sums: added here, or returned to the team's round
+        auto finish = [&](const Acc<T> &b, int cnt, bool nodes) {
+            if constexpr (TEAM) {
+                return b;
+            } else {
+                kahan_add<T, FIELDS>(S, C, b);
+                n_int += (unsigned long long)cnt * (unsigned long long)gr.y;
+                if (nodes) n_qint += (unsigned long long)cnt * (unsigned long long)gr.y;
+            }
+        };
         // evaluate list entries [0, cnt) of `list` (monopole: nodes >= 0, leaves as ~index)
         // Each slice of lanes sweeps one contiguous chunk of GS staged sources. Sources that may lie
         // within a softening length of the group (or coincide with a target) are staged as
@@ -814,8 +864,7 @@ __global__ void __launch_bounds__(MAX_WALK_WARPS * 32) __maxnreg__((walk_reg_cap
                 softened<T, FIELDS>(s.w, sm.sh[k], th, dx, dy, dz, dx * dx + dy * dy + dz * dz, b);
             }
             __syncwarp();
-            kahan_add<T, FIELDS>(S, C, b);
-            n_int += (unsigned long long)cnt * (unsigned long long)gr.y;
+            return finish(b, cnt, false);
         };
         // Quadrupole acceleration sweep with paired arithmetic (FP32, groups of 2 or more targets).
         // Sources are staged as pairs (2p, 2p + 1), each 16-byte word holding one quantity of both:
@@ -913,16 +962,11 @@ __global__ void __launch_bounds__(MAX_WALK_WARPS * 32) __maxnreg__((walk_reg_cap
                 f2_unpack(az, h0, h1);
                 b.v[3] = h0 + h1;
             }
-            kahan_add<T, FIELDS>(S, C, b);
-            n_int += (unsigned long long)cnt * (unsigned long long)gr.y;
-            n_qint += (unsigned long long)cnt * (unsigned long long)gr.y;
+            return finish(b, cnt, true);
         };
         auto eval_nodes = [&](const int *list, int cnt) {
             if constexpr (sizeof(T) == 4 && ((FIELDS & F_TID) == 0 || FIELDS == F_TID)) {
-                if (GS >= 2) {
-                    eval_nodes_paired(list, cnt);
-                    return;
-                }
+                if (GS >= 2) return eval_nodes_paired(list, cnt);
             }
             vec4<T> st = vec4<T>{FAR, FAR, FAR, T(0)}, q0 = vec4<T>{T(0), T(0), T(0), T(0)}, q1 = q0;
             if (lane < cnt) {
@@ -955,12 +999,29 @@ __global__ void __launch_bounds__(MAX_WALK_WARPS * 32) __maxnreg__((walk_reg_cap
                 }
             }
             __syncwarp();
-            kahan_add<T, FIELDS>(S, C, b);
-            n_int += (unsigned long long)cnt * (unsigned long long)gr.y;
-            n_qint += (unsigned long long)cnt * (unsigned long long)gr.y;
+            return finish(b, cnt, true);
         };
 
         unsigned g_mono = 0, g_quad = 0, g_tests = 0, g_steps = 0;  // this group's counters (warp-uniform)
+        // One batch of list entries: summed and added here, or, in a block that walks the group together, handed
+        // to the other warps, numbered in the order in which a single warp would sum them.
+        int round = 0, nbatch = 0;
+        auto emit = [&](const int *list, int cnt, bool nodes) {
+            team.entry[round & 1][nbatch][lane] = lane < cnt ? list[lane] : 0;
+            if (lane == 0) team.info[round & 1][nbatch] = cnt + (nodes ? 64 : 0);
+            nbatch++;
+            n_int += (unsigned long long)cnt * (unsigned long long)gr.y;
+            if (nodes) n_qint += (unsigned long long)cnt * (unsigned long long)gr.y;
+        };
+        auto take_leaves = [&](const int *list, int cnt) {
+            if constexpr (TEAM) emit(list, cnt, false);
+            else eval_batch(list, cnt);
+        };
+        auto take_nodes = [&](const int *list, int cnt) {
+            if constexpr (TEAM) emit(list, cnt, true);
+            else eval_nodes(list, cnt);
+        };
+
         int sp = 1, ni = 0, nn = 0;
         if (start >= 0) {
             if (lane == 0) sm.stack[0] = start;
@@ -970,10 +1031,48 @@ __global__ void __launch_bounds__(MAX_WALK_WARPS * 32) __maxnreg__((walk_reg_cap
             ni = 1;
         }
         __syncwarp();
-        bool overflow = false, runaway = false, heavy = false;
+        bool overflow = false, runaway = false, heavy = false, longer = false;
         // a traversal tests every node at most once, and each step tests at least one
         int64_t steps_left = a.step_limit > 0 && a.step_limit < a.ar.n_nodes + 2 ? a.step_limit : a.ar.n_nodes + 2;
-        for (;;) {
+        // Rounds of a block that walks the group together: in round k the first warp traverses and emits batches,
+        // the others sum round k - 1's, and the last one adds round k - 2's sums, in order; a round ends
+        // at a barrier. state: the first warp's word on the group; every warp returns it.
+        auto team_round = [&](int state) -> int {
+          if constexpr (TEAM) {
+            if (warp > 0 && round > 0) {
+                const int p = (round - 1) & 1, nb = team.nbatch[(round - 1) & 3];
+                for (int k = warp - 1; k < nb; k += TEAM_WARPS - 1) {
+                    const int info = team.info[p][k], cnt = info & 63;
+                    Acc<T> b;
+                    if (QUAD && info >= 64) b = eval_nodes(team.entry[p][k], cnt);
+                    else b = eval_batch(team.entry[p][k], cnt);
+                    int j = 0;
+#pragma unroll
+                    for (int c = 0; c < 10; c++)
+                        if (comp<FIELDS>(c)) team.sum[p][k][j++][lane] = (float)b.v[c];
+                }
+            }
+            if (warp == TEAM_WARPS - 1 && round > 1) {
+                const int p = round & 1, nb = team.nbatch[(round - 2) & 3];
+                for (int k = 0; k < nb; k++) {
+                    Acc<T> b;
+                    int j = 0;
+#pragma unroll
+                    for (int c = 0; c < 10; c++) b.v[c] = comp<FIELDS>(c) ? (T)team.sum[p][k][j++][lane] : T(0);
+                    kahan_add<T, FIELDS>(S, C, b);
+                }
+            }
+            if (warp == 0 && lane == 0) {
+                team.nbatch[round & 3] = nbatch;
+                team.state[round & 3] = state;
+            }
+            __syncthreads();
+            nbatch = 0;
+            return team.state[round++ & 3];
+          }
+          return state;
+        };
+        while (!TEAM || warp == 0) {
             if (--steps_left < 0) {
                 runaway = true;
                 break;
@@ -1084,28 +1183,50 @@ __global__ void __launch_bounds__(MAX_WALK_WARPS * 32) __maxnreg__((walk_reg_cap
                 __syncwarp();
             }
             while (ni >= 32) {
-                eval_batch(sm.ilist + ni - 32, 32);
+                take_leaves(sm.ilist + ni - 32, 32);
                 ni -= 32;
                 g_mono += 32;
             }
             if (QUAD) {
                 while (nn >= 32) {
-                    eval_nodes(sm.nlist + nn - 32, 32);
+                    take_nodes(sm.nlist + nn - 32, 32);
                     nn -= 32;
                     g_quad += 32;
                 }
             }
             if (sp == 0) break;
-            if (a.heavy && g_mono + g_quad > a.heavy_budget) {  // warp-uniform
-                heavy = true;
+            if (g_mono + g_quad > a.stop_budget) {  // warp-uniform
+                heavy = a.heavy && g_mono + g_quad > a.heavy_budget;
+                longer = !heavy;
                 break;
             }
+            if (TEAM && nbatch >= TEAM_ROUND) team_round(TEAM_RUN);
         }
-        if ((overflow && a.retry) || heavy) {
-            // handed to the large-stack pass or to the split walk; its counts so far are taken back
-            // so the statistics count the group once
+        bool team_stopped = false;
+        if constexpr (TEAM) {
+            int state = TEAM_RUN;
+            if (warp == 0) {
+                const bool stop = overflow || runaway || heavy;
+                if (!stop) {
+                    if (ni > 0) take_leaves(sm.ilist, ni);
+                    if (QUAD && nn > 0) take_nodes(sm.nlist, nn);
+                }
+                state = team_round(stop ? TEAM_STOP : TEAM_DONE);
+            } else {
+                while (state == TEAM_RUN) state = team_round(TEAM_RUN);
+            }
+            team_stopped = state == TEAM_STOP;
+            if (!team_stopped) {  // two more rounds sum and add the last round's batches
+                team_round(TEAM_DONE);
+                team_round(TEAM_DONE);
+            }
+        }
+        if ((overflow && a.retry) || heavy || longer) {
+            // handed to the large-stack pass, to the split walk or to a whole block; its counts so far
+            // are taken back so the statistics count the group once
             if (lane == 0) {
                 if (heavy) a.heavy[atomicAdd(a.heavy_count, 1)] = g;
+                else if (longer) a.team[atomicAdd(a.team_count, 1)] = g;
                 else a.retry[atomicAdd(a.retry_count, 1)] = g;
                 n_tests -= g_tests;
             }
@@ -1120,8 +1241,12 @@ __global__ void __launch_bounds__(MAX_WALK_WARPS * 32) __maxnreg__((walk_reg_cap
             __syncwarp();
             continue;
         }
-        if (ni > 0) eval_batch(sm.ilist, ni);
-        if (QUAD && nn > 0) eval_nodes(sm.nlist, nn);
+        if constexpr (TEAM) {
+            if (warp != TEAM_WARPS - 1 || team_stopped) continue;  // the last warp holds the sums
+        } else {
+            if (ni > 0) take_leaves(sm.ilist, ni);
+            if (QUAD && nn > 0) take_nodes(sm.nlist, nn);
+        }
         g_mono += ni;
         g_quad += QUAD ? nn : 0;
         if (a.gstats && lane == 0) {
@@ -1672,6 +1797,34 @@ static tg_status launch_walk(WalkArgs<T> &a, int warps, cudaStream_t st) {
     return TG_OK;
 }
 
+// The pass in which a whole block walks each group (TEAM): over the listed groups, or all of them.
+template <int FIELDS, bool QUAD>
+static tg_status launch_team(WalkArgs<float> &a, cudaStream_t st) {
+    const size_t smem = sizeof(WarpSmem<float, QUAD, STACK_SMALL>) * TEAM_WARPS + sizeof(TeamSmem<field_comps<FIELDS>()>);
+    auto kern = k_walk<float, FIELDS, QUAD, STACK_SMALL, true>;
+    TG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    int per_sm = 0;
+    TG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, TEAM_WARPS * 32, smem));
+    int64_t blocks = (int64_t)std::max(per_sm, 1) * num_sms();
+    if (!a.ngroups_dev) blocks = std::min(blocks, std::max<int64_t>(a.ngroups, 1));
+    { kern<<<(unsigned)blocks, TEAM_WARPS * 32, smem, st>>>(a); tg::note_launch(); }
+    TG_CUDA(cudaGetLastError());
+    return TG_OK;
+}
+
+static tg_status dispatch_team(WalkArgs<float> &a, int fields, bool quad, cudaStream_t st) {
+    const int fc = fields == F_TID ? F_TID : ((fields & F_TID) ? (F_POT | F_ACC | F_TID) : fields);  // as dispatch_walk
+    switch (fc) {
+        case F_POT: return quad ? launch_team<F_POT, true>(a, st) : launch_team<F_POT, false>(a, st);
+        case F_ACC: return quad ? launch_team<F_ACC, true>(a, st) : launch_team<F_ACC, false>(a, st);
+        case F_POT | F_ACC: return quad ? launch_team<F_POT | F_ACC, true>(a, st) : launch_team<F_POT | F_ACC, false>(a, st);
+        case F_TID: return quad ? launch_team<F_TID, true>(a, st) : launch_team<F_TID, false>(a, st);
+        default:
+            return quad ? launch_team<F_POT | F_ACC | F_TID, true>(a, st)
+                        : launch_team<F_POT | F_ACC | F_TID, false>(a, st);
+    }
+}
+
 template <typename T, int STACK>
 static tg_status dispatch_walk(WalkArgs<T> &a, int fields, bool quad, int warps, cudaStream_t st) {
     // Fields computed: potential and/or acceleration alone; the tidal tensor alone in FP32 (its own
@@ -1702,12 +1855,30 @@ static tg_status dispatch_walk(WalkArgs<T> &a, int fields, bool quad, int warps,
 
 // Scratch of one walk, in ints: queue, status, retry count, retry queue, then the retry list.
 constexpr int WS_QUEUE = 0, WS_STATUS = 1, WS_RETRY_COUNT = 2, WS_RETRY_QUEUE = 3, WS_REWALK_COUNT = 4,
-              WS_REWALK_QUEUE = 5, WS_HEAVY_COUNT = 6, WS_HEAVY_QUEUE = 7,
-              WS_RETRY_LIST = 8;  // then the retry list, the rewalk list and the heavy list
-inline int64_t walk_scratch_ints(int64_t ngroups) { return WS_RETRY_LIST + 3 * std::max<int64_t>(ngroups, 1); }
+              WS_REWALK_QUEUE = 5, WS_HEAVY_COUNT = 6, WS_HEAVY_QUEUE = 7, WS_TEAM_COUNT = 8, WS_TEAM_QUEUE = 9,
+              WS_RETRY_LIST = 10;  // then the retry list, the rewalk list, the heavy list and the team list
+inline int64_t walk_scratch_ints(int64_t ngroups) { return WS_RETRY_LIST + 4 * std::max<int64_t>(ngroups, 1); }
 // List entries after which a group counts as heavy (split_heavy walks): the median group of 8 at 1e6
 // Plummer particles evaluates ~1.9e3, the 99.9th percentile ~7e3.
 constexpr unsigned HEAVY_ENTRIES = 1u << 15;
+// Walks of consecutive targets whose long groups a whole block walks (TEAM in k_walk). A group that straddles
+// a jump of the Morton curve evaluates up to every particle, and one warp on it took longer than all the
+// others together: 12345 Plummer particles in groups of 8, one group of 12343 entries (the median is 1131) in
+// 0.68 ms. The block's sums are the warp's, bit for bit, so which groups it takes is a matter of time alone:
+//   * up to TEAM_ALL_GROUPS groups (every field at once: TEAM_ALL_GROUPS_FULL, its block fills an SM), which
+//     leave the GPU's warps idle, all of them, in one pass. ms, one warp each / long ones to blocks / all to
+//     blocks: 1001 particles 0.086 / 0.094 / 0.050, 12345 0.684 / 0.331 / 0.217, 30000 1.64 / 0.605 /
+//     0.534, 50000 (6250 groups) 1.93 / 0.805 / 1.047; every field, 6000 0.450 / 0.284 / 0.198, 12345 0.887 /
+//     0.380 / 0.404.
+//   * beyond, those past TEAM_MIN_ENTRIES entries or a quarter of the number of groups, about half of
+//     what one of the GPU's ~3600 resident warps evaluates in all: 1e5 uniform 0.851 -> 0.558, 3e5 Plummer
+//     2.20 -> 1.79 (budgets of 1024 and 1500: the median group stops too, 50000 0.91).
+// From TEAM_MAX_GROUPS groups on the warps' other work hides a long group (1e6 particles: 4.64 ms
+// without the pass, 5.48 with it). Groups of 1 or 2 targets do not straddle enough to pay (3000 single
+// targets 0.061, all to blocks 0.213).
+constexpr int64_t TEAM_ALL_GROUPS = 4000, TEAM_ALL_GROUPS_FULL = 1400, TEAM_MAX_GROUPS = 65536;
+constexpr int64_t TEAM_MIN_ENTRIES = 2048;
+constexpr int TEAM_MIN_TARGETS = 4;
 constexpr int ITEM_CAP = 1 << 16;  // items per heavy group
 
 // Enqueue a whole walk on st (no host synchronisation, so it can be captured): with the small
@@ -1727,6 +1898,7 @@ static tg_status enqueue_walk(WalkArgs<T> a, int fields, bool quad, int warps, i
     a.heavy_count = split_heavy ? scratch + WS_HEAVY_COUNT : nullptr;
     a.heavy_budget = loop_limits().heavy_entries > 0 ? (unsigned)std::min<long long>(loop_limits().heavy_entries, 1ll << 30)
                                                      : HEAVY_ENTRIES;
+    a.stop_budget = a.heavy ? a.heavy_budget : ~0u;
     a.step_limit = loop_limits().walk_steps;
     const bool budget = a.tol_group && a.err_budget > 0.f;
     a.rewalk = budget ? scratch + WS_RETRY_LIST + ng1 : nullptr;
@@ -1737,7 +1909,33 @@ static tg_status enqueue_walk(WalkArgs<T> a, int fields, bool quad, int warps, i
     } else {
         a.retry = scratch + WS_RETRY_LIST;
         a.retry_count = scratch + WS_RETRY_COUNT;
-        TG_TRY((dispatch_walk<T, STACK_SMALL>(a, fields, quad, warps, st)));
+        // groups of consecutive targets, FP32: the long ones take a block each
+        bool team = false;
+        if constexpr (sizeof(T) == 4)
+            team = a.group_order && a.gs >= TEAM_MIN_TARGETS && a.ngroups <= TEAM_MAX_GROUPS && !a.tol_group && !a.gstats;
+        const bool full = (fields & F_TID) && fields != F_TID;
+        const bool team_all = team && a.ngroups <= (full ? TEAM_ALL_GROUPS_FULL : TEAM_ALL_GROUPS);
+        if (team && !team_all) {
+            a.team = scratch + WS_RETRY_LIST + 3 * ng1;
+            a.team_count = scratch + WS_TEAM_COUNT;
+            a.stop_budget = std::min(a.stop_budget, (unsigned)std::max<int64_t>(TEAM_MIN_ENTRIES, a.ngroups / 4));
+        }
+        if (!team_all) TG_TRY((dispatch_walk<T, STACK_SMALL>(a, fields, quad, warps, st)));
+        if constexpr (sizeof(T) == 4) {
+            if (team) {
+                WalkArgs<T> m = a;
+                m.queue = scratch + WS_TEAM_QUEUE;
+                if (!team_all) {
+                    m.group_order = a.team;
+                    m.ngroups_dev = a.team_count;
+                }
+                m.team = m.team_count = nullptr;
+                m.stop_budget = a.heavy ? a.heavy_budget : ~0u;
+                TG_TRY(dispatch_team(m, fields, quad, st));
+            }
+        }
+        a.team = a.team_count = nullptr;
+        a.stop_budget = a.heavy ? a.heavy_budget : ~0u;
         WalkArgs<T> b = a;
         b.queue = scratch + WS_RETRY_QUEUE;
         b.group_order = scratch + WS_RETRY_LIST;  // retry list entries are group indices
@@ -1754,6 +1952,7 @@ static tg_status enqueue_walk(WalkArgs<T> a, int fields, bool quad, int warps, i
     r.retry = r.retry_count = nullptr;
     r.rewalk = r.rewalk_count = nullptr;
     r.heavy = r.heavy_count = nullptr;
+    r.stop_budget = ~0u;
     r.tol_group = nullptr;
     r.theta_group = nullptr;
     r.gerr = nullptr;
@@ -1772,6 +1971,7 @@ static tg_status walk_heavy(tg_tree_s *t, const WalkArgs<T> &a, Arena<T> &ar, in
     WalkArgs<T> b = a;
     b.retry = b.retry_count = nullptr;
     b.heavy = b.heavy_count = nullptr;
+    b.stop_budget = ~0u;
     b.rewalk = b.rewalk_count = nullptr;
     b.ngroups_dev = nullptr;
     b.queue = scratch + WS_HEAVY_QUEUE;

@@ -1,0 +1,60 @@
+"""Groups walked by a whole block against groups walked by one warp each, bit for bit: the same batches of
+list entries, summed apart and added in the same order. The walk of a tree that records per-group
+counters keeps one warp per group, so it is the other side; node tests and interactions agree too.
+
+Sizes: one short batch; one node; group counts on both sides of the lines between walking every group by
+block, the long ones only, and none (4000 groups, 1400 with every field, 65536), by targets per
+group; the accepted sets and fields against the oracle are in test_gpu_walk.py.
+"""
+
+import ctypes
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def tg():
+    import pytreegrav_gb300 as tg
+
+    return tg
+
+
+def walk(tree, per_warp, **kw):
+    from pytreegrav_gb300 import _lib
+
+    L = _lib.load()
+    _lib.check(L.tg_tree_record_group_stats(tree._h, int(per_warp)))
+    res = tree.fields(**kw)
+    s = tree.last_walk_stats()
+    _lib.check(L.tg_tree_record_group_stats(tree._h, 0))
+    return res, (s[0], s[1], s[3])
+
+
+@pytest.mark.parametrize("quadrupole", [False, True])
+@pytest.mark.parametrize("fields", [("potential",), ("accel",), ("potential", "accel"), ("tidal",),
+                                    ("potential", "accel", "tidal")])
+@pytest.mark.parametrize("n,gs", [(1, 8), (5, 4), (33, 8), (1200, 4), (11201, 8), (5599, 4), (32001, 8), (31999, 8),
+                                  (30000, 32)])
+def test_block_walk(tg, n, gs, fields, quadrupole):
+    from pytreegrav_gb300 import synthetic
+
+    x = synthetic.clustered(n, 3) if n > 100 else synthetic.plummer(n, 3)
+    rng = np.random.default_rng(n)
+    tree = tg.ConstructTree(x, rng.random(n) / n, 0.02 * rng.random(n), quadrupole=True)
+    kw = dict({k: True for k in fields}, quadrupole=quadrupole, group_size=gs, theta=0.6)
+    # (32000-entry groups would be split when no counters are kept: these systems stay below)
+    one, s1 = walk(tree, True, **kw)
+    block, s2 = walk(tree, False, **kw)
+    for k in one:
+        assert np.array_equal(one[k], block[k]), k
+    assert s1 == s2
+    xt = rng.normal(size=(257, 3)) * 5  # few targets of many sources
+    kw.update(pos=xt, soft=np.zeros(257), order="morton")
+    one, s1 = walk(tree, True, **kw)
+    block, s2 = walk(tree, False, **kw)
+    for k in one:
+        assert np.array_equal(one[k], block[k]), k
+    assert s1 == s2
