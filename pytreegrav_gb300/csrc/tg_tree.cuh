@@ -25,8 +25,9 @@ struct Arena {
     int64_t n_nodes = 0, n_leaves = 0;
     // per node
     // traversal record, two per node: (hi.x, hi.y, hi.z, size), (delta, hmax, first node child << 4 |
-    // node children, leaf start << 4 | leaves) -- the integers stored as the bit pattern of T
-    vec4<T> *n_trav = nullptr;
+    // node children, leaf start << 4 | leaves) -- FP32 in either precision (the acceptance test decides in FP32
+    // where it can), the integers stored as bit patterns
+    float4 *n_trav = nullptr;
     vec4<T> *n_pos = nullptr;   // interaction record: hi.xyz, M
     vec4<T> *n_lo = nullptr;    // lo.xyz, hmax
     vec4<T> *n_quad = nullptr;  // two per node: (xx, xy, xz, yy), (yz, zz, 0, 0)

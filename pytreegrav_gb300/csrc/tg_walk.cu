@@ -35,12 +35,6 @@ constexpr int STACK_LARGE = 4096;  // the large stack (fewer resident warps)
 constexpr int ILIST_CAP = 320;
 constexpr int NLIST_CAP = 64;
 
-// Integers carried in a traversal record, as the bit pattern of the record's element type.
-__device__ __forceinline__ float int_bits(int v, float) { return __int_as_float(v); }
-__device__ __forceinline__ double int_bits(int v, double) { return __longlong_as_double((long long)v); }
-__device__ __forceinline__ int bits_int(float x) { return __float_as_int(x); }
-__device__ __forceinline__ int bits_int(double x) { return (int)__double_as_longlong(x); }
-
 // ---------------------------------------------------------------------------------------------
 // Softening kernels (kernel.py:5-75) in the walk's precision.
 template <typename T>
@@ -87,7 +81,24 @@ __device__ __forceinline__ float rsqrt_t(float x) {
     asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
-__device__ __forceinline__ double rsqrt_t(double x) { return rsqrt(x); }
+// 1 / sqrt(x) to about an ulp in five FP64 operations (GB300 issues one per sub-partition every ~76 cycles):
+// the FP32 approximation y of the significand's, taken with an even exponent on the integer units, and one
+// step of Householder's third-order iteration, y + y e (1/2 + 3/8 e) with e = 1 - x y^2 (|e| < 2^-20: the next term is
+// 5/16 e^3). Zeros, subnormals, negative values, infinities and NaN take the library's.
+__device__ __forceinline__ double rsqrt_t(double x) {
+    const uint64_t u = (uint64_t)__double_as_longlong(x);
+    const uint32_t hi = (uint32_t)(u >> 32), E = hi >> 20;  // sign and exponent
+    if (E - 1u >= 2046u) return rsqrt(x);
+    const uint32_t odd = (E + 1u) & 1u;             // x = m 2^(E - 1023 - odd), 1 <= m < 4
+    const int half = (int)(E - 1023u - odd) / 2;    // exact: the difference is even
+    // m rounded down to 24 bits: an FP32 number
+    const float m = __uint_as_float(((127u + odd) << 23) | ((hi & 0xfffffu) << 3) | (uint32_t)((uint32_t)u >> 29));
+    const uint32_t yb = __float_as_uint(rsqrt_t(m));  // 1/2 < y <= 1
+    const double y = __longlong_as_double((long long)(((uint64_t)((yb >> 3) + ((896u - (uint32_t)half) << 20)) << 32) |
+                                                      (uint64_t)(yb << 29)));
+    const double e = fma(-(x * y), y, 1.0);
+    return fma(y * e, fma(0.375, e, 0.5), y);
+}
 __device__ __forceinline__ float sqrt_t(float x) { return sqrtf(x); }
 __device__ __forceinline__ double sqrt_t(double x) { return sqrt(x); }
 
@@ -138,6 +149,8 @@ __device__ __forceinline__ void split_hi_lo(double x, double &hi, double &lo) {
 // FP64 value in the walk precision (integer conversion for FP32).
 __device__ __forceinline__ float narrow(double x, float) { return d2f(x); }
 __device__ __forceinline__ double narrow(double x, double) { return x; }
+__device__ __forceinline__ float to_f32(float x) { return x; }
+__device__ __forceinline__ float to_f32(double x) { return d2f(x); }
 
 __global__ void k_arena_links(int64_t ntot, int64_t mtot, const int64_t *first, const int64_t *next, int4 *link,
                               int64_t *nleaf, int *bad) {
@@ -212,9 +225,10 @@ __global__ void k_arena_nodes(int64_t ntot, int64_t mtot, const double *coord, c
     ar.n_pos[j] = vec4<T>{hx, hy, hz, narrow(mass[f], T(0))};
     ar.n_lo[j] = vec4<T>{lx, ly, lz, hm};
     const int fc = lk.y > 0 ? lk.x : 0;
-    ar.n_trav[2 * j] = vec4<T>{hx, hy, hz, narrow(size[f], T(0))};
-    ar.n_trav[2 * j + 1] = vec4<T>{narrow(delta[f], T(0)), hm, int_bits((fc << 4) | lk.y, T(0)),
-                                   int_bits((lk.z << 4) | lk.w, T(0))};
+    // FP32 in either arena (in an FP32 one hx, hy, hz and hm already are): the test's margins cover the rounding
+    ar.n_trav[2 * j] = make_float4(to_f32(hx), to_f32(hy), to_f32(hz), d2f(size[f]));
+    ar.n_trav[2 * j + 1] = make_float4(d2f(delta[f]), to_f32(hm), __int_as_float((fc << 4) | lk.y),
+                                       __int_as_float((lk.z << 4) | lk.w));
     if (ar.n_tol) {  // log form: no underflow for tiny nodes; zero for massless or empty ones
         const float mf = d2f(mass[f]), sf = d2f(size[f]);
         float a3 = 0.f, a2 = 0.f;
@@ -256,7 +270,7 @@ tg_status build_arena_topology(tg_tree_s *t, Arena<T> &ar, cudaStream_t st) {
     }
     TG_CUDA(tg::dev_malloc((void **)&ar.n_pos, sizeof(vec4<T>) * M, st));
     TG_CUDA(tg::dev_malloc((void **)&ar.n_lo, sizeof(vec4<T>) * M, st));
-    TG_CUDA(tg::dev_malloc((void **)&ar.n_trav, sizeof(vec4<T>) * 2 * M, st));
+    TG_CUDA(tg::dev_malloc((void **)&ar.n_trav, sizeof(float4) * 2 * M, st));
     TG_CUDA(tg::dev_malloc((void **)&ar.n_link, sizeof(int4) * M, st));
     if (ar.has_quad) TG_CUDA(tg::dev_malloc((void **)&ar.n_quad, sizeof(vec4<T>) * 2 * M, st));
     if (sizeof(T) == 4) TG_CUDA(tg::dev_malloc((void **)&ar.n_tol, sizeof(float2) * M, st));
@@ -511,8 +525,19 @@ __device__ __forceinline__ void quad_terms(const T *q, T dx, T dy, T dz, T rinv,
 // Acceleration of an accepted node, monopole and quadrupole together (the sum of point_mass and
 // quad_terms for F_ACC): a += dx (m r^-3 + 2.5 A r^-7) - (Q dx) r^-5, with A = dx.Q.dx.
 template <typename T>
-__device__ __forceinline__ void acc_mono_quad(T m, const T *q, T dx, T dy, T dz, T rinv, Acc<T> &p) {
+__device__ __forceinline__ void acc_mono_quad(T m, const T *q, T dx, T dy, T dz, T r2, T rinv, Acc<T> &p) {
     T rinv2 = rinv * rinv;
+    if constexpr (sizeof(T) == 8) {  // r^-5 (t dx - Q dx), t = m r^2 + 2.5 A r^-2: one FP64 operation fewer
+        const T r5 = rinv * rinv2 * rinv2;
+        const T nx = fma(q[2], dz, fma(q[1], dy, q[0] * dx)), ny = fma(q[4], dz, fma(q[3], dy, q[1] * dx));
+        const T nz = fma(q[5], dz, fma(q[4], dy, q[2] * dx));
+        const T A = fma(dz, nz, fma(dy, ny, dx * nx));
+        const T t = fma(T(2.5) * A, rinv2, m * r2);
+        p.v[1] = fma(r5, fma(t, dx, -nx), p.v[1]);
+        p.v[2] = fma(r5, fma(t, dy, -ny), p.v[2]);
+        p.v[3] = fma(r5, fma(t, dz, -nz), p.v[3]);
+        return;
+    }
     T r3inv = rinv * rinv2;
     T r5inv = r3inv * rinv2;
     T r7inv = r5inv * rinv2;
@@ -547,9 +572,6 @@ __device__ __forceinline__ void kahan_add(Acc<T> &S, Acc<T> &C, const Acc<T> &b)
         }
     }
 }
-
-__device__ __forceinline__ float pow_fifth(float q) { return q > 0.f ? __powf(q, 0.2f) : 0.f; }
-__device__ __forceinline__ double pow_fifth(double q) { return q > 0.0 ? pow(q, 0.2) : 0.0; }
 
 // Exact FP64 acceptance, the expression of treewalk.py:22-25 on the group box r_min
 // (grouped_treewalk.py:209-231), each operation rounded once.
@@ -593,11 +615,13 @@ __device__ __forceinline__ void write_fields(double *o, int out_fields, const do
 // Register caps (registers are granted 8 per thread at a time): the FP32 quadrupole acceleration
 // walk with the small stack runs at 72, which with its shared memory lets 7 blocks of 4 warps share
 // an SM (6 at 80); the other small-stack walks at 80 (6 blocks of 4 warps, 3 of 8; 81 would round
-// to 88 and leave 5 or 2); large-stack walks uncapped.
+// to 88 and leave 5 or 2); FP64 walks, bound by the FP64 pipe at any occupancy, at 112 (4 blocks of 4
+// warps; 50000 particles 5.67 ms at 80 and 5.28 at 112); large-stack walks uncapped.
 template <typename T, int FIELDS, bool QUAD, int STACK, bool TEAM = false>
 constexpr int walk_reg_cap() {
     if (TEAM) return 128;  // two blocks of eight warps per SM
     if (STACK != STACK_SMALL) return 255;
+    if (sizeof(T) == 8) return 112;
     return (sizeof(T) == 4 && FIELDS == F_ACC && QUAD) ? 72 : 80;
 }
 template <typename T, int FIELDS, bool QUAD, int STACK, bool TEAM = false>
@@ -656,7 +680,8 @@ __global__ void __launch_bounds__(MAX_WALK_WARPS * 32) __maxnreg__((walk_reg_cap
         const T th = thv.w;
         // group box, relative (for the near-source test) and absolute (for the node tests)
         T rbmin[3] = {tx, ty, tz}, rbmax[3] = {tx, ty, tz};
-        T abmin[3] = {thv.x, thv.y, thv.z}, abmax[3] = {thv.x, thv.y, thv.z};
+        const float fx = to_f32(thv.x), fy = to_f32(thv.y), fz = to_f32(thv.z);
+        float abmin[3] = {fx, fy, fz}, abmax[3] = {fx, fy, fz};
         T hmax_g = th;
 #pragma unroll
         for (int o = 16; o; o >>= 1) {
@@ -699,21 +724,20 @@ __global__ void __launch_bounds__(MAX_WALK_WARPS * 32) __maxnreg__((walk_reg_cap
             __syncwarp();
             have_box_d = true;
         };
-        const T gscale = fabs(abmin[0]) + fabs(abmin[1]) + fabs(abmin[2]) + fabs(abmax[0]) + fabs(abmax[1]) +
-                         fabs(abmax[2]);
-        const T inv_theta = (T)(1.0 / theta);
+        const float gscale = fabs(abmin[0]) + fabs(abmin[1]) + fabs(abmin[2]) + fabs(abmax[0]) + fabs(abmax[1]) +
+                             fabs(abmax[2]);
+        const float hmax_f = to_f32(hmax_g);
+        const float inv_theta = (float)(1.0 / theta);
         const float tolg = a.tol_group ? a.tol_group[g] : 0.f;
-        const bool mass_aware = tolg > 0.f;  // warp-uniform
+        const bool mass_aware = sizeof(T) == 4 && tolg > 0.f;  // warp-uniform; the FP64 walk takes no tolerances
         const bool track_err = mass_aware && (FIELDS & F_ACC) && (a.gerr || a.rewalk);
         float err_est = 0.f;  // this lane's share of the group's truncation estimate
-        const T inv_tol = mass_aware ? (T)(1.0 / (double)tolg) : T(0);
-        // FP32: a node's mass-aware radius is its stored factor times tol^(-1/(p+2))
-        const float tol_k = (sizeof(T) == 4 && mass_aware) ? exp2f(-log2f(tolg) * (QUAD ? 0.2f : 0.25f)) : 0.f;
-        const T rel_eps = sizeof(T) == 4 ? T(1e-5) : T(0);
-        const T abs_eps = sizeof(T) == 4 ? T(1e-6) : T(0);
+        // a node's mass-aware radius is its stored factor times tol^(-1/(p+2))
+        const float tol_k = mass_aware ? exp2f(-log2f(tolg) * (QUAD ? 0.2f : 0.25f)) : 0.f;
+        const float rel_eps = 1e-5f, abs_eps = 1e-6f;
         // softening-path threshold: a source whose squared distance to the box exceeds this cannot
         // be within any target's softening length, nor coincide with a target
-        const T near_eps = (sizeof(T) == 4 ? T(4e-7) : T(1e-15)) * (gscale + T(1e-30));
+        const T near_eps = (sizeof(T) == 4 ? T(4e-7) : T(1e-15)) * ((T)gscale + T(1e-30));
 
         Acc<T> S, C;
 #pragma unroll
@@ -990,9 +1014,10 @@ __global__ void __launch_bounds__(MAX_WALK_WARPS * 32) __maxnreg__((walk_reg_cap
                 vec4<T> qa = sm.sq[2 * (k0 + i)], qb = sm.sq[2 * (k0 + i) + 1];
                 T qv[6] = {qa.x, qa.y, qa.z, qa.w, qb.x, qb.y};
                 T dx = s.x - tx, dy = s.y - ty, dz = s.z - tz;
-                T rinv = rsqrt_t(dx * dx + dy * dy + dz * dz);
+                const T r2 = dx * dx + dy * dy + dz * dz;
+                T rinv = rsqrt_t(r2);
                 if (FIELDS == F_ACC) {
-                    acc_mono_quad(s.w, qv, dx, dy, dz, rinv, b);
+                    acc_mono_quad(s.w, qv, dx, dy, dz, r2, rinv, b);
                 } else {
                     point_mass<T, FIELDS>(s.w, dx, dy, dz, rinv, b);
                     quad_terms<T, FIELDS>(qv, dx, dy, dz, rinv, b);
@@ -1085,50 +1110,42 @@ __global__ void __launch_bounds__(MAX_WALK_WARPS * 32) __maxnreg__((walk_reg_cap
                 const int node = lane < cnt ? sm.stack[sp - 1 - lane] : -1;
                 sp -= cnt;
                 bool acc = false, unsure = false;
-                vec4<T> r1 = vec4<T>{T(0), T(0), T(0), T(0)};
+                float4 r1 = make_float4(0.f, 0.f, 0.f, 0.f);
                 if (node >= 0) {
                     n_tests++;
-                    const vec4<T> p = a.ar.n_trav[2 * node];
+                    const float4 p = a.ar.n_trav[2 * node];
                     r1 = a.ar.n_trav[2 * node + 1];
                     float2 tq = make_float2(0.f, 0.f);
                     if constexpr (sizeof(T) == 4) {
                         if (mass_aware) tq = a.ar.n_tol[node];  // issued with the traversal record
                     }
-                    T dx = fmax(fmax(abmin[0] - p.x, p.x - abmax[0]), T(0));
-                    T dy = fmax(fmax(abmin[1] - p.y, p.y - abmax[1]), T(0));
-                    T dz = fmax(fmax(abmin[2] - p.z, p.z - abmax[2]), T(0));
-                    T r2 = dx * dx + dy * dy + dz * dz;
-                    T h = r1.y > hmax_g ? r1.y : hmax_g;
-                    T c1 = p.w * inv_theta + r1.x, c2 = h + T(0.6) * p.w + r1.x;
-                    T msp = T(0);  // M s^p of the node (tolerance test only)
+                    float dx = fmax(fmax(abmin[0] - p.x, p.x - abmax[0]), 0.f);
+                    float dy = fmax(fmax(abmin[1] - p.y, p.y - abmax[1]), 0.f);
+                    float dz = fmax(fmax(abmin[2] - p.z, p.z - abmax[2]), 0.f);
+                    float r2 = dx * dx + dy * dy + dz * dz;
+                    float h = r1.y > hmax_f ? r1.y : hmax_f;
+                    float c1 = p.w * inv_theta + r1.x, c2 = h + 0.6f * p.w + r1.x;
+                    float msp = 0.f;  // M s^p of the node (tolerance test only)
                     if (mass_aware) {
-                        if constexpr (sizeof(T) == 4) {
-                            const float av = QUAD ? tq.x : tq.y;
-                            const float av2 = av * av;
-                            msp = QUAD ? av2 * av2 * av : av2 * av2;
-                            c1 = fmax(p.w * inv_theta, av * tol_k) + r1.x;
-                        } else {
-                            msp = a.ar.n_pos[node].w * (QUAD ? p.w * p.w * p.w : p.w * p.w);
-                            const T q = msp * inv_tol;
-                            const T rc = QUAD ? pow_fifth(q) : sqrt(sqrt(q));
-                            c1 = fmax(p.w * inv_theta, rc) + r1.x;
-                        }
+                        const float av = QUAD ? tq.x : tq.y;
+                        const float av2 = av * av;
+                        msp = QUAD ? av2 * av2 * av : av2 * av2;
+                        c1 = fmax(p.w * inv_theta, av * tol_k) + r1.x;
                     }
-                    T crit = c1 > c2 ? c1 : c2;
+                    float crit = c1 > c2 ? c1 : c2;
                     // FP32 error bound: node positions near the boundary are within gscale + 2 crit of
                     // the origin, so the relative term covers their rounding
-                    T tol = rel_eps * crit + abs_eps * gscale;
-                    T hiq = crit + tol, loq = crit - tol;
+                    float tol = rel_eps * crit + abs_eps * gscale;
+                    float hiq = crit + tol, loq = crit - tol;
                     if (mass_aware) {  // no pytreegrav decision to reproduce
                         acc = r2 > crit * crit;
                         if (acc && track_err) {  // r - delta > rc >= 0 here; an estimate: approximate ops
-                            const float d = (float)r2 * rsqrt_t((float)r2) - (float)r1.x, d2 = d * d;
-                            err_est += __fdividef((float)msp, QUAD ? d2 * d2 * d : d2 * d2);
+                            const float d = r2 * rsqrt_t(r2) - r1.x, d2 = d * d;
+                            err_est += __fdividef(msp, QUAD ? d2 * d2 * d : d2 * d2);
                         }
                     }
-                    else if (sizeof(T) == 8) unsure = true;
                     else if (r2 > hiq * hiq) acc = true;
-                    else if (loq > T(0) && r2 < loq * loq) acc = false;
+                    else if (loq > 0.f && r2 < loq * loq) acc = false;
                     else unsure = true;
                 }
                 if (__any_sync(FULL, unsure)) {
@@ -1138,7 +1155,7 @@ __global__ void __launch_bounds__(MAX_WALK_WARPS * 32) __maxnreg__((walk_reg_cap
                                            sm.xbox[6], sm.xbox[7]);
                 }
                 const bool opn = node >= 0 && !acc;
-                const int cbits = opn ? bits_int(r1.z) : 0, lbits = opn ? bits_int(r1.w) : 0;
+                const int cbits = opn ? __float_as_int(r1.z) : 0, lbits = opn ? __float_as_int(r1.w) : 0;
                 const unsigned am = __ballot_sync(FULL, acc);
                 if (QUAD) {
                     if (acc) sm.nlist[nn + __popc(am & lt)] = node;
@@ -1666,7 +1683,7 @@ __global__ void __launch_bounds__(TOP_WARPS * 32) k_walk_top(TopArgs<T> a) {
         if (node >= 0) {
             acc = accept_exact(a.ntot + node, a.tc, a.ts, a.tsize, a.tdelta, bmin, bmax, hmax, theta);
             if (!acc) {
-                const int cb = bits_int(a.ar.n_trav[2 * node + 1].z), lb = bits_int(a.ar.n_trav[2 * node + 1].w);
+                const int cb = __float_as_int(a.ar.n_trav[2 * node + 1].z), lb = __float_as_int(a.ar.n_trav[2 * node + 1].w);
                 fc = cb >> 4;
                 nc = cb & 15;
                 ls = lb >> 4;
@@ -1881,6 +1898,17 @@ constexpr int64_t TEAM_MIN_ENTRIES = 2048;
 constexpr int TEAM_MIN_TARGETS = 4;
 constexpr int ITEM_CAP = 1 << 16;  // items per heavy group
 
+// FP64 walks of consecutive targets split sooner: one warp takes ~13 us for 32 entries of 8 targets, so a
+// group of 32768 was 13 ms of a 50000-particle walk's 18.3. About a third of what one warp evaluates in all
+// then bounds the tail, and below 2048 (the median is 1100 to 1900) splitting costs more than it
+// saves. ms at budgets of 32768 / 8192 / 4096 / 2048: 12345 particles 5.78 / 4.40 / 2.64 / 2.11, 50000 18.4 / 7.83
+// / 6.77 / 7.82, 2e5 33.7 / 27.3 / 28.8 / 48.
+template <typename T>
+static unsigned heavy_entries(const WalkArgs<T> &a) {
+    if (sizeof(T) == 4 || !a.group_order) return HEAVY_ENTRIES;
+    return (unsigned)std::min<int64_t>(12288, std::max<int64_t>(2048, a.ngroups / 2));
+}
+
 // Enqueue a whole walk on st (no host synchronisation, so it can be captured): with the small
 // first stack, the small-stack pass, then a large-stack pass over the groups that overflowed it
 // (an empty pass when none did); with the large first stack, one large-stack pass. scratch:
@@ -1897,7 +1925,7 @@ static tg_status enqueue_walk(WalkArgs<T> a, int fields, bool quad, int warps, i
     a.heavy = split_heavy ? scratch + WS_RETRY_LIST + 2 * ng1 : nullptr;
     a.heavy_count = split_heavy ? scratch + WS_HEAVY_COUNT : nullptr;
     a.heavy_budget = loop_limits().heavy_entries > 0 ? (unsigned)std::min<long long>(loop_limits().heavy_entries, 1ll << 30)
-                                                     : HEAVY_ENTRIES;
+                                                     : heavy_entries<T>(a);
     a.stop_budget = a.heavy ? a.heavy_budget : ~0u;
     a.step_limit = loop_limits().walk_steps;
     const bool budget = a.tol_group && a.err_budget > 0.f;
@@ -2099,7 +2127,7 @@ static int arena_exceeds_l2(const Arena<T> &ar) {
         if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev);
         if (l2 <= 0) l2 = 128 << 20;
     }
-    const int64_t bytes = ar.n_nodes * (int64_t)sizeof(vec4<T>) * (ar.n_quad ? 6 : 4) +
+    const int64_t bytes = ar.n_nodes * ((int64_t)sizeof(vec4<T>) * (ar.n_quad ? 4 : 2) + 2 * (int64_t)sizeof(float4)) +
                           ar.n_leaves * (int64_t)sizeof(vec4<T>) * 2 + (ar.n_tol ? ar.n_nodes * 8 : 0);
     return bytes > (int64_t)l2;
 }

@@ -1,4 +1,9 @@
-"""Groups walked by a whole block against groups walked by one warp each, bit for bit: the same batches of
+"""Walks of consecutive targets whose long groups do not stay with one warp.
+
+FP64 walks split them sooner than FP32 ones: fields against the oracle (1e-12, the FP64 walk's bar) at sizes
+whose longest groups are split, with softened targets.
+
+FP32: groups walked by a whole block against groups walked by one warp each, bit for bit: the same batches of
 list entries, summed apart and added in the same order. The walk of a tree that records per-group
 counters keeps one warp per group, so it is the other side; node tests and interactions agree too.
 
@@ -11,6 +16,8 @@ import ctypes
 
 import numpy as np
 import pytest
+
+from oracle import oracle as O
 
 pytestmark = pytest.mark.gpu
 
@@ -58,3 +65,22 @@ def test_block_walk(tg, n, gs, fields, quadrupole):
     for k in one:
         assert np.array_equal(one[k], block[k]), k
     assert s1 == s2
+
+
+@pytest.mark.parametrize("quadrupole", [False, True])
+@pytest.mark.parametrize("n,gs", [(40, 8), (3001, 8), (12345, 8), (12345, 1), (20011, 16)])
+def test_fp64_split(tg, n, gs, quadrupole):
+    from pytreegrav_gb300 import synthetic
+
+    x = synthetic.plummer(n, 17)
+    rng = np.random.default_rng(n)
+    m, h = rng.random(n) / n, np.where(rng.random(n) < 0.2, 0.0, 0.05 * rng.random(n))
+    kw = dict(potential=True, accel=True, tidal=True, theta=0.7, quadrupole=quadrupole, group_size=gs)
+    ref, _ = O.self_fields(x, m, h, nthreads=O.num_threads(), **kw)
+    got = tg.ConstructTree(x, m, h, quadrupole=quadrupole).fields(precision="fp64", **kw)
+    alone = tg.ConstructTree(x, m, h, quadrupole=quadrupole).fields(precision="fp64", **dict(kw, potential=False, tidal=False))
+    for k in ref:
+        a, b = got[k].reshape(n, -1), ref[k].reshape(n, -1)
+        assert np.sqrt(np.sum((a - b) ** 2)) < 1e-12 * np.sqrt(np.sum(b**2)), k
+    a, b = alone["accel"], ref["accel"]
+    assert np.sqrt(np.sum((a - b) ** 2)) < 1e-12 * np.sqrt(np.sum(b**2))
