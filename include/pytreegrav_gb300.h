@@ -261,6 +261,12 @@ tg_status tg_tree_correlation(tg_tree tree, int kind, const double *pos, const d
                               double boxsize, int weighted_binning, uint64_t seed, int mem, double *binsums,
                               double *wtsums, void *stream);
 
+/* The radial range behind the two-point functions' default bins (frontend.py:1091-1093): of the points'
+ * distances from their median position (numpy's median per coordinate), the one of the given rank from
+ * below (0 the smallest) and the largest, written to out[0] and out[1] (host memory). pos (n, 3), host or
+ * device per mem, finite; the values are numpy's, bit for bit. Synchronises `stream`. */
+tg_status tg_radial_range(const double *pos, int64_t n, int64_t rank, int mem, double *out, void *stream);
+
 /* Number of visible CUDA devices (0, not an error, when there is no driver or device); the check
  * behind pytreegrav.cuda.is_available (cuda.py:70-80). */
 tg_status tg_device_count(int *count);

@@ -67,6 +67,7 @@ EXPORTS = [
     "tg_tree_set_velocities",
     "tg_tree_copy_velocities",
     "tg_tree_correlation",
+    "tg_radial_range",
     "tg_device_count",
     "tg_sources_create",
     "tg_sources_bruteforce",
@@ -174,6 +175,7 @@ def _declare(L):
     L.tg_tree_copy_velocities.argtypes = [vp, vp, vp, vp]
     L.tg_tree_correlation.argtypes = [vp, ci, vp, vp, vp, i64, vp, ci, dbl, dbl, dbl, ci, ctypes.c_uint64, ci, vp,
                                       vp, vp]
+    L.tg_radial_range.argtypes = [vp, i64, i64, ci, vp, vp]
     L.tg_device_count.argtypes = [ctypes.POINTER(ci)]
     L.tg_sources_create.argtypes = [vp, vp, vp, i64, ci, vp, ctypes.POINTER(vp)]
     L.tg_sources_bruteforce.argtypes = [vp, vp, vp, i64, ci, dbl, ci, ci, vp, vp]

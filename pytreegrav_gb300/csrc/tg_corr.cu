@@ -20,6 +20,7 @@
 // One thread per target, each of a fixed set of threads accumulating its targets (a fixed stride) into
 // a private row of bins in device memory; rows are added per bin by a fixed-shape reduction, so the
 // result does not depend on timing.
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <new>
@@ -493,12 +494,135 @@ __global__ void __launch_bounds__(CORR_RED) k_corr_reduce(const double *rows, in
     if (t == 0) out[b] = sh[0];
 }
 
+// Order statistics by radix selection (tg_radial_range): 8 bits per pass from the top, every query's digit
+// histogram over the keys that share its prefix, the digit that holds its rank picked by the last block.
+// Points' columns: query q is rank[q] of column q / 2; one array of keys: query 0. Exact: the values
+// themselves come out, as numpy's partition gives them. Bound by the passes' launches and the picks (17
+// launches, ~8 us each at 2e5 points); a sort of four columns would write what nothing reads.
+constexpr int SEL_Q = 6, SEL_PASSES = 8, SEL_THREADS = 256;
+struct SelectState {
+    unsigned long long prefix[SEL_Q];
+    unsigned long long rank[SEL_Q];  // among the keys with the prefix
+    unsigned hist[SEL_PASSES][SEL_Q][256];
+    unsigned done[SEL_PASSES];
+};
+
+template <bool COLUMNS>
+__global__ void __launch_bounds__(SEL_THREADS) k_select(const double *pos, const unsigned long long *keys, int64_t n,
+                                                        int pass, SelectState *st) {
+    constexpr int Q = COLUMNS ? SEL_Q : 1;
+    __shared__ unsigned h[Q][256];
+    __shared__ bool last;
+    for (int i = threadIdx.x; i < Q * 256; i += SEL_THREADS) (&h[0][0])[i] = 0;
+    __syncthreads();
+    const int shift = 64 - 8 * (pass + 1);
+    unsigned long long prefix[Q];
+#pragma unroll
+    for (int q = 0; q < Q; q++) prefix[q] = st->prefix[q];
+    for (int64_t i = (int64_t)blockIdx.x * SEL_THREADS + threadIdx.x; i < n; i += (int64_t)gridDim.x * SEL_THREADS) {
+#pragma unroll
+        for (int c = 0; c < (COLUMNS ? 3 : 1); c++) {
+            const unsigned long long k = COLUMNS ? dbl_to_ordered(pos[3 * i + c]) : keys[i];
+#pragma unroll
+            for (int s = 0; s < (COLUMNS ? 2 : 1); s++) {
+                const int q = COLUMNS ? 2 * c + s : 0;
+                if (pass == 0 || (k ^ prefix[q]) >> (shift + 8) == 0) atomicAdd(&h[q][(k >> shift) & 255], 1u);
+            }
+        }
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < Q * 256; i += SEL_THREADS)
+        if ((&h[0][0])[i]) atomicAdd(&st->hist[pass][i >> 8][i & 255], (&h[0][0])[i]);
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(&st->done[pass], 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    const int q = threadIdx.x >> 5, lane = threadIdx.x & 31;  // a warp per query, eight digits per lane
+    if (q >= Q) return;
+    unsigned long long cnt[8], sum = 0;
+    for (int d = 0; d < 8; d++) sum += cnt[d] = __ldcg(&st->hist[pass][q][8 * lane + d]);
+    unsigned long long before = warp_inclusive_scan(sum) - sum;
+    const unsigned long long rank = st->rank[q];
+    __syncwarp();
+    for (int d = 0; d < 8; d++) {
+        if (rank >= before && rank < before + cnt[d]) {  // one lane's one digit
+            st->rank[q] = rank - before;
+            st->prefix[q] |= (unsigned long long)(8 * lane + d) << shift;
+        }
+        before += cnt[d];
+    }
+}
+
+// Keys of the points' distances from the selected medians, and the largest: numpy's median (the mean of the two
+// middle values, equal for an odd count) and sqrt(dx dx + dy dy + dz dz), each operation rounded once.
+__global__ void __launch_bounds__(SEL_THREADS) k_radial_keys(const double *pos, int64_t n, const SelectState *st,
+                                                             unsigned long long *keys, unsigned long long *largest) {
+    double med[3];
+    for (int c = 0; c < 3; c++)
+        med[c] = n & 1 ? ordered_to_dbl(st->prefix[2 * c])
+                       : dmul(dadd(ordered_to_dbl(st->prefix[2 * c]), ordered_to_dbl(st->prefix[2 * c + 1])), 0.5);
+    unsigned long long top = 0;
+    for (int64_t i = (int64_t)blockIdx.x * SEL_THREADS + threadIdx.x; i < n; i += (int64_t)gridDim.x * SEL_THREADS) {
+        const double d0 = dsub(pos[3 * i], med[0]), d1 = dsub(pos[3 * i + 1], med[1]), d2 = dsub(pos[3 * i + 2], med[2]);
+        const double r = __dsqrt_rn(dadd(dadd(dmul(d0, d0), dmul(d1, d1)), dmul(d2, d2)));
+        const unsigned long long k = dbl_to_ordered(r);
+        keys[i] = k;
+        top = k > top ? k : top;
+    }
+    for (int o = 16; o; o >>= 1) {
+        const unsigned long long u = __shfl_xor_sync(FULL, top, o);
+        top = u > top ? u : top;
+    }
+    if (lane_id() == 0) atomicMax(largest, top);
+}
+
 }  // namespace
 }  // namespace tg
 
 using namespace tg;
 
 extern "C" {
+
+tg_status tg_radial_range(const double *pos, int64_t n, int64_t rank, int mem, double *out, void *stream) {
+    if (!pos || !out || n < 1 || n > 0x7fffffffLL || rank < 0 || rank >= n ||
+        (mem != TG_MEM_HOST && mem != TG_MEM_DEVICE))
+        return TG_ERR_BAD_ARG;
+    cudaStream_t st = (cudaStream_t)stream;
+    DevArray<double> staged(st);
+    DevArray<SelectState> state(st);
+    DevArray<unsigned long long> keys(st);
+    const double *dp = pos;
+    if (mem == TG_MEM_HOST) {
+        TG_CUDA(staged.alloc(3 * n));
+        TG_CUDA(cudaMemcpyAsync(staged.p, pos, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, st));
+        dp = staged.p;
+    }
+    TG_CUDA(state.alloc(2));  // the columns', then the distances'
+    TG_CUDA(keys.alloc(n + 1));
+    unsigned long long *largest = keys.p + n;
+    unsigned long long ranks[SEL_Q], first = (unsigned long long)rank;
+    for (int q = 0; q < SEL_Q; q++) ranks[q] = (unsigned long long)((q & 1) || (n & 1) ? n / 2 : n / 2 - 1);
+    TG_CUDA(cudaMemsetAsync(state.p, 0, 2 * sizeof(SelectState), st));
+    TG_CUDA(cudaMemsetAsync(largest, 0, sizeof(unsigned long long), st));
+    TG_CUDA(cudaMemcpyAsync(state.p[0].rank, ranks, sizeof(ranks), cudaMemcpyHostToDevice, st));
+    TG_CUDA(cudaMemcpyAsync(state.p[1].rank, &first, sizeof(first), cudaMemcpyHostToDevice, st));
+    const int blocks = (int)std::min<int64_t>(div_up(n, 4 * SEL_THREADS), 2 * num_sms());
+    for (int p = 0; p < SEL_PASSES; p++) { k_select<true><<<blocks, SEL_THREADS, 0, st>>>(dp, nullptr, n, p, state.p); note_launch(); }
+    { k_radial_keys<<<blocks, SEL_THREADS, 0, st>>>(dp, n, state.p, keys.p, largest); note_launch(); }
+    for (int p = 0; p < SEL_PASSES; p++) { k_select<false><<<blocks, SEL_THREADS, 0, st>>>(nullptr, keys.p, n, p, state.p + 1); note_launch(); }
+    TG_CUDA(cudaGetLastError());
+    unsigned long long got[2];
+    TG_CUDA(cudaMemcpyAsync(got, state.p[1].prefix, sizeof(got[0]), cudaMemcpyDeviceToHost, st));
+    TG_CUDA(cudaMemcpyAsync(got + 1, largest, sizeof(got[0]), cudaMemcpyDeviceToHost, st));
+    TG_CUDA(cudaStreamSynchronize(st));
+    for (int k = 0; k < 2; k++) {  // ordered_to_dbl on the host
+        const unsigned long long b = (got[k] & 0x8000000000000000ull) ? (got[k] & 0x7fffffffffffffffull) : ~got[k];
+        memcpy(out + k, &b, sizeof(b));
+    }
+    return TG_OK;
+}
 
 tg_status tg_tree_set_velocities(tg_tree t, const double *vel, int mem, void *stream) {
     if (!t || !vel || (mem != TG_MEM_HOST && mem != TG_MEM_DEVICE)) return TG_ERR_BAD_ARG;

@@ -517,6 +517,15 @@ def morton_order(pos):
     return perm
 
 
+def radial_range(pos, rank):
+    """The rank-th smallest (from 0) and the largest of the points' distances from their median position."""
+    pos = _as_f64(pos, (-1, 3))
+    out = np.empty(2)
+    _lib.check(_lib.load().tg_radial_range(_lib.ptr(pos), len(pos), int(rank), _lib.TG_MEM_HOST, _lib.ptr(out), None),
+               "radial range")
+    return out[0], out[1]
+
+
 def bruteforce(pos_t, h_t, pos_s, m_s, h_s, potential=False, accel=False, tidal=False, mutual=False, G=1.0,
                precision="fp64"):
     """Direct summation on the GPU. mutual=True: targets are the sources, self excluded by index."""

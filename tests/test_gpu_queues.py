@@ -51,3 +51,21 @@ def test_corr_queue(tg, kind, n, nt, nbins):
     assert np.all(np.abs(b - bo) <= 1e-12 * np.maximum(scale, 1e-300))
     if kind != "density":
         assert np.all(np.abs(w - wo) <= 1e-12 * np.maximum(wo, 1e-300))
+
+
+@pytest.mark.parametrize("n", [11, 12, 255, 1024, 1025, 40001])
+@pytest.mark.parametrize("kind", ["normal", "lattice", "equal"])
+def test_radial_range(tg, n, kind):
+    """Ranks of the distances from the median position: numpy's values, bit for bit."""
+    from pytreegrav_gb300.tree import radial_range
+
+    rng = np.random.default_rng(n)
+    x = rng.normal(size=(n, 3)) * [1e-3, 1.0, 1e4] - [0.0, 3.0, 0.0]
+    if kind == "lattice":
+        x = np.round(x)  # many equal values, zeros of both signs
+    if kind == "equal":
+        x = np.full((n, 3), 0.25)
+    d = [x[:, k] - np.median(x[:, k]) for k in range(3)]
+    r = np.sort(np.sqrt(d[0] * d[0] + d[1] * d[1] + d[2] * d[2]))
+    for rank in (0, 10, n // 2, n - 1):
+        assert radial_range(x, rank) == (r[rank], r[-1])
