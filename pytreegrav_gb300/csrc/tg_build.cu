@@ -62,7 +62,11 @@ __global__ void __launch_bounds__(BB_THREADS) k_bbox(const double *pos, int64_t 
     int64_t tile0 = (int64_t)blockIdx.x * BB_THREADS * BB_ITEMS;
     if (tile0 >= n) return;
     int64_t tile1 = min(tile0 + (int64_t)BB_THREADS * BB_ITEMS, n) - 1;
-    int s0 = (int)find_seg(sys_off, nsys, tile0), s1 = (int)find_seg(sys_off, nsys, tile1);
+    int s0 = 0, s1 = 0;  // one system: sys_off is not read
+    if (nsys > 1) {
+        s0 = (int)find_seg(sys_off, nsys, tile0);
+        s1 = (int)find_seg(sys_off, nsys, tile1);
+    }
     if (s0 == s1) {
         unsigned long long lo[3] = {~0ull, ~0ull, ~0ull}, hi[3] = {0, 0, 0};
         for (int it = 0; it < BB_ITEMS; it++) {
@@ -1966,36 +1970,34 @@ tg_status ensure_quad64(tg_tree_s *T, cudaStream_t st) {
 
 // _morton_order (grouped_treewalk.py:269-275): stable order of points by their keys in their own
 // bounding cube. perm receives uint32 indices.
-tg_status morton_order_device(const double *pos, int64_t n, uint32_t *perm, cudaStream_t st) {
+// err_dev: a device int that receives a failed sort's flag, for a caller that reads it with its results (the
+// permutation is then the identity); null: this call reads its own, synchronises and reports it.
+tg_status morton_order_device(const double *pos, int64_t n, uint32_t *perm, cudaStream_t st, int *err_dev) {
     if (n <= 0) return TG_OK;
     if (n > 0x7fffffffLL) return TG_ERR_BAD_ARG;
-    const int64_t off[2] = {0, n};
-    DevArray<int64_t> sys_off(st);
-    DevArray<unsigned long long> mn(st), mx(st);
-    DevArray<double> center(st), size(st);
+    struct Cube {
+        unsigned long long mn[3], mx[3];
+        double center[3], size;
+        int err;
+    };
+    DevArray<Cube> cube(st);
     DevArray<uint64_t> keys(st);
-    DevArray<int> err(st);
-    TG_CUDA(sys_off.alloc(2));
-    TG_CUDA(mn.alloc(3));
-    TG_CUDA(mx.alloc(3));
-    TG_CUDA(center.alloc(3));
-    TG_CUDA(size.alloc(1));
+    TG_CUDA(cube.alloc(1));
     TG_CUDA(keys.alloc(n));
-    TG_CUDA(err.alloc(1));
-    TG_CUDA(cudaMemsetAsync(err.p, 0, sizeof(int), st));
-    TG_CUDA(cudaMemcpyAsync(sys_off.p, off, sizeof(int64_t) * 2, cudaMemcpyHostToDevice, st));
-    { k_bbox_init<<<1, 32, 0, st>>>(mn.p, mx.p, 1); tg::note_launch(); }
-    { k_bbox<<<div_up(n, BB_THREADS * BB_ITEMS), BB_THREADS, 0, st>>>(pos, n, sys_off.p, 1, mn.p, mx.p); tg::note_launch(); }
-    { k_bbox_finish<<<1, 32, 0, st>>>(mn.p, mx.p, 1, center.p, size.p); tg::note_launch(); }
-    { k_keys<<<LAUNCH(n)>>>(pos, n, sys_off.p, 1, center.p, size.p, keys.p, nullptr, perm); tg::note_launch(); }
+    TG_CUDA(cudaMemsetAsync(cube.p->mn, 0xff, sizeof(cube.p->mn), st));
+    TG_CUDA(cudaMemsetAsync(cube.p->mx, 0, sizeof(Cube) - sizeof(cube.p->mn), st));
+    int *err = err_dev ? err_dev : &cube.p->err;
+    { k_bbox<<<div_up(n, BB_THREADS * BB_ITEMS), BB_THREADS, 0, st>>>(pos, n, nullptr, 1, cube.p->mn, cube.p->mx); tg::note_launch(); }
+    { k_bbox_finish<<<1, 32, 0, st>>>(cube.p->mn, cube.p->mx, 1, cube.p->center, &cube.p->size); tg::note_launch(); }
+    { k_keys<<<LAUNCH(n)>>>(pos, n, nullptr, 1, cube.p->center, &cube.p->size, keys.p, nullptr, perm); tg::note_launch(); }
     TG_CUDA(cudaGetLastError());
-    tg_status rc = radix_sort_pairs(keys.p, perm, n, 63, st, err.p);
-    int bad = 0;
-    if (rc == TG_OK) TG_CUDA(cudaMemcpyAsync(&bad, err.p, sizeof(int), cudaMemcpyDeviceToHost, st));
-    // the host array `off` must outlive its copy, also on error
+    TG_TRY(radix_sort_pairs(keys.p, perm, n, 63, st, err));
+    if (err_dev) return TG_OK;
+    void *host = nullptr;
+    TG_TRY(host_words(&host));
+    TG_CUDA(cudaMemcpyAsync(host, err, sizeof(int), cudaMemcpyDeviceToHost, st));
     TG_CUDA(cudaStreamSynchronize(st));
-    TG_TRY(rc);
-    if (bad) {
+    if (*(const int *)host) {
         set_last_error_msg("radix sort: a tile's look-back did not complete within its bound");
         return TG_ERR_QUEUE_TIMEOUT;
     }

@@ -11,7 +11,7 @@ tg_status build_tree(tg_tree_s *T, const double *pos, const double *m, const dou
                      const std::vector<int64_t> &sys_off_host, int quadrupole, int compute_moments,
                      const int *nonfinite, cudaStream_t st, cudaEvent_t m_h_ready);
 tg_status tree_side_stream(tg_tree_s *t);
-tg_status morton_order_device(const double *pos, int64_t n, uint32_t *perm, cudaStream_t st);
+tg_status morton_order_device(const double *pos, int64_t n, uint32_t *perm, cudaStream_t st, int *err_dev);
 template <typename T>
 tg_status build_arena(tg_tree_s *t, Arena<T> &ar, cudaStream_t st);
 template <typename T>
@@ -56,7 +56,7 @@ __global__ void k_u32_to_i64(const uint32_t *a, int64_t n, int64_t *b) {
 }
 
 __global__ void k_gather_targets(const uint32_t *perm, int64_t n, const double *pos, const double *h, double *pos_s,
-                                 double *h_s) {
+                                 double *h_s, int64_t *scatter) {
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     int64_t o = perm[i];
@@ -64,6 +64,7 @@ __global__ void k_gather_targets(const uint32_t *perm, int64_t n, const double *
     pos_s[3 * i + 1] = pos[3 * o + 1];
     pos_s[3 * i + 2] = pos[3 * o + 2];
     h_s[i] = h ? h[o] : 0.0;
+    scatter[i] = o;
 }
 
 // Device copies of caller arrays (or the caller's own device pointers), freed on scope exit.
@@ -98,11 +99,12 @@ tg_status check_finite(const double *const *arrs, const int64_t *counts, int k, 
     TG_CUDA(cudaMemsetAsync(flag, 0, sizeof(int), st));
     for (int q = 0; q < k; q++)
         if (arrs[q] && counts[q] > 0) { k_nonfinite<<<div_up(counts[q], 256), 256, 0, st>>>(arrs[q], counts[q], flag); tg::note_launch(); }
-    int hflag = 0;
-    TG_CUDA(cudaMemcpyAsync(&hflag, flag, sizeof(int), cudaMemcpyDeviceToHost, st));
+    void *host = nullptr;
+    TG_TRY(host_words(&host));
+    TG_CUDA(cudaMemcpyAsync(host, flag, sizeof(int), cudaMemcpyDeviceToHost, st));
     TG_CUDA(cudaFreeAsync(flag, st));
     TG_CUDA(cudaStreamSynchronize(st));
-    return hflag ? TG_ERR_NONFINITE : TG_OK;
+    return *(const int *)host ? TG_ERR_NONFINITE : TG_OK;
 }
 
 void destroy(tg_tree_s *t) {
@@ -115,7 +117,6 @@ void destroy(tg_tree_s *t) {
     f(t->first); f(t->next); f(t->walk_idx); f(t->parent); f(t->node_range); f(t->cell_center);
     free_arena(t->arena32, st);
     free_arena(t->arena64, st);
-    if (t->stats_dev) cudaFreeAsync(t->stats_dev, st);
     f(t->groups); f(t->group_root); f(t->group_node); f(t->gstats); f(t->gerr); f(t->sort_err); f(t->vel); f(t->vdisp); f(t->quad32); f(t->lvl_list); f(t->fdepth); f(t->own32);
     release_stream(t->side);  // back to the library's pool, its queued work still to run
     release_event(t->ev_fork, false, t->dev);
@@ -335,7 +336,7 @@ tg_status tg_tree_fields(tg_tree t, const double *pos, const double *h, int64_t 
             ngroups = t->ngroups;
         } else {
             TG_TRY(make_groups(t, t->sys_off, group_size, &groups, &groot, &ngroups, st));
-            TG_TRY(make_cost_order(t->coord, groups, ngroups, &gorder, st, t->sort_err));
+            if (group_size > 1) TG_TRY(make_cost_order(t->coord, groups, ngroups, &gorder, st, t->sort_err));
             wg = groups;
             wr = groot;
         }
@@ -357,12 +358,11 @@ tg_status tg_tree_fields(tg_tree t, const double *pos, const double *h, int64_t 
         if (order == TG_ORDER_MORTON) {
             uint32_t *perm = nullptr;
             TG_CUDA(tg::dev_malloc((void **)&perm, sizeof(uint32_t) * n, st));
-            TG_TRY(morton_order_device(dp.ptr, n, perm, st));
+            TG_TRY(morton_order_device(dp.ptr, n, perm, st, t->sort_err));  // reported with the walk's results
             TG_CUDA(tg::dev_malloc((void **)&sp, sizeof(double) * 3 * n, st));
             TG_CUDA(tg::dev_malloc((void **)&sh, sizeof(double) * n, st));
             TG_CUDA(tg::dev_malloc((void **)&scatter, sizeof(int64_t) * n, st));
-            { k_gather_targets<<<div_up(n, 256), 256, 0, st>>>(perm, n, dp.ptr, dh.ptr, sp, sh); tg::note_launch(); }
-            { k_u32_to_i64<<<div_up(n, 256), 256, 0, st>>>(perm, n, scatter); tg::note_launch(); }
+            { k_gather_targets<<<div_up(n, 256), 256, 0, st>>>(perm, n, dp.ptr, dh.ptr, sp, sh, scatter); tg::note_launch(); }
             TG_CUDA(cudaGetLastError());
             TG_CUDA(cudaFreeAsync(perm, st));
         } else {
@@ -372,7 +372,7 @@ tg_status tg_tree_fields(tg_tree t, const double *pos, const double *h, int64_t 
         }
         std::vector<int64_t> toff = {0, n};
         TG_TRY(make_groups(t, toff, group_size, &groups, &groot, &ngroups, st));
-        TG_TRY(make_cost_order(sp ? sp : dp.ptr, groups, ngroups, &gorder, st, t->sort_err));
+        if (group_size > 1) TG_TRY(make_cost_order(sp ? sp : dp.ptr, groups, ngroups, &gorder, st, t->sort_err));
         if (mem == TG_MEM_HOST) TG_CUDA(tg::dev_malloc((void **)&dout, sizeof(double) * nt * W, st));
         else dout = out;
         rc = run_walk(t, sp ? sp : dp.ptr, sh, nt, groups, groot, gorder, ngroups, scatter, fields, quadrupole, theta, G,
@@ -427,7 +427,7 @@ tg_status tg_morton_order(const double *pos, int64_t n, int mem, int64_t *perm, 
     DevArray<uint32_t> p32(st);
     DevArray<int64_t> p64buf(st);
     TG_CUDA(p32.alloc(n));
-    TG_TRY(morton_order_device(dp.ptr, n, p32.p, st));
+    TG_TRY(morton_order_device(dp.ptr, n, p32.p, st, nullptr));
     int64_t *p64 = perm;
     if (mem == TG_MEM_HOST) {
         TG_CUDA(p64buf.alloc(n));

@@ -194,6 +194,43 @@ __device__ __forceinline__ T warp_inclusive_scan(T v) {
     return v;
 }
 
+// Exclusive prefix of one value per tile by decoupled look-back, for kernels that scan in one pass. Called by
+// one whole warp of the tile's block with the tile's sum (the same on every lane); tiles are numbered by an
+// atomic counter, so every earlier one belongs to a block already running. A status word holds a flag
+// (bits 62-63: the tile's own sum, or the sum up to and with it) and the value; zeroed before the kernel. The
+// wait for a word is bounded: if it runs out, redo() gives the prefix from the input itself.
+constexpr unsigned long long SCAN_OWN = 1ull << 62, SCAN_UPTO = 2ull << 62, SCAN_VALUE = (1ull << 62) - 1;
+template <class Redo>
+__device__ __forceinline__ long long scan_look_back(long long sum, int tile, unsigned long long *status, long long spins,
+                                                    Redo redo) {
+    volatile unsigned long long *st = status;
+    const int lane = lane_id();
+    if (tile == 0) {
+        if (lane == 0) st[0] = SCAN_UPTO | (unsigned long long)sum;
+        return 0;
+    }
+    if (lane == 0) st[tile] = SCAN_OWN | (unsigned long long)sum;
+    long long before = 0;
+    bool ok = true;
+    for (int j = tile - 1;; j -= 32) {  // 32 earlier tiles at a time, nearest first
+        const int k = j - lane;
+        unsigned long long w = SCAN_UPTO;
+        if (k >= 0) w = st[k];
+        for (long long s = 0; (w >> 62) == 0 && s < spins; s++) w = st[k];
+        ok = !__any_sync(FULL, (w >> 62) == 0);
+        if (!ok) break;
+        const unsigned upto = __ballot_sync(FULL, (w >> 62) == 2);
+        long long v = !upto || lane <= __ffs(upto) - 1 ? (long long)(w & SCAN_VALUE) : 0;
+#pragma unroll
+        for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(FULL, v, o);
+        before += v;
+        if (upto) break;
+    }
+    if (!ok) before = redo();
+    if (lane == 0) st[tile] = SCAN_UPTO | (unsigned long long)(before + sum);
+    return before;
+}
+
 inline int div_up(int64_t a, int64_t b) { return (int)((a + b - 1) / b); }
 
 // Device-wide helpers implemented in tg_scan.cu / tg_sort.cu.
@@ -219,6 +256,14 @@ struct LoopLimits {
 LoopLimits &loop_limits();
 
 int num_sms();
+
+// A few words of page-locked host memory per thread (HOST_WORDS_BYTES), for reading results back without the
+// driver's staging: copies into it are asynchronous, so several share one synchronisation. A call has the
+// words from its copies to its last read; nothing is kept in them between calls.
+constexpr size_t HOST_WORDS_BYTES = 4096;
+tg_status host_words(void **p);
+// Polls of one look-back word in a one-pass scan.
+long long scan_spins();
 
 // The unique id of the calling thread's current CUDA context (the driver's cuCtxGetCurrent and
 // cuCtxGetId, reached through the runtime's entry-point query so that the library needs no link to

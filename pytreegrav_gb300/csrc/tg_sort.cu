@@ -149,6 +149,28 @@ void release_event(cudaEvent_t e, bool timing, int dev) {
     res_pool(dev).events[timing ? 1 : 0].push_back(e);
 }
 
+namespace {
+struct HostWords {
+    void *p = nullptr;
+    unsigned long long ctx = 0;
+    ~HostWords() {  // the thread ends: given back, unless its context has gone (and the memory with it)
+        if (p && current_cuda_context_id() == ctx) cudaFreeHost(p);
+    }
+};
+}  // namespace
+
+tg_status host_words(void **p) {
+    static thread_local HostWords w;
+    const unsigned long long ctx = current_cuda_context_id();
+    if (w.p && w.ctx != ctx) w.p = nullptr;  // a new context: the old memory died with the old one
+    if (!w.p) {
+        TG_CUDA(cudaHostAlloc(&w.p, HOST_WORDS_BYTES, cudaHostAllocPortable));
+        w.ctx = current_cuda_context_id();
+    }
+    *p = w.p;
+    return TG_OK;
+}
+
 cudaError_t dev_malloc(void **p, size_t bytes, cudaStream_t s) {
     constexpr int MAX_DEVICES = 64;
     static std::mutex mu;
@@ -187,7 +209,7 @@ cudaError_t dev_malloc(void **p, size_t bytes, cudaStream_t s) {
 }
 
 // ---------------------------------------------------------------------------------------------
-// Exclusive scan: block sums -> scan of block sums (one CTA) -> per-block scan plus carry.
+// Exclusive scan in one pass (decoupled look-back over tiles of 2048).
 constexpr int SCAN_THREADS = 256;
 constexpr int SCAN_ITEMS = 8;
 constexpr int SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;
@@ -212,46 +234,15 @@ __device__ T block_exclusive_scan(T v, T *total) {
 }
 
 template <typename T>
-__global__ void scan_block_sums(const T *in, int64_t n, T *sums) {
+__global__ void __launch_bounds__(SCAN_THREADS) k_scan(const T *in, T *out, int64_t n, T *total,
+                                                       unsigned long long *status, int *counter, long long spins) {
     __shared__ T tot;
-    int64_t base = (int64_t)blockIdx.x * SCAN_TILE + (int64_t)threadIdx.x * SCAN_ITEMS;
-    T v = 0;
-#pragma unroll
-    for (int i = 0; i < SCAN_ITEMS; i++)
-        if (base + i < n) v += in[base + i];
-    block_exclusive_scan(v, &tot);
-    if (threadIdx.x == 0) sums[blockIdx.x] = tot;
-}
-
-template <typename T>
-__global__ void scan_sums_single(T *sums, int64_t nb, T *total) {
-    __shared__ T tot;
-    T carry = 0;
-    for (int64_t base = 0; base < nb; base += SCAN_TILE) {
-        int64_t i0 = base + (int64_t)threadIdx.x * SCAN_ITEMS;
-        T vals[SCAN_ITEMS];
-        T v = 0;
-#pragma unroll
-        for (int i = 0; i < SCAN_ITEMS; i++) {
-            vals[i] = (i0 + i < nb) ? sums[i0 + i] : T(0);
-            v += vals[i];
-        }
-        T ex = block_exclusive_scan(v, &tot) + carry;
-#pragma unroll
-        for (int i = 0; i < SCAN_ITEMS; i++) {
-            if (i0 + i < nb) sums[i0 + i] = ex;
-            ex += vals[i];
-        }
-        carry += tot;
-        __syncthreads();
-    }
-    if (threadIdx.x == 0 && total) *total = carry;
-}
-
-template <typename T>
-__global__ void scan_apply(const T *in, T *out, int64_t n, const T *sums) {
-    __shared__ T tot;
-    int64_t base = (int64_t)blockIdx.x * SCAN_TILE + (int64_t)threadIdx.x * SCAN_ITEMS;
+    __shared__ long long before_s;
+    __shared__ int tile_s;
+    if (threadIdx.x == 0) tile_s = atomicAdd(counter, 1);
+    __syncthreads();
+    const int tile = tile_s;
+    const int64_t base = (int64_t)tile * SCAN_TILE + (int64_t)threadIdx.x * SCAN_ITEMS;
     T vals[SCAN_ITEMS];
     T v = 0;
 #pragma unroll
@@ -259,7 +250,21 @@ __global__ void scan_apply(const T *in, T *out, int64_t n, const T *sums) {
         vals[i] = (base + i < n) ? in[base + i] : T(0);
         v += vals[i];
     }
-    T ex = block_exclusive_scan(v, &tot) + sums[blockIdx.x];
+    T ex = block_exclusive_scan(v, &tot);
+    if (threadIdx.x < 32) {
+        const long long before = scan_look_back((long long)tot, tile, status, spins, [&]() {
+            long long sum = 0;
+            for (int64_t i = threadIdx.x; i < (int64_t)tile * SCAN_TILE; i += 32) sum += in[i];
+            for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(FULL, sum, o);
+            return sum;
+        });
+        if (threadIdx.x == 0) {
+            before_s = before;
+            if (total && (int64_t)(tile + 1) * SCAN_TILE >= n) *total = (T)(before + (long long)tot);
+        }
+    }
+    __syncthreads();
+    ex += (T)before_s;
 #pragma unroll
     for (int i = 0; i < SCAN_ITEMS; i++) {
         if (base + i < n) out[base + i] = ex;
@@ -273,14 +278,13 @@ static tg_status exclusive_scan(const T *in, T *out, int64_t n, T *total_dev, cu
         if (total_dev) TG_CUDA(cudaMemsetAsync(total_dev, 0, sizeof(T), s));
         return TG_OK;
     }
-    int64_t nb = (n + SCAN_TILE - 1) / SCAN_TILE;
-    T *sums = nullptr;
-    TG_CUDA(tg::dev_malloc((void **)&sums, sizeof(T) * nb, s));
-    { scan_block_sums<T><<<(unsigned)nb, SCAN_THREADS, 0, s>>>(in, n, sums); tg::note_launch(); }
-    { scan_sums_single<T><<<1, SCAN_THREADS, 0, s>>>(sums, nb, total_dev); tg::note_launch(); }
-    { scan_apply<T><<<(unsigned)nb, SCAN_THREADS, 0, s>>>(in, out, n, sums); tg::note_launch(); }
+    const int64_t nb = (n + SCAN_TILE - 1) / SCAN_TILE;
+    unsigned long long *status = nullptr;  // then the tile counter
+    TG_CUDA(tg::dev_malloc((void **)&status, sizeof(unsigned long long) * (nb + 1), s));
+    TG_CUDA(cudaMemsetAsync(status, 0, sizeof(unsigned long long) * (nb + 1), s));
+    { k_scan<T><<<(unsigned)nb, SCAN_THREADS, 0, s>>>(in, out, n, total_dev, status, (int *)(status + nb), scan_spins()); tg::note_launch(); }
     TG_CUDA(cudaGetLastError());
-    TG_CUDA(cudaFreeAsync(sums, s));
+    TG_CUDA(cudaFreeAsync(status, s));
     return TG_OK;
 }
 
@@ -570,6 +574,8 @@ __global__ void k_sort_fallback(uint64_t *keys, uint32_t *vals, int64_t n, const
         vals[i] = (uint32_t)i;
     }
 }
+
+long long scan_spins() { return loop_limits().sort_spin > 0 ? loop_limits().sort_spin : SPIN_LIMIT; }
 
 tg_status radix_sort_pairs(uint64_t *keys, uint32_t *vals, int64_t n, int bits, cudaStream_t s, int *err) {
     if (n <= 1 || bits <= 0) return TG_OK;

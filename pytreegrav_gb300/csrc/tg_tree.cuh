@@ -96,7 +96,6 @@ struct tg_tree_s {
     // made on the side stream beside the first grouping; null until then.
     float4 *own32 = nullptr;
     tg::WalkStats last_stats;
-    int64_t *stats_dev = nullptr;  // 8 counters
 
     // Tree grouping (TG_GROUP_TREE, TG_ORDER_TREE) at group size groups_G, made on first use and
     // kept: groups as (first target, count) in start order, each group's system root and the node

@@ -21,6 +21,7 @@
 // point-mass path; the rest take the full softened path. Each lane sums a batch in registers and
 // adds the batch total into a Kahan-compensated accumulator.
 #include <algorithm>
+#include <cstring>
 #include <new>
 #include <type_traits>
 #include <vector>
@@ -152,43 +153,79 @@ __device__ __forceinline__ double narrow(double x, double) { return x; }
 __device__ __forceinline__ float to_f32(float x) { return x; }
 __device__ __forceinline__ float to_f32(double x) { return d2f(x); }
 
-__global__ void k_arena_links(int64_t ntot, int64_t mtot, const int64_t *first, const int64_t *next, int4 *link,
-                              int64_t *nleaf, int *bad) {
-    int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= mtot) return;
-    int64_t f = ntot + j, stop = next[f];
-    int fc = -1, nc = 0, nl = 0, steps = 0;
-    for (int64_t c = first[f]; c != stop && c >= 0; c = next[c]) {
-        if (++steps > 8) {  // an octree node has at most 8 children
-            atomicOr(bad, 1);
-            break;
+// Node links with the leaf ranges' starts: a node's particle children counted and scanned in one pass (it was six
+// launches, each its ~2 us gap and ramp). The ranges must be a partition of the particles.
+constexpr int LINK_THREADS = 256;
+__global__ void __launch_bounds__(LINK_THREADS) k_arena_links(int64_t ntot, int64_t mtot, const int64_t *first,
+                                                              const int64_t *next, int4 *link, int *bad,
+                                                              unsigned long long *status, int *counter, long long spins) {
+    __shared__ int warp_sum[LINK_THREADS / 32];
+    __shared__ long long before_s;
+    __shared__ int tile_s;
+    if (threadIdx.x == 0) tile_s = atomicAdd(counter, 1);
+    __syncthreads();
+    const int tile = tile_s, lane = lane_id(), w = threadIdx.x >> 5;
+    const int64_t j = (int64_t)tile * LINK_THREADS + threadIdx.x;
+    auto children = [&](int64_t node, int &fc, int &nc, int *flags) {
+        int nl = 0, steps = 0;
+        fc = -1, nc = 0;
+        const int64_t f = ntot + node, stop = next[f];
+        for (int64_t c = first[f]; c != stop && c >= 0; c = next[c]) {
+            if (++steps > 8) {  // an octree node has at most 8 children
+                *flags |= 1;
+                break;
+            }
+            if (c < ntot) nl++;
+            else {
+                if (nc == 0) fc = (int)(c - ntot);
+                else if (c - ntot != fc + nc) *flags |= 2;  // node children must be consecutive
+                nc++;
+            }
         }
-        if (c < ntot) nl++;
-        else {
-            if (nc == 0) fc = (int)(c - ntot);
-            else if (c - ntot != fc + nc) atomicOr(bad, 2);  // node children must be consecutive
-            nc++;
+        return nl;
+    };
+    int fc = -1, nc = 0, nl = 0, flags = 0;
+    if (j < mtot) nl = children(j, fc, nc, &flags);
+    if (nc > 0 && (fc < 0 || fc + nc > mtot)) flags |= 4;
+    const int inc = warp_inclusive_scan(nl);
+    if (lane == 31) warp_sum[w] = inc;
+    __syncthreads();
+    int below = 0, tot = 0;
+#pragma unroll
+    for (int k = 0; k < LINK_THREADS / 32; k++) {
+        below += k < w ? warp_sum[k] : 0;
+        tot += warp_sum[k];
+    }
+    if (w == 0) {
+        const long long before = scan_look_back(tot, tile, status, spins, [&]() {
+            long long sum = 0;
+            int a, b, c = 0;
+            for (int64_t k = lane; k < (int64_t)tile * LINK_THREADS; k += 32) sum += children(k, a, b, &c);
+            for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(FULL, sum, o);
+            return sum;
+        });
+        if (lane == 0) {
+            before_s = before;
+            if ((int64_t)(tile + 1) * LINK_THREADS >= mtot && before + tot != ntot) flags |= 8;  // one leaf each
         }
     }
-    if (nc > 0 && (fc < 0 || fc + nc > mtot)) atomicOr(bad, 4);
-    link[j] = make_int4(fc, nc, 0, nl);
-    nleaf[j] = nl;
+    __syncthreads();
+    const long long ls = before_s + below + inc - nl;
+    // the records hold leaf starts below 2^27; others come from invalid links, and the leaf fill bounds them
+    if (j < mtot) link[j] = make_int4(fc, nc, ls > 0x7fffffffLL ? -1 : (int)ls, nl);
+    if (flags) atomicOr(bad, flags);
 }
 
 // Leaf ranges: each node's particle children, in chain order, copied to its range of the leaf
-// arrays; the range start also goes into the node's link. Reads particle data only, which is final
-// before the moment pass.
+// arrays. Reads particle data only, which is final before the moment pass.
 template <typename T>
 __global__ void k_arena_leaves(int64_t ntot, int64_t mtot, const int64_t *first, const int64_t *next,
-                               const double *coord, const double *mass, const double *soft,
-                               const int64_t *leaf_start, Arena<T> ar) {
+                               const double *coord, const double *mass, const double *soft, Arena<T> ar) {
     int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= mtot) return;
     int64_t f = ntot + j, stop = next[f];
-    int64_t ls = leaf_start[j];
-    int4 lk = ar.n_link[j];
-    lk.z = (int)ls;
-    ar.n_link[j] = lk;
+    const int4 lk = ar.n_link[j];
+    const int64_t ls = lk.z;
     if (ls < 0 || ls + lk.w > ar.n_leaves) {  // leaf ranges from invalid links: nothing written
         atomicOr(ar.bad, 16);
         return;
@@ -251,13 +288,8 @@ __global__ void k_arena_nodes(int64_t ntot, int64_t mtot, const double *coord, c
     }
 }
 
-// Every particle must be exactly one node's leaf.
-__global__ void k_arena_total(const int64_t *ltot, int64_t ntot, int *bad) {
-    if (threadIdx.x == 0 && *ltot != ntot) atomicOr(bad, 8);
-}
-
 // The arena's topology part: allocation, node links, leaf ranges (validated on the device, see
-// k_arena_total) and the leaf records. Needs no moments.
+// k_arena_links) and the leaf records. Needs no moments.
 template <typename T>
 tg_status build_arena_topology(tg_tree_s *t, Arena<T> &ar, cudaStream_t st) {
     const int64_t M = t->mtot, N = t->ntot;
@@ -276,23 +308,18 @@ tg_status build_arena_topology(tg_tree_s *t, Arena<T> &ar, cudaStream_t st) {
     if (sizeof(T) == 4) TG_CUDA(tg::dev_malloc((void **)&ar.n_tol, sizeof(float2) * M, st));
     TG_CUDA(tg::dev_malloc((void **)&ar.l_pos, sizeof(vec4<T>) * N, st));
     TG_CUDA(tg::dev_malloc((void **)&ar.l_lo, sizeof(vec4<T>) * N, st));
-    int64_t *nleaf = nullptr, *lstart = nullptr, *ltot = nullptr;
-    TG_CUDA(tg::dev_malloc((void **)&nleaf, sizeof(int64_t) * M, st));
-    TG_CUDA(tg::dev_malloc((void **)&lstart, sizeof(int64_t) * M, st));
-    TG_CUDA(tg::dev_malloc((void **)&ltot, sizeof(int64_t), st));
     TG_CUDA(tg::dev_malloc((void **)&ar.bad, sizeof(int), st));
     TG_CUDA(cudaMemsetAsync(ar.bad, 0, sizeof(int), st));
+    const int tiles = div_up(M, LINK_THREADS);
+    DevArray<unsigned long long> status(st);  // then the tile counter
+    TG_CUDA(status.alloc(tiles + 1));
+    TG_CUDA(cudaMemsetAsync(status.p, 0, sizeof(unsigned long long) * (tiles + 1), st));
     // validated on the device: the fill writes only in-range leaf ranges, and every walk checks the
     // flag before it reads the arena (no host synchronisation here)
-    { k_arena_links<<<div_up(M, 256), 256, 0, st>>>(N, M, t->first, t->next, ar.n_link, nleaf, ar.bad); tg::note_launch(); }
-    TG_TRY(exclusive_scan_i64(nleaf, lstart, M, ltot, st));
-    { k_arena_total<<<1, 32, 0, st>>>(ltot, N, ar.bad); tg::note_launch(); }
-    TG_CUDA(cudaFreeAsync(ltot, st));
-    { k_arena_leaves<T><<<div_up(M, 256), 256, 0, st>>>(N, M, t->first, t->next, t->coord, t->mass, t->soft, lstart,
-                                                       ar); tg::note_launch(); }
+    { k_arena_links<<<tiles, LINK_THREADS, 0, st>>>(N, M, t->first, t->next, ar.n_link, ar.bad, status.p,
+                                                    (int *)(status.p + tiles), scan_spins()); tg::note_launch(); }
+    { k_arena_leaves<T><<<div_up(M, 256), 256, 0, st>>>(N, M, t->first, t->next, t->coord, t->mass, t->soft, ar); tg::note_launch(); }
     TG_CUDA(cudaGetLastError());
-    TG_CUDA(cudaFreeAsync(nleaf, st));
-    TG_CUDA(cudaFreeAsync(lstart, st));
     return TG_OK;
 }
 
@@ -1339,6 +1366,16 @@ __global__ void k_make_groups(const int64_t *sys_off, int nsys, int gs, const in
     }
 }
 
+// The groups of one system's n targets, with nothing to copy or wait for first (1e5 single targets: 50 us in one
+// block and ~30 us of copies before it, 3 us here).
+__global__ void k_make_groups_one(int64_t n, int gs, int root, int64_t ngroups, int2 *groups, int *group_root) {
+    const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (g >= ngroups) return;
+    const int64_t t = g * gs;
+    groups[g] = make_int2((int)t, (int)(n - t < gs ? n - t : gs));
+    group_root[g] = root;
+}
+
 // Engine grouping: groups are taken from the tree, so a group never straddles a jump of the Morton
 // curve. A system root with at most G particles is one group. Every node with more than G
 // particles emits its children, in order, packed greedily into runs of at most G particles; a child
@@ -1568,7 +1605,7 @@ __global__ void k_group_cost_keys(const double *tpos, const int2 *groups, int64_
         }
     float d = (float)sqrt((hi[0] - lo[0]) * (hi[0] - lo[0]) + (hi[1] - lo[1]) * (hi[1] - lo[1]) +
                           (hi[2] - lo[2]) * (hi[2] - lo[2]));
-    keys[g] = (uint64_t)(0xffffffffu - __float_as_uint(d));
+    keys[g] = (uint64_t)(0xffffu - (__float_as_uint(d) >> 15));  // exponent and top 8 fraction bits: two sort passes
     vals[g] = (uint32_t)g;
 }
 __global__ void k_group_start_keys(const int2 *groups, int64_t ngroups, uint64_t *keys, uint32_t *vals) {
@@ -1870,10 +1907,11 @@ static tg_status dispatch_walk(WalkArgs<T> &a, int fields, bool quad, int warps,
     }
 }
 
-// Scratch of one walk, in ints: queue, status, retry count, retry queue, then the retry list.
-constexpr int WS_QUEUE = 0, WS_STATUS = 1, WS_RETRY_COUNT = 2, WS_RETRY_QUEUE = 3, WS_REWALK_COUNT = 4,
-              WS_REWALK_QUEUE = 5, WS_HEAVY_COUNT = 6, WS_HEAVY_QUEUE = 7, WS_TEAM_COUNT = 8, WS_TEAM_QUEUE = 9,
-              WS_RETRY_LIST = 10;  // then the retry list, the rewalk list, the heavy list and the team list
+// Scratch of one walk, in ints: the statistics, the queues, counts and status word, then the lists.
+constexpr int WS_STATS = 0;  // 8 64-bit counters
+constexpr int WS_QUEUE = 16, WS_STATUS = 17, WS_RETRY_COUNT = 18, WS_RETRY_QUEUE = 19, WS_REWALK_COUNT = 20,
+              WS_REWALK_QUEUE = 21, WS_HEAVY_COUNT = 22, WS_HEAVY_QUEUE = 23, WS_TEAM_COUNT = 24, WS_TEAM_QUEUE = 25,
+              WS_RETRY_LIST = 26;  // then the retry list, the rewalk list, the heavy list and the team list
 inline int64_t walk_scratch_ints(int64_t ngroups) { return WS_RETRY_LIST + 4 * std::max<int64_t>(ngroups, 1); }
 // List entries after which a group counts as heavy (split_heavy walks): the median group of 8 at 1e6
 // Plummer particles evaluates ~1.9e3, the 99.9th percentile ~7e3.
@@ -1896,7 +1934,6 @@ constexpr unsigned HEAVY_ENTRIES = 1u << 15;
 constexpr int64_t TEAM_ALL_GROUPS = 4000, TEAM_ALL_GROUPS_FULL = 1400, TEAM_MAX_GROUPS = 65536;
 constexpr int64_t TEAM_MIN_ENTRIES = 2048;
 constexpr int TEAM_MIN_TARGETS = 4;
-constexpr int ITEM_CAP = 1 << 16;  // items per heavy group
 
 // FP64 walks of consecutive targets split sooner: one warp takes ~13 us for 32 entries of 8 targets, so a
 // group of 32768 was 13 ms of a 50000-particle walk's 18.3. About a third of what one warp evaluates in all
@@ -1918,6 +1955,7 @@ static tg_status enqueue_walk(WalkArgs<T> a, int fields, bool quad, int warps, i
                               cudaStream_t st, bool split_heavy = false) {
     TG_CUDA(cudaMemsetAsync(scratch, 0, sizeof(int) * WS_RETRY_LIST, st));
     const int64_t ng1 = std::max<int64_t>(a.ngroups, 1);
+    a.stats = reinterpret_cast<unsigned long long *>(scratch + WS_STATS);
     a.queue = scratch + WS_QUEUE;
     a.status = scratch + WS_STATUS;
     a.ngroups_dev = nullptr;
@@ -2083,12 +2121,20 @@ static tg_status walk_heavy(tg_tree_s *t, const WalkArgs<T> &a, Arena<T> &ar, in
     return TG_OK;
 }
 
-// Run a walk and time it on the stream; *status_out receives the device status word. With
-// split_heavy, groups past the entry budget are walked by walk_heavy.
+// What a walk's host side reads back: the scratch's head (statistics, status word, counts) and the tree's sort
+// flag, with one synchronisation through page-locked words (four copies and four waits through the driver's
+// staging took ~50 us after each walk).
+struct WalkReadback {
+    int head[WS_RETRY_LIST];
+    int sort_bad;
+};
+
+// Run a walk, time it on the stream and read its results back. With split_heavy, groups past the entry
+// budget are walked by walk_heavy.
 template <typename T>
 static tg_status walk_with_fallback(tg_tree_s *t, WalkArgs<T> &a, Arena<T> &ar, int fields, bool quad, int warps,
-                                    int first_stack, int *scratch, bool split_heavy, cudaStream_t st, int *status_out,
-                                    float *kernel_ms) {
+                                    int first_stack, int *scratch, bool split_heavy, cudaStream_t st,
+                                    WalkReadback *back, float *kernel_ms) {
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     struct Events {  // back to the pool on every exit
         cudaEvent_t *a, *b;
@@ -2099,22 +2145,30 @@ static tg_status walk_with_fallback(tg_tree_s *t, WalkArgs<T> &a, Arena<T> &ar, 
     } evs{&e0, &e1};
     TG_CUDA(pool_event(&e0, true));
     TG_CUDA(pool_event(&e1, true));
-    TG_CUDA(cudaEventRecord(e0, st));
-    tg_status rc = enqueue_walk<T>(a, fields, quad, warps, first_stack, scratch, st, split_heavy);
-    int hdr[WS_RETRY_LIST] = {0};
-    if (rc == TG_OK && split_heavy) {
-        TG_CUDA(cudaMemcpyAsync(hdr, scratch, sizeof(hdr), cudaMemcpyDeviceToHost, st));
+    void *words = nullptr;
+    TG_TRY(host_words(&words));
+    static_assert(sizeof(WalkReadback) <= HOST_WORDS_BYTES, "a walk's read-back must fit the host words");
+    WalkReadback *host = static_cast<WalkReadback *>(words);
+    auto read_back = [&]() -> tg_status {
+        TG_CUDA(cudaEventRecord(e1, st));
+        host->sort_bad = 0;
+        TG_CUDA(cudaMemcpyAsync(host->head, scratch, sizeof(host->head), cudaMemcpyDeviceToHost, st));
+        if (t->sort_err) TG_CUDA(cudaMemcpyAsync(&host->sort_bad, t->sort_err, sizeof(int), cudaMemcpyDeviceToHost, st));
         TG_CUDA(cudaStreamSynchronize(st));
-        if (hdr[WS_HEAVY_COUNT] > 0)
-            rc = walk_heavy<T>(t, a, ar, fields, quad, warps, scratch, hdr[WS_HEAVY_COUNT], st);
+        *back = *host;
+        return TG_OK;
+    };
+    TG_CUDA(cudaEventRecord(e0, st));
+    TG_TRY(enqueue_walk<T>(a, fields, quad, warps, first_stack, scratch, st, split_heavy));
+    TG_TRY(read_back());
+    if (split_heavy && back->head[WS_HEAVY_COUNT] > 0) {
+        a.stats = reinterpret_cast<unsigned long long *>(scratch + WS_STATS);
+        a.status = scratch + WS_STATUS;
+        TG_TRY(walk_heavy<T>(t, a, ar, fields, quad, warps, scratch, back->head[WS_HEAVY_COUNT], st));
+        TG_TRY(read_back());
     }
-    TG_CUDA(cudaEventRecord(e1, st));
-    int status = 0;
-    TG_CUDA(cudaMemcpyAsync(&status, scratch + WS_STATUS, sizeof(int), cudaMemcpyDeviceToHost, st));
-    TG_CUDA(cudaStreamSynchronize(st));
     TG_CUDA(cudaEventElapsedTime(kernel_ms, e0, e1));
-    *status_out = status;
-    return rc;
+    return TG_OK;
 }
 
 // Whether a walk arena is larger than the GPU's L2 (the walk then prefetches the records it queues).
@@ -2139,12 +2193,10 @@ tg_status run_walk(tg_tree_s *t, const double *tpos, const double *th, int64_t n
                    int quadrupole, double theta, double G, int group_size, int precision, const float *theta_group,
                    const float *tol_group, double *out, cudaStream_t st) {
     int w = ((fields & F_POT) ? 1 : 0) + ((fields & F_ACC) ? 3 : 0) + ((fields & F_TID) ? 9 : 0);
-    if (!t->stats_dev) TG_CUDA(tg::dev_malloc((void **)&t->stats_dev, sizeof(unsigned long long) * 8, st));
     int *scratch = nullptr;
     TG_CUDA(tg::dev_malloc((void **)&scratch, sizeof(int) * walk_scratch_ints(ngroups), st));
-    TG_CUDA(cudaMemsetAsync(t->stats_dev, 0, sizeof(unsigned long long) * 8, st));
     tg_status rc = TG_OK;
-    int status = 0;
+    WalkReadback back;
     float kms = 0.f;
     unsigned *gstats = nullptr;
     if (t->record_group_stats) {
@@ -2182,7 +2234,6 @@ tg_status run_walk(tg_tree_s *t, const double *tpos, const double *th, int64_t n
         a.gerr = gerr;
         a.rewalk_theta = t->rewalk_theta;
         a.out_fields = fields; a.out_w = w; a.out = out; a.gs = group_size;
-        a.stats = (unsigned long long *)t->stats_dev;
         a.gstats = gstats;
         a.prefetch = arena_exceeds_l2(t->arena64);
         vec4<double> *thi = nullptr, *tlo = nullptr;
@@ -2192,8 +2243,7 @@ tg_status run_walk(tg_tree_s *t, const double *tpos, const double *th, int64_t n
         a.thi = thi;
         a.tlo = tlo;
         rc = walk_with_fallback<double>(t, a, t->arena64, fields, quadrupole != 0, t->walk_warps, t->walk_stack,
-                                        scratch, split_heavy, st, &status,
-                                        &kms);
+                                        scratch, split_heavy, st, &back, &kms);
         cudaFreeAsync(thi, st);
         cudaFreeAsync(tlo, st);
     } else {
@@ -2209,7 +2259,6 @@ tg_status run_walk(tg_tree_s *t, const double *tpos, const double *th, int64_t n
         a.gerr = gerr;
         a.rewalk_theta = t->rewalk_theta;
         a.out_fields = fields; a.out_w = w; a.out = out; a.gs = group_size;
-        a.stats = (unsigned long long *)t->stats_dev;
         a.gstats = gstats;
         a.prefetch = arena_exceeds_l2(t->arena32);
         vec4<float> *thi = nullptr, *tlo = nullptr;
@@ -2225,18 +2274,15 @@ tg_status run_walk(tg_tree_s *t, const double *tpos, const double *th, int64_t n
             a.tlo = tlo;
         }
         rc = walk_with_fallback<float>(t, a, t->arena32, fields, quadrupole != 0, t->walk_warps, t->walk_stack,
-                                       scratch, split_heavy, st, &status,
-                                       &kms);
+                                       scratch, split_heavy, st, &back, &kms);
         if (thi) cudaFreeAsync(thi, st);
         if (tlo) cudaFreeAsync(tlo, st);
     }
+    TG_CUDA(cudaFreeAsync(scratch, st));
     if (rc != TG_OK) return rc;
     unsigned long long stats[8];
-    int sort_bad = 0;
-    TG_CUDA(cudaMemcpyAsync(stats, t->stats_dev, sizeof(stats), cudaMemcpyDeviceToHost, st));
-    if (t->sort_err) TG_CUDA(cudaMemcpyAsync(&sort_bad, t->sort_err, sizeof(int), cudaMemcpyDeviceToHost, st));
-    TG_CUDA(cudaFreeAsync(scratch, st));
-    TG_CUDA(cudaStreamSynchronize(st));
+    memcpy(stats, back.head + WS_STATS, sizeof(stats));
+    const int status = back.head[WS_STATUS], sort_bad = back.sort_bad;
     t->last_stats.interactions = (int64_t)stats[0];
     t->last_stats.node_tests = (int64_t)stats[1];
     t->last_stats.max_stack = (int64_t)stats[2];
@@ -2381,7 +2427,7 @@ tg_status make_cost_order(const double *tpos, const int2 *groups, int64_t ngroup
     TG_CUDA(tg::dev_malloc((void **)order, sizeof(int) * std::max<int64_t>(ngroups, 1), st));
     { k_group_cost_keys<<<div_up(ngroups, 256), 256, 0, st>>>(tpos, groups, ngroups, keys, (uint32_t *)*order); tg::note_launch(); }
     TG_CUDA(cudaGetLastError());
-    TG_TRY(radix_sort_pairs(keys, (uint32_t *)*order, ngroups, 32, st, sort_err));
+    TG_TRY(radix_sort_pairs(keys, (uint32_t *)*order, ngroups, 16, st, sort_err));
     TG_CUDA(cudaFreeAsync(keys, st));
     return TG_OK;
 }
@@ -2396,6 +2442,14 @@ tg_status make_groups(tg_tree_s *t, const std::vector<int64_t> &sys_off_host, in
         roots[s] = (int)t->sys_node_off[s];
     }
     *ngroups = goff[nsys];
+    if (nsys == 1) {  // nothing to copy, nothing to wait for
+        const int64_t ng1 = std::max<int64_t>(*ngroups, 1);
+        TG_CUDA(tg::dev_malloc((void **)groups, sizeof(int2) * ng1, st));
+        TG_CUDA(tg::dev_malloc((void **)group_root, sizeof(int) * ng1, st));
+        { k_make_groups_one<<<div_up(ng1, 256), 256, 0, st>>>(sys_off_host[1], gs, roots[0], *ngroups, *groups, *group_root); tg::note_launch(); }
+        TG_CUDA(cudaGetLastError());
+        return TG_OK;
+    }
     int64_t *d_sys = nullptr, *d_goff = nullptr;
     int *d_roots = nullptr;
     TG_CUDA(tg::dev_malloc((void **)groups, sizeof(int2) * std::max<int64_t>(*ngroups, 1), st));
@@ -2488,8 +2542,6 @@ tg_status tg_walk_graph_create(tg_tree t, int fields, int quadrupole, double the
     }
     if ((rc = build_arena(t, t->arena32, cs)) != TG_OK) return fail(rc);
     const int64_t n = t->ntot;
-    if (!t->stats_dev && dev_malloc((void **)&t->stats_dev, sizeof(unsigned long long) * 8, cs) != cudaSuccess)
-        return fail(TG_ERR_OOM);
     if (dev_malloc((void **)&g->thi, sizeof(float4) * std::max<int64_t>(n, 1), cs) != cudaSuccess ||
         dev_malloc((void **)&g->tlo, sizeof(float4) * std::max<int64_t>(n, 1), cs) != cudaSuccess ||
         dev_malloc((void **)&g->scratch, sizeof(int) * walk_scratch_ints(ng), cs) != cudaSuccess)
@@ -2514,15 +2566,13 @@ tg_status tg_walk_graph_create(tg_tree t, int fields, int quadrupole, double the
     a.out_fields = fields;
     a.out_w = ((fields & F_POT) ? 1 : 0) + ((fields & F_ACC) ? 3 : 0) + ((fields & F_TID) ? 9 : 0);
     a.out = out; a.gs = group_size;
-    a.stats = (unsigned long long *)t->stats_dev;
     a.gstats = nullptr;
     a.thi = g->thi;
     a.tlo = g->tlo;
     const int64_t launches0 = launches_so_far();
     if (cudaStreamBeginCapture(cs, cudaStreamCaptureModeRelaxed) != cudaSuccess) return fail(TG_ERR_CUDA);
     rc = TG_OK;
-    if (cudaMemsetAsync(t->stats_dev, 0, sizeof(unsigned long long) * 8, cs) != cudaSuccess) rc = TG_ERR_CUDA;
-    if (rc == TG_OK) rc = enqueue_walk<float>(a, fields, quadrupole != 0, t->walk_warps, t->walk_stack, g->scratch, cs);
+    rc = enqueue_walk<float>(a, fields, quadrupole != 0, t->walk_warps, t->walk_stack, g->scratch, cs);
     cudaError_t ce = cudaStreamEndCapture(cs, &g->graph);
     note_launches(launches0 - launches_so_far());  // recorded, not run
     if (rc != TG_OK) return fail(rc);

@@ -84,3 +84,26 @@ def test_fp64_split(tg, n, gs, quadrupole):
         assert np.sqrt(np.sum((a - b) ** 2)) < 1e-12 * np.sqrt(np.sum(b**2)), k
     a, b = alone["accel"], ref["accel"]
     assert np.sqrt(np.sum((a - b) ** 2)) < 1e-12 * np.sqrt(np.sum(b**2))
+
+
+@pytest.mark.parametrize("n", [1, 257, 3001, 100003])
+def test_scan_that_does_not_wait(tg, n):
+    """The walk arena's one-pass scan of leaf counts when a tile gives up waiting for the tiles before it: the
+    prefix then comes from the input itself, so the walk is the same. (Groups of one target: nothing else of
+    this walk waits.)"""
+    from pytreegrav_gb300 import _lib, synthetic
+
+    L = _lib.load()
+    L.tg_set_loop_limits.argtypes = [ctypes.c_int64] * 4
+    x = synthetic.plummer(n, 5)
+    m, h = np.full(n, 1.0 / n), np.full(n, 0.01)
+    kw = dict(accel=True, group_size=1, theta=0.9)
+    ref = tg.ConstructTree(x, m, h).fields(**kw)["accel"]
+    for _ in range(3):
+        tree = tg.ConstructTree(x, m, h)
+        L.tg_set_loop_limits(1, 0, 0, 0)
+        try:
+            got = tree.fields(**kw)["accel"]
+        finally:
+            L.tg_set_loop_limits(0, 0, 0, 0)
+        assert np.array_equal(got, ref)
