@@ -49,14 +49,6 @@ __device__ __forceinline__ int64_t find_seg(const int64_t *off, int nseg, int64_
 
 // ---------------------------------------------------------------------------------------------
 // Bounding cube (octree.py:539-574): exact min/max through order-preserving integer atomics.
-__global__ void k_bbox_init(unsigned long long *mn, unsigned long long *mx, int nsys) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < 3 * nsys) {
-        mn[i] = ~0ull;
-        mx[i] = 0ull;
-    }
-}
-
 __global__ void __launch_bounds__(BB_THREADS) k_bbox(const double *pos, int64_t n, const int64_t *sys_off, int nsys,
                                                      unsigned long long *mn, unsigned long long *mx) {
     int64_t tile0 = (int64_t)blockIdx.x * BB_THREADS * BB_ITEMS;
@@ -120,10 +112,8 @@ __global__ void __launch_bounds__(BB_THREADS) k_bbox(const double *pos, int64_t 
     }
 }
 
-__global__ void k_bbox_finish(const unsigned long long *mn, const unsigned long long *mx, int nsys, double *center,
-                              double *size) {
-    int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= nsys) return;
+__device__ __forceinline__ void bounding_cube(const unsigned long long *mn, const unsigned long long *mx, int s,
+                                              double *center, double *size) {
     double lo[3], hi[3];
     for (int k = 0; k < 3; k++) {
         lo[k] = ordered_to_dbl(mn[3 * s + k]);
@@ -134,6 +124,11 @@ __global__ void k_bbox_finish(const unsigned long long *mn, const unsigned long 
     if (dsub(hi[1], lo[1]) > sz) sz = dsub(hi[1], lo[1]);
     if (dsub(hi[2], lo[2]) > sz) sz = dsub(hi[2], lo[2]);
     size[s] = sz;
+}
+__global__ void k_bbox_finish(const unsigned long long *mn, const unsigned long long *mx, int nsys, double *center,
+                              double *size) {
+    int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s < nsys) bounding_cube(mn, mx, s, center, size);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -211,20 +206,23 @@ __global__ void k_sys_of(const uint32_t *vals, int64_t n, const int64_t *sys_off
 }
 
 // _permute_particles (octree.py:577-603)
-// sort_err set (the sort gave up and left the identity permutation): the keys stay the sort's
-// fallback keys i, so that every later kernel sees sorted keys (the build then reports the error).
+// sort_err set (the sort gave up): the identity permutation, and keys i, so that every later kernel sees
+// sorted keys and valid indices (the build then reports the error). keys_in null: keys_sorted holds the
+// sorted keys already.
 __global__ void k_gather(const uint32_t *perm, int64_t n, const double *pos, const double *m, const double *h,
                          const uint64_t *keys_in, double *coord, double *mass, double *soft, uint64_t *keys_sorted,
                          int64_t *walk_idx, const int *sort_err) {
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    int64_t o = perm[i];
+    const bool bad = *sort_err != 0;
+    int64_t o = bad ? i : (int64_t)perm[i];
     coord[3 * i] = pos[3 * o];
     coord[3 * i + 1] = pos[3 * o + 1];
     coord[3 * i + 2] = pos[3 * o + 2];
     mass[i] = m ? m[o] : 0.0;
     soft[i] = h ? h[o] : 0.0;
-    keys_sorted[i] = *sort_err ? (uint64_t)i : keys_in[o];
+    if (bad) keys_sorted[i] = (uint64_t)i;
+    else if (keys_in) keys_sorted[i] = keys_in[o];
     walk_idx[i] = o;
 }
 
@@ -276,32 +274,82 @@ __device__ __forceinline__ void elem_loc(const RoundView &v, int64_t e, int &s, 
     i = v.seg_lo[s] + (e - v.eoff[s]);
 }
 
-__global__ void k_levels(RoundView v, int64_t E, const uint64_t *keys, int8_t *L) {
-    int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= E) return;
-    int s;
-    int64_t i;
-    elem_loc(v, e, s, i);
-    L[e] = (i + 1 < v.seg_hi[s]) ? (int8_t)pair_level(keys[i], keys[i + 1]) : (int8_t)-1;
-}
-
 // lowest level of a node starting at element e (e's particle i); root level 0 only at a segment
 // start whose root is created this round.
 __device__ __forceinline__ int lvl0(const RoundView &v, const int8_t *L, int s, int64_t e, int64_t i) {
     if (i == v.seg_lo[s]) return v.seg_root[s] >= 0 ? 1 : 0;
     return L[e - 1] + 1;
 }
+// nodes starting at an element: levels lo .. hi (a one-particle system still has its root)
+__device__ __forceinline__ int node_count(int lo, int hi) {
+    if (lo == 0 && hi < 0) hi = 0;
+    return hi >= lo ? hi - lo + 1 : 0;
+}
 
-__global__ void k_counts(RoundView v, int64_t E, const int8_t *L, int64_t *cnt) {
-    int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= E) return;
-    int s;
-    int64_t i;
-    elem_loc(v, e, s, i);
-    int lo = lvl0(v, L, s, e, i);
-    int hi = L[e];
-    if (lo == 0 && hi < 0) hi = 0;  // a one-particle system still has its root
-    cnt[e] = hi >= lo ? (hi - lo + 1) : 0;
+// The round's levels L and the exclusive prefix sum of its elements' node counts, in one pass over the keys
+// (decoupled look-back; levels, counts and a three-launch scan took five launches and four more arrays'
+// traffic: 37 us of a 1e6 build). The round's node total goes to *total.
+constexpr int LV_THREADS = 256, LV_ITEMS = 4, LV_TILE = LV_THREADS * LV_ITEMS;
+__global__ void __launch_bounds__(LV_THREADS) k_levels(RoundView v, int64_t E, const uint64_t *keys, int8_t *L,
+                                                       int *nstart, unsigned long long *total,
+                                                       unsigned long long *status, int *counter, long long spins) {
+    __shared__ int warp_sum[LV_THREADS / 32];
+    __shared__ long long before_s;
+    __shared__ int tile_s;
+    if (threadIdx.x == 0) tile_s = atomicAdd(counter, 1);
+    __syncthreads();
+    const int tile = tile_s, lane = lane_id(), w = threadIdx.x >> 5;
+    auto element = [&](int64_t e, int &level) {  // the element's node count
+        int s;
+        int64_t i;
+        elem_loc(v, e, s, i);
+        const uint64_t k = keys[i];
+        level = i + 1 < v.seg_hi[s] ? pair_level(k, keys[i + 1]) : -1;
+        const int lo = i == v.seg_lo[s] ? (v.seg_root[s] >= 0 ? 1 : 0) : pair_level(keys[i - 1], k) + 1;
+        return node_count(lo, level);
+    };
+    const int64_t e0 = (int64_t)tile * LV_TILE + (int64_t)threadIdx.x * LV_ITEMS;
+    int cnt[LV_ITEMS], mine = 0;
+#pragma unroll
+    for (int q = 0; q < LV_ITEMS; q++) {
+        cnt[q] = 0;
+        if (e0 + q < E) {
+            int level;
+            cnt[q] = element(e0 + q, level);
+            L[e0 + q] = (int8_t)level;
+        }
+        mine += cnt[q];
+    }
+    const int inc = warp_inclusive_scan(mine);
+    if (lane == 31) warp_sum[w] = inc;
+    __syncthreads();
+    int below = 0, tot = 0;
+#pragma unroll
+    for (int k = 0; k < LV_THREADS / 32; k++) {
+        below += k < w ? warp_sum[k] : 0;
+        tot += warp_sum[k];
+    }
+    if (w == 0) {
+        const long long before = scan_look_back(tot, tile, status, spins, [&]() {
+            long long sum = 0;
+            int level;
+            for (int64_t e = lane; e < (int64_t)tile * LV_TILE; e += 32) sum += element(e, level);
+            for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(FULL, sum, o);
+            return sum;
+        });
+        if (lane == 0) {
+            before_s = before;
+            if ((int64_t)(tile + 1) * LV_TILE >= E) *total = (unsigned long long)(before + tot);
+        }
+    }
+    __syncthreads();
+    long long run = before_s + below + inc - mine;
+#pragma unroll
+    for (int q = 0; q < LV_ITEMS; q++) {
+        // clamped: such a round fits no slot array, k_nodes skips it and the host refuses it
+        if (e0 + q < E) nstart[e0 + q] = (int)min(run, 0x7fffffffll);
+        run += cnt[q];
+    }
 }
 
 // last index in [a, b) with prefix(key, level) == p (keys sorted): upper bound - 1
@@ -347,7 +395,7 @@ __device__ __forceinline__ int64_t gallop_lower_prefix(const uint64_t *keys, int
 }
 
 // slot of the node at `level` containing particle i (level >= lvl0 of the segment root)
-__device__ __forceinline__ int64_t node_at(const RoundView &v, const int8_t *L, const int64_t *nstart,
+__device__ __forceinline__ int64_t node_at(const RoundView &v, const int8_t *L, const int *nstart,
                                            int64_t slot_base, const uint64_t *keys, int s, int64_t i, int level) {
     if (level == 0 && v.seg_root[s] >= 0) return v.seg_root[s];
     int64_t lo = v.seg_lo[s];
@@ -357,7 +405,7 @@ __device__ __forceinline__ int64_t node_at(const RoundView &v, const int8_t *L, 
 }
 
 // NextBranch reference of an element whose particle range ends at e_end (exclusive)
-__device__ __forceinline__ int64_t next_after(const RoundView &v, const int8_t *L, const int64_t *nstart,
+__device__ __forceinline__ int64_t next_after(const RoundView &v, const int8_t *L, const int *nstart,
                                               int64_t slot_base, int s, int64_t e_end_particle) {
     if (e_end_particle >= v.seg_hi[s]) return v.seg_next[s];
     int64_t pe = v.eoff[s] + (e_end_particle - v.seg_lo[s]);
@@ -365,25 +413,38 @@ __device__ __forceinline__ int64_t next_after(const RoundView &v, const int8_t *
     return (outer <= L[pe]) ? node_ref(slot_base + nstart[pe]) : e_end_particle;
 }
 
+// Particle i's parent slot and NextBranch reference.
+__device__ __forceinline__ void place_particle(const RoundView &v, const int8_t *L, const int *nstart, int64_t slot_base,
+                                               const uint64_t *keys, int s, int64_t e, int64_t i, int64_t *p_parent,
+                                               int64_t *p_next) {
+    int lprev = (i == v.seg_lo[s]) ? -1 : L[e - 1];
+    int K = max(lprev, (int)L[e]);
+    if (K >= MAX_LEVEL) return;  // inside a key-exhausted run: the next round places it
+    if (K < 0) K = 0;            // lone particle of its segment: child of the root
+    p_parent[i] = node_at(v, L, nstart, slot_base, keys, s, i, K);
+    p_next[i] = next_after(v, L, nstart, slot_base, s, i + 1);
+}
+
 // Node slots beyond nd.cap are not written (the host sees the round's node total, grows the slot
 // arrays and runs the round's node kernels again); so are exhausted-run entries beyond exh_cap.
-__global__ void k_nodes(RoundView v, int64_t E, const int8_t *L, const int64_t *nstart, const int64_t *cnt,
-                        int64_t slot_base, const uint64_t *keys, Nodes nd, int64_t *exhausted,
-                        unsigned long long *n_exhausted, int64_t exh_cap, int64_t *root_first) {
+__global__ void k_nodes(RoundView v, int64_t E, const int8_t *L, const int *nstart, int64_t slot_base,
+                        const uint64_t *keys, Nodes nd, int64_t *exhausted, unsigned long long *n_exhausted,
+                        int64_t exh_cap, int64_t *root_first, int64_t *p_parent, int64_t *p_next) {
     int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= E) return;
-    if (slot_base + nstart[e] + cnt[e] > nd.cap) return;
     int s;
     int64_t i;
     elem_loc(v, e, s, i);
+    place_particle(v, L, nstart, slot_base, keys, s, e, i, p_parent, p_next);
     int l0 = lvl0(v, L, s, e, i);
+    const int64_t nc = node_count(l0, L[e]);
+    if (slot_base + nstart[e] + nc > nd.cap) return;
     uint64_t key = keys[i];
     int64_t seg_lo = v.seg_lo[s], seg_hi = v.seg_hi[s];
     // existing segment root (a re-keyed node): its first child is the level-1 run at seg_lo
     if (i == seg_lo && v.seg_root[s] >= 0) {
         root_first[s] = (1 <= L[e]) ? node_ref(slot_base + nstart[e]) : i;
     }
-    const int64_t nc = cnt[e];
     const int64_t slot0 = slot_base + nstart[e];
     for (int64_t j = 0; j < nc; j++) {
         int k = l0 + (int)j;
@@ -480,21 +541,6 @@ __global__ void __launch_bounds__(CENTER_BLOCK) k_node_centers(RoundView v, Node
     nd.center[3 * slot + 1] = c1;
     nd.center[3 * slot + 2] = c2;
     nd.size[slot] = sz;
-}
-
-__global__ void k_particles(RoundView v, int64_t E, const int8_t *L, const int64_t *nstart, int64_t slot_base,
-                            const uint64_t *keys, int64_t *p_parent, int64_t *p_next) {
-    int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= E) return;
-    int s;
-    int64_t i;
-    elem_loc(v, e, s, i);
-    int lprev = (i == v.seg_lo[s]) ? -1 : L[e - 1];
-    int K = max(lprev, (int)L[e]);
-    if (K >= MAX_LEVEL) return;  // inside a key-exhausted run: the next round places it
-    if (K < 0) K = 0;            // lone particle of its segment: child of the root
-    p_parent[i] = node_at(v, L, nstart, slot_base, keys, s, i, K);
-    p_next[i] = next_after(v, L, nstart, slot_base, s, i + 1);
 }
 
 __global__ void k_set_root_first(const int64_t *seg_root, const int64_t *root_first, int nseg, int64_t *nd_first) {
@@ -633,12 +679,9 @@ __device__ __forceinline__ bool ref_ok(int64_t r, int64_t N, int64_t M) {
     if (r == -1) return true;
     return (-r - 2) < M;
 }
-__global__ void k_validate_links(int64_t NE, const int64_t *first, const int64_t *next, const int64_t *parent,
-                                 int *bad) {
-    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= NE) return;
-    bool ok = first[i] >= -1 && first[i] < NE && next[i] >= -1 && next[i] < NE && parent[i] >= -1 && parent[i] < NE;
-    if (!ok) atomicOr(bad, 4);
+// final links: elements of the arena, or none
+__device__ __forceinline__ bool links_ok(int64_t NE, int64_t first, int64_t next, int64_t parent) {
+    return first >= -1 && first < NE && next >= -1 && next < NE && parent >= -1 && parent < NE;
 }
 
 // Values the host reads back after a split round, gathered so that one copy (one synchronisation)
@@ -648,15 +691,20 @@ struct BuildSummary {
     unsigned long long nodes;  // node slots made by the round (its scan total)
     unsigned long long n_exh;  // key-exhausted runs found by the round
     int bad;                   // invalid references (bit flags)
-    int nonfinite;             // the input check's flag, copied in before the read-back
+    int nonfinite;             // the input check's flag
     int depth_hist[DEPTH_CAP + 1];
+};
+// Section starts of the depth lists, from the histogram.
+struct LevelOffsets {
+    int at[DEPTH_CAP + 1];
 };
 
 // Slot validation (as above) plus the depth histogram, over the slots [0, M) with
 // M = M_base + *M_round (clamped to the slot capacity).
 __global__ void k_summarize_slots(Nodes nd, int64_t M_base, const unsigned long long *M_round, const int64_t *p_parent,
-                                  const int64_t *p_next, int64_t N, BuildSummary *sum) {
+                                  const int64_t *p_next, int64_t N, BuildSummary *sum, const int *nonfinite) {
     __shared__ int hist[DEPTH_CAP + 1];
+    if (nonfinite && blockIdx.x == 0 && threadIdx.x == 0) sum->nonfinite = *nonfinite;
     for (int b = threadIdx.x; b <= DEPTH_CAP; b += blockDim.x) hist[b] = 0;
     __syncthreads();
     int64_t M = M_base + (M_round ? (int64_t)*M_round : 0);
@@ -684,11 +732,6 @@ __global__ void k_sys_node_counts(const int32_t *nd_sys, int64_t M, int64_t *cnt
     int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (c < M) atomicAdd((unsigned long long *)&cnt[nd_sys[c]], 1ull);
 }
-__global__ void k_single_sys_node_off(int64_t *sys_node_off, int64_t M) {
-    sys_node_off[0] = 0;
-    sys_node_off[1] = M;
-}
-
 // ---------------------------------------------------------------------------------------------
 // Numbering.
 struct NumberingBits {
@@ -703,8 +746,7 @@ struct NumberingBits {
 // instead of the first particle, which saves sort passes. (A bucket chain hangs all its nodes on one
 // allocating parent, so it needs the full first-particle rank.)
 __global__ void k_number_keys(Nodes nd, int64_t count, const int64_t *sys_off, NumberingBits b, uint64_t root_key,
-                              int compact, uint64_t *keys, uint32_t *vals, int64_t *root_slot_of_sys,
-                              int *nonroot_count) {
+                              int compact, uint64_t *keys, uint32_t *vals, int64_t *root_slot_of_sys) {
     int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= count) return;
     int s = nd.sys[c];
@@ -723,11 +765,10 @@ __global__ void k_number_keys(Nodes nd, int64_t count, const int64_t *sys_off, N
                  ((uint64_t)nd.depth[ap] << low) | sib;
     keys[c] = k;
     vals[c] = (uint32_t)c;
-    atomicAdd(nonroot_count, 1);
 }
 
-// sort_err set (the numbering sort left the identity, roots not last): every slot keeps its own
-// index, a bijection onto the node range, so the arrays written from it stay in bounds.
+// sort_err set (the numbering sort gave up): every slot keeps its own index, a bijection onto the node
+// range, so the arrays written from it stay in bounds. sys_node_off null: one system, offset 0.
 __global__ void k_final_index(const uint32_t *vals, int64_t count, const int32_t *nd_sys, int64_t ntot,
                               const int64_t *sys_node_off, int64_t *final_of_slot, const int64_t *root_slot_of_sys,
                               int nsys, const int *sort_err) {
@@ -741,7 +782,7 @@ __global__ void k_final_index(const uint32_t *vals, int64_t count, const int32_t
         int s = nd_sys[c];
         if (q < count - nsys) final_of_slot[c] = ntot + q + s + 1;
     }
-    if (q < nsys) final_of_slot[root_slot_of_sys[q]] = ntot + sys_node_off[q];
+    if (q < nsys) final_of_slot[root_slot_of_sys[q]] = ntot + (sys_node_off ? sys_node_off[q] : 0);
 }
 
 __device__ __forceinline__ int64_t resolve(int64_t ref, const int64_t *final_of_slot) {
@@ -750,18 +791,44 @@ __device__ __forceinline__ int64_t resolve(int64_t ref, const int64_t *final_of_
     return final_of_slot[-ref - 2];
 }
 
-// Besides the node arrays, files every node into the list of its depth (lvl_list, sections at
-// lvl_off[d]; depths >= DEPTH_CAP share the last section) for the level-by-level moment pass.
-__global__ void k_write_nodes(Nodes nd, int64_t count, const int64_t *final_of_slot, double *coord, double *size,
-                              double *mass, double *soft, double *delta, int64_t *first, int64_t *next,
-                              int64_t *parent, int2 *range, double *cell, int64_t ntot, const int *lvl_off,
-                              int *lvl_cursor, int32_t *lvl_list, int8_t *fdepth) {
+// The final arrays: blocks [0, node_blocks) write the nodes, the others the particles, so both run together;
+// the links are checked as they are written. Besides the node arrays, every node is filed into the list of
+// its depth (lvl_list, sections at off.at[d]; depths >= DEPTH_CAP share the last section) for the
+// level-by-level moment pass.
+struct FinalArrays {
+    double *coord, *mass, *soft, *size, *delta;
+    int64_t *first, *next, *parent;
+    int2 *range;
+    double *cell;
+};
+__global__ void k_write(Nodes nd, int64_t count, int64_t ntot, int node_blocks, const int64_t *final_of_slot,
+                        FinalArrays o, LevelOffsets off, int *lvl_cursor, int32_t *lvl_list, int8_t *fdepth,
+                        const int64_t *p_parent, const int64_t *p_next, const double *pc, const double *pm,
+                        const double *ps, int *bad) {
+    const int64_t NE = ntot + count;
+    if ((int)blockIdx.x >= node_blocks) {  // particles: the Morton-ordered data and the resolved links
+        const int64_t i = (int64_t)(blockIdx.x - node_blocks) * blockDim.x + threadIdx.x;
+        if (i >= ntot) return;
+        const int64_t next = resolve(p_next[i], final_of_slot), parent = final_of_slot[p_parent[i]];
+        o.coord[3 * i] = pc[3 * i];
+        o.coord[3 * i + 1] = pc[3 * i + 1];
+        o.coord[3 * i + 2] = pc[3 * i + 2];
+        o.mass[i] = pm[i];
+        o.soft[i] = ps[i];
+        o.first[i] = -1;
+        o.next[i] = next;
+        o.parent[i] = parent;
+        o.size[i] = 0.0;
+        o.delta[i] = 0.0;
+        if (!links_ok(NE, -1, next, parent)) atomicOr(bad, 4);
+        return;
+    }
     int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= count) return;
     int64_t f = final_of_slot[c];
-    mass[f] = 0.0;  // the moment pass fills these
-    soft[f] = 0.0;
-    delta[f] = 0.0;
+    o.mass[f] = 0.0;  // the moment pass fills these
+    o.soft[f] = 0.0;
+    o.delta[f] = 0.0;
     {
         int d = nd.depth[c];
         d = d < 0 ? 0 : (d > DEPTH_CAP ? DEPTH_CAP : d);
@@ -770,39 +837,24 @@ __global__ void k_write_nodes(Nodes nd, int64_t count, const int64_t *final_of_s
         int base = 0;
         if (lane_id() == leader) base = atomicAdd(&lvl_cursor[d], __popc(peers));
         base = __shfl_sync(peers, base, leader);
-        lvl_list[lvl_off[d] + base + __popc(peers & lanemask_lt())] = (int32_t)(f - ntot);
+        lvl_list[off.at[d] + base + __popc(peers & lanemask_lt())] = (int32_t)(f - ntot);
         fdepth[f - ntot] = (int8_t)d;
     }
-    range[f - ntot] = make_int2((int)nd.lo[c], (int)nd.hi[c]);
-    cell[3 * (f - ntot)] = nd.center[3 * c];
-    cell[3 * (f - ntot) + 1] = nd.center[3 * c + 1];
-    cell[3 * (f - ntot) + 2] = nd.center[3 * c + 2];
-    coord[3 * f] = nd.center[3 * c];
-    coord[3 * f + 1] = nd.center[3 * c + 1];
-    coord[3 * f + 2] = nd.center[3 * c + 2];
-    size[f] = nd.size[c];
-    first[f] = resolve(nd.first[c], final_of_slot);
-    next[f] = resolve(nd.next[c], final_of_slot);
-    parent[f] = nd.parent[c] < 0 ? -1 : final_of_slot[nd.parent[c]];
-}
-
-// Particle rows of the final arrays, the Morton-ordered coordinates, masses and softenings included.
-__global__ void k_write_particles(int64_t ntot, const int64_t *p_parent, const int64_t *p_next,
-                                  const int64_t *final_of_slot, const double *pc, const double *pm, const double *ps,
-                                  double *coord, double *mass, double *soft, int64_t *first, int64_t *next,
-                                  int64_t *parent, double *size, double *delta) {
-    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= ntot) return;
-    coord[3 * i] = pc[3 * i];
-    coord[3 * i + 1] = pc[3 * i + 1];
-    coord[3 * i + 2] = pc[3 * i + 2];
-    mass[i] = pm[i];
-    soft[i] = ps[i];
-    first[i] = -1;
-    next[i] = resolve(p_next[i], final_of_slot);
-    parent[i] = final_of_slot[p_parent[i]];
-    size[i] = 0.0;
-    delta[i] = 0.0;
+    o.range[f - ntot] = make_int2((int)nd.lo[c], (int)nd.hi[c]);
+    const double c0 = nd.center[3 * c], c1 = nd.center[3 * c + 1], c2 = nd.center[3 * c + 2];
+    o.cell[3 * (f - ntot)] = c0;
+    o.cell[3 * (f - ntot) + 1] = c1;
+    o.cell[3 * (f - ntot) + 2] = c2;
+    o.coord[3 * f] = c0;
+    o.coord[3 * f + 1] = c1;
+    o.coord[3 * f + 2] = c2;
+    o.size[f] = nd.size[c];
+    const int64_t first = resolve(nd.first[c], final_of_slot), next = resolve(nd.next[c], final_of_slot);
+    const int64_t parent = nd.parent[c] < 0 ? -1 : final_of_slot[nd.parent[c]];
+    o.first[f] = first;
+    o.next[f] = next;
+    o.parent[f] = parent;
+    if (!links_ok(NE, first, next, parent)) atomicOr(bad, 4);
 }
 
 // Children of every node in the order the moment sums take them (octree.py:199-292): particle
@@ -1299,17 +1351,6 @@ __global__ void k_quad64_deep(MomentArgs a, const int32_t *list, int count, cons
     }
 }
 
-// Section offsets of the level lists from the depth histogram; cursors reset.
-__global__ void k_level_offsets(const BuildSummary *sum, int *lvl_off, int *lvl_cursor) {
-    if (threadIdx.x != 0) return;
-    int run = 0;
-    for (int d = 0; d <= DEPTH_CAP; d++) {
-        lvl_off[d] = run;
-        lvl_cursor[d] = 0;
-        run += sum->depth_hist[d];
-    }
-}
-
 // compute_moments=False: node masses/softenings hold only the particles folded in by the split.
 __global__ void k_fold_only(MomentArgs a) {
     int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1370,60 +1411,88 @@ static void dfree(T *&p, cudaStream_t s) {
     p = nullptr;
 }
 
-static tg_status segs_alloc(Segs &g, int n, cudaStream_t s) {
+// Several device arrays in one allocation: lay them out twice, first to size it.
+struct Carve {
+    unsigned char *base = nullptr;
+    size_t used = 0;
+    template <typename T>
+    void take(T *&p, int64_t n) {
+        used = (used + 255) & ~(size_t)255;
+        p = base ? reinterpret_cast<T *>(base + used) : nullptr;
+        used += sizeof(T) * (size_t)std::max<int64_t>(n, 1);
+    }
+};
+template <class Lay>
+static cudaError_t carve(DevArray<unsigned char> &mem, Lay lay) {
+    Carve c;
+    lay(c);
+    mem.reset();
+    cudaError_t e = mem.alloc((int64_t)c.used);
+    if (e != cudaSuccess) return e;
+    Carve d;
+    d.base = mem.p;
+    lay(d);
+    return cudaSuccess;
+}
+
+static void segs_lay(Carve &c, Segs &g, int n) {
     g.n = n;
-    TG_TRY(dalloc(&g.lo, n, s));
-    TG_TRY(dalloc(&g.hi, n, s));
-    TG_TRY(dalloc(&g.root, n, s));
-    TG_TRY(dalloc(&g.center, 3 * n, s));
-    TG_TRY(dalloc(&g.size, n, s));
-    TG_TRY(dalloc(&g.depth0, n, s));
-    TG_TRY(dalloc(&g.next_ref, n, s));
-    TG_TRY(dalloc(&g.sys, n, s));
-    TG_TRY(dalloc(&g.eoff, n + 1, s));
-    return TG_OK;
+    c.take(g.lo, n);
+    c.take(g.hi, n);
+    c.take(g.root, n);
+    c.take(g.center, 3 * (int64_t)n);
+    c.take(g.size, n);
+    c.take(g.depth0, n);
+    c.take(g.next_ref, n);
+    c.take(g.sys, n);
+    c.take(g.eoff, (int64_t)n + 1);
 }
-static void segs_free(Segs &g, cudaStream_t s) {
-    dfree(g.lo, s); dfree(g.hi, s); dfree(g.root, s); dfree(g.center, s); dfree(g.size, s);
-    dfree(g.depth0, s); dfree(g.next_ref, s); dfree(g.sys, s); dfree(g.eoff, s);
-    g.n = 0;
+static void nodes_lay(Carve &c, Nodes &nd, int64_t cap) {
+    nd.cap = cap;
+    c.take(nd.lo, cap);
+    c.take(nd.hi, cap);
+    c.take(nd.parent, cap);
+    c.take(nd.first, cap);
+    c.take(nd.next, cap);
+    c.take(nd.aparent, cap);
+    c.take(nd.rank, cap);
+    c.take(nd.digit, cap);
+    c.take(nd.depth, cap);
+    c.take(nd.sys, cap);
+    c.take(nd.seg, cap);
+    c.take(nd.level, cap);
+    c.take(nd.center, 3 * cap);
+    c.take(nd.size, cap);
 }
-
-template <typename T>
-static tg_status grow_copy(T **p, int64_t old_n, int64_t new_n, int width, cudaStream_t s) {
-    T *q = nullptr;
-    TG_TRY(dalloc(&q, new_n * width, s));
-    if (*p && old_n > 0) TG_CUDA(cudaMemcpyAsync(q, *p, sizeof(T) * old_n * width, cudaMemcpyDeviceToDevice, s));
-    dfree(*p, s);
-    *p = q;
-    return TG_OK;
-}
-
-static tg_status nodes_reserve(Nodes &nd, int64_t need, cudaStream_t s) {
+// Room for `need` slots: nd's filled slots copied into a larger allocation, which replaces the one in mem.
+static tg_status nodes_reserve(DevArray<unsigned char> &mem, Nodes &nd, int64_t need, cudaStream_t st) {
     if (need <= nd.cap) return TG_OK;
-    int64_t nc = std::max<int64_t>(need, nd.cap + nd.cap / 2 + 64);
-    TG_TRY(grow_copy(&nd.lo, nd.count, nc, 1, s));
-    TG_TRY(grow_copy(&nd.hi, nd.count, nc, 1, s));
-    TG_TRY(grow_copy(&nd.parent, nd.count, nc, 1, s));
-    TG_TRY(grow_copy(&nd.first, nd.count, nc, 1, s));
-    TG_TRY(grow_copy(&nd.next, nd.count, nc, 1, s));
-    TG_TRY(grow_copy(&nd.aparent, nd.count, nc, 1, s));
-    TG_TRY(grow_copy(&nd.rank, nd.count, nc, 1, s));
-    TG_TRY(grow_copy(&nd.digit, nd.count, nc, 1, s));
-    TG_TRY(grow_copy(&nd.depth, nd.count, nc, 1, s));
-    TG_TRY(grow_copy(&nd.sys, nd.count, nc, 1, s));
-    TG_TRY(grow_copy(&nd.seg, nd.count, nc, 1, s));
-    TG_TRY(grow_copy(&nd.level, nd.count, nc, 1, s));
-    TG_TRY(grow_copy(&nd.center, nd.count, nc, 3, s));
-    TG_TRY(grow_copy(&nd.size, nd.count, nc, 1, s));
-    nd.cap = nc;
+    const int64_t cap = std::max<int64_t>(need, nd.cap + nd.cap / 2 + 64);
+    DevArray<unsigned char> grown(st);
+    Nodes q = nd;
+    TG_CUDA(carve(grown, [&](Carve &c) { nodes_lay(c, q, cap); }));
+    auto copy = [&](auto *dst, const auto *src, int width) {
+        return cudaMemcpyAsync(dst, src, sizeof(*dst) * (size_t)(nd.count * width), cudaMemcpyDeviceToDevice, st);
+    };
+    if (nd.count > 0) {
+        TG_CUDA(copy(q.lo, nd.lo, 1));
+        TG_CUDA(copy(q.hi, nd.hi, 1));
+        TG_CUDA(copy(q.parent, nd.parent, 1));
+        TG_CUDA(copy(q.first, nd.first, 1));
+        TG_CUDA(copy(q.next, nd.next, 1));
+        TG_CUDA(copy(q.aparent, nd.aparent, 1));
+        TG_CUDA(copy(q.rank, nd.rank, 1));
+        TG_CUDA(copy(q.digit, nd.digit, 1));
+        TG_CUDA(copy(q.depth, nd.depth, 1));
+        TG_CUDA(copy(q.sys, nd.sys, 1));
+        TG_CUDA(copy(q.seg, nd.seg, 1));
+        TG_CUDA(copy(q.level, nd.level, 1));
+        TG_CUDA(copy(q.center, nd.center, 3));
+        TG_CUDA(copy(q.size, nd.size, 1));
+    }
+    mem.swap(grown);
+    nd = q;
     return TG_OK;
-}
-static void nodes_free(Nodes &nd, cudaStream_t s) {
-    dfree(nd.lo, s); dfree(nd.hi, s); dfree(nd.parent, s); dfree(nd.first, s); dfree(nd.next, s);
-    dfree(nd.aparent, s); dfree(nd.rank, s); dfree(nd.digit, s); dfree(nd.depth, s); dfree(nd.sys, s); dfree(nd.seg, s);
-    dfree(nd.level, s);
-    dfree(nd.center, s); dfree(nd.size, s);
 }
 
 static RoundView view_of(const Segs &g) {
@@ -1448,19 +1517,26 @@ static int64_t reference_capacity(int64_t npart, int64_t required) {
     return cap;
 }
 
-__global__ void k_init_root_segs(Segs g, const int64_t *sys_off, const double *center, const double *size) {
-    int s = blockIdx.x * blockDim.x + threadIdx.x;
+// The bounding cubes' centres and sizes, and round 0's segments: one per system. One system's offsets (0, n) are
+// written here too.
+__global__ void k_root_segs(const unsigned long long *mn, const unsigned long long *mx, int64_t *sys_off, int64_t n,
+                            Segs g) {
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= g.n) return;
-    g.lo[s] = sys_off[s];
-    g.hi[s] = sys_off[s + 1];
+    bounding_cube(mn, mx, s, g.center, g.size);
+    const int64_t lo = g.n == 1 ? 0 : sys_off[s], hi = g.n == 1 ? n : sys_off[s + 1];
+    if (g.n == 1) {
+        sys_off[0] = lo;
+        sys_off[1] = hi;
+    }
+    g.lo[s] = lo;
+    g.hi[s] = hi;
     g.root[s] = -1;
-    g.center[3 * s] = center[3 * s];
-    g.center[3 * s + 1] = center[3 * s + 1];
-    g.center[3 * s + 2] = center[3 * s + 2];
-    g.size[s] = size[s];
     g.depth0[s] = 0;
     g.next_ref[s] = -1;
     g.sys[s] = s;
+    g.eoff[s] = lo;
+    if (s == g.n - 1) g.eoff[g.n] = hi;
 }
 
 #define LAUNCH(n) div_up((n), 256), 256, 0, st
@@ -1468,6 +1544,9 @@ __global__ void k_init_root_segs(Segs g, const int64_t *sys_off, const double *c
 // Build the whole arena. pos/m/h are device pointers (m/h may be null). m_h_ready (may be null):
 // an event after which m and h may be read; the build waits for it only where it first reads them
 // (the gather into Morton order), so their upload overlaps the bounding cube, keys and sort.
+// The temporaries whose sizes are known up front are one allocation, as are those that need the node
+// count, and the tree's own arrays: a build made ~50 allocations and as many frees, whose host time a small
+// build waits for (with the fused launches below, 12345 particles with their walk: 842 -> 735 us).
 tg_status build_tree(tg_tree_s *T, const double *pos, const double *m, const double *h,
                      const std::vector<int64_t> &sys_off_host, int quadrupole, int compute_moments,
                      const int *nonfinite, cudaStream_t st, cudaEvent_t m_h_ready) {
@@ -1491,102 +1570,142 @@ tg_status build_tree(tg_tree_s *T, const double *pos, const double *m, const dou
     T->has_quads = quadrupole;
     T->compute_moments = compute_moments;
     T->stream = st;
+    void *host = nullptr;  // read-backs
+    TG_TRY(host_words(&host));
 
-    int64_t *sys_off = nullptr;
-    TG_TRY(dalloc(&sys_off, nsys + 1, st));
-    TG_CUDA(cudaMemcpyAsync(sys_off, sys_off_host.data(), sizeof(int64_t) * (nsys + 1), cudaMemcpyHostToDevice, st));
-    TG_TRY(dalloc(&T->sort_err, 1, st));  // every sort of this tree reports here
-    TG_CUDA(cudaMemsetAsync(T->sort_err, 0, sizeof(int), st));
-
-    // 1. bounding cubes
-    unsigned long long *mn = nullptr, *mx = nullptr;
-    double *center = nullptr, *size = nullptr;
-    TG_TRY(dalloc(&mn, 3 * nsys, st));
-    TG_TRY(dalloc(&mx, 3 * nsys, st));
-    TG_TRY(dalloc(&center, 3 * nsys, st));
-    TG_TRY(dalloc(&size, nsys, st));
-    { k_bbox_init<<<LAUNCH(3 * nsys)>>>(mn, mx, nsys); tg::note_launch(); }
-    { k_bbox<<<div_up(N, BB_THREADS * BB_ITEMS), BB_THREADS, 0, st>>>(pos, N, sys_off, nsys, mn, mx); tg::note_launch(); }
-    { k_bbox_finish<<<LAUNCH(nsys)>>>(mn, mx, nsys, center, size); tg::note_launch(); }
-    TG_CUDA(cudaGetLastError());
-
-    // 2. keys and stable sort (system id as the most significant digit when batched)
+    // zeroed together: the summary, the depth lists' cursors, the level scan's status words and counter, the
+    // cubes' maxima and (kept with the tree) the sorts' error word
+    const int lv_tiles = div_up(N, LV_TILE);
+    const int64_t cap0 = N + N / 2 + 16;  // node slots, grown if needed
+    int64_t exh_cap = N / 2 + 1;          // key-exhausted runs hold at least two particles each
+    BuildSummary *sum = nullptr;
+    int *lvl_cursor = nullptr;
+    unsigned long long *lv_status = nullptr, *mn = nullptr, *mx = nullptr;
+    int64_t *sys_off = nullptr, *p_parent = nullptr, *p_next = nullptr, *exh = nullptr, *root_first = nullptr;
     uint64_t *keys = nullptr, *keys_orig = nullptr;
     uint32_t *perm = nullptr;
-    TG_TRY(dalloc(&keys, N, st));
-    TG_TRY(dalloc(&keys_orig, N, st));
-    TG_TRY(dalloc(&perm, N, st));
-    { k_keys<<<LAUNCH(N)>>>(pos, N, sys_off, nsys, center, size, keys, keys_orig, perm); tg::note_launch(); }
+    double *pc = nullptr, *pm = nullptr, *ps = nullptr;
+    int8_t *L = nullptr;
+    int *nstart = nullptr;
+    Nodes nd;
+    Segs sg;
+    DevArray<unsigned char> temps(st);
+    TG_CUDA(carve(temps, [&](Carve &c) {
+        c.take(sum, 1);
+        c.take(lvl_cursor, DEPTH_CAP + 1);
+        c.take(lv_status, lv_tiles + 1);
+        c.take(mx, 3 * nsys);
+        c.take(mn, 3 * nsys);
+        c.take(sys_off, nsys + 1);
+        c.take(keys, N);
+        if (nsys > 1) c.take(keys_orig, N);
+        c.take(perm, N);
+        c.take(pc, 3 * N);
+        c.take(pm, N);
+        c.take(ps, N);
+        c.take(L, N);
+        c.take(nstart, N);
+        c.take(exh, exh_cap);
+        c.take(root_first, nsys);
+        c.take(p_parent, N);
+        c.take(p_next, N);
+        segs_lay(c, sg, nsys);
+        nodes_lay(c, nd, cap0);
+    }));
+    // what replaces parts of it: slots that grow, the segments and lists of later rounds
+    DevArray<unsigned char> slots(st), round_mem(st);
+    const size_t head = (size_t)((unsigned char *)mn - temps.p);
+    TG_CUDA(cudaMemsetAsync(temps.p, 0, head, st));
+    TG_CUDA(cudaMemsetAsync(mn, 0xff, sizeof(unsigned long long) * 3 * nsys, st));
+    TG_TRY(dalloc(&T->sort_err, 1, st));  // every sort of this tree reports here
+    TG_CUDA(cudaMemsetAsync(T->sort_err, 0, sizeof(int), st));
+    TG_TRY(dalloc(&T->walk_idx, N, st));
+
+    // 1. bounding cubes
+    if (nsys > 1)
+        TG_CUDA(cudaMemcpyAsync(sys_off, sys_off_host.data(), sizeof(int64_t) * (nsys + 1), cudaMemcpyHostToDevice, st));
+    { k_bbox<<<div_up(N, BB_THREADS * BB_ITEMS), BB_THREADS, 0, st>>>(pos, N, sys_off, nsys, mn, mx); tg::note_launch(); }
+    { k_root_segs<<<LAUNCH(nsys)>>>(mn, mx, sys_off, N, sg); tg::note_launch(); }
+
+    // 2. keys and stable sort (system id as the most significant digit when batched)
+    { k_keys<<<LAUNCH(N)>>>(pos, N, sys_off, nsys, sg.center, sg.size, keys, keys_orig, perm); tg::note_launch(); }
     TG_CUDA(cudaGetLastError());
-    TG_TRY(radix_sort_pairs(keys, perm, N, 63, st, T->sort_err));
+    TG_TRY(radix_sort_pairs(keys, perm, N, 63, st, T->sort_err, nsys == 1));
     if (nsys > 1) {
         { k_sys_of<<<LAUNCH(N)>>>(perm, N, sys_off, nsys, keys); tg::note_launch(); }
         TG_TRY(radix_sort_pairs(keys, perm, N, sysbits, st, T->sort_err));
     }
 
-    // 3. arena element arrays; particles gathered into Morton order
-    const int64_t cap0 = N + N / 2 + 16;  // node slots, grown if needed
-    TG_TRY(dalloc(&T->walk_idx, N, st));
-    double *pc = nullptr, *pm = nullptr, *ps = nullptr;
-    TG_TRY(dalloc(&pc, 3 * N, st));
-    TG_TRY(dalloc(&pm, N, st));
-    TG_TRY(dalloc(&ps, N, st));
-    uint64_t *keys_sorted = keys;  // reuse
+    // 3. particles gathered into Morton order
     if (m_h_ready) TG_CUDA(cudaStreamWaitEvent(st, m_h_ready, 0));
-    { k_gather<<<LAUNCH(N)>>>(perm, N, pos, m, h, keys_orig, pc, pm, ps, keys_sorted, T->walk_idx, T->sort_err); tg::note_launch(); }
+    { k_gather<<<LAUNCH(N)>>>(perm, N, pos, m, h, keys_orig, pc, pm, ps, keys, T->walk_idx, T->sort_err); tg::note_launch(); }
     TG_CUDA(cudaGetLastError());
-    dfree(keys_orig, st);
 
     // 4. split rounds
-    Nodes nd;
-    TG_TRY(nodes_reserve(nd, cap0, st));
-    int64_t *p_parent = nullptr, *p_next = nullptr;
-    TG_TRY(dalloc(&p_parent, N, st));
-    TG_TRY(dalloc(&p_next, N, st));
-    Segs sg;
-    TG_TRY(segs_alloc(sg, nsys, st));
-    { k_init_root_segs<<<LAUNCH(nsys)>>>(sg, sys_off, center, size); tg::note_launch(); }
-    TG_CUDA(cudaGetLastError());
-    int64_t *exh = nullptr;
     int n_exh = 0;
-    int64_t *root_first = nullptr;
     int has_coincident = 0;
     // What the host reads back after a round; final (covering every slot) once a round leaves no
     // key-exhausted run. The common case, one round and no buckets, synchronises here once.
-    BuildSummary *sum = nullptr;
-    TG_TRY(dalloc(&sum, 1, st));
     BuildSummary hs;
     memset(&hs, 0, sizeof(hs));
+    static_assert(sizeof(BuildSummary) <= HOST_WORDS_BYTES, "the summary must fit the host words");
+    auto read_summary = [&]() -> tg_status {
+        TG_CUDA(cudaMemcpyAsync(host, sum, sizeof(BuildSummary), cudaMemcpyDeviceToHost, st));
+        TG_CUDA(cudaStreamSynchronize(st));
+        memcpy(&hs, host, sizeof(hs));
+        return TG_OK;
+    };
     bool summary_final = false;
     BuildSide *side = nullptr;  // k_node_centers of the last round runs there when set
     bool centers_forked = false;
-    // Non-finite input is reported once the build has run to its end and freed its memory: every
-    // kernel stays in bounds on such input (keys of NaN quantize to 0, every link is checked).
+    // work that reads the temporaries on the side stream is waited for before they are freed, also on errors
+    struct Join {
+        BuildSide *&side;
+        const bool &forked;
+        cudaStream_t st;
+        ~Join() {
+            if (forked) cudaStreamWaitEvent(st, side->join, 0);
+        }
+    } join{side, centers_forked, st};
+    // Non-finite input is reported once the build has run to its end: every kernel stays in bounds on
+    // such input (keys of NaN quantize to 0, every link is checked).
     bool nonfinite_seen = false;
 
     for (int round = 0; round <= MORTON_MAX_ROUNDS; round++) {
         // element offsets of the segments; round 0's segments are the systems
         int64_t E = N;
-        if (round == 0) {
-            TG_CUDA(cudaMemcpyAsync(sg.eoff, sys_off, sizeof(int64_t) * (nsys + 1), cudaMemcpyDeviceToDevice, st));
-        } else {
-            int64_t *sizes = nullptr;
-            TG_TRY(dalloc(&sizes, sg.n, st));
-            { k_seg_sizes<<<LAUNCH(sg.n)>>>(sg.lo, sg.hi, sg.n, sizes); tg::note_launch(); }
-            TG_TRY(exclusive_scan_i64(sizes, sg.eoff, sg.n, sg.eoff + sg.n, st));
-            dfree(sizes, st);
-            TG_CUDA(cudaMemcpyAsync(&E, sg.eoff + sg.n, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+        if (round > 0) {
+            DevArray<int64_t> sizes(st);
+            TG_CUDA(sizes.alloc(sg.n));
+            { k_seg_sizes<<<LAUNCH(sg.n)>>>(sg.lo, sg.hi, sg.n, sizes.p); tg::note_launch(); }
+            TG_TRY(exclusive_scan_i64(sizes.p, sg.eoff, sg.n, sg.eoff + sg.n, st));
+            TG_CUDA(cudaMemcpyAsync(host, sg.eoff + sg.n, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
             TG_CUDA(cudaStreamSynchronize(st));
+            E = *(const int64_t *)host;
+            if (E < 0 || E > N) {
+                set_last_error_msg("internal error: octree build made segments larger than its particles");
+                return TG_ERR_CUDA;
+            }
         }
         RoundView v = view_of(sg);
 
         if (round > 0) {
             // re-key the exhausted runs relative to their cells and sort each run stably
-            uint64_t *rk = nullptr, *rk_elem = nullptr;
+            uint64_t *rk = nullptr, *rk_elem = nullptr, *tk = nullptr;
             uint32_t *rv = nullptr;
-            TG_TRY(dalloc(&rk, E, st));
-            TG_TRY(dalloc(&rk_elem, E, st));
-            TG_TRY(dalloc(&rv, E, st));
+            double *tc = nullptr, *tm = nullptr, *ts = nullptr;
+            int64_t *tw = nullptr;
+            DevArray<unsigned char> rekey(st);
+            TG_CUDA(carve(rekey, [&](Carve &c) {
+                c.take(rk, E);
+                c.take(rk_elem, E);
+                c.take(rv, E);
+                c.take(tc, 3 * E);
+                c.take(tm, E);
+                c.take(ts, E);
+                c.take(tw, E);
+                c.take(tk, E);
+            }));
             { k_rekey_keys<<<LAUNCH(E)>>>(v, E, pc, rk, rv); tg::note_launch(); }
             TG_CUDA(cudaMemcpyAsync(rk_elem, rk, sizeof(uint64_t) * E, cudaMemcpyDeviceToDevice, st));
             TG_TRY(radix_sort_pairs(rk, rv, E, 63, st, T->sort_err));
@@ -1594,60 +1713,37 @@ tg_status build_tree(tg_tree_s *T, const double *pos, const double *m, const dou
                 { k_rekey_segkeys<<<LAUNCH(E)>>>(v, rv, E, rk); tg::note_launch(); }
                 TG_TRY(radix_sort_pairs(rk, rv, E, bits_for(sg.n - 1), st, T->sort_err));
             }
-            double *tc = nullptr, *tm = nullptr, *ts = nullptr;
-            int64_t *tw = nullptr;
-            uint64_t *tk = nullptr;
-            TG_TRY(dalloc(&tc, 3 * E, st));
-            TG_TRY(dalloc(&tm, E, st));
-            TG_TRY(dalloc(&ts, E, st));
-            TG_TRY(dalloc(&tw, E, st));
-            TG_TRY(dalloc(&tk, E, st));
             { k_rekey_gather<<<LAUNCH(E)>>>(v, E, rv, pc, pm, ps, T->walk_idx, rk_elem, tc, tm, ts, tw, tk, T->sort_err); tg::note_launch(); }
-            { k_rekey_scatter<<<LAUNCH(E)>>>(v, E, tc, tm, ts, tw, tk, pc, pm, ps, T->walk_idx, keys_sorted); tg::note_launch(); }
+            { k_rekey_scatter<<<LAUNCH(E)>>>(v, E, tc, tm, ts, tw, tk, pc, pm, ps, T->walk_idx, keys); tg::note_launch(); }
             TG_CUDA(cudaGetLastError());
-            dfree(rk, st); dfree(rk_elem, st); dfree(rv, st);
-            dfree(tc, st); dfree(tm, st); dfree(ts, st); dfree(tw, st); dfree(tk, st);
         }
 
-        int8_t *L = nullptr;
-        int64_t *cnt = nullptr, *nstart = nullptr;
-        TG_TRY(dalloc(&L, E, st));
-        TG_TRY(dalloc(&cnt, E, st));
-        TG_TRY(dalloc(&nstart, E, st));
-        TG_CUDA(cudaMemsetAsync(sum, 0, sizeof(BuildSummary), st));
-        { k_levels<<<LAUNCH(E)>>>(v, E, keys_sorted, L); tg::note_launch(); }
-        { k_counts<<<LAUNCH(E)>>>(v, E, L, cnt); tg::note_launch(); }
-        TG_CUDA(cudaGetLastError());
-        TG_TRY(exclusive_scan_i64(cnt, nstart, E, (int64_t *)&sum->nodes, st));
         const int64_t slot_base = nd.count;
-        dfree(exh, st);
-        dfree(root_first, st);
-        int64_t exh_cap = std::max<int64_t>(nd.cap - slot_base, 1);
-        TG_TRY(dalloc(&exh, exh_cap, st));
-        TG_TRY(dalloc(&root_first, sg.n, st));
+        const int tiles = div_up(E, LV_TILE);
+        if (round > 0) {
+            TG_CUDA(cudaMemsetAsync(sum, 0, sizeof(BuildSummary), st));
+            TG_CUDA(cudaMemsetAsync(lv_status, 0, sizeof(unsigned long long) * (lv_tiles + 1), st));
+        }
+        { k_levels<<<tiles, LV_THREADS, 0, st>>>(v, E, keys, L, nstart, &sum->nodes, lv_status,
+                                                 (int *)(lv_status + lv_tiles), scan_spins()); tg::note_launch(); }
         // The round's nodes, particle links and the summary, read back with one copy. Slots that
         // do not fit are skipped by k_nodes; the host then grows the arrays and runs it again.
         auto run_round = [&]() -> tg_status {
-            { k_nodes<<<LAUNCH(E)>>>(v, E, L, nstart, cnt, slot_base, keys_sorted, nd, exh, &sum->n_exh, exh_cap,
-                                     root_first); tg::note_launch(); }
-            { k_particles<<<LAUNCH(E)>>>(v, E, L, nstart, slot_base, keys_sorted, p_parent, p_next); tg::note_launch(); }
+            { k_nodes<<<LAUNCH(E)>>>(v, E, L, nstart, slot_base, keys, nd, exh, &sum->n_exh, exh_cap, root_first,
+                                     p_parent, p_next); tg::note_launch(); }
             if (round > 0) { k_set_root_first<<<LAUNCH(sg.n)>>>(sg.root, root_first, sg.n, nd.first); tg::note_launch(); }
             { k_summarize_slots<<<LAUNCH(std::max<int64_t>(nd.cap, N))>>>(nd, slot_base, &sum->nodes, p_parent, p_next,
-                                                                       N, sum); tg::note_launch(); }
+                                                                       N, sum, nonfinite); tg::note_launch(); }
             TG_CUDA(cudaGetLastError());
-            if (nonfinite) TG_CUDA(cudaMemcpyAsync(&sum->nonfinite, nonfinite, sizeof(int), cudaMemcpyDeviceToDevice, st));
-            TG_CUDA(cudaMemcpyAsync(&hs, sum, sizeof(BuildSummary), cudaMemcpyDeviceToHost, st));
-            TG_CUDA(cudaStreamSynchronize(st));
+            TG_TRY(read_summary());
             if (hs.nonfinite) nonfinite_seen = true;
             return TG_OK;
         };
         TG_TRY(run_round());
         const int64_t Mr = (int64_t)hs.nodes;
+        if (slot_base + Mr > 0x7fffffffLL) return TG_ERR_BAD_ARG;
         if (slot_base + Mr > nd.cap) {
-            TG_TRY(nodes_reserve(nd, slot_base + Mr, st));
-            dfree(exh, st);
-            exh_cap = std::max<int64_t>(Mr, 1);
-            TG_TRY(dalloc(&exh, exh_cap, st));
+            TG_TRY(nodes_reserve(slots, nd, slot_base + Mr, st));
             TG_CUDA(cudaMemsetAsync(&sum->n_exh, 0, sizeof(unsigned long long), st));
             TG_CUDA(cudaMemsetAsync(&sum->bad, 0, sizeof(int) * (2 + DEPTH_CAP + 1), st));
             TG_TRY(run_round());
@@ -1655,7 +1751,7 @@ tg_status build_tree(tg_tree_s *T, const double *pos, const double *m, const dou
         nd.count = slot_base + Mr;
         if (Mr > 0) {
             // the last round's centres (nothing re-keys or grows the slots after it) run beside the
-            // node numbering, which does not read them; k_write_nodes joins them
+            // node numbering, which does not read them; k_write joins them
             cudaStream_t cs = st;
             if (hs.n_exh == 0) {
                 TG_TRY(build_side(side));
@@ -1663,47 +1759,52 @@ tg_status build_tree(tg_tree_s *T, const double *pos, const double *m, const dou
                 TG_CUDA(cudaStreamWaitEvent(side->s, side->fork, 0));
                 cs = side->s;
             }
-            { k_node_centers<<<div_up(Mr, CENTER_BLOCK), CENTER_BLOCK, 0, cs>>>(v, nd, slot_base, Mr, keys_sorted); tg::note_launch(); }
+            { k_node_centers<<<div_up(Mr, CENTER_BLOCK), CENTER_BLOCK, 0, cs>>>(v, nd, slot_base, Mr, keys); tg::note_launch(); }
             if (cs != st) {
                 TG_CUDA(cudaEventRecord(side->join, cs));
                 centers_forked = true;
             }
         }
         n_exh = (int)hs.n_exh;
-        dfree(L, st); dfree(cnt, st); dfree(nstart, st);
         if (n_exh == 0) {
             summary_final = true;
             break;
         }
         if (round < MORTON_MAX_ROUNDS) {
-            segs_free(sg, st);
-            TG_TRY(segs_alloc(sg, n_exh, st));
-            { k_make_segs<<<LAUNCH(n_exh)>>>(exh, n_exh, nd, sg); tg::note_launch(); }
+            // the next round's segments and lists replace this round's
+            DevArray<unsigned char> next_mem(st);
+            Segs next;
+            int64_t *next_exh = nullptr;
+            TG_CUDA(carve(next_mem, [&](Carve &c) {
+                segs_lay(c, next, n_exh);
+                c.take(next_exh, exh_cap);
+                c.take(root_first, n_exh);
+            }));
+            { k_make_segs<<<LAUNCH(n_exh)>>>(exh, n_exh, nd, next); tg::note_launch(); }
             TG_CUDA(cudaGetLastError());
+            round_mem.swap(next_mem);
+            sg = next;
+            exh = next_exh;
         }
     }
-    if (!centers_forked) segs_free(sg, st);  // else k_node_centers still reads them: freed after the join
-    dfree(root_first, st);
 
     // 5. buckets for runs still exhausted after three re-keys
     int n_bucket = (n_exh > 0) ? n_exh : 0;
     if (n_bucket > 0) {
         has_coincident = 1;
-        int64_t *nchain = nullptr, *choff = nullptr, *chtot = nullptr;
-        TG_TRY(dalloc(&nchain, n_bucket, st));
-        TG_TRY(dalloc(&choff, n_bucket, st));
-        TG_TRY(dalloc(&chtot, 1, st));
-        { k_bucket_counts<<<LAUNCH(n_bucket)>>>(exh, n_bucket, nd.lo, nd.hi, nchain); tg::note_launch(); }
-        TG_TRY(exclusive_scan_i64(nchain, choff, n_bucket, chtot, st));
-        int64_t nch = 0;
-        TG_CUDA(cudaMemcpyAsync(&nch, chtot, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+        DevArray<int64_t> nchain(st), choff(st);
+        TG_CUDA(nchain.alloc(n_bucket));
+        TG_CUDA(choff.alloc(n_bucket + 1));
+        { k_bucket_counts<<<LAUNCH(n_bucket)>>>(exh, n_bucket, nd.lo, nd.hi, nchain.p); tg::note_launch(); }
+        TG_TRY(exclusive_scan_i64(nchain.p, choff.p, n_bucket, choff.p + n_bucket, st));
+        TG_CUDA(cudaMemcpyAsync(host, choff.p + n_bucket, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
         TG_CUDA(cudaStreamSynchronize(st));
+        const int64_t nch = *(const int64_t *)host;
         int64_t slot_base = nd.count;
-        TG_TRY(nodes_reserve(nd, slot_base + nch, st));
-        { k_bucket<<<LAUNCH(n_bucket)>>>(exh, n_bucket, choff, slot_base, nd, p_parent, p_next); tg::note_launch(); }
+        TG_TRY(nodes_reserve(slots, nd, slot_base + nch, st));
+        { k_bucket<<<LAUNCH(n_bucket)>>>(exh, n_bucket, choff.p, slot_base, nd, p_parent, p_next); tg::note_launch(); }
         TG_CUDA(cudaGetLastError());
         nd.count = slot_base + nch;
-        dfree(nchain, st); dfree(choff, st); dfree(chtot, st);
     }
     T->has_coincident = has_coincident;
 
@@ -1711,99 +1812,95 @@ tg_status build_tree(tg_tree_s *T, const double *pos, const double *m, const dou
     if (!summary_final) {  // buckets were made after the last summary: validate every slot again
         TG_CUDA(cudaMemsetAsync(sum, 0, sizeof(BuildSummary), st));
         { k_summarize_slots<<<LAUNCH(std::max<int64_t>(nd.count, N))>>>(nd, nd.count, nullptr, p_parent, p_next, N,
-                                                                      sum); tg::note_launch(); }
+                                                                      sum, nonfinite); tg::note_launch(); }
         TG_CUDA(cudaGetLastError());
-        TG_CUDA(cudaMemcpyAsync(&hs, sum, sizeof(BuildSummary), cudaMemcpyDeviceToHost, st));
-        TG_CUDA(cudaStreamSynchronize(st));
+        TG_TRY(read_summary());
     }
     if (hs.bad) {
         if (nonfinite_seen) return TG_ERR_NONFINITE;
         set_last_error_msg("internal error: octree build produced an invalid node reference");
         return TG_ERR_CUDA;
     }
-    const int64_t M = nd.count;
+    const int64_t M = nd.count, NE = N + M;
     T->mtot = M;
     uint64_t *nkeys = nullptr;
     uint32_t *nvals = nullptr;
-    int64_t *root_slot = nullptr, *final_of_slot = nullptr, *sys_node_off = nullptr;
-    int *nonroot = nullptr;
-    TG_TRY(dalloc(&nkeys, M, st));
-    TG_TRY(dalloc(&nvals, M, st));
-    TG_TRY(dalloc(&root_slot, nsys, st));
-    TG_TRY(dalloc(&final_of_slot, M, st));
-    TG_TRY(dalloc(&sys_node_off, nsys + 1, st));
-    TG_TRY(dalloc(&nonroot, 1, st));
-    TG_CUDA(cudaMemsetAsync(nonroot, 0, sizeof(int), st));
+    int64_t *root_slot = nullptr, *final_of_slot = nullptr, *sys_node_off = nullptr, *ncnt = nullptr;
+    unsigned long long *req = nullptr;
+    DevArray<unsigned char> numbering(st), arrays(st);
+    TG_CUDA(carve(numbering, [&](Carve &c) {
+        c.take(nkeys, M);
+        c.take(nvals, M);
+        c.take(root_slot, nsys);
+        c.take(final_of_slot, M);
+        if (nsys > 1) {
+            c.take(sys_node_off, nsys + 1);
+            c.take(ncnt, nsys);
+        }
+        if (n_bucket > 0) c.take(req, nsys);
+    }));
+    TG_CUDA(carve(arrays, [&](Carve &c) {
+        c.take(T->coord, 3 * NE);
+        c.take(T->mass, NE);
+        c.take(T->size, NE);
+        c.take(T->delta, NE);
+        c.take(T->soft, NE);
+        c.take(T->first, NE);
+        c.take(T->next, NE);
+        c.take(T->parent, NE);
+        c.take(T->node_range, M);
+        c.take(T->cell_center, 3 * M);
+    }));
+    T->arrays = arrays.p;  // the tree's from here on
+    arrays.p = nullptr;
     const int compact = n_bucket == 0;
     const int key_bits = sysbits + nb.lb + nb.db + (compact ? 3 : nb.lb);
     const int sort_bits = key_bits < 64 ? key_bits + 1 : 64;
     const uint64_t root_key = key_bits < 64 ? (1ull << key_bits) : ~0ull;
-    { k_number_keys<<<LAUNCH(M)>>>(nd, M, sys_off, nb, root_key, compact, nkeys, nvals, root_slot, nonroot); tg::note_launch(); }
+    { k_number_keys<<<LAUNCH(M)>>>(nd, M, sys_off, nb, root_key, compact, nkeys, nvals, root_slot); tg::note_launch(); }
     TG_CUDA(cudaGetLastError());
-    TG_TRY(radix_sort_pairs(nkeys, nvals, M, sort_bits, st, T->sort_err));
+    TG_TRY(radix_sort_pairs(nkeys, nvals, M, sort_bits, st, T->sort_err, true));
     // per-system node offsets (roots first within each system's block), on the device; the host
     // copy is read with the final synchronisation
     if (nsys == 1) {
-        { k_single_sys_node_off<<<1, 1, 0, st>>>(sys_node_off, M); tg::note_launch(); }
         T->sys_node_off = {0, M};
     } else {
-        int64_t *ncnt = nullptr;
-        TG_TRY(dalloc(&ncnt, nsys, st));
         TG_CUDA(cudaMemsetAsync(ncnt, 0, sizeof(int64_t) * nsys, st));
         { k_sys_node_counts<<<LAUNCH(M)>>>(nd.sys, M, ncnt); tg::note_launch(); }
         TG_CUDA(cudaGetLastError());
         TG_TRY(exclusive_scan_i64(ncnt, sys_node_off, nsys, sys_node_off + nsys, st));
-        dfree(ncnt, st);
         T->sys_node_off.assign(nsys + 1, 0);
     }
     { k_final_index<<<LAUNCH(std::max<int64_t>(M, nsys))>>>(nvals, M, nd.sys, N, sys_node_off, final_of_slot, root_slot,
                                                          nsys, T->sort_err); tg::note_launch(); }
     TG_CUDA(cudaGetLastError());
     // capacity (NumNodes) per system: bucket reservations, read with the final synchronisation
-    unsigned long long *req = nullptr;
     if (n_bucket > 0) {
-        TG_TRY(dalloc(&req, nsys, st));
         TG_CUDA(cudaMemsetAsync(req, 0, sizeof(unsigned long long) * nsys, st));
         { k_bucket_requirement<<<LAUNCH(n_bucket)>>>(exh, n_bucket, nd, sys_off, nb, nkeys, M, N, req); tg::note_launch(); }
         TG_CUDA(cudaGetLastError());
     }
-    dfree(exh, st);
 
     // 7. final arrays; every node also goes into the list of its depth
-    const int64_t NE = N + M;
-    TG_TRY(dalloc(&T->coord, 3 * NE, st));
-    TG_TRY(dalloc(&T->mass, NE, st));
-    TG_TRY(dalloc(&T->size, NE, st));
-    TG_TRY(dalloc(&T->delta, NE, st));
-    TG_TRY(dalloc(&T->soft, NE, st));
-    TG_TRY(dalloc(&T->first, NE, st));
-    TG_TRY(dalloc(&T->next, NE, st));
-    TG_TRY(dalloc(&T->parent, NE, st));
-    TG_TRY(dalloc(&T->node_range, M, st));
-    TG_TRY(dalloc(&T->cell_center, 3 * M, st));
-    int *lvl = nullptr;  // section offsets, then cursors, of the depth lists
-    int32_t *lvl_list = nullptr;
-    int8_t *fdepth = nullptr;
-    TG_TRY(dalloc(&lvl, 2 * (DEPTH_CAP + 1), st));
-    TG_TRY(dalloc(&lvl_list, M, st));
-    TG_TRY(dalloc(&fdepth, M, st));
-    { k_level_offsets<<<1, 32, 0, st>>>(sum, lvl, lvl + DEPTH_CAP + 1); tg::note_launch(); }
-    if (centers_forked) {
-        TG_CUDA(cudaStreamWaitEvent(st, side->join, 0));
-        segs_free(sg, st);
+    DevArray<int32_t> lvl_mem(st);
+    DevArray<int8_t> depth_mem(st);
+    TG_CUDA(lvl_mem.alloc(M));
+    TG_CUDA(depth_mem.alloc(M));
+    int32_t *lvl_list = lvl_mem.p;
+    int8_t *fdepth = depth_mem.p;
+    T->lvl_off.assign(DEPTH_CAP + 2, 0);
+    LevelOffsets lo;
+    for (int d = 0; d <= DEPTH_CAP; d++) {
+        lo.at[d] = T->lvl_off[d];
+        T->lvl_off[d + 1] = T->lvl_off[d] + hs.depth_hist[d];
     }
-    { k_write_nodes<<<LAUNCH(M)>>>(nd, M, final_of_slot, T->coord, T->size, T->mass, T->soft, T->delta, T->first,
-                                 T->next, T->parent, T->node_range, T->cell_center, N, lvl, lvl + DEPTH_CAP + 1,
-                                 lvl_list, fdepth); tg::note_launch(); }
-    { k_write_particles<<<LAUNCH(N)>>>(N, p_parent, p_next, final_of_slot, pc, pm, ps, T->coord, T->mass, T->soft,
-                                     T->first, T->next, T->parent, T->size, T->delta); tg::note_launch(); }
-    dfree(pc, st); dfree(pm, st); dfree(ps, st);
-    TG_CUDA(cudaMemsetAsync(&sum->bad, 0, sizeof(int), st));
-    { k_validate_links<<<LAUNCH(NE)>>>(NE, T->first, T->next, T->parent, &sum->bad); tg::note_launch(); }
+    if (centers_forked) TG_CUDA(cudaStreamWaitEvent(st, side->join, 0));
+    FinalArrays fa{T->coord, T->mass, T->soft, T->size, T->delta, T->first, T->next, T->parent, T->node_range,
+                   T->cell_center};
+    const int node_blocks = div_up(M, 256);
+    { k_write<<<node_blocks + div_up(N, 256), 256, 0, st>>>(nd, M, N, node_blocks, final_of_slot, fa, lo, lvl_cursor,
+                                                            lvl_list, fdepth, p_parent, p_next, pc, pm, ps, &sum->bad); tg::note_launch(); }
     TG_CUDA(cudaGetLastError());
-    nodes_free(nd, st);
-    dfree(p_parent, st); dfree(p_next, st); dfree(nkeys, st); dfree(nvals, st); dfree(root_slot, st);
-    dfree(final_of_slot, st); dfree(nonroot, st); dfree(keys, st); dfree(perm, st);
 
     // 8. the one closing synchronisation, ahead of the moment pass (nothing the host needs comes from
     // it): link check, per-system node offsets, bucket reservations. The moment pass is then enqueued
@@ -1814,19 +1911,17 @@ tg_status build_tree(tg_tree_s *T, const double *pos, const double *m, const dou
         TG_CUDA(pool_event(&T->ev_built, false));
     }
     TG_CUDA(cudaEventRecord(T->ev_topo, st));
-    int links_bad = 0, sort_bad = 0;
     std::vector<unsigned long long> rq(nsys, 0);
-    TG_CUDA(cudaMemcpyAsync(&sort_bad, T->sort_err, sizeof(int), cudaMemcpyDeviceToHost, st));
-    TG_CUDA(cudaMemcpyAsync(&links_bad, &sum->bad, sizeof(int), cudaMemcpyDeviceToHost, st));
+    int *flags = (int *)host;  // the sorts' word, the links'
+    TG_CUDA(cudaMemcpyAsync(flags, T->sort_err, sizeof(int), cudaMemcpyDeviceToHost, st));
+    TG_CUDA(cudaMemcpyAsync(flags + 1, &sum->bad, sizeof(int), cudaMemcpyDeviceToHost, st));
     if (nsys > 1)
         TG_CUDA(cudaMemcpyAsync(T->sys_node_off.data(), sys_node_off, sizeof(int64_t) * (nsys + 1),
                                 cudaMemcpyDeviceToHost, st));
     if (req) TG_CUDA(cudaMemcpyAsync(rq.data(), req, sizeof(unsigned long long) * nsys, cudaMemcpyDeviceToHost, st));
-    dfree(req, st); dfree(sum, st); dfree(sys_node_off, st);
-    dfree(sys_off, st); dfree(mn, st); dfree(mx, st); dfree(center, st); dfree(size, st);
     TG_CUDA(cudaStreamSynchronize(st));
+    const int sort_bad = flags[0], links_bad = flags[1];
     if (nonfinite_seen || sort_bad || links_bad) {
-        dfree(lvl, st); dfree(lvl_list, st); dfree(fdepth, st);
         if (nonfinite_seen) return TG_ERR_NONFINITE;
         if (sort_bad) {
             set_last_error_msg("radix sort: a tile's look-back did not complete within its bound");
@@ -1860,21 +1955,24 @@ tg_status build_tree(tg_tree_s *T, const double *pos, const double *m, const dou
         if (compute_moments) a.quad32 = T->quad32;  // every node's is written by the pass below
         else TG_CUDA(cudaMemsetAsync(T->quad32, 0, sizeof(float4) * 2 * M, st));
     }
-    T->lvl_off.assign(DEPTH_CAP + 2, 0);
-    for (int d = 0; d <= DEPTH_CAP; d++) T->lvl_off[d + 1] = T->lvl_off[d] + hs.depth_hist[d];
+    DevArray<unsigned char> moments(st);
     if (compute_moments) {
         const int *off = T->lvl_off.data();
         // every node's children once, in summation order
+        const int ndeep = hs.depth_hist[DEPTH_CAP];
         int32_t *kids = nullptr;
         int8_t *nk = nullptr;
-        TG_TRY(dalloc(&kids, 8 * M, st));
-        TG_TRY(dalloc(&nk, M, st));
+        TG_CUDA(carve(moments, [&](Carve &c) {
+            c.take(kids, 8 * M);
+            c.take(nk, M);
+            c.take(a.acc, 3 * M);
+            if (ndeep > 0) {
+                c.take(a.nchild, M);
+                c.take(a.arrived, M);
+            }
+        }));
         { k_kids<<<LAUNCH(M)>>>(N, M, T->first, T->next, kids, nk); tg::note_launch(); }
-        TG_TRY(dalloc(&a.acc, 3 * M, st));
-        const int ndeep = hs.depth_hist[DEPTH_CAP];
         if (ndeep > 0) {
-            TG_TRY(dalloc(&a.nchild, M, st));
-            TG_TRY(dalloc(&a.arrived, M, st));
             TG_CUDA(cudaMemsetAsync(a.nchild, 0, sizeof(int) * M, st));
             TG_CUDA(cudaMemsetAsync(a.arrived, 0, sizeof(int) * M, st));
             { k_count_node_children<<<LAUNCH(M)>>>(N, M, T->parent, a.nchild); tg::note_launch(); }
@@ -1899,19 +1997,16 @@ tg_status build_tree(tg_tree_s *T, const double *pos, const double *m, const dou
             tg::note_launch();
         }
         TG_CUDA(cudaGetLastError());
-        dfree(kids, st); dfree(nk, st);
-        dfree(a.acc, st); dfree(a.nchild, st); dfree(a.arrived, st);
     } else {
         { k_fold_only<<<LAUNCH(M)>>>(a); tg::note_launch(); }
         TG_CUDA(cudaGetLastError());
     }
 
-    dfree(lvl, st);
     if (quadrupole && compute_moments) {  // kept for the FP64 quadrupole pass
         T->lvl_list = lvl_list;
         T->fdepth = fdepth;
-    } else {
-        dfree(lvl_list, st); dfree(fdepth, st);
+        lvl_mem.p = nullptr;
+        depth_mem.p = nullptr;
     }
     TG_CUDA(cudaEventRecord(T->ev_built, st));
     return TG_OK;

@@ -113,8 +113,7 @@ void destroy(tg_tree_s *t) {
     auto f = [&](void *p) {
         if (p) cudaFreeAsync(p, st);
     };
-    f(t->coord); f(t->mass); f(t->size); f(t->delta); f(t->soft); f(t->quad);
-    f(t->first); f(t->next); f(t->walk_idx); f(t->parent); f(t->node_range); f(t->cell_center);
+    f(t->arrays); f(t->quad); f(t->walk_idx);
     free_arena(t->arena32, st);
     free_arena(t->arena64, st);
     f(t->groups); f(t->group_root); f(t->group_node); f(t->gstats); f(t->gerr); f(t->sort_err); f(t->vel); f(t->vdisp); f(t->quad32); f(t->lvl_list); f(t->fdepth); f(t->own32);

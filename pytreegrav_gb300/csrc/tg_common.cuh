@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <utility>
 
 #include "../../include/pytreegrav_gb300.h"
 
@@ -243,7 +244,10 @@ tg_status exclusive_scan_i32(const int32_t *in, int32_t *out, int64_t n, cudaStr
 // look-back that does not complete within its bound sets *err (a device int the caller owns and
 // reads back with its results; nonzero: the sort failed) and leaves keys[i] = i and vals[i] = i, a
 // sorted, well-formed result, so every later kernel stays in bounds.
-tg_status radix_sort_pairs(uint64_t *keys, uint32_t *vals, int64_t n, int bits, cudaStream_t s, int *err);
+// caller_falls_back: the pairs are left as the passes left them on a failure (some places never written), and the
+// caller's next kernel takes the identity instead when *err is set (then one launch fewer).
+tg_status radix_sort_pairs(uint64_t *keys, uint32_t *vals, int64_t n, int bits, cudaStream_t s, int *err,
+                           bool caller_falls_back = false);
 
 // Bounds of the library's bounded device loops, overridable (tg_set_loop_limits in the measurement
 // header) so that tests can make each one run out; 0 selects the built-in bound. Process-wide.
@@ -303,8 +307,14 @@ struct DevArray {
     T *p = nullptr;
     cudaStream_t st = nullptr;
     explicit DevArray(cudaStream_t s) : st(s) {}
-    ~DevArray() {
+    ~DevArray() { reset(); }
+    void reset() {
         if (p) cudaFreeAsync(p, st);
+        p = nullptr;
+    }
+    void swap(DevArray &o) {
+        std::swap(p, o.p);
+        std::swap(st, o.st);
     }
     DevArray(const DevArray &) = delete;
     DevArray &operator=(const DevArray &) = delete;

@@ -434,27 +434,45 @@ constexpr unsigned long long ST_TAGS = 63ull << 56, ST_VAL = (1ull << 56) - 1;
 constexpr long long SPIN_LIMIT = 1ll << 22;
 constexpr int LB = TG_OS_LB;  // predecessors read per look-back round trip
 
-__global__ void __launch_bounds__(256) k_sort_hist_all(const uint64_t *keys, int64_t n, int npass, int *hist) {
+// Every pass's digit histogram from one read of the keys; the last block to finish scans each pass's 256 counts
+// in place (exclusive), which took a launch of its own.
+constexpr int HIST_THREADS = 256;
+__global__ void __launch_bounds__(HIST_THREADS) k_sort_hist(const uint64_t *keys, int64_t n, int npass, int *hist,
+                                                            int *done) {
     __shared__ int h[MAX_PASSES * RS_BINS];
-    for (int i = threadIdx.x; i < npass * RS_BINS; i += blockDim.x) h[i] = 0;
+    __shared__ int tot[MAX_PASSES * RS_BINS / 32];
+    __shared__ bool last;
+    for (int i = threadIdx.x; i < npass * RS_BINS; i += HIST_THREADS) h[i] = 0;
     __syncthreads();
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    for (int64_t i = (int64_t)blockIdx.x * HIST_THREADS + threadIdx.x; i < n; i += (int64_t)gridDim.x * HIST_THREADS) {
         const uint64_t k = keys[i];
         for (int p = 0; p < npass; p++) atomicAdd(&h[p * RS_BINS + (int)((k >> (8 * p)) & (RS_BINS - 1))], 1);
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < npass * RS_BINS; i += blockDim.x)
+    for (int i = threadIdx.x; i < npass * RS_BINS; i += HIST_THREADS)
         if (h[i]) atomicAdd(&hist[i], h[i]);
-}
-
-// Exclusive scan of each pass's 256 digit counts, in place. One block of 256 threads.
-__global__ void k_sort_digit_offsets(int *hist, int npass) {
-    __shared__ int tot;
-    for (int p = 0; p < npass; p++) {
-        int v = hist[p * RS_BINS + threadIdx.x];
-        int ex = block_exclusive_scan(v, &tot);
-        hist[p * RS_BINS + threadIdx.x] = ex;
-        __syncthreads();
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(done, 1) == (int)gridDim.x - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    const int lane = lane_id(), w = threadIdx.x >> 5;
+    int v[MAX_PASSES], inc[MAX_PASSES];
+#pragma unroll
+    for (int p = 0; p < MAX_PASSES; p++) {
+        if (p >= npass) break;
+        v[p] = __ldcg(&hist[p * RS_BINS + threadIdx.x]);
+        inc[p] = warp_inclusive_scan(v[p]);
+        if (lane == 31) tot[p * (RS_BINS / 32) + w] = inc[p];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int p = 0; p < MAX_PASSES; p++) {
+        if (p >= npass) break;
+        int below = 0;
+        for (int k = 0; k < w; k++) below += tot[p * (RS_BINS / 32) + k];
+        hist[p * RS_BINS + threadIdx.x] = below + inc[p] - v[p];
     }
 }
 
@@ -557,6 +575,7 @@ __global__ void __launch_bounds__(RS_THREADS, 4) k_onesweep(const uint64_t *keys
         const uint64_t k = skey[i];
         const int d = (int)((k >> shift) & (RS_BINS - 1));
         const int pos = prefix[d] + (i - lstart[d]);
+        if ((unsigned)pos >= (unsigned)n) continue;  // only after a look-back that gave up (garbage keys)
         keys_out[pos] = k;
         vals_out[pos] = sval[i];
     }
@@ -577,45 +596,46 @@ __global__ void k_sort_fallback(uint64_t *keys, uint32_t *vals, int64_t n, const
 
 long long scan_spins() { return loop_limits().sort_spin > 0 ? loop_limits().sort_spin : SPIN_LIMIT; }
 
-tg_status radix_sort_pairs(uint64_t *keys, uint32_t *vals, int64_t n, int bits, cudaStream_t s, int *err) {
+tg_status radix_sort_pairs(uint64_t *keys, uint32_t *vals, int64_t n, int bits, cudaStream_t s, int *err,
+                           bool caller_falls_back) {
     if (n <= 1 || bits <= 0) return TG_OK;
     if (n > (int64_t)0x7fffffff || !err) return TG_ERR_BAD_ARG;
     const long long spin_limit = loop_limits().sort_spin > 0 ? loop_limits().sort_spin : SPIN_LIMIT;
     const int ntiles = div_up(n, OS_TILE);
     const int npass = std::min((bits + 7) / 8, MAX_PASSES);
-    uint64_t *k2 = nullptr;
-    uint32_t *v2 = nullptr;
-    unsigned char *scr = nullptr;
+    // one allocation: status words, histograms, tile counters, the histogram's and the error word (zeroed), then
+    // the other halves of the key and value buffers
     const size_t st_bytes = sizeof(unsigned long long) * (size_t)ntiles * RS_BINS;
     const size_t hist_bytes = sizeof(int) * MAX_PASSES * RS_BINS;
-    TG_CUDA(tg::dev_malloc((void **)&k2, sizeof(uint64_t) * n, s));
-    TG_CUDA(tg::dev_malloc((void **)&v2, sizeof(uint32_t) * n, s));
-    TG_CUDA(tg::dev_malloc((void **)&scr, st_bytes + hist_bytes + sizeof(int) * (MAX_PASSES + 1), s));
+    const size_t head = (st_bytes + hist_bytes + sizeof(int) * (MAX_PASSES + 2) + 255) / 256 * 256;
+    const size_t key_bytes = (sizeof(uint64_t) * (size_t)n + 255) / 256 * 256;
+    unsigned char *scr = nullptr;
+    TG_CUDA(tg::dev_malloc((void **)&scr, head + key_bytes + sizeof(uint32_t) * (size_t)n, s));
     unsigned long long *status = (unsigned long long *)scr;
     int *hist = (int *)(scr + st_bytes);
     int *counters = hist + MAX_PASSES * RS_BINS;
-    int *local_err = counters + MAX_PASSES;
-    TG_CUDA(cudaMemsetAsync(scr, 0, st_bytes + hist_bytes + sizeof(int) * (MAX_PASSES + 1), s));
-    const int hblocks = (int)std::min<int64_t>(div_up(n, 256 * 16), (int64_t)num_sms() * 4);
-    { k_sort_hist_all<<<hblocks, 256, 0, s>>>(keys, n, npass, hist); tg::note_launch(); }
-    { k_sort_digit_offsets<<<1, RS_BINS, 0, s>>>(hist, npass); tg::note_launch(); }
+    int *done = counters + MAX_PASSES;
+    int *local_err = caller_falls_back ? err : done + 1;
+    uint64_t *k2 = (uint64_t *)(scr + head);
+    uint32_t *v2 = (uint32_t *)(scr + head + key_bytes);
+    TG_CUDA(cudaMemsetAsync(scr, 0, head, s));
+    const int hblocks = (int)std::min<int64_t>(div_up(n, HIST_THREADS * 4), (int64_t)num_sms() * 4);
+    { k_sort_hist<<<hblocks, HIST_THREADS, 0, s>>>(keys, n, npass, hist, done); tg::note_launch(); }
     uint64_t *kin = keys, *kout = k2;
     uint32_t *vin = vals, *vout = v2;
     for (int p = 0; p < npass; p++) {
         { k_onesweep<<<ntiles, RS_THREADS, 0, s>>>(kin, vin, n, 8 * p, p, hist + p * RS_BINS, status, counters + p, kout,
                                                    vout, local_err, spin_limit); tg::note_launch(); }
-        TG_CUDA(cudaGetLastError());
         uint64_t *tk = kin; kin = kout; kout = tk;
         uint32_t *tv = vin; vin = vout; vout = tv;
     }
+    TG_CUDA(cudaGetLastError());
     if (kin != keys) {
         TG_CUDA(cudaMemcpyAsync(keys, kin, sizeof(uint64_t) * n, cudaMemcpyDeviceToDevice, s));
         TG_CUDA(cudaMemcpyAsync(vals, vin, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, s));
     }
-    { k_sort_fallback<<<std::min(div_up(n, 256), 4 * num_sms()), 256, 0, s>>>(keys, vals, n, local_err, err); tg::note_launch(); }
+    if (!caller_falls_back) { k_sort_fallback<<<std::min(div_up(n, 256), 4 * num_sms()), 256, 0, s>>>(keys, vals, n, local_err, err); tg::note_launch(); }
     TG_CUDA(cudaGetLastError());
-    TG_CUDA(cudaFreeAsync(k2, s));
-    TG_CUDA(cudaFreeAsync(v2, s));
     TG_CUDA(cudaFreeAsync(scr, s));
     return TG_OK;
 }

@@ -63,7 +63,9 @@ struct tg_tree_s {
     std::vector<int64_t> sys_capacity;  // host: NumNodes per system (reference capacity rule)
     cudaStream_t stream = nullptr;
 
-    // Octree arrays over the arena: particles [0, ntot), nodes [ntot, ntot + mtot).
+    // Octree arrays over the arena: particles [0, ntot), nodes [ntot, ntot + mtot). coord to cell_center but
+    // quad, quad32 and walk_idx lie in one allocation (arrays).
+    unsigned char *arrays = nullptr;
     double *coord = nullptr;   // 3 per element
     double *mass = nullptr;
     double *size = nullptr;
