@@ -33,7 +33,6 @@ Differences a caller can see, all deliberate:
 import warnings
 
 import numpy as np
-from numpy import zeros
 
 from . import _lib
 from .tree import Octree, bruteforce, morton_order, radial_range
@@ -86,6 +85,13 @@ def _bf_precision(device):
     return "fp32" if device == "cuda" else "fp64"
 
 
+def _softening(h):
+    """Softening lengths as float64, or None for zeros, which the library fills in on the GPU: uploading an array
+    of zeros made here costs the first touch of each of its pages (structure function of 200000 particles 6.64 ms
+    with it, 6.46 without)."""
+    return None if h is None else np.atleast_1d(_f64(h))
+
+
 def _check_tree(tree):
     if not isinstance(tree, Octree):
         raise TypeError("tree must be an Octree built by pytreegrav_gb300.ConstructTree")
@@ -107,9 +113,7 @@ def ConstructTree(pos, m=None, softening=None, quadrupole=False, vel=None, compu
         compute_moments = False
     else:
         m = np.atleast_1d(_f64(m))
-    if softening is None:
-        softening = zeros(len(pos))
-    softening = np.atleast_1d(_f64(softening))
+    softening = _softening(softening)
     # non-finite positions, masses or softenings are found by the library's device-side check
     # (TG_ERR_NONFINITE), which frontend.py:123-125's print-and-raise then reports
     try:
@@ -128,9 +132,7 @@ def _self_field(key, pos, m, softening, G, theta, tree, return_tree, method, qua
     valueTestMethod(method)
     pos = np.atleast_2d(_f64(pos))
     m = np.atleast_1d(_f64(m))
-    if softening is None:
-        softening = np.zeros_like(m)
-    softening = np.atleast_1d(_f64(softening))
+    softening = _softening(softening)
     if method == "adaptive":
         method = "tree" if (tree is not None or len(pos) > parallel_threshold) else "bruteforce"
     if device is not None:
@@ -169,15 +171,11 @@ def _target_field(key, pos_target, pos_source, m_source, softening_target, softe
     if tree is None and (pos_source is None or m_source is None):
         raise ValueError("Must pass either pos_source & m_source or source tree.")
     pos_target = np.atleast_2d(_f64(pos_target))
-    if softening_target is None:
-        softening_target = zeros(len(pos_target))
-    softening_target = np.atleast_1d(_f64(softening_target))
+    softening_target = _softening(softening_target)
     if pos_source is not None:
         pos_source = np.atleast_2d(_f64(pos_source))
         m_source = np.atleast_1d(_f64(m_source))
-        if softening_source is None:
-            softening_source = zeros(len(pos_source))
-        softening_source = np.atleast_1d(_f64(softening_source))
+        softening_source = _softening(softening_source)
     if method == "adaptive":
         if pos_source is None or len(pos_target) * len(pos_source) > 10**6:
             method = "tree"
@@ -261,9 +259,7 @@ class Field:
                  precision="fp32", grouping="blocks", learned=None, error_ratio=None):
         pos = np.atleast_2d(_f64(pos))
         m = np.atleast_1d(_f64(m))
-        if softening is None:
-            softening = np.zeros_like(m)
-        softening = np.atleast_1d(_f64(softening))
+        softening = _softening(softening)
         self.G = G
         self.theta = theta
         self.quadrupole = quadrupole
@@ -293,9 +289,7 @@ class Field:
             return self.tree.fields(order="tree", grouping=self.grouping, learned=self.learned,
                                     error_ratio=self.error_ratio, **kw)
         pos_target = np.atleast_2d(_f64(pos_target))
-        if softening_target is None:
-            softening_target = zeros(len(pos_target))
-        softening_target = np.atleast_1d(_f64(softening_target))
+        softening_target = _softening(softening_target)
         return self.tree.fields(pos_target, softening_target, order="morton", grouping=self.grouping,
                                 learned=self.learned, error_ratio=self.error_ratio, **kw)
 
@@ -432,7 +426,7 @@ def _corr(kind, pos, m, v, rbins, max_bin_size_ratio, theta, tree, boxsize, weig
         rbins = _rbins_of(pos)
     rbins = np.ascontiguousarray(_f64(rbins))
     if tree is None:
-        tree = ConstructTree(pos, _f64(m), zeros(len(pos)), vel=v)
+        tree = ConstructTree(pos, _f64(m), vel=v)
         bs, ws = tree.correlation(kind, None, rbins, max_bin_size_ratio=max_bin_size_ratio, theta=theta,
                                   boxsize=boxsize, weighted_binning=weighted_binning, seed=seed)
     else:

@@ -79,7 +79,7 @@ class Octree:
         pos = _as_f64(pos, (-1, 3))
         n = len(pos)
         m = _as_f64(m, (n,))
-        softening = np.zeros(n) if softening is None else _as_f64(softening, (n,))
+        softening = None if softening is None else _as_f64(softening, (n,))
         offsets = np.ascontiguousarray(offsets, np.int64)
         handle = ctypes.c_void_p()
         rc = L.tg_tree_build_batched(_lib.ptr(pos), _lib.ptr(m), _lib.ptr(softening), _lib.ptr(offsets),
@@ -186,7 +186,7 @@ class Octree:
         else:
             pos = _as_f64(pos, (-1, 3))
             n = len(pos)
-            soft = np.zeros(n) if soft is None else _as_f64(soft, (n,))
+            soft = None if soft is None else _as_f64(soft, (n,))
             pos_p, soft_p = _lib.ptr(pos), _lib.ptr(soft)
         out = np.empty((n, W))
         if n == 0:
@@ -378,7 +378,7 @@ class TargetSet:
         self.tree = tree  # the source tree must outlive the set
         pos = _as_f64(pos, (-1, 3))
         n = len(pos)
-        soft = np.zeros(n) if soft is None else _as_f64(soft, (n,))
+        soft = None if soft is None else _as_f64(soft, (n,))
         self.n = n
         self.group_size = int(group_size)
         self._h = ctypes.c_void_p()
@@ -535,12 +535,12 @@ def bruteforce(pos_t, h_t, pos_s, m_s, h_s, potential=False, accel=False, tidal=
     pos_s = _as_f64(pos_s, (-1, 3))
     ns = len(pos_s)
     m_s = _as_f64(m_s, (ns,))
-    h_s = np.zeros(ns) if h_s is None else _as_f64(h_s, (ns,))
+    h_s = None if h_s is None else _as_f64(h_s, (ns,))
     if mutual:
         pos_t, h_t = pos_s, h_s
     else:
         pos_t = _as_f64(pos_t, (-1, 3))
-        h_t = np.zeros(len(pos_t)) if h_t is None else _as_f64(h_t, (len(pos_t),))
+        h_t = None if h_t is None else _as_f64(h_t, (len(pos_t),))
     nt = len(pos_t)
     W = int(bool(potential)) + 3 * int(bool(accel)) + 9 * int(bool(tidal))
     out = np.empty((nt, W))
