@@ -48,7 +48,10 @@ __device__ __forceinline__ int64_t find_seg(const int64_t *off, int nseg, int64_
 }
 
 // ---------------------------------------------------------------------------------------------
-// Bounding cube (octree.py:539-574): exact min/max through order-preserving integer atomics.
+// Bounding cube (octree.py:539-574): exact min/max through order-preserving integer atomics. A tile that holds
+// parts of several systems (tiles hold 2048 points) took six atomics per particle:
+// 1024 systems of 3900 particles 174 us, now 30. Tiles of BB_SEGS systems or more still do.
+constexpr int BB_SEGS = 8;
 __global__ void __launch_bounds__(BB_THREADS) k_bbox(const double *pos, int64_t n, const int64_t *sys_off, int nsys,
                                                      unsigned long long *mn, unsigned long long *mx) {
     int64_t tile0 = (int64_t)blockIdx.x * BB_THREADS * BB_ITEMS;
@@ -59,43 +62,48 @@ __global__ void __launch_bounds__(BB_THREADS) k_bbox(const double *pos, int64_t 
         s0 = (int)find_seg(sys_off, nsys, tile0);
         s1 = (int)find_seg(sys_off, nsys, tile1);
     }
-    if (s0 == s1) {
-        unsigned long long lo[3] = {~0ull, ~0ull, ~0ull}, hi[3] = {0, 0, 0};
-        for (int it = 0; it < BB_ITEMS; it++) {
-            int64_t i = tile0 + (int64_t)it * BB_THREADS + threadIdx.x;
-            if (i <= tile1) {
+    if (s1 - s0 < BB_SEGS) {  // the tile's part of each system in turn: one reduction and six atomics per system
+        __shared__ unsigned long long slo[3][BB_THREADS / 32], shi[3][BB_THREADS / 32];
+        const int w = threadIdx.x >> 5;
+        for (int s = s0; s <= s1; s++) {
+            const int64_t a = nsys > 1 ? max(tile0, sys_off[s]) : tile0;
+            const int64_t b = nsys > 1 ? min(tile1 + 1, sys_off[s + 1]) : tile1 + 1;
+            unsigned long long lo[3] = {~0ull, ~0ull, ~0ull}, hi[3] = {0, 0, 0};
+            for (int it = 0; it < BB_ITEMS; it++) {
+                const int64_t i = a + (int64_t)it * BB_THREADS + threadIdx.x;
+                if (i < b) {
 #pragma unroll
-                for (int k = 0; k < 3; k++) {
-                    unsigned long long u = dbl_to_ordered(pos[3 * i + k]);
-                    lo[k] = min(lo[k], u);
-                    hi[k] = max(hi[k], u);
+                    for (int k = 0; k < 3; k++) {
+                        unsigned long long u = dbl_to_ordered(pos[3 * i + k]);
+                        lo[k] = min(lo[k], u);
+                        hi[k] = max(hi[k], u);
+                    }
                 }
             }
-        }
 #pragma unroll
-        for (int k = 0; k < 3; k++) {
-            for (int o = 16; o; o >>= 1) {
-                lo[k] = min(lo[k], __shfl_xor_sync(FULL, lo[k], o));
-                hi[k] = max(hi[k], __shfl_xor_sync(FULL, hi[k], o));
-            }
-        }
-        __shared__ unsigned long long slo[3][BB_THREADS / 32], shi[3][BB_THREADS / 32];
-        int w = threadIdx.x >> 5;
-        if (lane_id() == 0)
             for (int k = 0; k < 3; k++) {
-                slo[k][w] = lo[k];
-                shi[k][w] = hi[k];
+                for (int o = 16; o; o >>= 1) {
+                    lo[k] = min(lo[k], __shfl_xor_sync(FULL, lo[k], o));
+                    hi[k] = max(hi[k], __shfl_xor_sync(FULL, hi[k], o));
+                }
             }
-        __syncthreads();
-        if (threadIdx.x < 3) {
-            int k = threadIdx.x;
-            unsigned long long a = ~0ull, b = 0;
-            for (int ww = 0; ww < BB_THREADS / 32; ww++) {
-                a = min(a, slo[k][ww]);
-                b = max(b, shi[k][ww]);
+            if (lane_id() == 0)
+                for (int k = 0; k < 3; k++) {
+                    slo[k][w] = lo[k];
+                    shi[k][w] = hi[k];
+                }
+            __syncthreads();
+            if (threadIdx.x < 3) {
+                int k = threadIdx.x;
+                unsigned long long mlo = ~0ull, mhi = 0;
+                for (int ww = 0; ww < BB_THREADS / 32; ww++) {
+                    mlo = min(mlo, slo[k][ww]);
+                    mhi = max(mhi, shi[k][ww]);
+                }
+                atomicMin(&mn[3 * s + k], mlo);
+                atomicMax(&mx[3 * s + k], mhi);
             }
-            atomicMin(&mn[3 * s0 + k], a);
-            atomicMax(&mx[3 * s0 + k], b);
+            __syncthreads();
         }
     } else {
         for (int it = 0; it < BB_ITEMS; it++) {
@@ -183,8 +191,9 @@ __device__ __forceinline__ uint64_t morton_key(double x, double y, double z, con
     return morton_key(x, y, z, key_cell(c, size));
 }
 
+// cells: the systems' key cells, when there are several.
 __global__ void k_keys(const double *pos, int64_t n, const int64_t *sys_off, int nsys, const double *center,
-                       const double *size, uint64_t *keys, uint64_t *keys_copy, uint32_t *vals) {
+                       const double *size, const KeyCell *cells, uint64_t *keys, uint64_t *keys_copy, uint32_t *vals) {
     __shared__ KeyCell one;  // one system: its cell (with the division) formed once per block
     if (nsys == 1) {
         if (threadIdx.x == 0) one = key_cell(center, size[0]);
@@ -193,7 +202,7 @@ __global__ void k_keys(const double *pos, int64_t n, const int64_t *sys_off, int
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     int s = nsys > 1 ? (int)find_seg(sys_off, nsys, i) : 0;
-    const KeyCell kc = nsys == 1 ? one : key_cell(center + 3 * s, size[s]);
+    const KeyCell kc = nsys == 1 ? one : cells[s];
     uint64_t k = morton_key(pos[3 * i], pos[3 * i + 1], pos[3 * i + 2], kc);
     keys[i] = k;
     if (keys_copy) keys_copy[i] = k;
@@ -209,18 +218,27 @@ __global__ void k_sys_of(const uint32_t *vals, int64_t n, const int64_t *sys_off
 // sort_err set (the sort gave up): the identity permutation, and keys i, so that every later kernel sees
 // sorted keys and valid indices (the build then reports the error). keys_in null: keys_sorted holds the
 // sorted keys already.
+// Infinities and NaNs among the inputs set *nonfinite: every value passes through here once (checking them ahead
+// of the build read them all again: 62 us for 4e6 particles).
+__device__ __forceinline__ bool nonfinite_bits(double x) {  // the all-ones exponent, on the integer units
+    return (~(unsigned long long)__double_as_longlong(x) & 0x7ff0000000000000ull) == 0;
+}
 __global__ void k_gather(const uint32_t *perm, int64_t n, const double *pos, const double *m, const double *h,
                          const uint64_t *keys_in, double *coord, double *mass, double *soft, uint64_t *keys_sorted,
-                         int64_t *walk_idx, const int *sort_err) {
+                         int64_t *walk_idx, const int *sort_err, int *nonfinite) {
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const bool bad = *sort_err != 0;
     int64_t o = bad ? i : (int64_t)perm[i];
-    coord[3 * i] = pos[3 * o];
-    coord[3 * i + 1] = pos[3 * o + 1];
-    coord[3 * i + 2] = pos[3 * o + 2];
-    mass[i] = m ? m[o] : 0.0;
-    soft[i] = h ? h[o] : 0.0;
+    const double x = pos[3 * o], y = pos[3 * o + 1], z = pos[3 * o + 2];
+    const double mi = m ? m[o] : 0.0, hi = h ? h[o] : 0.0;
+    coord[3 * i] = x;
+    coord[3 * i + 1] = y;
+    coord[3 * i + 2] = z;
+    mass[i] = mi;
+    soft[i] = hi;
+    if (nonfinite_bits(x) || nonfinite_bits(y) || nonfinite_bits(z) || nonfinite_bits(mi) || nonfinite_bits(hi))
+        atomicOr(nonfinite, 1);
     if (bad) keys_sorted[i] = (uint64_t)i;
     else if (keys_in) keys_sorted[i] = keys_in[o];
     walk_idx[i] = o;
@@ -727,11 +745,6 @@ __global__ void k_summarize_slots(Nodes nd, int64_t M_base, const unsigned long 
         if (hist[b]) atomicAdd(&sum->depth_hist[b], hist[b]);
 }
 
-// Node slots per system -> node offsets (exclusive scan done by the caller).
-__global__ void k_sys_node_counts(const int32_t *nd_sys, int64_t M, int64_t *cnt) {
-    int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c < M) atomicAdd((unsigned long long *)&cnt[nd_sys[c]], 1ull);
-}
 // ---------------------------------------------------------------------------------------------
 // Numbering.
 struct NumberingBits {
@@ -768,10 +781,13 @@ __global__ void k_number_keys(Nodes nd, int64_t count, const int64_t *sys_off, N
 }
 
 // sort_err set (the numbering sort gave up): every slot keeps its own index, a bijection onto the node
-// range, so the arrays written from it stay in bounds. sys_node_off null: one system, offset 0.
-__global__ void k_final_index(const uint32_t *vals, int64_t count, const int32_t *nd_sys, int64_t ntot,
-                              const int64_t *sys_node_off, int64_t *final_of_slot, const int64_t *root_slot_of_sys,
-                              int nsys, const int *sort_err) {
+// range, so the arrays written from it stay in bounds. sys_node_off (null for one system) receives the systems'
+// node offsets: the roots sort last, so system q's other nodes start where its keys do (the system is the keys'
+// top part, from sys_shift), behind q roots. (Counting them by an atomic per node took 287 us for 1024 systems of
+// 3900 particles.)
+__global__ void k_final_index(const uint64_t *sorted_keys, const uint32_t *vals, int64_t count, const int32_t *nd_sys,
+                              int64_t ntot, int sys_shift, int64_t *sys_node_off, int64_t *final_of_slot,
+                              const int64_t *root_slot_of_sys, int nsys, const int *sort_err) {
     int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (*sort_err) {
         if (q < count) final_of_slot[q] = ntot + q;
@@ -782,7 +798,21 @@ __global__ void k_final_index(const uint32_t *vals, int64_t count, const int32_t
         int s = nd_sys[c];
         if (q < count - nsys) final_of_slot[c] = ntot + q + s + 1;
     }
-    if (q < nsys) final_of_slot[root_slot_of_sys[q]] = ntot + (sys_node_off ? sys_node_off[q] : 0);
+    if (q < nsys) {
+        int64_t off = 0;
+        if (sys_node_off) {
+            int64_t a = 0, z = count - nsys;
+            while (a < z) {
+                const int64_t mid = (a + z) >> 1;
+                if ((int64_t)(sorted_keys[mid] >> sys_shift) < q) a = mid + 1;
+                else z = mid;
+            }
+            off = a + q;
+            sys_node_off[q] = off;
+            if (q == 0) sys_node_off[nsys] = count;
+        }
+        final_of_slot[root_slot_of_sys[q]] = ntot + off;
+    }
 }
 
 __device__ __forceinline__ int64_t resolve(int64_t ref, const int64_t *final_of_slot) {
@@ -1517,13 +1547,15 @@ static int64_t reference_capacity(int64_t npart, int64_t required) {
     return cap;
 }
 
-// The bounding cubes' centres and sizes, and round 0's segments: one per system. One system's offsets (0, n) are
-// written here too.
+// The bounding cubes' centres and sizes, the systems' key cells (formed by every particle's thread, their FP64
+// divisions were two thirds of k_keys: 123 us for 1024 systems of 3900 particles, now 52 us), and round 0's
+// segments: one per system. One system's offsets (0, n) are written here too.
 __global__ void k_root_segs(const unsigned long long *mn, const unsigned long long *mx, int64_t *sys_off, int64_t n,
-                            Segs g) {
+                            KeyCell *cells, Segs g) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= g.n) return;
     bounding_cube(mn, mx, s, g.center, g.size);
+    if (g.n > 1) cells[s] = key_cell(g.center + 3 * s, g.size[s]);
     const int64_t lo = g.n == 1 ? 0 : sys_off[s], hi = g.n == 1 ? n : sys_off[s + 1];
     if (g.n == 1) {
         sys_off[0] = lo;
@@ -1541,15 +1573,14 @@ __global__ void k_root_segs(const unsigned long long *mn, const unsigned long lo
 
 #define LAUNCH(n) div_up((n), 256), 256, 0, st
 
-// Build the whole arena. pos/m/h are device pointers (m/h may be null). m_h_ready (may be null):
-// an event after which m and h may be read; the build waits for it only where it first reads them
-// (the gather into Morton order), so their upload overlaps the bounding cube, keys and sort.
+// Build the whole arena. pos is a device pointer; stage_mh gives the device pointers of the masses and
+// softenings (null: none) and the event (null: none) after which they may be read. It is called once the
+// bounding cube, keys and sort are queued, so that their upload overlaps them.
 // The temporaries whose sizes are known up front are one allocation, as are those that need the node
 // count, and the tree's own arrays: a build made ~50 allocations and as many frees, whose host time a small
 // build waits for (with the fused launches below, 12345 particles with their walk: 842 -> 735 us).
-tg_status build_tree(tg_tree_s *T, const double *pos, const double *m, const double *h,
-                     const std::vector<int64_t> &sys_off_host, int quadrupole, int compute_moments,
-                     const int *nonfinite, cudaStream_t st, cudaEvent_t m_h_ready) {
+tg_status build_tree(tg_tree_s *T, const double *pos, const StageMH &stage_mh,
+                     const std::vector<int64_t> &sys_off_host, int quadrupole, int compute_moments, cudaStream_t st) {
     const int nsys = (int)sys_off_host.size() - 1;
     const int64_t N = sys_off_host.back();
     if (N < 1 || nsys < 1) return TG_ERR_BAD_ARG;
@@ -1573,16 +1604,17 @@ tg_status build_tree(tg_tree_s *T, const double *pos, const double *m, const dou
     void *host = nullptr;  // read-backs
     TG_TRY(host_words(&host));
 
-    // zeroed together: the summary, the depth lists' cursors, the level scan's status words and counter, the
+    // zeroed together: the summary, the depth lists' cursors, the input check's flag, the level scan's status words and counter, the
     // cubes' maxima and (kept with the tree) the sorts' error word
     const int lv_tiles = div_up(N, LV_TILE);
     const int64_t cap0 = N + N / 2 + 16;  // node slots, grown if needed
     int64_t exh_cap = N / 2 + 1;          // key-exhausted runs hold at least two particles each
     BuildSummary *sum = nullptr;
-    int *lvl_cursor = nullptr;
+    int *lvl_cursor = nullptr, *nonfinite = nullptr;
     unsigned long long *lv_status = nullptr, *mn = nullptr, *mx = nullptr;
     int64_t *sys_off = nullptr, *p_parent = nullptr, *p_next = nullptr, *exh = nullptr, *root_first = nullptr;
     uint64_t *keys = nullptr, *keys_orig = nullptr;
+    KeyCell *cells = nullptr;
     uint32_t *perm = nullptr;
     double *pc = nullptr, *pm = nullptr, *ps = nullptr;
     int8_t *L = nullptr;
@@ -1593,12 +1625,16 @@ tg_status build_tree(tg_tree_s *T, const double *pos, const double *m, const dou
     TG_CUDA(carve(temps, [&](Carve &c) {
         c.take(sum, 1);
         c.take(lvl_cursor, DEPTH_CAP + 1);
+        c.take(nonfinite, 1);
         c.take(lv_status, lv_tiles + 1);
         c.take(mx, 3 * nsys);
         c.take(mn, 3 * nsys);
         c.take(sys_off, nsys + 1);
         c.take(keys, N);
-        if (nsys > 1) c.take(keys_orig, N);
+        if (nsys > 1) {
+            c.take(keys_orig, N);
+            c.take(cells, nsys);
+        }
         c.take(perm, N);
         c.take(pc, 3 * N);
         c.take(pm, N);
@@ -1625,10 +1661,10 @@ tg_status build_tree(tg_tree_s *T, const double *pos, const double *m, const dou
     if (nsys > 1)
         TG_CUDA(cudaMemcpyAsync(sys_off, sys_off_host.data(), sizeof(int64_t) * (nsys + 1), cudaMemcpyHostToDevice, st));
     { k_bbox<<<div_up(N, BB_THREADS * BB_ITEMS), BB_THREADS, 0, st>>>(pos, N, sys_off, nsys, mn, mx); tg::note_launch(); }
-    { k_root_segs<<<LAUNCH(nsys)>>>(mn, mx, sys_off, N, sg); tg::note_launch(); }
+    { k_root_segs<<<LAUNCH(nsys)>>>(mn, mx, sys_off, N, cells, sg); tg::note_launch(); }
 
     // 2. keys and stable sort (system id as the most significant digit when batched)
-    { k_keys<<<LAUNCH(N)>>>(pos, N, sys_off, nsys, sg.center, sg.size, keys, keys_orig, perm); tg::note_launch(); }
+    { k_keys<<<LAUNCH(N)>>>(pos, N, sys_off, nsys, sg.center, sg.size, cells, keys, keys_orig, perm); tg::note_launch(); }
     TG_CUDA(cudaGetLastError());
     TG_TRY(radix_sort_pairs(keys, perm, N, 63, st, T->sort_err, nsys == 1));
     if (nsys > 1) {
@@ -1637,8 +1673,12 @@ tg_status build_tree(tg_tree_s *T, const double *pos, const double *m, const dou
     }
 
     // 3. particles gathered into Morton order
+    const double *m = nullptr, *h = nullptr;
+    cudaEvent_t m_h_ready = nullptr;
+    TG_TRY(stage_mh(m, h, m_h_ready));
     if (m_h_ready) TG_CUDA(cudaStreamWaitEvent(st, m_h_ready, 0));
-    { k_gather<<<LAUNCH(N)>>>(perm, N, pos, m, h, keys_orig, pc, pm, ps, keys, T->walk_idx, T->sort_err); tg::note_launch(); }
+    { k_gather<<<LAUNCH(N)>>>(perm, N, pos, m, h, keys_orig, pc, pm, ps, keys, T->walk_idx,
+                               T->sort_err, nonfinite); tg::note_launch(); }
     TG_CUDA(cudaGetLastError());
 
     // 4. split rounds
@@ -1825,7 +1865,7 @@ tg_status build_tree(tg_tree_s *T, const double *pos, const double *m, const dou
     T->mtot = M;
     uint64_t *nkeys = nullptr;
     uint32_t *nvals = nullptr;
-    int64_t *root_slot = nullptr, *final_of_slot = nullptr, *sys_node_off = nullptr, *ncnt = nullptr;
+    int64_t *root_slot = nullptr, *final_of_slot = nullptr, *sys_node_off = nullptr;
     unsigned long long *req = nullptr;
     DevArray<unsigned char> numbering(st), arrays(st);
     TG_CUDA(carve(numbering, [&](Carve &c) {
@@ -1833,10 +1873,7 @@ tg_status build_tree(tg_tree_s *T, const double *pos, const double *m, const dou
         c.take(nvals, M);
         c.take(root_slot, nsys);
         c.take(final_of_slot, M);
-        if (nsys > 1) {
-            c.take(sys_node_off, nsys + 1);
-            c.take(ncnt, nsys);
-        }
+        if (nsys > 1) c.take(sys_node_off, nsys + 1);
         if (n_bucket > 0) c.take(req, nsys);
     }));
     TG_CUDA(carve(arrays, [&](Carve &c) {
@@ -1860,19 +1897,15 @@ tg_status build_tree(tg_tree_s *T, const double *pos, const double *m, const dou
     { k_number_keys<<<LAUNCH(M)>>>(nd, M, sys_off, nb, root_key, compact, nkeys, nvals, root_slot); tg::note_launch(); }
     TG_CUDA(cudaGetLastError());
     TG_TRY(radix_sort_pairs(nkeys, nvals, M, sort_bits, st, T->sort_err, true));
-    // per-system node offsets (roots first within each system's block), on the device; the host
-    // copy is read with the final synchronisation
+    // per-system node offsets (roots first within each system's block): k_final_index makes them on the device,
+    // the host copy is read with the final synchronisation
     if (nsys == 1) {
         T->sys_node_off = {0, M};
     } else {
-        TG_CUDA(cudaMemsetAsync(ncnt, 0, sizeof(int64_t) * nsys, st));
-        { k_sys_node_counts<<<LAUNCH(M)>>>(nd.sys, M, ncnt); tg::note_launch(); }
-        TG_CUDA(cudaGetLastError());
-        TG_TRY(exclusive_scan_i64(ncnt, sys_node_off, nsys, sys_node_off + nsys, st));
         T->sys_node_off.assign(nsys + 1, 0);
     }
-    { k_final_index<<<LAUNCH(std::max<int64_t>(M, nsys))>>>(nvals, M, nd.sys, N, sys_node_off, final_of_slot, root_slot,
-                                                         nsys, T->sort_err); tg::note_launch(); }
+    { k_final_index<<<LAUNCH(std::max<int64_t>(M, nsys))>>>(nkeys, nvals, M, nd.sys, N, key_bits - sysbits,
+                                                         sys_node_off, final_of_slot, root_slot, nsys, T->sort_err); tg::note_launch(); }
     TG_CUDA(cudaGetLastError());
     // capacity (NumNodes) per system: bucket reservations, read with the final synchronisation
     if (n_bucket > 0) {
@@ -2084,7 +2117,7 @@ tg_status morton_order_device(const double *pos, int64_t n, uint32_t *perm, cuda
     int *err = err_dev ? err_dev : &cube.p->err;
     { k_bbox<<<div_up(n, BB_THREADS * BB_ITEMS), BB_THREADS, 0, st>>>(pos, n, nullptr, 1, cube.p->mn, cube.p->mx); tg::note_launch(); }
     { k_bbox_finish<<<1, 32, 0, st>>>(cube.p->mn, cube.p->mx, 1, cube.p->center, &cube.p->size); tg::note_launch(); }
-    { k_keys<<<LAUNCH(n)>>>(pos, n, nullptr, 1, cube.p->center, &cube.p->size, keys.p, nullptr, perm); tg::note_launch(); }
+    { k_keys<<<LAUNCH(n)>>>(pos, n, nullptr, 1, cube.p->center, &cube.p->size, nullptr, keys.p, nullptr, perm); tg::note_launch(); }
     TG_CUDA(cudaGetLastError());
     TG_TRY(radix_sort_pairs(keys.p, perm, n, 63, st, err));
     if (err_dev) return TG_OK;

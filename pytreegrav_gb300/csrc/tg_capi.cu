@@ -7,9 +7,8 @@
 #include "tg_tree.cuh"
 
 namespace tg {
-tg_status build_tree(tg_tree_s *T, const double *pos, const double *m, const double *h,
-                     const std::vector<int64_t> &sys_off_host, int quadrupole, int compute_moments,
-                     const int *nonfinite, cudaStream_t st, cudaEvent_t m_h_ready);
+tg_status build_tree(tg_tree_s *T, const double *pos, const StageMH &stage_mh,
+                     const std::vector<int64_t> &sys_off_host, int quadrupole, int compute_moments, cudaStream_t st);
 tg_status tree_side_stream(tg_tree_s *t);
 tg_status morton_order_device(const double *pos, int64_t n, uint32_t *perm, cudaStream_t st, int *err_dev);
 template <typename T>
@@ -40,14 +39,6 @@ __device__ __forceinline__ bool nonfinite_bits(const double *p) {
 __global__ void k_nonfinite(const double *a, int64_t n, int *flag) {
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n && nonfinite_bits(a + i)) atomicOr(flag, 1);
-}
-
-// Any non-finite value among positions (3n), masses (n, may be NULL) and softenings (n, may be NULL).
-__global__ void k_nonfinite3(const double *pos, const double *m, const double *h, int64_t n, int *flag) {
-    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= 5 * n) return;
-    const double *p = i < 3 * n ? pos + i : (i < 4 * n ? (m ? m + (i - 3 * n) : nullptr) : (h ? h + (i - 4 * n) : nullptr));
-    if (p && nonfinite_bits(p)) atomicOr(flag, 1);
 }
 
 __global__ void k_u32_to_i64(const uint32_t *a, int64_t n, int64_t *b) {
@@ -160,41 +151,38 @@ static tg_status build_common(const double *pos, const double *m, const double *
     tg_status rc = TG_OK;
     {
         DevBuf dp, dm, dh;
-        int *flag = nullptr;
         cudaEvent_t m_h_ready = nullptr;
+        // Masses and softenings come in once the build has queued the sort of the positions, on the tree's side
+        // stream when they are uploaded: the copies overlap the sort, and so does the host's part in them. The
+        // build waits for m_h_ready where it first reads them.
+        auto stage_mh = [&](const double *&md, const double *&hd, cudaEvent_t &ready) -> tg_status {
+            const bool side = mem == TG_MEM_HOST && (m || h);
+            cudaStream_t ms = side ? t->side : st;
+            TG_TRY(stage_in(m, n, mem, ms, dm));
+            TG_TRY(stage_in(h, n, mem, ms, dh));
+            if (side) {
+                dm.st = dh.st = st;  // freed on st, after the build's last read
+                TG_CUDA(cudaEventRecord(t->ev_join, t->side));
+                m_h_ready = t->ev_join;
+            }
+            md = dm.ptr;
+            hd = dh.ptr;
+            ready = m_h_ready;
+            return TG_OK;
+        };
         auto stage = [&]() -> tg_status {
             TG_TRY(stage_in(pos, 3 * n, mem, st, dp));
-            // the input check runs ahead of the build on the stream; the build reads its flag back
-            // with its first summary and reports non-finite input with its closing read-back
-            TG_CUDA(tg::dev_malloc((void **)&flag, sizeof(int), st));
-            TG_CUDA(cudaMemsetAsync(flag, 0, sizeof(int), st));
             if (mem == TG_MEM_HOST && (m || h)) {
-                { k_nonfinite<<<div_up(3 * n, 256), 256, 0, st>>>(dp.ptr, 3 * n, flag); tg::note_launch(); }
-                // masses and softenings are uploaded (and checked) on the tree's side stream while
-                // the build sorts the positions; the build waits for them where it first reads them
                 TG_TRY(tree_side_stream(t));
                 TG_CUDA(cudaEventRecord(t->ev_fork, st));
                 TG_CUDA(cudaStreamWaitEvent(t->side, t->ev_fork, 0));
-                TG_TRY(stage_in(m, n, mem, t->side, dm));
-                TG_TRY(stage_in(h, n, mem, t->side, dh));
-                dm.st = dh.st = st;  // freed on st, after the build's last read
-                if (dm.ptr) { k_nonfinite<<<div_up(n, 256), 256, 0, t->side>>>(dm.ptr, n, flag); tg::note_launch(); }
-                if (dh.ptr) { k_nonfinite<<<div_up(n, 256), 256, 0, t->side>>>(dh.ptr, n, flag); tg::note_launch(); }
-                TG_CUDA(cudaEventRecord(t->ev_join, t->side));
-                m_h_ready = t->ev_join;
-            } else {
-                TG_TRY(stage_in(m, n, mem, st, dm));
-                TG_TRY(stage_in(h, n, mem, st, dh));
-                { k_nonfinite3<<<div_up(5 * n, 256), 256, 0, st>>>(dp.ptr, dm.ptr, dh.ptr, n, flag); tg::note_launch(); }
             }
-            TG_CUDA(cudaGetLastError());
             return TG_OK;
         };
         rc = stage();
-        if (rc == TG_OK) rc = build_tree(t, dp.ptr, dm.ptr, dh.ptr, off, quadrupole, compute_moments, flag, st, m_h_ready);
+        if (rc == TG_OK) rc = build_tree(t, dp.ptr, stage_mh, off, quadrupole, compute_moments, st);
         // st is ordered after the side stream's uploads before anything staged is freed
         if (m_h_ready) cudaStreamWaitEvent(st, m_h_ready, 0);
-        if (flag) cudaFreeAsync(flag, st);
     }
     if (rc != TG_OK) {
         destroy(t);

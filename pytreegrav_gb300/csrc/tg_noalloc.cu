@@ -32,13 +32,14 @@
 
 namespace tg {
 
+struct KeyCell;
 // Kernels defined in tg_build.cu (bounding cube, Morton keys) and tg_sort.cu (radix passes).
 __global__ void k_bbox(const double *pos, int64_t n, const int64_t *sys_off, int nsys, unsigned long long *mn,
                        unsigned long long *mx);
 __global__ void k_bbox_finish(const unsigned long long *mn, const unsigned long long *mx, int nsys, double *center,
                               double *size);
 __global__ void k_keys(const double *pos, int64_t n, const int64_t *sys_off, int nsys, const double *center,
-                       const double *size, uint64_t *keys, uint64_t *keys_copy, uint32_t *vals);
+                       const double *size, const KeyCell *cells, uint64_t *keys, uint64_t *keys_copy, uint32_t *vals);
 __global__ void radix_hist(const uint64_t *keys, int64_t n, int shift, int ntiles, int *hist);
 __global__ void radix_scatter(const uint64_t *keys, const uint32_t *vals, int64_t n, int shift, int ntiles,
                               const int *offs, uint64_t *keys_out, uint32_t *vals_out);
@@ -237,7 +238,7 @@ extern "C" tg_status tg_morton_order_noalloc(const double *pos, int64_t n, int64
     // Bounding cube and keys, then stable radix passes over the 63 key bits.
     { k_bbox<<<div_up(n, BBOX_POINTS), BBOX_THREADS, 0, st>>>(pos, n, sys_off, 1, mn, mx); tg::note_launch(); }
     { k_bbox_finish<<<1, 32, 0, st>>>(mn, mx, 1, center, size); tg::note_launch(); }
-    { k_keys<<<div_up(n, 256), 256, 0, st>>>(pos, n, sys_off, 1, center, size, keys[0], nullptr, vals[0]); tg::note_launch(); }
+    { k_keys<<<div_up(n, 256), 256, 0, st>>>(pos, n, sys_off, 1, center, size, nullptr, keys[0], nullptr, vals[0]); tg::note_launch(); }
     const int ntiles = div_up(n, SORT_TILE);
     int cur = 0;
     for (int shift = 0; shift < KEY_BITS; shift += 8) {

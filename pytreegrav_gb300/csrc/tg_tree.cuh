@@ -1,12 +1,16 @@
 // Device-resident octree and the walk arena derived from it.
 #pragma once
 
+#include <functional>
 #include <type_traits>
 #include <vector>
 
 #include "tg_common.cuh"
 
 namespace tg {
+
+// Device pointers of a build's masses and softenings (null: none) and the event after which they may be read.
+typedef std::function<tg_status(const double *&m, const double *&h, cudaEvent_t &ready)> StageMH;
 
 // 32-byte FP64 quadruple (the CUDA double4 vector type is deprecated in CUDA 13).
 struct alignas(32) D4 {
