@@ -1703,10 +1703,14 @@ tg_status build_tree(tg_tree_s *T, const double *pos, const StageMH &stage_mh,
     // 2. keys and stable sort (system id as the most significant digit when batched)
     { k_keys<<<LAUNCH(N)>>>(pos, N, sys_off, nsys, sg.center, sg.size, cells, keys, keys_orig, perm); tg::note_launch(); }
     TG_CUDA(cudaGetLastError());
-    TG_TRY(radix_sort_pairs(keys, perm, N, 63, st, T->sort_err, nsys == 1));
+    SortedPairs by_key(st), by_sys(st);  // the first may keep the build's keys
+    TG_TRY(radix_sort_pairs(keys, perm, N, 63, st, T->sort_err, nsys == 1, &by_key));
+    keys = by_key.keys;
+    perm = by_key.vals;
     if (nsys > 1) {
         { k_sys_of<<<LAUNCH(N)>>>(perm, N, sys_off, nsys, keys); tg::note_launch(); }
-        TG_TRY(radix_sort_pairs(keys, perm, N, sysbits, st, T->sort_err));
+        TG_TRY(radix_sort_pairs(keys, perm, N, sysbits, st, T->sort_err, false, &by_sys));
+        perm = by_sys.vals;
     }
 
     // 3. particles gathered into Morton order
@@ -1933,7 +1937,10 @@ tg_status build_tree(tg_tree_s *T, const double *pos, const StageMH &stage_mh,
     const uint64_t root_key = key_bits < 64 ? (1ull << key_bits) : ~0ull;
     { k_number_keys<<<LAUNCH(M)>>>(nd, M, sys_off, nb, root_key, compact, nkeys, nvals, root_slot); tg::note_launch(); }
     TG_CUDA(cudaGetLastError());
-    TG_TRY(radix_sort_pairs(nkeys, nvals, M, sort_bits, st, T->sort_err, true));
+    SortedPairs numbered(st);
+    TG_TRY(radix_sort_pairs(nkeys, nvals, M, sort_bits, st, T->sort_err, true, &numbered));
+    nkeys = numbered.keys;
+    nvals = numbered.vals;
     // per-system node offsets (roots first within each system's block): k_final_index makes them on the device,
     // the host copy is read with the final synchronisation
     if (nsys == 1) {
@@ -2156,7 +2163,10 @@ tg_status morton_order_device(const double *pos, int64_t n, uint32_t *perm, cuda
     { k_bbox_finish<<<1, 32, 0, st>>>(cube.p->mn, cube.p->mx, 1, cube.p->center, &cube.p->size); tg::note_launch(); }
     { k_keys<<<LAUNCH(n)>>>(pos, n, nullptr, 1, cube.p->center, &cube.p->size, nullptr, keys.p, nullptr, perm); tg::note_launch(); }
     TG_CUDA(cudaGetLastError());
-    TG_TRY(radix_sort_pairs(keys.p, perm, n, 63, st, err));
+    SortedPairs sorted(st);
+    TG_TRY(radix_sort_pairs(keys.p, perm, n, 63, st, err, false, &sorted));
+    if (sorted.vals != perm)
+        TG_CUDA(cudaMemcpyAsync(perm, sorted.vals, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, st));
     if (err_dev) return TG_OK;
     void *host = nullptr;
     TG_TRY(host_words(&host));

@@ -246,8 +246,11 @@ tg_status exclusive_scan_i32(const int32_t *in, int32_t *out, int64_t n, cudaStr
 // sorted, well-formed result, so every later kernel stays in bounds.
 // caller_falls_back: the pairs are left as the passes left them on a failure (some places never written), and the
 // caller's next kernel takes the identity instead when *err is set (then one launch fewer).
+// left: the sorted pairs are left wherever the last pass put them, in keys and vals or in the sort's scratch, which
+// *left then keeps (an odd number of passes otherwise ends with a copy).
+struct SortedPairs;
 tg_status radix_sort_pairs(uint64_t *keys, uint32_t *vals, int64_t n, int bits, cudaStream_t s, int *err,
-                           bool caller_falls_back = false);
+                           bool caller_falls_back = false, SortedPairs *left = nullptr);
 
 // Bounds of the library's bounded device loops, overridable (tg_set_loop_limits in the measurement
 // header) so that tests can make each one run out; 0 selects the built-in bound. Process-wide.
@@ -319,6 +322,13 @@ struct DevArray {
     DevArray(const DevArray &) = delete;
     DevArray &operator=(const DevArray &) = delete;
     cudaError_t alloc(int64_t n) { return dev_malloc((void **)&p, sizeof(T) * (size_t)(n > 1 ? n : 1), st); }
+};
+
+struct SortedPairs {
+    DevArray<unsigned char> mem;
+    uint64_t *keys = nullptr;
+    uint32_t *vals = nullptr;
+    explicit SortedPairs(cudaStream_t s) : mem(s) {}
 };
 
 // Counts kernel launches (every launch site calls it; read through tg_launch_count()).

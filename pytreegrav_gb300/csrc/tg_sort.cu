@@ -412,44 +412,52 @@ __global__ void __launch_bounds__(RS_THREADS) radix_scatter(const uint64_t *keys
 // One-sweep passes (decoupled look-back). All digit histograms come from one read of the keys;
 // then each pass is one kernel: a CTA takes the next tile from an atomic counter (so every earlier
 // tile belongs to a CTA that is already running), ranks its keys stably as above, publishes its
-// per-digit count, looks back over earlier tiles' published words for its exclusive prefix, and
-// scatters. A look-back spin is bounded; running out sets the sort's own error word instead of
-// hanging, and the sort then leaves the identity permutation (k_sort_fallback).
+// per-digit count, orders its tile by digit in shared memory, looks back over earlier tiles' published words for
+// its exclusive prefix, and writes the tile out. A look-back spin is bounded; running out sets the sort's own
+// error word instead of hanging, and the sort then leaves the identity permutation (k_sort_fallback).
+// Digits have up to nine bits (63 key bits: seven passes; a sort's bits are shared out evenly over its passes).
+// A pass is bound by the chain of one tile (load, rank, publish, look back, write) with the ~300 tiles that fit the
+// SMs, a third of the copy bandwidth: hence few instructions per key (lanes of equal digits find one another by
+// an OR into a word per digit, ~12 instructions where ballots over the digit's bits took ~45) and the tile's own
+// reordering before the look-back, which then finds its predecessors further on. Tiles of 512 threads x 8
+// keys: Morton order of 1e6 points 264 us, 8e6 940 us (ballots, 8-bit digits, 256 threads x 8: 298 and 1136;
+// this kernel with 8-bit digits 256 and 963, but slower builds below 1e6). From LONG_SORT pairs 12 keys per thread:
+// longer runs of a digit to write (8e6 points 879 us; 1e6 266).
 
-constexpr int MAX_PASSES = 8;
-#ifndef TG_OS_ROUNDS
-#define TG_OS_ROUNDS 8
-#endif
-#ifndef TG_OS_LB
-#define TG_OS_LB 4
-#endif
-constexpr int OS_ROUNDS = TG_OS_ROUNDS;             // keys per thread in a one-sweep pass
-constexpr int OS_WARP_KEYS = OS_ROUNDS * 32;
-constexpr int OS_TILE = RS_WARPS * OS_WARP_KEYS;   // 2048 keys per CTA (8 per thread; measured against 2, 4 and 16)
+constexpr int OS_BITS = 9, OS_BINS = 1 << OS_BITS;
+constexpr int MAX_PASSES = (64 + OS_BITS - 1) / OS_BITS;
+constexpr int OS_WARPS = 16, OS_THREADS = OS_WARPS * 32;
+static_assert(OS_THREADS == OS_BINS, "a thread per digit");
+constexpr int64_t LONG_SORT = 3 << 20;
+template <int ROUNDS>  // keys per thread
+struct OsTile {
+    static constexpr int WARP_KEYS = ROUNDS * 32, KEYS = OS_WARPS * WARP_KEYS;
+};
 // A status word: flag (bits 62-63: aggregate or inclusive), the pass it belongs to (bits 56-61, pass + 1),
 // value (bits 0-55). Words of an earlier pass read as not yet published, so the status array is
 // cleared once per sort rather than once per pass.
 constexpr unsigned long long ST_AGG = 1ull << 62, ST_INC = 2ull << 62, ST_FLAGS = 3ull << 62;
 constexpr unsigned long long ST_TAGS = 63ull << 56, ST_VAL = (1ull << 56) - 1;
 constexpr long long SPIN_LIMIT = 1ll << 22;
-constexpr int LB = TG_OS_LB;  // predecessors read per look-back round trip
+constexpr int LB = 4;  // predecessors read per look-back round trip
 
-// Every pass's digit histogram from one read of the keys; the last block to finish scans each pass's 256 counts
+// Every pass's digit histogram from one read of the keys; the last block to finish scans each pass's counts
 // in place (exclusive), which took a launch of its own.
-constexpr int HIST_THREADS = 256;
-__global__ void __launch_bounds__(HIST_THREADS) k_sort_hist(const uint64_t *keys, int64_t n, int npass, int *hist,
-                                                            int *done) {
-    __shared__ int h[MAX_PASSES * RS_BINS];
-    __shared__ int tot[MAX_PASSES * RS_BINS / 32];
+constexpr int HIST_THREADS = OS_BINS / 2;
+__global__ void __launch_bounds__(HIST_THREADS) k_sort_hist(const uint64_t *keys, int64_t n, int npass, int width,
+                                                            int *hist, int *done) {
+    __shared__ int h[MAX_PASSES * OS_BINS];
+    __shared__ int tot[MAX_PASSES * HIST_THREADS / 32];
     __shared__ bool last;
-    for (int i = threadIdx.x; i < npass * RS_BINS; i += HIST_THREADS) h[i] = 0;
+    for (int i = threadIdx.x; i < npass * OS_BINS; i += HIST_THREADS) h[i] = 0;
     __syncthreads();
+    const unsigned mask = (1u << width) - 1;
     for (int64_t i = (int64_t)blockIdx.x * HIST_THREADS + threadIdx.x; i < n; i += (int64_t)gridDim.x * HIST_THREADS) {
         const uint64_t k = keys[i];
-        for (int p = 0; p < npass; p++) atomicAdd(&h[p * RS_BINS + (int)((k >> (8 * p)) & (RS_BINS - 1))], 1);
+        for (int p = 0; p < npass; p++) atomicAdd(&h[p * OS_BINS + ((unsigned)(k >> (width * p)) & mask)], 1);
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < npass * RS_BINS; i += HIST_THREADS)
+    for (int i = threadIdx.x; i < npass * OS_BINS; i += HIST_THREADS)
         if (h[i]) atomicAdd(&hist[i], h[i]);
     __threadfence();
     __syncthreads();
@@ -458,126 +466,162 @@ __global__ void __launch_bounds__(HIST_THREADS) k_sort_hist(const uint64_t *keys
     if (!last) return;
     __threadfence();
     const int lane = lane_id(), w = threadIdx.x >> 5;
-    int v[MAX_PASSES], inc[MAX_PASSES];
+    int2 v[MAX_PASSES];
+    int inc[MAX_PASSES];
 #pragma unroll
     for (int p = 0; p < MAX_PASSES; p++) {
         if (p >= npass) break;
-        v[p] = __ldcg(&hist[p * RS_BINS + threadIdx.x]);
-        inc[p] = warp_inclusive_scan(v[p]);
-        if (lane == 31) tot[p * (RS_BINS / 32) + w] = inc[p];
+        v[p] = __ldcg(reinterpret_cast<const int2 *>(hist + p * OS_BINS) + threadIdx.x);
+        inc[p] = warp_inclusive_scan(v[p].x + v[p].y);
+        if (lane == 31) tot[p * (HIST_THREADS / 32) + w] = inc[p];
     }
     __syncthreads();
 #pragma unroll
     for (int p = 0; p < MAX_PASSES; p++) {
         if (p >= npass) break;
-        int below = 0;
-        for (int k = 0; k < w; k++) below += tot[p * (RS_BINS / 32) + k];
-        hist[p * RS_BINS + threadIdx.x] = below + inc[p] - v[p];
+        int below = inc[p] - v[p].x - v[p].y;
+        for (int k = 0; k < w; k++) below += tot[p * (HIST_THREADS / 32) + k];
+        reinterpret_cast<int2 *>(hist + p * OS_BINS)[threadIdx.x] = make_int2(below, below + v[p].x);
     }
 }
 
-__global__ void __launch_bounds__(RS_THREADS, 4) k_onesweep(const uint64_t *keys, const uint32_t *vals, int64_t n,
-                                                         int shift, int pass, const int *digit_off,
-                                                         unsigned long long *status, int *tile_counter,
-                                                         uint64_t *keys_out, uint32_t *vals_out, int *err,
-                                                         long long spin_limit) {
+template <int ROUNDS>
+struct alignas(16) OsSmem {
+    unsigned short wcount[OS_WARPS][OS_BINS];  // a warp's digit counts, then its first positions within the tile
+    int prefix[OS_BINS];                       // the digit's place in the output, less lstart
+    int warp_sum[OS_WARPS];
+    int tile;
+    union alignas(16) {  // cleared 16 bytes at a time
+        unsigned peers[OS_WARPS][OS_BINS];  // while ranking: a warp's lanes with the digit
+        struct {
+            uint64_t key[OsTile<ROUNDS>::KEYS];  // the tile in digit order
+            uint32_t val[OsTile<ROUNDS>::KEYS];
+        };
+    };
+};
+template <int ROUNDS>
+__global__ void __launch_bounds__(OS_THREADS, 2)
+    k_onesweep(const uint64_t *keys, const uint32_t *vals, int64_t n, int shift, int width, int pass, const int *digit_off,
+               unsigned long long *status, int *tile_counter, uint64_t *keys_out, uint32_t *vals_out, int *err,
+               long long spin_limit) {
     const unsigned long long tag = (unsigned long long)(pass + 1) << 56;
-    __shared__ int wcount[RS_WARPS][RS_BINS];
-    __shared__ int prefix[RS_BINS];
-    __shared__ int lstart[RS_BINS];  // the digit's first position within the tile
-    __shared__ uint64_t skey[OS_TILE];
-    __shared__ uint32_t sval[OS_TILE];
-    __shared__ int tile_s;
-    if (threadIdx.x == 0) tile_s = atomicAdd(tile_counter, 1);
-    for (int i = threadIdx.x; i < RS_WARPS * RS_BINS; i += RS_THREADS) (&wcount[0][0])[i] = 0;
+    extern __shared__ __align__(16) unsigned char os_raw[];
+    OsSmem<ROUNDS> &sm = *reinterpret_cast<OsSmem<ROUNDS> *>(os_raw);
+    constexpr int TILE = OsTile<ROUNDS>::KEYS;
+    if (threadIdx.x == 0) sm.tile = atomicAdd(tile_counter, 1);
+    const int w = threadIdx.x >> 5, lane = lane_id();
+    const unsigned lt = lanemask_lt(), mask = (1u << width) - 1;
+    unsigned short *wc = sm.wcount[w];
+    unsigned *peers = sm.peers[w];
+    for (int i = lane; i < OS_BINS / 8; i += 32) reinterpret_cast<uint4 *>(wc)[i] = make_uint4(0, 0, 0, 0);
+    for (int i = lane; i < OS_BINS / 4; i += 32) reinterpret_cast<uint4 *>(peers)[i] = make_uint4(0, 0, 0, 0);
     __syncthreads();
-    const int t = tile_s;
-    const int w = threadIdx.x >> 5;
-    const int64_t wbase = (int64_t)t * OS_TILE + (int64_t)w * OS_WARP_KEYS;
-    int digit[OS_ROUNDS], rank[OS_ROUNDS];
-    uint64_t kv[OS_ROUNDS];
-    uint32_t vv[OS_ROUNDS];  // values loaded with the keys, so the scatter reads nothing from memory
-    {
-        const int lane = lane_id();
+    const int t = sm.tile;
+    const int64_t tbase = (int64_t)t * TILE;
+    const int cnt = n - tbase < TILE ? (int)(n - tbase) : TILE;
+    const int wofs = w * OsTile<ROUNDS>::WARP_KEYS + lane;
+    const uint64_t *kp = keys + tbase;
+    const uint32_t *vp = vals + tbase;
+    int place[ROUNDS];  // rank within the warp's keys of the digit (low half), the digit (high half)
+    uint64_t kv[ROUNDS];
+    uint32_t vv[ROUNDS];  // values loaded with the keys, so the scatter reads nothing from memory
 #pragma unroll
-        for (int r = 0; r < OS_ROUNDS; r++) {
-            const int64_t i = wbase + r * 32 + lane;
-            kv[r] = i < n ? __ldg(keys + i) : 0ull;
-            vv[r] = i < n ? __ldg(vals + i) : 0u;
-        }
+    for (int r = 0; r < ROUNDS; r++) {
+        const int i = wofs + r * 32;
+        kv[r] = i < cnt ? __ldg(kp + i) : 0ull;
+        vv[r] = i < cnt ? __ldg(vp + i) : 0u;
     }
-    rank_loaded_slice<OS_ROUNDS>(kv, n, wbase, shift, wcount[w], digit, rank);
+    // ranks round by round: the lanes of one digit find one another through a word per digit
+#pragma unroll
+    for (int r = 0; r < ROUNDS; r++) {
+        const bool in = wofs + r * 32 < cnt;
+        const int d = (int)((unsigned)(kv[r] >> shift) & mask);
+        if (in) atomicOr(&peers[d], 1u << lane);
+        __syncwarp();
+        unsigned m = 0;
+        int base = 0;
+        if (in) {
+            m = peers[d];
+            base = wc[d];
+        }
+        __syncwarp();
+        if (in && (31 - __clz(m)) == lane) {
+            peers[d] = 0;
+            wc[d] = (unsigned short)(base + __popc(m));
+        }
+        __syncwarp();
+        place[r] = d << 16 | (base + __popc(m & lt));
+    }
     __syncthreads();
-    {  // one thread per digit: offsets of the warps within the tile, then the tile's prefix
-        const int d = threadIdx.x;
-        int run = 0;
+    // a thread per digit: its counts per warp become the warps' first places within the tile
+    const int d = threadIdx.x;
+    int run = 0;
 #pragma unroll
-        for (int ww = 0; ww < RS_WARPS; ww++) {
-            int c = wcount[ww][d];
-            wcount[ww][d] = run;
-            run += c;
-        }
-        volatile unsigned long long *st = status + (int64_t)t * RS_BINS + d;
-        long long acc = 0;
-        if (t == 0) {
-            *st = ST_INC | tag | (unsigned long long)run;
-        } else {
-            *st = ST_AGG | tag | (unsigned long long)run;
-            // earlier tiles publish their aggregate without waiting on anyone, so each wait ends
-            // once that tile's CTA (already running: it took its tile before this one) has ranked.
-            // The words of LB predecessors are read together (independent loads, one round trip),
-            // then summed in order up to the first inclusive one.
-            bool done = false;
-            for (int64_t j = t - 1; j >= 0 && !done; j -= LB) {
-                unsigned long long w[LB];
+    for (int ww = 0; ww < OS_WARPS; ww++) run += sm.wcount[ww][d];
+    volatile unsigned long long *st = status + (int64_t)t * OS_BINS + d;
+    *st = (t == 0 ? ST_INC : ST_AGG) | tag | (unsigned long long)run;
+    const int inc = warp_inclusive_scan(run);
+    if (lane == 31) sm.warp_sum[w] = inc;
+    __syncthreads();
+    int start = inc - run;
 #pragma unroll
-                for (int k = 0; k < LB; k++)
-                    w[k] = j - k >= 0 ? ((const volatile unsigned long long *)status)[(j - k) * RS_BINS + d] : 0ull;
+    for (int ww = 0; ww < OS_WARPS; ww++) start += ww < w ? sm.warp_sum[ww] : 0;
+    int first = start;
 #pragma unroll
-                for (int k = 0; k < LB; k++) {
-                    if (done || j - k < 0) break;
-                    unsigned long long wd = w[k];
-                    const volatile unsigned long long *src = status + (j - k) * RS_BINS + d;
-                    auto ready = [tag](unsigned long long x) { return (x & ST_FLAGS) && (x & ST_TAGS) == tag; };
-                    for (long long spins = 0; !ready(wd) && spins < spin_limit; spins++) wd = *src;
-                    if (!ready(wd)) {
-                        atomicExch(err, 1);
-                        done = true;
-                        break;
-                    }
-                    acc += (long long)(wd & ST_VAL);
-                    if ((wd & ST_FLAGS) == ST_INC) done = true;
-                }
-            }
-            *st = ST_INC | tag | (unsigned long long)(acc + run);
-        }
-        prefix[d] = digit_off[d] + (int)acc;
-        __shared__ int tot_s;
-        lstart[d] = block_exclusive_scan(run, &tot_s);
+    for (int ww = 0; ww < OS_WARPS; ww++) {
+        const int c = sm.wcount[ww][d];
+        sm.wcount[ww][d] = (unsigned short)first;
+        first += c;
     }
     __syncthreads();
     // the tile in digit order in shared memory, then written out: keys of one digit go to consecutive
     // places, so consecutive threads write consecutive words instead of one scattered sector each
-    const int lane = lane_id();
 #pragma unroll
-    for (int r = 0; r < OS_ROUNDS; r++) {
-        const int64_t i = wbase + r * 32 + lane;
-        if (i < n) {
-            const int loc = lstart[digit[r]] + wcount[w][digit[r]] + rank[r];
-            skey[loc] = kv[r];
-            sval[loc] = vv[r];
+    for (int r = 0; r < ROUNDS; r++) {
+        if (wofs + r * 32 < cnt) {
+            const int loc = wc[place[r] >> 16] + (place[r] & 0xffff);
+            sm.key[loc] = kv[r];
+            sm.val[loc] = vv[r];
         }
     }
+    // earlier tiles publish their counts without waiting on anyone, so each wait ends once that tile's CTA
+    // (already running: it took its tile before this one) has ranked. The words of LB predecessors are read
+    // together (independent loads, one round trip), then summed in order up to the first inclusive one.
+    long long acc = 0;
+    bool done = false;
+    for (int64_t j = t - 1; j >= 0 && !done; j -= LB) {
+        unsigned long long word[LB];
+#pragma unroll
+        for (int k = 0; k < LB; k++)
+            word[k] = j - k >= 0 ? ((const volatile unsigned long long *)status)[(j - k) * OS_BINS + d] : 0ull;
+#pragma unroll
+        for (int k = 0; k < LB; k++) {
+            if (done || j - k < 0) break;
+            unsigned long long wd = word[k];
+            const volatile unsigned long long *src = status + (j - k) * OS_BINS + d;
+            auto ready = [tag](unsigned long long x) { return (x & ST_FLAGS) && (x & ST_TAGS) == tag; };
+            for (long long spins = 0; !ready(wd) && spins < spin_limit; spins++) wd = *src;
+            if (!ready(wd)) {
+                atomicExch(err, 1);
+                done = true;
+                break;
+            }
+            acc += (long long)(wd & ST_VAL);
+            if ((wd & ST_FLAGS) == ST_INC) done = true;
+        }
+    }
+    if (t > 0) *st = ST_INC | tag | (unsigned long long)(acc + run);
+    sm.prefix[d] = digit_off[d] + (int)acc - start;
     __syncthreads();
-    const int64_t rest = n - (int64_t)t * OS_TILE;
-    const int cnt = rest < OS_TILE ? (int)rest : OS_TILE;
-    for (int i = threadIdx.x; i < cnt; i += RS_THREADS) {
-        const uint64_t k = skey[i];
-        const int d = (int)((k >> shift) & (RS_BINS - 1));
-        const int pos = prefix[d] + (i - lstart[d]);
-        if ((unsigned)pos >= (unsigned)n) continue;  // only after a look-back that gave up (garbage keys)
+#pragma unroll
+    for (int r = 0; r < ROUNDS; r++) {
+        const int i = r * OS_THREADS + threadIdx.x;
+        if (i >= cnt) break;
+        const uint64_t k = sm.key[i];
+        const unsigned pos = (unsigned)(sm.prefix[(unsigned)(k >> shift) & mask] + i);
+        if (pos >= (unsigned)n) continue;  // only after a look-back that gave up (garbage keys)
         keys_out[pos] = k;
-        vals_out[pos] = sval[i];
+        vals_out[pos] = sm.val[i];
     }
 }
 
@@ -597,46 +641,60 @@ __global__ void k_sort_fallback(uint64_t *keys, uint32_t *vals, int64_t n, const
 long long scan_spins() { return loop_limits().sort_spin > 0 ? loop_limits().sort_spin : SPIN_LIMIT; }
 
 tg_status radix_sort_pairs(uint64_t *keys, uint32_t *vals, int64_t n, int bits, cudaStream_t s, int *err,
-                           bool caller_falls_back) {
+                           bool caller_falls_back, SortedPairs *left) {
+    if (left) {
+        left->keys = keys;
+        left->vals = vals;
+    }
     if (n <= 1 || bits <= 0) return TG_OK;
     if (n > (int64_t)0x7fffffff || !err) return TG_ERR_BAD_ARG;
     const long long spin_limit = loop_limits().sort_spin > 0 ? loop_limits().sort_spin : SPIN_LIMIT;
-    const int ntiles = div_up(n, OS_TILE);
-    const int npass = std::min((bits + 7) / 8, MAX_PASSES);
+    const bool lng = n >= LONG_SORT;
+    const int ntiles = div_up(n, lng ? OsTile<12>::KEYS : OsTile<8>::KEYS);
+    const int npass = (bits + OS_BITS - 1) / OS_BITS, width = (bits + npass - 1) / npass;
     // one allocation: status words, histograms, tile counters, the histogram's and the error word (zeroed), then
     // the other halves of the key and value buffers
-    const size_t st_bytes = sizeof(unsigned long long) * (size_t)ntiles * RS_BINS;
-    const size_t hist_bytes = sizeof(int) * MAX_PASSES * RS_BINS;
+    const size_t st_bytes = sizeof(unsigned long long) * (size_t)ntiles * OS_BINS;
+    const size_t hist_bytes = sizeof(int) * MAX_PASSES * OS_BINS;
     const size_t head = (st_bytes + hist_bytes + sizeof(int) * (MAX_PASSES + 2) + 255) / 256 * 256;
     const size_t key_bytes = (sizeof(uint64_t) * (size_t)n + 255) / 256 * 256;
-    unsigned char *scr = nullptr;
-    TG_CUDA(tg::dev_malloc((void **)&scr, head + key_bytes + sizeof(uint32_t) * (size_t)n, s));
+    DevArray<unsigned char> own(s), &mem = left ? left->mem : own;
+    mem.reset();
+    TG_CUDA(mem.alloc((int64_t)(head + key_bytes + sizeof(uint32_t) * (size_t)n)));
+    unsigned char *scr = mem.p;
     unsigned long long *status = (unsigned long long *)scr;
     int *hist = (int *)(scr + st_bytes);
-    int *counters = hist + MAX_PASSES * RS_BINS;
+    int *counters = hist + MAX_PASSES * OS_BINS;
     int *done = counters + MAX_PASSES;
     int *local_err = caller_falls_back ? err : done + 1;
     uint64_t *k2 = (uint64_t *)(scr + head);
     uint32_t *v2 = (uint32_t *)(scr + head + key_bytes);
     TG_CUDA(cudaMemsetAsync(scr, 0, head, s));
     const int hblocks = (int)std::min<int64_t>(div_up(n, HIST_THREADS * 4), (int64_t)num_sms() * 4);
-    { k_sort_hist<<<hblocks, HIST_THREADS, 0, s>>>(keys, n, npass, hist, done); tg::note_launch(); }
+    { k_sort_hist<<<hblocks, HIST_THREADS, 0, s>>>(keys, n, npass, width, hist, done); tg::note_launch(); }
+    auto pass = lng ? k_onesweep<12> : k_onesweep<8>;
+    const int smem = lng ? (int)sizeof(OsSmem<12>) : (int)sizeof(OsSmem<8>);
+    TG_CUDA(cudaFuncSetAttribute(pass, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     uint64_t *kin = keys, *kout = k2;
     uint32_t *vin = vals, *vout = v2;
     for (int p = 0; p < npass; p++) {
-        { k_onesweep<<<ntiles, RS_THREADS, 0, s>>>(kin, vin, n, 8 * p, p, hist + p * RS_BINS, status, counters + p, kout,
-                                                   vout, local_err, spin_limit); tg::note_launch(); }
+        { pass<<<ntiles, OS_THREADS, smem, s>>>(kin, vin, n, width * p, width, p, hist + p * OS_BINS, status, counters + p,
+                                                kout, vout, local_err, spin_limit); tg::note_launch(); }
         uint64_t *tk = kin; kin = kout; kout = tk;
         uint32_t *tv = vin; vin = vout; vout = tv;
     }
     TG_CUDA(cudaGetLastError());
-    if (kin != keys) {
+    if (left) {
+        left->keys = kin;
+        left->vals = vin;
+    } else if (kin != keys) {
         TG_CUDA(cudaMemcpyAsync(keys, kin, sizeof(uint64_t) * n, cudaMemcpyDeviceToDevice, s));
         TG_CUDA(cudaMemcpyAsync(vals, vin, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, s));
+        kin = keys;
+        vin = vals;
     }
-    if (!caller_falls_back) { k_sort_fallback<<<std::min(div_up(n, 256), 4 * num_sms()), 256, 0, s>>>(keys, vals, n, local_err, err); tg::note_launch(); }
+    if (!caller_falls_back) { k_sort_fallback<<<std::min(div_up(n, 256), 4 * num_sms()), 256, 0, s>>>(kin, vin, n, local_err, err); tg::note_launch(); }
     TG_CUDA(cudaGetLastError());
-    TG_CUDA(cudaFreeAsync(scr, s));
     return TG_OK;
 }
 

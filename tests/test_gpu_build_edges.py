@@ -38,3 +38,20 @@ def test_tree_is_the_oracles(kind, n):
     assert t.NumNodes == ref.NumNodes
     for f in FIELDS:
         assert np.array_equal(getattr(t, f), getattr(ref, f)), f
+
+
+@pytest.mark.parametrize("kind", ["uniform", "one digit", "duplicates"])
+@pytest.mark.parametrize("n", [2, 31, 511, 513, 4095, 4096, 4097, 8193, 70000, 3 * 2**20 + 1])
+def test_morton_order_is_the_oracles(kind, n):
+    """The radix sort at the edges of its tiles (4096 pairs; 6144 in long sorts), with digits all alike in most passes and with equal
+    keys, whose order must be kept: integers, so equal."""
+    import pytreegrav_gb300 as tg
+
+    rng = np.random.default_rng(n)
+    x = rng.random((n, 3))
+    if kind == "one digit":  # all but the corners of the cube within one cell of level 17
+        x = 0.3 + 1e-6 * x
+        x[0], x[-1] = 0.0, 1.0
+    if kind == "duplicates":
+        x = x[rng.integers(0, max(n // 50, 1), n)]
+    assert np.array_equal(tg.morton_order(x), O.morton_order(x))
