@@ -276,10 +276,6 @@ __device__ __forceinline__ int pair_level(uint64_t a, uint64_t b) {
     return l > MAX_LEVEL ? MAX_LEVEL : l;
 }
 
-__device__ __forceinline__ uint64_t prefix(uint64_t key, int level) {
-    return level <= 0 ? 0 : (key >> (63 - 3 * level));
-}
-
 struct RoundView {
     const int64_t *seg_lo, *seg_hi, *seg_root, *seg_next, *eoff;
     const double *seg_center, *seg_size;
@@ -308,9 +304,11 @@ __device__ __forceinline__ int node_count(int lo, int hi) {
 // (decoupled look-back; levels, counts and a three-launch scan took five launches and four more arrays'
 // traffic: 37 us of a 1e6 build). The round's node total goes to *total.
 constexpr int LV_THREADS = 256, LV_ITEMS = 4, LV_TILE = LV_THREADS * LV_ITEMS;
+// elem_of_slot receives the element of each of the round's first slot_cap nodes.
 __global__ void __launch_bounds__(LV_THREADS) k_levels(RoundView v, int64_t E, const uint64_t *keys, int8_t *L,
-                                                       int *nstart, unsigned long long *total,
-                                                       unsigned long long *status, int *counter, long long spins) {
+                                                       int *nstart, int *elem_of_slot, int64_t slot_cap,
+                                                       unsigned long long *total, unsigned long long *status,
+                                                       int *counter, long long spins) {
     __shared__ int warp_sum[LV_THREADS / 32];
     __shared__ long long before_s;
     __shared__ int tile_s;
@@ -366,50 +364,59 @@ __global__ void __launch_bounds__(LV_THREADS) k_levels(RoundView v, int64_t E, c
     for (int q = 0; q < LV_ITEMS; q++) {
         // clamped: such a round fits no slot array, k_nodes skips it and the host refuses it
         if (e0 + q < E) nstart[e0 + q] = (int)min(run, 0x7fffffffll);
+        for (int c = 0; c < cnt[q]; c++)
+            if (run + c < slot_cap) elem_of_slot[run + c] = (int)(e0 + q);
         run += cnt[q];
     }
 }
 
-// last index in [a, b) with prefix(key, level) == p (keys sorted): upper bound - 1
-__device__ __forceinline__ int64_t upper_prefix(const uint64_t *keys, int64_t a, int64_t b, uint64_t p, int level) {
-    while (a < b) {
-        int64_t mid = (a + b) >> 1;
-        if (prefix(keys[mid], level) <= p) a = mid + 1;
-        else b = mid;
-    }
-    return a;
-}
-// upper_prefix over [a, b) by galloping from a: cheap when the answer lies near a.
-__device__ __forceinline__ int64_t gallop_upper_prefix(const uint64_t *keys, int64_t a, int64_t b, uint64_t p,
-                                                       int level) {
-    int64_t step = 1;
-    while (a + step - 1 < b && prefix(keys[a + step - 1], level) <= p) {
-        a += step;
-        step <<= 1;
-    }
-    int64_t e = a + step - 1;
-    return upper_prefix(keys, a, e < b ? e : b, p, level);
-}
-__device__ __forceinline__ int64_t lower_prefix(const uint64_t *keys, int64_t a, int64_t b, uint64_t p, int level) {
-    while (a < b) {
-        int64_t mid = (a + b) >> 1;
-        if (prefix(keys[mid], level) < p) a = mid + 1;
-        else b = mid;
-    }
-    return a;
+// elem_of_slot again, for slot arrays that grew.
+__global__ void k_slot_elems(RoundView v, int64_t E, const int8_t *L, const int *nstart, int *elem_of_slot,
+                             int64_t slot_cap) {
+    const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= E) return;
+    int s;
+    int64_t i;
+    elem_loc(v, e, s, i);
+    const int nc = node_count(lvl0(v, L, s, e, i), L[e]);
+    for (int c = 0; c < nc; c++)
+        if ((int64_t)nstart[e] + c < slot_cap) elem_of_slot[(int64_t)nstart[e] + c] = (int)e;
 }
 
-// lower_prefix over [a, b] where keys[b] has prefix p, by galloping down from b: cheap when the
-// run of prefix p starts near b (a node's particles end at or after i, and most runs are short).
-__device__ __forceinline__ int64_t gallop_lower_prefix(const uint64_t *keys, int64_t a, int64_t b, uint64_t p,
-                                                       int level) {
-    int64_t step = 1;
-    while (b - step >= a && prefix(keys[b - step], level) >= p) {
-        b -= step;
+// The key bits below `level`: keys with k's prefix at a level are those in [k & ~mask, k | mask].
+__device__ __forceinline__ uint64_t below_mask(int level) { return level <= 0 ? ~0ull : (1ull << (63 - 3 * level)) - 1; }
+
+// End of the run of keys <= top that starts at a (keys sorted), within [a, b), by galloping from a: cheap when the
+// run is short.
+__device__ __forceinline__ int64_t run_end(const uint64_t *keys, int64_t a, int64_t b, uint64_t top) {
+    unsigned lo = (unsigned)a, hi = (unsigned)b, step = 1;
+    while (lo + step - 1 < hi && keys[lo + step - 1] <= top) {
+        lo += step;
         step <<= 1;
     }
-    const int64_t lo = b - step + 1 > a ? b - step + 1 : a;  // keys[b - step] (if >= a) is below p
-    return lower_prefix(keys, lo, b, p, level);
+    hi = min(lo + step - 1, hi);
+    while (lo < hi) {
+        const unsigned mid = (lo + hi) >> 1;
+        if (keys[mid] <= top) lo = mid + 1;
+        else hi = mid;
+    }
+    return (int64_t)lo;
+}
+// Start of the run of keys >= bottom that ends at b, where keys[b] >= bottom, within [a, b], by galloping down.
+__device__ __forceinline__ int64_t run_begin(const uint64_t *keys, int64_t a, int64_t b, uint64_t bottom) {
+    int lo = (int)a, hi = (int)b;
+    unsigned step = 1;
+    while (step <= (unsigned)(hi - lo) && keys[hi - (int)step] >= bottom) {
+        hi -= (int)step;
+        step <<= 1;
+    }
+    if (step <= (unsigned)(hi - lo)) lo = hi - (int)step + 1;  // that key is below
+    while (lo < hi) {
+        const int mid = lo + ((hi - lo) >> 1);
+        if (keys[mid] < bottom) lo = mid + 1;
+        else hi = mid;
+    }
+    return hi;
 }
 
 // slot of the node at `level` containing particle i (level >= lvl0 of the segment root)
@@ -417,7 +424,7 @@ __device__ __forceinline__ int64_t node_at(const RoundView &v, const int8_t *L, 
                                            int64_t slot_base, const uint64_t *keys, int s, int64_t i, int level) {
     if (level == 0 && v.seg_root[s] >= 0) return v.seg_root[s];
     int64_t lo = v.seg_lo[s];
-    int64_t p_lo = gallop_lower_prefix(keys, lo, i, prefix(keys[i], level), level);
+    int64_t p_lo = run_begin(keys, lo, i, keys[i] & ~below_mask(level));
     int64_t pe = v.eoff[s] + (p_lo - lo);
     return slot_base + nstart[pe] + (level - lvl0(v, L, s, pe, p_lo));
 }
@@ -431,72 +438,124 @@ __device__ __forceinline__ int64_t next_after(const RoundView &v, const int8_t *
     return (outer <= L[pe]) ? node_ref(slot_base + nstart[pe]) : e_end_particle;
 }
 
-// Particle i's parent slot and NextBranch reference.
-__device__ __forceinline__ void place_particle(const RoundView &v, const int8_t *L, const int *nstart, int64_t slot_base,
-                                               const uint64_t *keys, int s, int64_t e, int64_t i, int64_t *p_parent,
-                                               int64_t *p_next) {
-    int lprev = (i == v.seg_lo[s]) ? -1 : L[e - 1];
-    int K = max(lprev, (int)L[e]);
-    if (K >= MAX_LEVEL) return;  // inside a key-exhausted run: the next round places it
-    if (K < 0) K = 0;            // lone particle of its segment: child of the root
-    p_parent[i] = node_at(v, L, nstart, slot_base, keys, s, i, K);
-    p_next[i] = next_after(v, L, nstart, slot_base, s, i + 1);
+// ---------------------------------------------------------------------------------------------
+// Index validation: every slot or particle reference the later kernels dereference is checked
+// once; a bad one stops the build with an error instead of an out-of-bounds access.
+__device__ __forceinline__ bool ref_ok(int64_t r, int64_t N, int64_t M) {
+    if (r >= 0) return r < N;
+    if (r == -1) return true;
+    return (-r - 2) < M;
+}
+// final links: elements of the arena, or none
+__device__ __forceinline__ bool links_ok(int64_t NE, int64_t first, int64_t next, int64_t parent) {
+    return first >= -1 && first < NE && next >= -1 && next < NE && parent >= -1 && parent < NE;
+}
+__device__ __forceinline__ bool slot_ok(int64_t N, int64_t M, int64_t parent, int64_t aparent, int64_t first,
+                                        int64_t next, int64_t lo, int64_t hi) {
+    return parent >= -1 && parent < M && aparent >= -1 && aparent < M && ref_ok(first, N, M) && ref_ok(next, N, M) &&
+           first != -1 && lo >= 0 && hi <= N && lo < hi;
+}
+__device__ __forceinline__ bool particle_ok(int64_t N, int64_t M, int64_t parent, int64_t next) {
+    return parent >= 0 && parent < M && ref_ok(next, N, M);
 }
 
-// Node slots beyond nd.cap are not written (the host sees the round's node total, grows the slot
-// arrays and runs the round's node kernels again); so are exhausted-run entries beyond exh_cap.
-__global__ void k_nodes(RoundView v, int64_t E, const int8_t *L, const int *nstart, int64_t slot_base,
-                        const uint64_t *keys, Nodes nd, int64_t *exhausted, unsigned long long *n_exhausted,
-                        int64_t exh_cap, int64_t *root_first, int64_t *p_parent, int64_t *p_next) {
-    int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= E) return;
-    int s;
-    int64_t i;
-    elem_loc(v, e, s, i);
-    place_particle(v, L, nstart, slot_base, keys, s, e, i, p_parent, p_next);
-    int l0 = lvl0(v, L, s, e, i);
-    const int64_t nc = node_count(l0, L[e]);
-    if (slot_base + nstart[e] + nc > nd.cap) return;
-    uint64_t key = keys[i];
-    int64_t seg_lo = v.seg_lo[s], seg_hi = v.seg_hi[s];
-    // existing segment root (a re-keyed node): its first child is the level-1 run at seg_lo
-    if (i == seg_lo && v.seg_root[s] >= 0) {
-        root_first[s] = (1 <= L[e]) ? node_ref(slot_base + nstart[e]) : i;
+// Values the host reads back after a split round, gathered so that one copy (one synchronisation)
+// serves them all. depth_hist counts node slots per depth; depths >= DEPTH_CAP share the last bin.
+constexpr int DEPTH_CAP = 48;
+struct BuildSummary {
+    unsigned long long nodes;  // node slots made by the round (its scan total)
+    unsigned long long n_exh;  // key-exhausted runs found by the round
+    int bad;                   // invalid references (bit flags)
+    int nonfinite;             // the input check's flag
+    int depth_hist[DEPTH_CAP + 1];
+};
+// Section starts of the depth lists, from the histogram.
+struct LevelOffsets {
+    int at[DEPTH_CAP + 1];
+};
+__device__ __forceinline__ int depth_bin(int d) { return d < 0 ? 0 : (d > DEPTH_CAP ? DEPTH_CAP : d); }
+
+// Blocks [0, elem_blocks): every element's parent slot and NextBranch reference. The others: a thread per
+// node slot of the round (*total of them; the grid covers the slot arrays). Slots beyond nd.cap do not exist: the
+// host sees the round's node total, grows the slot arrays and runs this again; exhausted-run entries
+// beyond exh_cap are not written either. check (a first round, whose slots are all there are): slots and
+// particles are validated and the depths counted as they are made; a slot with exhausted keys has no first child
+// yet, but then another round follows and k_summarize_slots goes over everything.
+// A thread per element that makes the element's nodes spends most lanes idle (half the elements make none, some
+// several) and its warp on the longest search among them: 8e6 particles 518 us and 126 for the checks, this
+// 232 in all.
+constexpr int NODE_THREADS = 256;
+__global__ void __launch_bounds__(NODE_THREADS)
+    k_nodes(RoundView v, int64_t E, int elem_blocks, const int8_t *L, const int *nstart, const int *elem_of_slot,
+            int64_t slot_base, const unsigned long long *total, const uint64_t *keys, Nodes nd, int64_t *exhausted,
+            unsigned long long *n_exhausted, int64_t exh_cap, int64_t *root_first, int64_t *p_parent, int64_t *p_next,
+            int64_t N, BuildSummary *check, const int *nonfinite) {
+    __shared__ int hist[DEPTH_CAP + 1];
+    const int64_t M = slot_base + (int64_t)*total;  // all slots, this round's included
+    if ((int)blockIdx.x < elem_blocks) {
+        const int64_t e = (int64_t)blockIdx.x * NODE_THREADS + threadIdx.x;
+        if (check && nonfinite && e == 0) check->nonfinite = *nonfinite;
+        if (e >= E) return;
+        int s;
+        int64_t i;
+        elem_loc(v, e, s, i);
+        const int lev = L[e];
+        // existing segment root (a re-keyed node): its first child is the level-1 run at seg_lo
+        if (i == v.seg_lo[s] && v.seg_root[s] >= 0) root_first[s] = (1 <= lev) ? node_ref(slot_base + nstart[e]) : i;
+        int K = max(i == v.seg_lo[s] ? -1 : (int)L[e - 1], lev);
+        if (K >= MAX_LEVEL) return;  // inside a key-exhausted run: the next round places it
+        if (K < 0) K = 0;            // lone particle of its segment: child of the root
+        const int64_t parent = node_at(v, L, nstart, slot_base, keys, s, i, K);
+        const int64_t next = next_after(v, L, nstart, slot_base, s, i + 1);
+        p_parent[i] = parent;
+        p_next[i] = next;
+        if (check && !particle_ok(N, M, parent, next)) atomicOr(&check->bad, 2);
+        return;
     }
-    const int64_t slot0 = slot_base + nstart[e];
-    for (int64_t j = 0; j < nc; j++) {
-        int k = l0 + (int)j;
-        int64_t slot = slot0 + j;
+    const int64_t c0 = (int64_t)((int)blockIdx.x - elem_blocks) * NODE_THREADS;
+    const int64_t count = min((int64_t)*total, nd.cap - slot_base);
+    if (c0 >= count) return;
+    for (int b = threadIdx.x; b <= DEPTH_CAP; b += NODE_THREADS) hist[b] = 0;
+    __syncthreads();
+    const int64_t c = c0 + threadIdx.x;
+    if (c < count) {
+        const int64_t e = elem_of_slot[c], slot = slot_base + c;
+        int s;
+        int64_t i;
+        elem_loc(v, e, s, i);
+        const int j = (int)(c - nstart[e]), k = lvl0(v, L, s, e, i) + j, lev = L[e];
+        const uint64_t key = keys[i];
+        // the element's nodes are nested runs starting at i: all but the first have the previous slot as parent
+        const int64_t par = k == 0 ? -1 : (j > 0 ? slot - 1 : node_at(v, L, nstart, slot_base, keys, s, i, k - 1));
+        const int64_t hi = k == 0 ? v.seg_hi[s] : run_end(keys, i + 1, v.seg_hi[s], key | below_mask(k));
+        const int64_t next = next_after(v, L, nstart, slot_base, s, hi);
+        const int64_t first = k == MAX_LEVEL ? -1 : (k + 1 <= lev ? node_ref(slot + 1) : i);
+        const int depth = v.seg_depth0[s] + k;
+        if (k == MAX_LEVEL) {  // first: set by the re-key round or the bucket
+            unsigned long long q = atomicAdd(n_exhausted, 1ull);
+            if ((int64_t)q < exh_cap) exhausted[q] = slot;
+        }
         nd.lo[slot] = i;
+        nd.hi[slot] = hi;
         nd.level[slot] = (int8_t)k;
-        nd.depth[slot] = v.seg_depth0[s] + k;
+        nd.depth[slot] = depth;
         nd.sys[slot] = v.seg_sys[s];
-        // the element's nodes are nested runs starting at i: all but the first have the
-        // previous slot as parent
-        int64_t par = (k == 0) ? -1 : (j > 0 ? slot - 1 : node_at(v, L, nstart, slot_base, keys, s, i, k - 1));
         nd.parent[slot] = par;
         nd.aparent[slot] = par;
         nd.rank[slot] = i;
         nd.digit[slot] = k > 0 ? (int8_t)((key >> (63 - 3 * k)) & 7) : (int8_t)0;
         nd.seg[slot] = s;
-        if (k == MAX_LEVEL) {
-            nd.first[slot] = -1;  // set by the re-key round or the bucket
-            unsigned long long q = atomicAdd(n_exhausted, 1ull);
-            if ((int64_t)q < exh_cap) exhausted[q] = slot;
-        } else {
-            nd.first[slot] = (k + 1 <= L[e]) ? node_ref(slot + 1) : i;
+        nd.first[slot] = first;
+        nd.next[slot] = next;
+        if (check) {
+            if (!slot_ok(N, M, par, par, first, next, i, hi)) atomicOr(&check->bad, 1);
+            atomicAdd(&hist[depth_bin(depth)], 1);
         }
     }
-    // run ends, deepest first: a shallower run ends at or after the deeper one, so each search
-    // gallops on from the previous end
-    int64_t hi = i + 1;
-    for (int64_t j = nc - 1; j >= 0; j--) {
-        int k = l0 + (int)j;
-        int64_t slot = slot0 + j;
-        hi = (k == 0) ? seg_hi : gallop_upper_prefix(keys, hi, seg_hi, prefix(key, k), k);
-        nd.hi[slot] = hi;
-        nd.next[slot] = next_after(v, L, nstart, slot_base, s, hi);
-    }
+    __syncthreads();
+    if (!check) return;
+    for (int b = threadIdx.x; b <= DEPTH_CAP; b += NODE_THREADS)
+        if (hist[b]) atomicAdd(&check->depth_hist[b], hist[b]);
 }
 
 // x * 2^-q for q in {1, 2}, exactly: an exponent decrement when x and the result are normal
@@ -727,35 +786,8 @@ __global__ void k_bucket(const int64_t *exh, int n, const int64_t *chain_off, in
 }
 
 // ---------------------------------------------------------------------------------------------
-// Index validation: every slot or particle reference the later kernels dereference is checked
-// once; a bad one stops the build with an error instead of an out-of-bounds access.
-__device__ __forceinline__ bool ref_ok(int64_t r, int64_t N, int64_t M) {
-    if (r >= 0) return r < N;
-    if (r == -1) return true;
-    return (-r - 2) < M;
-}
-// final links: elements of the arena, or none
-__device__ __forceinline__ bool links_ok(int64_t NE, int64_t first, int64_t next, int64_t parent) {
-    return first >= -1 && first < NE && next >= -1 && next < NE && parent >= -1 && parent < NE;
-}
-
-// Values the host reads back after a split round, gathered so that one copy (one synchronisation)
-// serves them all. depth_hist counts node slots per depth; depths >= DEPTH_CAP share the last bin.
-constexpr int DEPTH_CAP = 48;
-struct BuildSummary {
-    unsigned long long nodes;  // node slots made by the round (its scan total)
-    unsigned long long n_exh;  // key-exhausted runs found by the round
-    int bad;                   // invalid references (bit flags)
-    int nonfinite;             // the input check's flag
-    int depth_hist[DEPTH_CAP + 1];
-};
-// Section starts of the depth lists, from the histogram.
-struct LevelOffsets {
-    int at[DEPTH_CAP + 1];
-};
-
-// Slot validation (as above) plus the depth histogram, over the slots [0, M) with
-// M = M_base + *M_round (clamped to the slot capacity).
+// Slot and particle validation plus the depth histogram, over the slots [0, M) with M = M_base + *M_round
+// (clamped to the slot capacity), for builds of more than one round or with buckets.
 __global__ void k_summarize_slots(Nodes nd, int64_t M_base, const unsigned long long *M_round, const int64_t *p_parent,
                                   const int64_t *p_next, int64_t N, BuildSummary *sum, const int *nonfinite) {
     __shared__ int hist[DEPTH_CAP + 1];
@@ -766,17 +798,11 @@ __global__ void k_summarize_slots(Nodes nd, int64_t M_base, const unsigned long 
     if (M > nd.cap) M = nd.cap;
     int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (c < M) {
-        bool ok = nd.parent[c] >= -1 && nd.parent[c] < M && nd.aparent[c] >= -1 && nd.aparent[c] < M &&
-                  ref_ok(nd.first[c], N, M) && ref_ok(nd.next[c], N, M) && nd.first[c] != -1 && nd.lo[c] >= 0 &&
-                  nd.hi[c] <= N && nd.lo[c] < nd.hi[c];
-        if (!ok) atomicOr(&sum->bad, 1);
-        int d = nd.depth[c];
-        atomicAdd(&hist[d < 0 ? 0 : (d > DEPTH_CAP ? DEPTH_CAP : d)], 1);
+        if (!slot_ok(N, M, nd.parent[c], nd.aparent[c], nd.first[c], nd.next[c], nd.lo[c], nd.hi[c]))
+            atomicOr(&sum->bad, 1);
+        atomicAdd(&hist[depth_bin(nd.depth[c])], 1);
     }
-    if (c < N) {
-        bool ok = p_parent[c] >= 0 && p_parent[c] < M && ref_ok(p_next[c], N, M);
-        if (!ok) atomicOr(&sum->bad, 2);
-    }
+    if (c < N && !particle_ok(N, M, p_parent[c], p_next[c])) atomicOr(&sum->bad, 2);
     __syncthreads();
     for (int b = threadIdx.x; b <= DEPTH_CAP; b += blockDim.x)
         if (hist[b]) atomicAdd(&sum->depth_hist[b], hist[b]);
@@ -1655,7 +1681,7 @@ tg_status build_tree(tg_tree_s *T, const double *pos, const StageMH &stage_mh,
     uint32_t *perm = nullptr;
     double *pc = nullptr, *pm = nullptr, *ps = nullptr;
     int8_t *L = nullptr;
-    int *nstart = nullptr;
+    int *nstart = nullptr, *elem_of_slot = nullptr;
     Nodes nd;
     Segs sg;
     DevArray<unsigned char> temps(st);
@@ -1678,6 +1704,7 @@ tg_status build_tree(tg_tree_s *T, const double *pos, const StageMH &stage_mh,
         c.take(ps, N);
         c.take(L, N);
         c.take(nstart, N);
+        c.take(elem_of_slot, cap0);
         c.take(exh, exh_cap);
         c.take(root_first, nsys);
         c.take(p_parent, N);
@@ -1686,7 +1713,7 @@ tg_status build_tree(tg_tree_s *T, const double *pos, const StageMH &stage_mh,
         nodes_lay(c, nd, cap0);
     }));
     // what replaces parts of it: slots that grow, the segments and lists of later rounds
-    DevArray<unsigned char> slots(st), round_mem(st);
+    DevArray<unsigned char> slots(st), elem_mem(st), round_mem(st);
     const size_t head = (size_t)((unsigned char *)mn - temps.p);
     TG_CUDA(cudaMemsetAsync(temps.p, 0, head, st));
     TG_CUDA(cudaMemsetAsync(mn, 0xff, sizeof(unsigned long long) * 3 * nsys, st));
@@ -1805,16 +1832,20 @@ tg_status build_tree(tg_tree_s *T, const double *pos, const StageMH &stage_mh,
             TG_CUDA(cudaMemsetAsync(sum, 0, sizeof(BuildSummary), st));
             TG_CUDA(cudaMemsetAsync(lv_status, 0, sizeof(unsigned long long) * (lv_tiles + 1), st));
         }
-        { k_levels<<<tiles, LV_THREADS, 0, st>>>(v, E, keys, L, nstart, &sum->nodes, lv_status,
-                                                 (int *)(lv_status + lv_tiles), scan_spins()); tg::note_launch(); }
+        { k_levels<<<tiles, LV_THREADS, 0, st>>>(v, E, keys, L, nstart, elem_of_slot, nd.cap - slot_base, &sum->nodes,
+                                                 lv_status, (int *)(lv_status + lv_tiles), scan_spins()); tg::note_launch(); }
         // The round's nodes, particle links and the summary, read back with one copy. Slots that
         // do not fit are skipped by k_nodes; the host then grows the arrays and runs it again.
         auto run_round = [&]() -> tg_status {
-            { k_nodes<<<LAUNCH(E)>>>(v, E, L, nstart, slot_base, keys, nd, exh, &sum->n_exh, exh_cap, root_first,
-                                     p_parent, p_next); tg::note_launch(); }
-            if (round > 0) { k_set_root_first<<<LAUNCH(sg.n)>>>(sg.root, root_first, sg.n, nd.first); tg::note_launch(); }
-            { k_summarize_slots<<<LAUNCH(std::max<int64_t>(nd.cap, N))>>>(nd, slot_base, &sum->nodes, p_parent, p_next,
-                                                                       N, sum, nonfinite); tg::note_launch(); }
+            const int elem_blocks = div_up(E, NODE_THREADS);
+            { k_nodes<<<elem_blocks + div_up(nd.cap - slot_base, NODE_THREADS), NODE_THREADS, 0, st>>>(
+                v, E, elem_blocks, L, nstart, elem_of_slot, slot_base, &sum->nodes, keys, nd, exh, &sum->n_exh, exh_cap,
+                root_first, p_parent, p_next, N, round == 0 ? sum : nullptr, nonfinite); tg::note_launch(); }
+            if (round > 0) {
+                { k_set_root_first<<<LAUNCH(sg.n)>>>(sg.root, root_first, sg.n, nd.first); tg::note_launch(); }
+                { k_summarize_slots<<<LAUNCH(std::max<int64_t>(nd.cap, N))>>>(nd, slot_base, &sum->nodes, p_parent, p_next,
+                                                                           N, sum, nonfinite); tg::note_launch(); }
+            }
             TG_CUDA(cudaGetLastError());
             TG_TRY(read_summary());
             if (hs.nonfinite) nonfinite_seen = true;
@@ -1825,6 +1856,8 @@ tg_status build_tree(tg_tree_s *T, const double *pos, const StageMH &stage_mh,
         if (slot_base + Mr > 0x7fffffffLL) return TG_ERR_BAD_ARG;
         if (slot_base + Mr > nd.cap) {
             TG_TRY(nodes_reserve(slots, nd, slot_base + Mr, st));
+            TG_CUDA(carve(elem_mem, [&](Carve &c) { c.take(elem_of_slot, nd.cap); }));
+            { k_slot_elems<<<LAUNCH(E)>>>(v, E, L, nstart, elem_of_slot, nd.cap - slot_base); tg::note_launch(); }
             TG_CUDA(cudaMemsetAsync(&sum->n_exh, 0, sizeof(unsigned long long), st));
             TG_CUDA(cudaMemsetAsync(&sum->bad, 0, sizeof(int) * (2 + DEPTH_CAP + 1), st));
             TG_TRY(run_round());
