@@ -54,6 +54,7 @@ __device__ __forceinline__ int64_t find_seg(const int64_t *off, int nseg, int64_
 constexpr int BB_SEGS = 8;
 __global__ void __launch_bounds__(BB_THREADS) k_bbox(const double *pos, int64_t n, const int64_t *sys_off, int nsys,
                                                      unsigned long long *mn, unsigned long long *mx) {
+    chain_next();
     int64_t tile0 = (int64_t)blockIdx.x * BB_THREADS * BB_ITEMS;
     if (tile0 >= n) return;
     int64_t tile1 = min(tile0 + (int64_t)BB_THREADS * BB_ITEMS, n) - 1;
@@ -135,6 +136,8 @@ __device__ __forceinline__ void bounding_cube(const unsigned long long *mn, cons
 }
 __global__ void k_bbox_finish(const unsigned long long *mn, const unsigned long long *mx, int nsys, double *center,
                               double *size) {
+    chain_wait();
+    chain_next();
     int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s < nsys) bounding_cube(mn, mx, s, center, size);
 }
@@ -194,6 +197,8 @@ __device__ __forceinline__ uint64_t morton_key(double x, double y, double z, con
 // cells: the systems' key cells, when there are several.
 __global__ void k_keys(const double *pos, int64_t n, const int64_t *sys_off, int nsys, const double *center,
                        const double *size, const KeyCell *cells, uint64_t *keys, uint64_t *keys_copy, uint32_t *vals) {
+    chain_wait();
+    chain_next();
     __shared__ KeyCell one;  // one system: its cell (with the division) formed once per block
     if (nsys == 1) {
         if (threadIdx.x == 0) one = key_cell(center, size[0]);
@@ -210,6 +215,8 @@ __global__ void k_keys(const double *pos, int64_t n, const int64_t *sys_off, int
 }
 
 __global__ void k_sys_of(const uint32_t *vals, int64_t n, const int64_t *sys_off, int nsys, uint64_t *out) {
+    chain_wait();
+    chain_next();
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) out[i] = (uint64_t)find_seg(sys_off, nsys, vals[i]);
 }
@@ -226,6 +233,8 @@ __device__ __forceinline__ bool nonfinite_bits(double x) {  // the all-ones expo
 __global__ void k_gather(const uint32_t *perm, int64_t n, const double *pos, const double *m, const double *h,
                          const uint64_t *keys_in, double *coord, double *mass, double *soft, uint64_t *keys_sorted,
                          int64_t *walk_idx, const int *sort_err, int *nonfinite) {
+    chain_wait();
+    chain_next();
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const bool bad = *sort_err != 0;
@@ -309,6 +318,8 @@ __global__ void __launch_bounds__(LV_THREADS) k_levels(RoundView v, int64_t E, c
                                                        int *nstart, int *elem_of_slot, int64_t slot_cap,
                                                        unsigned long long *total, unsigned long long *status,
                                                        int *counter, long long spins) {
+    chain_wait();
+    chain_next();
     __shared__ int warp_sum[LV_THREADS / 32];
     __shared__ long long before_s;
     __shared__ int tile_s;
@@ -490,6 +501,8 @@ __global__ void __launch_bounds__(NODE_THREADS)
             int64_t slot_base, const unsigned long long *total, const uint64_t *keys, Nodes nd, int64_t *exhausted,
             unsigned long long *n_exhausted, int64_t exh_cap, int64_t *root_first, int64_t *p_parent, int64_t *p_next,
             int64_t N, BuildSummary *check, const int *nonfinite) {
+    chain_wait();
+    chain_next();
     __shared__ int hist[DEPTH_CAP + 1];
     const int64_t M = slot_base + (int64_t)*total;  // all slots, this round's included
     if ((int)blockIdx.x < elem_blocks) {
@@ -790,6 +803,8 @@ __global__ void k_bucket(const int64_t *exh, int n, const int64_t *chain_off, in
 // (clamped to the slot capacity), for builds of more than one round or with buckets.
 __global__ void k_summarize_slots(Nodes nd, int64_t M_base, const unsigned long long *M_round, const int64_t *p_parent,
                                   const int64_t *p_next, int64_t N, BuildSummary *sum, const int *nonfinite) {
+    chain_wait();
+    chain_next();
     __shared__ int hist[DEPTH_CAP + 1];
     if (nonfinite && blockIdx.x == 0 && threadIdx.x == 0) sum->nonfinite = *nonfinite;
     for (int b = threadIdx.x; b <= DEPTH_CAP; b += blockDim.x) hist[b] = 0;
@@ -823,6 +838,8 @@ struct NumberingBits {
 // allocating parent, so it needs the full first-particle rank.)
 __global__ void k_number_keys(Nodes nd, int64_t count, const int64_t *sys_off, NumberingBits b, uint64_t root_key,
                               int compact, uint64_t *keys, uint32_t *vals, int64_t *root_slot_of_sys) {
+    chain_wait();
+    chain_next();
     int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= count) return;
     int s = nd.sys[c];
@@ -851,6 +868,8 @@ __global__ void k_number_keys(Nodes nd, int64_t count, const int64_t *sys_off, N
 __global__ void k_final_index(const uint64_t *sorted_keys, const uint32_t *vals, int64_t count, const int32_t *nd_sys,
                               int64_t ntot, int sys_shift, int64_t *sys_node_off, int64_t *final_of_slot,
                               const int64_t *root_slot_of_sys, int nsys, const int *sort_err) {
+    chain_wait();
+    chain_next();
     int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (*sort_err) {
         if (q < count) final_of_slot[q] = ntot + q;
@@ -898,6 +917,8 @@ __global__ void k_write(Nodes nd, int64_t count, int64_t ntot, int node_blocks, 
                         FinalArrays o, LevelOffsets off, int *lvl_cursor, int32_t *lvl_list, int8_t *fdepth,
                         const int64_t *p_parent, const int64_t *p_next, const double *pc, const double *pm,
                         const double *ps, int *bad) {
+    chain_wait();
+    chain_next();
     const int64_t NE = ntot + count;
     if ((int)blockIdx.x >= node_blocks) {  // particles: the Morton-ordered data and the resolved links
         const int64_t i = (int64_t)(blockIdx.x - node_blocks) * blockDim.x + threadIdx.x;
@@ -957,6 +978,8 @@ __global__ void k_write(Nodes nd, int64_t count, int64_t ntot, int node_blocks, 
 // places the node children from the back, so no local array is needed.
 __global__ void k_kids(int64_t ntot, int64_t mtot, const int64_t *first, const int64_t *next, int32_t *kids,
                        int8_t *nk) {
+    chain_wait();
+    chain_next();
     const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= mtot) return;
     const int64_t f = ntot + j, stop = next[f], ne = ntot + mtot;
@@ -1191,6 +1214,8 @@ __device__ __forceinline__ void node_moments_kids(const MomentArgs &a, int64_t j
 template <int MOM_BLOCK>
 __global__ void __launch_bounds__(MOM_BLOCK) k_moments_sorted(MomentArgs a, const int32_t *list, int count,
                                                               const int32_t *kids, const int8_t *nk) {
+    chain_wait();
+    chain_next();
     __shared__ int bin[9];
     __shared__ int order[MOM_BLOCK];
     const int t = threadIdx.x;
@@ -1231,10 +1256,14 @@ constexpr int WIDE_MAX_LEVEL = 12288;  // levels up to this many nodes use k_mom
 
 __global__ void __launch_bounds__(WIDE_THREADS) k_moments_wide(MomentArgs a, const int32_t *list, int count,
                                                               const int32_t *kids, const int8_t *nk) {
+    chain_wait();
+    chain_next();
     __shared__ double s_m[8][WIDE_NODES], s_t[3][8][WIDE_NODES], s_h[8][WIDE_NODES];  // child terms
     __shared__ double s_sum[5][WIDE_NODES], s_com[3][WIDE_NODES];
     __shared__ float s_q[6][8][WIDE_NODES];  // the children's FP32 quadrupole terms
     __shared__ int8_t s_use[8][WIDE_NODES];  // child enters the sums (a particle, or a node of nonzero mass)
+    chain_wait();
+    chain_next();
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int idx = blockIdx.x * WIDE_NODES + lane;
     const int64_t N = a.ntot;
@@ -1417,6 +1446,8 @@ __device__ __forceinline__ void node_quad64(const MomentArgs &a, int64_t j, cons
 }
 
 __global__ void k_quad64_level(MomentArgs a, const int32_t *list, int count, const int32_t *kids, const int8_t *nk) {
+    chain_wait();
+    chain_next();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= count) return;
     const int64_t j = list[i];
@@ -1615,6 +1646,8 @@ static int64_t reference_capacity(int64_t npart, int64_t required) {
 // segments: one per system. One system's offsets (0, n) are written here too.
 __global__ void k_root_segs(const unsigned long long *mn, const unsigned long long *mx, int64_t *sys_off, int64_t n,
                             KeyCell *cells, Segs g) {
+    chain_wait();
+    chain_next();
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= g.n) return;
     bounding_cube(mn, mx, s, g.center, g.size);
@@ -1725,17 +1758,18 @@ tg_status build_tree(tg_tree_s *T, const double *pos, const StageMH &stage_mh,
     if (nsys > 1)
         TG_CUDA(cudaMemcpyAsync(sys_off, sys_off_host.data(), sizeof(int64_t) * (nsys + 1), cudaMemcpyHostToDevice, st));
     { k_bbox<<<div_up(N, BB_THREADS * BB_ITEMS), BB_THREADS, 0, st>>>(pos, N, sys_off, nsys, mn, mx); tg::note_launch(); }
-    { k_root_segs<<<LAUNCH(nsys)>>>(mn, mx, sys_off, N, cells, sg); tg::note_launch(); }
+    TG_CHAIN(k_root_segs, div_up(nsys, 256), 256, 0, st, mn, mx, sys_off, N, cells, sg);
 
     // 2. keys and stable sort (system id as the most significant digit when batched)
-    { k_keys<<<LAUNCH(N)>>>(pos, N, sys_off, nsys, sg.center, sg.size, cells, keys, keys_orig, perm); tg::note_launch(); }
+    TG_CHAIN(k_keys, div_up(N, 256), 256, 0, st, pos, N, sys_off, nsys, sg.center, sg.size, cells, keys, keys_orig,
+             perm);
     TG_CUDA(cudaGetLastError());
     SortedPairs by_key(st), by_sys(st);  // the first may keep the build's keys
     TG_TRY(radix_sort_pairs(keys, perm, N, 63, st, T->sort_err, nsys == 1, &by_key));
     keys = by_key.keys;
     perm = by_key.vals;
     if (nsys > 1) {
-        { k_sys_of<<<LAUNCH(N)>>>(perm, N, sys_off, nsys, keys); tg::note_launch(); }
+        TG_CHAIN(k_sys_of, div_up(N, 256), 256, 0, st, perm, N, sys_off, nsys, keys);
         TG_TRY(radix_sort_pairs(keys, perm, N, sysbits, st, T->sort_err, false, &by_sys));
         perm = by_sys.vals;
     }
@@ -1745,8 +1779,8 @@ tg_status build_tree(tg_tree_s *T, const double *pos, const StageMH &stage_mh,
     cudaEvent_t m_h_ready = nullptr;
     TG_TRY(stage_mh(m, h, m_h_ready));
     if (m_h_ready) TG_CUDA(cudaStreamWaitEvent(st, m_h_ready, 0));
-    { k_gather<<<LAUNCH(N)>>>(perm, N, pos, m, h, keys_orig, pc, pm, ps, keys, T->walk_idx,
-                               T->sort_err, nonfinite); tg::note_launch(); }
+    TG_CHAIN(k_gather, div_up(N, 256), 256, 0, st, perm, N, pos, m, h, keys_orig, pc, pm, ps, keys, T->walk_idx,
+             T->sort_err, nonfinite);
     TG_CUDA(cudaGetLastError());
 
     // 4. split rounds
@@ -1832,19 +1866,19 @@ tg_status build_tree(tg_tree_s *T, const double *pos, const StageMH &stage_mh,
             TG_CUDA(cudaMemsetAsync(sum, 0, sizeof(BuildSummary), st));
             TG_CUDA(cudaMemsetAsync(lv_status, 0, sizeof(unsigned long long) * (lv_tiles + 1), st));
         }
-        { k_levels<<<tiles, LV_THREADS, 0, st>>>(v, E, keys, L, nstart, elem_of_slot, nd.cap - slot_base, &sum->nodes,
-                                                 lv_status, (int *)(lv_status + lv_tiles), scan_spins()); tg::note_launch(); }
+        TG_CHAIN(k_levels, tiles, LV_THREADS, 0, st, v, E, keys, L, nstart, elem_of_slot, nd.cap - slot_base,
+                 &sum->nodes, lv_status, (int *)(lv_status + lv_tiles), scan_spins());
         // The round's nodes, particle links and the summary, read back with one copy. Slots that
         // do not fit are skipped by k_nodes; the host then grows the arrays and runs it again.
         auto run_round = [&]() -> tg_status {
             const int elem_blocks = div_up(E, NODE_THREADS);
-            { k_nodes<<<elem_blocks + div_up(nd.cap - slot_base, NODE_THREADS), NODE_THREADS, 0, st>>>(
-                v, E, elem_blocks, L, nstart, elem_of_slot, slot_base, &sum->nodes, keys, nd, exh, &sum->n_exh, exh_cap,
-                root_first, p_parent, p_next, N, round == 0 ? sum : nullptr, nonfinite); tg::note_launch(); }
+            TG_CHAIN(k_nodes, elem_blocks + div_up(nd.cap - slot_base, NODE_THREADS), NODE_THREADS, 0, st, v, E,
+                     elem_blocks, L, nstart, elem_of_slot, slot_base, &sum->nodes, keys, nd, exh, &sum->n_exh,
+                     exh_cap, root_first, p_parent, p_next, N, round == 0 ? sum : nullptr, nonfinite);
             if (round > 0) {
                 { k_set_root_first<<<LAUNCH(sg.n)>>>(sg.root, root_first, sg.n, nd.first); tg::note_launch(); }
-                { k_summarize_slots<<<LAUNCH(std::max<int64_t>(nd.cap, N))>>>(nd, slot_base, &sum->nodes, p_parent, p_next,
-                                                                           N, sum, nonfinite); tg::note_launch(); }
+                TG_CHAIN(k_summarize_slots, div_up(std::max<int64_t>(nd.cap, N), 256), 256, 0, st, nd, slot_base,
+                         &sum->nodes, p_parent, p_next, N, sum, nonfinite);
             }
             TG_CUDA(cudaGetLastError());
             TG_TRY(read_summary());
@@ -1925,8 +1959,8 @@ tg_status build_tree(tg_tree_s *T, const double *pos, const StageMH &stage_mh,
     // 6. reference numbering
     if (!summary_final) {  // buckets were made after the last summary: validate every slot again
         TG_CUDA(cudaMemsetAsync(sum, 0, sizeof(BuildSummary), st));
-        { k_summarize_slots<<<LAUNCH(std::max<int64_t>(nd.count, N))>>>(nd, nd.count, nullptr, p_parent, p_next, N,
-                                                                      sum, nonfinite); tg::note_launch(); }
+        TG_CHAIN(k_summarize_slots, div_up(std::max<int64_t>(nd.count, N), 256), 256, 0, st, nd, nd.count, nullptr,
+                 p_parent, p_next, N, sum, nonfinite);
         TG_CUDA(cudaGetLastError());
         TG_TRY(read_summary());
     }
@@ -1968,7 +2002,8 @@ tg_status build_tree(tg_tree_s *T, const double *pos, const StageMH &stage_mh,
     const int key_bits = sysbits + nb.lb + nb.db + (compact ? 3 : nb.lb);
     const int sort_bits = key_bits < 64 ? key_bits + 1 : 64;
     const uint64_t root_key = key_bits < 64 ? (1ull << key_bits) : ~0ull;
-    { k_number_keys<<<LAUNCH(M)>>>(nd, M, sys_off, nb, root_key, compact, nkeys, nvals, root_slot); tg::note_launch(); }
+    TG_CHAIN(k_number_keys, div_up(M, 256), 256, 0, st, nd, M, sys_off, nb, root_key, compact, nkeys, nvals,
+             root_slot);
     TG_CUDA(cudaGetLastError());
     SortedPairs numbered(st);
     TG_TRY(radix_sort_pairs(nkeys, nvals, M, sort_bits, st, T->sort_err, true, &numbered));
@@ -1981,8 +2016,8 @@ tg_status build_tree(tg_tree_s *T, const double *pos, const StageMH &stage_mh,
     } else {
         T->sys_node_off.assign(nsys + 1, 0);
     }
-    { k_final_index<<<LAUNCH(std::max<int64_t>(M, nsys))>>>(nkeys, nvals, M, nd.sys, N, key_bits - sysbits,
-                                                         sys_node_off, final_of_slot, root_slot, nsys, T->sort_err); tg::note_launch(); }
+    TG_CHAIN(k_final_index, div_up(std::max<int64_t>(M, nsys), 256), 256, 0, st, nkeys, nvals, M, nd.sys, N,
+             key_bits - sysbits, sys_node_off, final_of_slot, root_slot, nsys, T->sort_err);
     TG_CUDA(cudaGetLastError());
     // capacity (NumNodes) per system: bucket reservations, read with the final synchronisation
     if (n_bucket > 0) {
@@ -2008,8 +2043,8 @@ tg_status build_tree(tg_tree_s *T, const double *pos, const StageMH &stage_mh,
     FinalArrays fa{T->coord, T->mass, T->soft, T->size, T->delta, T->first, T->next, T->parent, T->node_range,
                    T->cell_center};
     const int node_blocks = div_up(M, 256);
-    { k_write<<<node_blocks + div_up(N, 256), 256, 0, st>>>(nd, M, N, node_blocks, final_of_slot, fa, lo, lvl_cursor,
-                                                            lvl_list, fdepth, p_parent, p_next, pc, pm, ps, &sum->bad); tg::note_launch(); }
+    TG_CHAIN(k_write, node_blocks + div_up(N, 256), 256, 0, st, nd, M, N, node_blocks, final_of_slot, fa, lo,
+             lvl_cursor, lvl_list, fdepth, p_parent, p_next, pc, pm, ps, &sum->bad);
     TG_CUDA(cudaGetLastError());
 
     // 8. the one closing synchronisation, ahead of the moment pass (nothing the host needs comes from
@@ -2081,7 +2116,7 @@ tg_status build_tree(tg_tree_s *T, const double *pos, const StageMH &stage_mh,
                 c.take(a.arrived, M);
             }
         }));
-        { k_kids<<<LAUNCH(M)>>>(N, M, T->first, T->next, kids, nk); tg::note_launch(); }
+        TG_CHAIN(k_kids, div_up(M, 256), 256, 0, st, N, M, T->first, T->next, kids, nk);
         if (ndeep > 0) {
             TG_CUDA(cudaMemsetAsync(a.nchild, 0, sizeof(int) * M, st));
             TG_CUDA(cudaMemsetAsync(a.arrived, 0, sizeof(int) * M, st));
@@ -2096,15 +2131,10 @@ tg_status build_tree(tg_tree_s *T, const double *pos, const StageMH &stage_mh,
             const int c = hs.depth_hist[d];
             if (c <= 0) continue;
             const int32_t *lst = lvl_list + off[d];
-            if (c <= WIDE_MAX_LEVEL)
-                k_moments_wide<<<div_up(c, WIDE_NODES), WIDE_THREADS, 0, st>>>(a, lst, c, kids, nk);
-            else if (div_up(c, 256) >= want)
-                k_moments_sorted<256><<<div_up(c, 256), 256, 0, st>>>(a, lst, c, kids, nk);
-            else if (div_up(c, 128) >= want)
-                k_moments_sorted<128><<<div_up(c, 128), 128, 0, st>>>(a, lst, c, kids, nk);
-            else
-                k_moments_sorted<64><<<div_up(c, 64), 64, 0, st>>>(a, lst, c, kids, nk);
-            tg::note_launch();
+            if (c <= WIDE_MAX_LEVEL) TG_CHAIN(k_moments_wide, div_up(c, WIDE_NODES), WIDE_THREADS, 0, st, a, lst, c, kids, nk);
+            else if (div_up(c, 256) >= want) TG_CHAIN(k_moments_sorted<256>, div_up(c, 256), 256, 0, st, a, lst, c, kids, nk);
+            else if (div_up(c, 128) >= want) TG_CHAIN(k_moments_sorted<128>, div_up(c, 128), 128, 0, st, a, lst, c, kids, nk);
+            else TG_CHAIN(k_moments_sorted<64>, div_up(c, 64), 64, 0, st, a, lst, c, kids, nk);
         }
         TG_CUDA(cudaGetLastError());
     } else {
@@ -2151,7 +2181,7 @@ tg_status ensure_quad64(tg_tree_s *T, cudaStream_t st) {
     int8_t *nk = nullptr;
     TG_TRY(dalloc(&kids, 8 * M, st));
     TG_TRY(dalloc(&nk, M, st));
-    { k_kids<<<LAUNCH(M)>>>(N, M, T->first, T->next, kids, nk); tg::note_launch(); }
+    TG_CHAIN(k_kids, div_up(M, 256), 256, 0, st, N, M, T->first, T->next, kids, nk);
     const int ndeep = off[DEPTH_CAP + 1] - off[DEPTH_CAP];
     if (ndeep > 0) {
         TG_TRY(dalloc(&a.nchild, M, st));
@@ -2164,7 +2194,7 @@ tg_status ensure_quad64(tg_tree_s *T, cudaStream_t st) {
     for (int d = DEPTH_CAP - 1; d >= 0; d--) {
         const int c = off[d + 1] - off[d];
         if (c <= 0) continue;
-        { k_quad64_level<<<div_up(c, 64), 64, 0, st>>>(a, T->lvl_list + off[d], c, kids, nk); tg::note_launch(); }
+        TG_CHAIN(k_quad64_level, div_up(c, 64), 64, 0, st, a, T->lvl_list + off[d], c, kids, nk);
     }
     TG_CUDA(cudaGetLastError());
     dfree(kids, st); dfree(nk, st); dfree(a.nchild, st); dfree(a.arrived, st);
@@ -2193,8 +2223,9 @@ tg_status morton_order_device(const double *pos, int64_t n, uint32_t *perm, cuda
     TG_CUDA(cudaMemsetAsync(cube.p->mx, 0, sizeof(Cube) - sizeof(cube.p->mn), st));
     int *err = err_dev ? err_dev : &cube.p->err;
     { k_bbox<<<div_up(n, BB_THREADS * BB_ITEMS), BB_THREADS, 0, st>>>(pos, n, nullptr, 1, cube.p->mn, cube.p->mx); tg::note_launch(); }
-    { k_bbox_finish<<<1, 32, 0, st>>>(cube.p->mn, cube.p->mx, 1, cube.p->center, &cube.p->size); tg::note_launch(); }
-    { k_keys<<<LAUNCH(n)>>>(pos, n, nullptr, 1, cube.p->center, &cube.p->size, nullptr, keys.p, nullptr, perm); tg::note_launch(); }
+    TG_CHAIN(k_bbox_finish, 1, 32, 0, st, cube.p->mn, cube.p->mx, 1, cube.p->center, &cube.p->size);
+    TG_CHAIN(k_keys, div_up(n, 256), 256, 0, st, pos, n, nullptr, 1, cube.p->center, &cube.p->size, nullptr, keys.p,
+             nullptr, perm);
     TG_CUDA(cudaGetLastError());
     SortedPairs sorted(st);
     TG_TRY(radix_sort_pairs(keys.p, perm, n, 63, st, err, false, &sorted));

@@ -36,6 +36,7 @@ constexpr uint32_t LINK_NONE = 0xffffffffu;  // elements number below 2^32 - 1 (
 __device__ __forceinline__ uint32_t pack_link(int64_t e) { return e < 0 ? LINK_NONE : (uint32_t)e; }
 
 __global__ void k_column_prep(ColumnTree t, float4 *rec) {
+    chain_next();
     const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= t.nelem) return;
     float4 a, b;
@@ -196,6 +197,8 @@ __device__ double column_walk(const ColumnTree &t, bool active, const double *p,
 __global__ void __launch_bounds__(COL_THREADS, COL_BLOCKS_PER_SM) k_column_rays(ColumnTree t, const double *pos, int64_t n,
                                                              const double *rays, int64_t nrays, int64_t ray_stride,
                                                              double *out, int *runaway) {
+    chain_wait();
+    chain_next();
     __shared__ uint32_t queue[COL_QUEUE][COL_THREADS];
     const int64_t pair = (int64_t)blockIdx.x * COL_THREADS + threadIdx.x;
     const bool active = pair < n * nrays;
@@ -430,8 +433,8 @@ tg_status tg_tree_column_density(tg_tree t, const double *pos, int64_t n, const 
         ct.rec = fcopy;
         k_column_prep<<<div_up(ct.nelem, 256), 256, 0, st>>>(ct, fcopy);
         note_launch();
-        k_column_rays<<<div_up(n * nrays, COL_THREADS), COL_THREADS, 0, st>>>(ct, dpos, n, drays, nrays, ray_stride, dout, flag);
-        note_launch();
+        TG_CHAIN(k_column_rays, div_up(n * nrays, COL_THREADS), COL_THREADS, 0, st, ct, dpos, n, drays, nrays,
+                 ray_stride, dout, flag);
     }
     TG_CUDA(cudaGetLastError());
     int hflag = 0;

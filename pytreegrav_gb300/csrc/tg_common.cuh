@@ -232,6 +232,36 @@ __device__ __forceinline__ long long scan_look_back(long long sum, int tile, uns
     return before;
 }
 
+// Kernels that follow one another closely in a stream: launched with launch_after, a kernel's blocks come up while
+// the one before is still finishing; chain_wait (first, in every block, before any memory is touched) then waits
+// for that kernel's completion, which includes that of all before it, and chain_next lets the following kernel come
+// up in its turn, once every block here has got past its wait. A kernel without chain_wait must not be
+// launched this way. Saves most of the ~2 us and of the ramp between two dependent kernels: build of 12345 particles (49
+// launches) 322 -> 244 us, with its walk 673 -> 574; build of 1e6 688 -> 636.
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+template <class... P, class... A>
+inline cudaError_t launch_after(void (*kernel)(P...), int64_t grid, int block, size_t smem, cudaStream_t s, A... args) {
+    cudaLaunchConfig_t c = {};
+    c.gridDim = dim3((unsigned)grid);
+    c.blockDim = dim3((unsigned)block);
+    c.dynamicSmemBytes = smem;
+    c.stream = s;
+    cudaLaunchAttribute a[1];
+    a[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    a[0].val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = a;
+    c.numAttrs = 1;
+    return cudaLaunchKernelEx(&c, kernel, P(args)...);
+}
+
+// launch_after in a function that returns a tg_status, counted as a launch.
+#define TG_CHAIN(...)                             \
+    do {                                          \
+        TG_CUDA(tg::launch_after(__VA_ARGS__));   \
+        tg::note_launch();                        \
+    } while (0)
+
 inline int div_up(int64_t a, int64_t b) { return (int)((a + b - 1) / b); }
 
 // Device-wide helpers implemented in tg_scan.cu / tg_sort.cu.

@@ -45,6 +45,8 @@ __device__ __forceinline__ double nearest_image(double x, double box) {
 
 // Depth of every node (root 0) by climbing parent links; a climb longer than the bound sets *bad.
 __global__ void k_node_depth(int64_t ntot, int64_t mtot, const int64_t *parent, int *depth, int *maxdepth, int *bad) {
+    chain_wait();
+    chain_next();
     const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= mtot) return;
     int d = 0;
@@ -60,6 +62,7 @@ __global__ void k_node_depth(int64_t ntot, int64_t mtot, const int64_t *parent, 
 
 // Particle velocities in tree (walk) order, and zero dispersion for particles.
 __global__ void k_gather_vel(int64_t ntot, const int64_t *walk_idx, const double *vel_in, double *vel) {
+    chain_next();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= ntot) return;
     const int64_t o = walk_idx[i];
@@ -73,6 +76,8 @@ __global__ void k_gather_vel(int64_t ntot, const int64_t *walk_idx, const double
 // over m, children in chain order, each operation rounded once. disp is per element (particles 0).
 __global__ void k_vel_level(int64_t ntot, int64_t mtot, int level, const int *depth, const int64_t *first,
                             const int64_t *next, const double *mass, double *vel, double *disp) {
+    chain_wait();
+    chain_next();
     const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= mtot || depth[j] != level) return;
     const int64_t f = ntot + j, stop = next[f], ne = ntot + mtot;
@@ -328,6 +333,8 @@ __device__ __forceinline__ int bin_screen(const CorrArgs &a, float r, float er) 
 constexpr int CORR_QUEUE = 16;  // entries per lane (8 to 32: within 4 %)
 
 __global__ void __launch_bounds__(CORR_THREADS, CORR_BLOCKS_PER_SM) k_corr(CorrArgs a) {
+    chain_wait();
+    chain_next();
     __shared__ uint32_t q_elem[CORR_QUEUE][CORR_THREADS];
     __shared__ uint16_t q_bin[CORR_QUEUE][CORR_THREADS];
     const int tid = blockIdx.x * blockDim.x + threadIdx.x;
@@ -452,6 +459,7 @@ __global__ void __launch_bounds__(CORR_THREADS, CORR_BLOCKS_PER_SM) k_corr(CorrA
 // max(s / theta + delta, 0.6 s + delta), formed in FP64 and rounded.
 __global__ void k_corr_prep(int64_t ntot, int64_t nelem, const double *coord, const double *size, const double *delta,
                             const int64_t *next, const int64_t *first, double theta, float4 *rec) {
+    chain_next();
     const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= nelem) return;
     float hx, lx, hy, ly, hz, lz;
@@ -470,6 +478,8 @@ __global__ void k_corr_prep(int64_t ntot, int64_t nelem, const double *coord, co
 }
 
 __global__ void k_corr_whole(const double *rbins, int nbins, double mbr, long long *whole, float *whole32) {
+    chain_wait();
+    chain_next();
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b >= nbins) return;
     const double w = dmul(mbr, dsub(rbins[b + 1], rbins[b]));
@@ -481,6 +491,8 @@ __global__ void k_corr_whole(const double *rbins, int nbins, double mbr, long lo
 // One block per output value (bin sums, then weight sums): thread t adds rows t, t + CORR_RED, ...
 // in order, then a fixed-shape tree adds the threads' sums.
 __global__ void __launch_bounds__(CORR_RED) k_corr_reduce(const double *rows, int nrows, int nbins, double *out) {
+    chain_wait();
+    chain_next();
     __shared__ double sh[CORR_RED];
     const int b = blockIdx.x, t = threadIdx.x;
     double s = 0.0;
@@ -510,6 +522,8 @@ struct SelectState {
 template <bool COLUMNS>
 __global__ void __launch_bounds__(SEL_THREADS) k_select(const double *pos, const unsigned long long *keys, int64_t n,
                                                         int pass, SelectState *st) {
+    chain_wait();
+    chain_next();
     constexpr int Q = COLUMNS ? SEL_Q : 1;
     __shared__ unsigned h[Q][256];
     __shared__ bool last;
@@ -559,6 +573,8 @@ __global__ void __launch_bounds__(SEL_THREADS) k_select(const double *pos, const
 // middle values, equal for an odd count) and sqrt(dx dx + dy dy + dz dz), each operation rounded once.
 __global__ void __launch_bounds__(SEL_THREADS) k_radial_keys(const double *pos, int64_t n, const SelectState *st,
                                                              unsigned long long *keys, unsigned long long *largest) {
+    chain_wait();
+    chain_next();
     double med[3];
     for (int c = 0; c < 3; c++)
         med[c] = n & 1 ? ordered_to_dbl(st->prefix[2 * c])
@@ -609,9 +625,10 @@ tg_status tg_radial_range(const double *pos, int64_t n, int64_t rank, int mem, d
     TG_CUDA(cudaMemcpyAsync(state.p[0].rank, ranks, sizeof(ranks), cudaMemcpyHostToDevice, st));
     TG_CUDA(cudaMemcpyAsync(state.p[1].rank, &first, sizeof(first), cudaMemcpyHostToDevice, st));
     const int blocks = (int)std::min<int64_t>(div_up(n, 4 * SEL_THREADS), 2 * num_sms());
-    for (int p = 0; p < SEL_PASSES; p++) { k_select<true><<<blocks, SEL_THREADS, 0, st>>>(dp, nullptr, n, p, state.p); note_launch(); }
-    { k_radial_keys<<<blocks, SEL_THREADS, 0, st>>>(dp, n, state.p, keys.p, largest); note_launch(); }
-    for (int p = 0; p < SEL_PASSES; p++) { k_select<false><<<blocks, SEL_THREADS, 0, st>>>(nullptr, keys.p, n, p, state.p + 1); note_launch(); }
+    for (int p = 0; p < SEL_PASSES; p++) TG_CHAIN(k_select<true>, blocks, SEL_THREADS, 0, st, dp, nullptr, n, p, state.p);
+    TG_CHAIN(k_radial_keys, blocks, SEL_THREADS, 0, st, dp, n, state.p, keys.p, largest);
+    for (int p = 0; p < SEL_PASSES; p++)
+        TG_CHAIN(k_select<false>, blocks, SEL_THREADS, 0, st, nullptr, keys.p, n, p, state.p + 1);
     TG_CUDA(cudaGetLastError());
     unsigned long long got[2];
     TG_CUDA(cudaMemcpyAsync(got, state.p[1].prefix, sizeof(got[0]), cudaMemcpyDeviceToHost, st));
@@ -644,7 +661,7 @@ tg_status tg_tree_set_velocities(tg_tree t, const double *vel, int mem, void *st
     TG_CUDA(depth.alloc(M));
     TG_CUDA(flags.alloc(2));
     TG_CUDA(cudaMemsetAsync(flags.p, 0, 2 * sizeof(int), st));
-    if (M > 0) { k_node_depth<<<div_up(M, 256), 256, 0, st>>>(N, M, t->parent, depth.p, flags.p, flags.p + 1); note_launch(); }
+    if (M > 0) TG_CHAIN(k_node_depth, div_up(M, 256), 256, 0, st, N, M, t->parent, depth.p, flags.p, flags.p + 1);
     TG_CUDA(cudaGetLastError());
     int hf[2] = {0, 0};
     TG_CUDA(cudaMemcpyAsync(hf, flags.p, sizeof(hf), cudaMemcpyDeviceToHost, st));
@@ -654,8 +671,8 @@ tg_status tg_tree_set_velocities(tg_tree t, const double *vel, int mem, void *st
         return TG_ERR_ITER_LIMIT;
     }
     for (int d = hf[0]; d >= 0; d--) {
-        k_vel_level<<<div_up(M, 256), 256, 0, st>>>(N, M, d, depth.p, t->first, t->next, t->mass, t->vel, t->vdisp);
-        note_launch();
+        TG_CHAIN(k_vel_level, div_up(M, 256), 256, 0, st, N, M, d, depth.p, t->first, t->next, t->mass, t->vel,
+                 t->vdisp);
     }
     TG_CUDA(cudaGetLastError());
     TG_CUDA(cudaStreamSynchronize(st));
@@ -765,7 +782,7 @@ tg_status tg_tree_correlation(tg_tree t, int kind, const double *pos, const doub
     TG_CUDA(whole32.alloc(nbins));
     { k_corr_prep<<<div_up(a.nelem, 256), 256, 0, st>>>(t->ntot, a.nelem, t->coord, t->size, t->delta, t->next, t->first,
                                                           theta, rec.p); note_launch(); }
-    { k_corr_whole<<<div_up(nbins, 256), 256, 0, st>>>(a.rbins, nbins, max_bin_size_ratio, whole.p, whole32.p); note_launch(); }
+    TG_CHAIN(k_corr_whole, div_up(nbins, 256), 256, 0, st, a.rbins, nbins, max_bin_size_ratio, whole.p, whole32.p);
     a.rec = rec.p;
     a.whole = whole.p;
     a.whole32 = whole32.p;
@@ -785,8 +802,8 @@ tg_status tg_tree_correlation(tg_tree t, int kind, const double *pos, const doub
         a.tscale32 = (float)((double)nbins / (std::log10(rbn) - std::log10(rb0)));
         a.box32 = (float)boxsize;
     }
-    { k_corr<<<div_up(nrows, CORR_THREADS), CORR_THREADS, 0, st>>>(a); note_launch(); }
-    { k_corr_reduce<<<2 * nbins, CORR_RED, 0, st>>>(rows.p, a.nrows, nbins, dout.p); note_launch(); }
+    TG_CHAIN(k_corr, div_up(nrows, CORR_THREADS), CORR_THREADS, 0, st, a);
+    TG_CHAIN(k_corr_reduce, 2 * nbins, CORR_RED, 0, st, rows.p, a.nrows, nbins, dout.p);
     TG_CUDA(cudaGetLastError());
     const cudaMemcpyKind kd = host ? cudaMemcpyDeviceToHost : cudaMemcpyDeviceToDevice;
     TG_CUDA(cudaMemcpyAsync(binsums, dout.p, sizeof(double) * nbins, kd, st));

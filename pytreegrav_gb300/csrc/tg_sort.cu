@@ -449,6 +449,8 @@ __global__ void __launch_bounds__(HIST_THREADS) k_sort_hist(const uint64_t *keys
     __shared__ int h[MAX_PASSES * OS_BINS];
     __shared__ int tot[MAX_PASSES * HIST_THREADS / 32];
     __shared__ bool last;
+    chain_wait();
+    chain_next();
     for (int i = threadIdx.x; i < npass * OS_BINS; i += HIST_THREADS) h[i] = 0;
     __syncthreads();
     const unsigned mask = (1u << width) - 1;
@@ -508,6 +510,8 @@ __global__ void __launch_bounds__(OS_THREADS, 2)
     extern __shared__ __align__(16) unsigned char os_raw[];
     OsSmem<ROUNDS> &sm = *reinterpret_cast<OsSmem<ROUNDS> *>(os_raw);
     constexpr int TILE = OsTile<ROUNDS>::KEYS;
+    chain_wait();
+    chain_next();
     if (threadIdx.x == 0) sm.tile = atomicAdd(tile_counter, 1);
     const int w = threadIdx.x >> 5, lane = lane_id();
     const unsigned lt = lanemask_lt(), mask = (1u << width) - 1;
@@ -629,6 +633,8 @@ __global__ void __launch_bounds__(OS_THREADS, 2)
 // written), every value becomes its own index and every key its own position -- sorted pairs and a
 // valid permutation, so every later kernel sees well-formed input -- and the caller's flag is set.
 __global__ void k_sort_fallback(uint64_t *keys, uint32_t *vals, int64_t n, const int *local_err, int *err) {
+    chain_wait();
+    chain_next();
     if (!*local_err) return;
     const int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i0 == 0) atomicExch(err, 1);
@@ -671,15 +677,15 @@ tg_status radix_sort_pairs(uint64_t *keys, uint32_t *vals, int64_t n, int bits, 
     uint32_t *v2 = (uint32_t *)(scr + head + key_bytes);
     TG_CUDA(cudaMemsetAsync(scr, 0, head, s));
     const int hblocks = (int)std::min<int64_t>(div_up(n, HIST_THREADS * 4), (int64_t)num_sms() * 4);
-    { k_sort_hist<<<hblocks, HIST_THREADS, 0, s>>>(keys, n, npass, width, hist, done); tg::note_launch(); }
+    TG_CHAIN(k_sort_hist, hblocks, HIST_THREADS, 0, s, keys, n, npass, width, hist, done);
     auto pass = lng ? k_onesweep<12> : k_onesweep<8>;
     const int smem = lng ? (int)sizeof(OsSmem<12>) : (int)sizeof(OsSmem<8>);
     TG_CUDA(cudaFuncSetAttribute(pass, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     uint64_t *kin = keys, *kout = k2;
     uint32_t *vin = vals, *vout = v2;
     for (int p = 0; p < npass; p++) {
-        { pass<<<ntiles, OS_THREADS, smem, s>>>(kin, vin, n, width * p, width, p, hist + p * OS_BINS, status, counters + p,
-                                                kout, vout, local_err, spin_limit); tg::note_launch(); }
+        TG_CHAIN(pass, ntiles, OS_THREADS, smem, s, kin, vin, n, width * p, width, p, hist + p * OS_BINS, status,
+                 counters + p, kout, vout, local_err, spin_limit);
         uint64_t *tk = kin; kin = kout; kout = tk;
         uint32_t *tv = vin; vin = vout; vout = tv;
     }
@@ -693,7 +699,8 @@ tg_status radix_sort_pairs(uint64_t *keys, uint32_t *vals, int64_t n, int bits, 
         kin = keys;
         vin = vals;
     }
-    if (!caller_falls_back) { k_sort_fallback<<<std::min(div_up(n, 256), 4 * num_sms()), 256, 0, s>>>(kin, vin, n, local_err, err); tg::note_launch(); }
+    if (!caller_falls_back) TG_CHAIN(k_sort_fallback, std::min(div_up(n, 256), 4 * num_sms()), 256, 0, s, kin, vin, n,
+                                     local_err, err);
     TG_CUDA(cudaGetLastError());
     return TG_OK;
 }

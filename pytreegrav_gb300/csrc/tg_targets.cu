@@ -48,6 +48,8 @@ int width_of(int fields) { return ((fields & 1) ? 1 : 0) + ((fields & 2) ? 3 : 0
 __global__ void k_target_src_nodes(int64_t ntot, int64_t mtot, const double *cell, const double *size, Arena<float> ar,
                                    const int2 *node_range, const double *tpos, const int2 *groups, int64_t ng, int G,
                                    int *node, int *nsub, int *sublen) {
+    chain_wait();
+    chain_next();
     const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= ng) return;
     const int2 gr = groups[g];
@@ -124,6 +126,8 @@ __global__ void k_target_src_nodes(int64_t ntot, int64_t mtot, const double *cel
 // offset off[g], in start order.
 __global__ void k_split_groups(const int2 *groups, const int *gnode, int64_t ng, const int *nsub, const int *sublen,
                                const int *off, int2 *out, int *out_root, int *out_node) {
+    chain_wait();
+    chain_next();
     const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= ng) return;
     const int2 gr = groups[g];
@@ -145,10 +149,9 @@ tg_status targets_src_nodes(tg_targets_s *ts, cudaStream_t st) {
     const int64_t ng = tt->ngroups;
     TG_CUDA(dev_malloc((void **)&ts->src_node, sizeof(int) * std::max<int64_t>(ng, 1), st));
     if (ng > 0) {
-        k_target_src_nodes<<<div_up(ng, 128), 128, 0, st>>>(src->ntot, src->mtot, src->cell_center, src->size,
-                                                            src->arena32, src->node_range, tt->coord, tt->groups, ng,
-                                                            ts->group_size, ts->src_node, nullptr, nullptr);
-        note_launch();
+        TG_CHAIN(k_target_src_nodes, div_up(ng, 128), 128, 0, st, src->ntot, src->mtot, src->cell_center, src->size,
+                 src->arena32, src->node_range, tt->coord, tt->groups, ng, ts->group_size, ts->src_node, nullptr,
+                 nullptr);
         TG_CUDA(cudaGetLastError());
     }
     return TG_OK;
@@ -168,9 +171,8 @@ tg_status targets_refine_groups(tg_targets_s *ts, cudaStream_t st) {
     TG_CUDA(sublen.alloc(ng));
     TG_CUDA(off.alloc(ng + 1));
     TG_CUDA(cudaMemsetAsync(nsub.p + ng, 0, sizeof(int), st));
-    { k_target_src_nodes<<<div_up(ng, 128), 128, 0, st>>>(src->ntot, src->mtot, src->cell_center, src->size,
-                                                         src->arena32, src->node_range, tt->coord, tt->groups, ng,
-                                                         ts->group_size, node.p, nsub.p, sublen.p); note_launch(); }
+    TG_CHAIN(k_target_src_nodes, div_up(ng, 128), 128, 0, st, src->ntot, src->mtot, src->cell_center, src->size,
+             src->arena32, src->node_range, tt->coord, tt->groups, ng, ts->group_size, node.p, nsub.p, sublen.p);
     TG_CUDA(cudaGetLastError());
     TG_TRY(exclusive_scan_i32(nsub.p, off.p, ng + 1, st));
     int total = 0;
@@ -182,8 +184,8 @@ tg_status targets_refine_groups(tg_targets_s *ts, cudaStream_t st) {
     TG_CUDA(dev_malloc((void **)&groups, sizeof(int2) * total, st));
     TG_CUDA(dev_malloc((void **)&root, sizeof(int) * total, st));
     TG_CUDA(dev_malloc((void **)&gnode, sizeof(int) * total, st));
-    { k_split_groups<<<div_up(ng, 128), 128, 0, st>>>(tt->groups, tt->group_node, ng, nsub.p, sublen.p, off.p, groups,
-                                                     root, gnode); note_launch(); }
+    TG_CHAIN(k_split_groups, div_up(ng, 128), 128, 0, st, tt->groups, tt->group_node, ng, nsub.p, sublen.p, off.p,
+             groups, root, gnode);
     TG_CUDA(cudaGetLastError());
     cudaFreeAsync(tt->groups, st);
     cudaFreeAsync(tt->group_root, st);

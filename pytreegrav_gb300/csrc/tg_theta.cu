@@ -58,6 +58,8 @@ __global__ void k_copy_groups(const int2 *groups, const int *node, int64_t ng, i
 // centre (float3 + pad). One block; *ntop receives the count.
 __global__ void k_top_nodes(Arena<float> ar, int64_t ntot, const double *coord, const double *mass,
                             const double *size, int *top, int *ntop, float4 *rec, float *hs2, float4 *origin) {
+    chain_wait();
+    chain_next();
     __shared__ int cur[TOP_MAX], nxt[TOP_MAX], fr[TOP_MAX];
     __shared__ int ncur, nnxt, nout;
     if (ar.bad && *ar.bad) {  // the arena is invalid (the walk reports it): no frontier
@@ -132,6 +134,8 @@ __global__ void k_features(int64_t ntot, const double *coord, const double *mass
                            int64_t ngroups,
                            const float4 *rec, const float *hs2, const int *ntop_p, const float4 *origin, int quad,
                            float log10n, float *feat, unsigned long long *field_sums) {
+    chain_wait();
+    chain_next();
     // the tolerance unit's sums, added per block and then once to field_sums
     __shared__ unsigned long long red[2];
     if (threadIdx.x == 0) red[0] = red[1] = 0ull;
@@ -443,6 +447,8 @@ struct TolOut {
 __global__ void __launch_bounds__(INF_WARPS * 32) k_theta_infer(ModelDev md, const float *feat, int64_t n,
                                                                 float loglam, float tmin, float tmax, float *theta,
                                                                 TolOut ts) {
+    chain_wait();
+    chain_next();
     __shared__ uint32_t sw1[H * NF / 2], sw2[H * H / 2];
     __shared__ float sb1[H], sb2[H], sw3[H], smu[NF], sis[NF];
     __shared__ float sscale;
@@ -534,6 +540,8 @@ __global__ void k_to_bf16_pairs(const float *w, int npairs, uint32_t *out) {
 
 // Non-finite or out-of-range outputs (a damaged model) are replaced by `fallback`.
 __global__ void k_theta_guard(float *theta, int64_t n, float fallback, float tmin, float tmax) {
+    chain_wait();
+    chain_next();
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     float v = theta[i];
@@ -591,12 +599,12 @@ tg_status features_of_groups(tg_tree_s *t, const double *tcoord, const double *t
     float *hs2 = (float *)(origin + 1);
     unsigned long long *sums = field_sums ? field_sums : (unsigned long long *)(origin + 1 + TOP_MAX / 4);
     TG_CUDA(cudaMemsetAsync(sums, 0, 2 * sizeof(unsigned long long), st));
-    { k_top_nodes<<<1, 256, 0, st>>>(t->arena32, t->ntot, t->coord, t->mass, t->size, top + 1, top, rec, hs2, origin); note_launch(); }
+    TG_CHAIN(k_top_nodes, 1, 256, 0, st, t->arena32, t->ntot, t->coord, t->mass, t->size, top + 1, top, rec, hs2,
+             origin);
     if (ng > 0) {
-        k_features<<<div_up(ng * 32, 256), 256, 0, st>>>(t->ntot, t->coord, t->mass, t->size, tcoord, tsoft, groups,
-                                                         group_node, ng, rec, hs2, top, origin, quadrupole,
-                                                         (float)log10((double)t->ntot), feat, sums);
-        note_launch();
+        TG_CHAIN(k_features, div_up(ng * 32, 256), 256, 0, st, t->ntot, t->coord, t->mass, t->size, tcoord, tsoft,
+                 groups, group_node, ng, rec, hs2, top, origin, quadrupole, (float)log10((double)t->ntot), feat,
+                 sums);
     }
     TG_CUDA(cudaGetLastError());
     TG_CUDA(cudaFreeAsync(scr, st));
@@ -638,7 +646,7 @@ tg_status infer_device(const tg_theta_model_s *m, const float *feat, int64_t n, 
     if (n <= 0) return TG_OK;
     const int64_t tiles = (n + 15) / 16;
     const int grid = (int)std::min<int64_t>((tiles + INF_WARPS - 1) / INF_WARPS, (int64_t)num_sms() * 8);
-    { k_theta_infer<<<grid, INF_WARPS * 32, 0, st>>>(m->dev, feat, n, loglam, m->tmin, m->tmax, theta, ts); note_launch(); }
+    TG_CHAIN(k_theta_infer, grid, INF_WARPS * 32, 0, st, m->dev, feat, n, loglam, m->tmin, m->tmax, theta, ts);
     TG_CUDA(cudaGetLastError());
     return TG_OK;
 }
@@ -671,7 +679,8 @@ tg_status learned_walk(tg_tree_s *t, FeatFn feats, const double *tpos, const dou
         if (m->kind == TG_THETA_KIND_ANGLE) {
             TG_CUDA(dev_malloc((void **)&tg_theta, sizeof(float) * ng1, st));
             TG_TRY(infer_device(m, feat, ng, log10_lambda, tg_theta, st));
-            { k_theta_guard<<<div_up(ng, 256), 256, 0, st>>>(tg_theta, ng, (float)theta_fallback, m->tmin, m->tmax); note_launch(); }
+            TG_CHAIN(k_theta_guard, div_up(ng, 256), 256, 0, st, tg_theta, ng, (float)theta_fallback, m->tmin,
+                     m->tmax);
             TG_CUDA(cudaGetLastError());
         } else {  // the tolerances straight from the inference (tolerances_device's values)
             TG_CUDA(dev_malloc((void **)&tol, sizeof(float) * ng1, st));

@@ -159,6 +159,8 @@ constexpr int LINK_THREADS = 256;
 __global__ void __launch_bounds__(LINK_THREADS) k_arena_links(int64_t ntot, int64_t mtot, const int64_t *first,
                                                               const int64_t *next, int4 *link, int *bad,
                                                               unsigned long long *status, int *counter, long long spins) {
+    chain_wait();
+    chain_next();
     __shared__ int warp_sum[LINK_THREADS / 32];
     __shared__ long long before_s;
     __shared__ int tile_s;
@@ -221,6 +223,8 @@ __global__ void __launch_bounds__(LINK_THREADS) k_arena_links(int64_t ntot, int6
 template <typename T>
 __global__ void k_arena_leaves(int64_t ntot, int64_t mtot, const int64_t *first, const int64_t *next,
                                const double *coord, const double *mass, const double *soft, Arena<T> ar) {
+    chain_wait();
+    chain_next();
     int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= mtot) return;
     int64_t f = ntot + j, stop = next[f];
@@ -250,6 +254,8 @@ template <typename T>
 __global__ void k_arena_nodes(int64_t ntot, int64_t mtot, const double *coord, const double *mass,
                               const double *soft, const double *size, const double *delta, const double *quad,
                               const float4 *quad32, Arena<T> ar) {
+    chain_wait();
+    chain_next();
     int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= mtot) return;
     const int64_t f = ntot + j;
@@ -316,9 +322,9 @@ tg_status build_arena_topology(tg_tree_s *t, Arena<T> &ar, cudaStream_t st) {
     TG_CUDA(cudaMemsetAsync(status.p, 0, sizeof(unsigned long long) * (tiles + 1), st));
     // validated on the device: the fill writes only in-range leaf ranges, and every walk checks the
     // flag before it reads the arena (no host synchronisation here)
-    { k_arena_links<<<tiles, LINK_THREADS, 0, st>>>(N, M, t->first, t->next, ar.n_link, ar.bad, status.p,
-                                                    (int *)(status.p + tiles), scan_spins()); tg::note_launch(); }
-    { k_arena_leaves<T><<<div_up(M, 256), 256, 0, st>>>(N, M, t->first, t->next, t->coord, t->mass, t->soft, ar); tg::note_launch(); }
+    TG_CHAIN(k_arena_links, tiles, LINK_THREADS, 0, st, N, M, t->first, t->next, ar.n_link, ar.bad, status.p,
+             (int *)(status.p + tiles), scan_spins());
+    TG_CHAIN(k_arena_leaves<T>, div_up(M, 256), 256, 0, st, N, M, t->first, t->next, t->coord, t->mass, t->soft, ar);
     TG_CUDA(cudaGetLastError());
     return TG_OK;
 }
@@ -328,8 +334,8 @@ template <typename T>
 tg_status build_arena_nodes(tg_tree_s *t, Arena<T> &ar, cudaStream_t st) {
     const int64_t M = t->mtot, N = t->ntot;
     if (sizeof(T) == 8 && ar.n_quad) TG_TRY(ensure_quad64(t, st));
-    { k_arena_nodes<T><<<div_up(M, 256), 256, 0, st>>>(N, M, t->coord, t->mass, t->soft, t->size, t->delta, t->quad,
-                                                      t->quad32, ar); tg::note_launch(); }
+    TG_CHAIN(k_arena_nodes<T>, div_up(M, 256), 256, 0, st, N, M, t->coord, t->mass, t->soft, t->size, t->delta,
+             t->quad, t->quad32, ar);
     TG_CUDA(cudaGetLastError());
     ar.built = true;
     return TG_OK;
@@ -654,6 +660,8 @@ constexpr int walk_reg_cap() {
 template <typename T, int FIELDS, bool QUAD, int STACK, bool TEAM = false>
 __global__ void __launch_bounds__(MAX_WALK_WARPS * 32) __maxnreg__((walk_reg_cap<T, FIELDS, QUAD, STACK, TEAM>()))
     k_walk(WalkArgs<T> a) {
+    chain_wait();
+    chain_next();
     extern __shared__ unsigned char smem_raw[];
     WarpSmem<T, QUAD, STACK> &sm = reinterpret_cast<WarpSmem<T, QUAD, STACK> *>(smem_raw)[threadIdx.x >> 5];
     // a block that walks one group together: its shared part lies behind the warps'
@@ -1369,6 +1377,7 @@ __global__ void k_make_groups(const int64_t *sys_off, int nsys, int gs, const in
 // The groups of one system's n targets, with nothing to copy or wait for first (1e5 single targets: 50 us in one
 // block and ~30 us of copies before it, 3 us here).
 __global__ void k_make_groups_one(int64_t n, int gs, int root, int64_t ngroups, int2 *groups, int *group_root) {
+    chain_next();
     const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= ngroups) return;
     const int64_t t = g * gs;
@@ -1397,6 +1406,8 @@ __global__ void k_tree_groups_mark(int64_t ntot, int64_t mtot, const int2 *node_
                                    const int64_t *next, const int64_t *parent, int G, const int64_t *sys_off,
                                    const int64_t *sys_node_off, int nsys, int2 *groups, int *group_root,
                                    int *group_node, unsigned long long *count, LargeNode *large, int *nlarge) {
+    chain_wait();
+    chain_next();
     const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const bool valid = j < mtot;
     int2 r = make_int2(0, 0);
@@ -1464,6 +1475,8 @@ __device__ __forceinline__ unsigned long long warp_max_key(unsigned long long u)
 __global__ void k_tree_groups_large(int64_t ntot, const int2 *node_range, const double *cell, const double *size,
                                     const double *coord, int G, const LargeNode *large, const int *nlarge,
                                     int2 *groups, int *group_root, int *group_node, unsigned long long *count) {
+    chain_wait();
+    chain_next();
     typedef unsigned long long u64;
     const int lane = lane_id();
     const int n = *nlarge;
@@ -1592,6 +1605,8 @@ __global__ void k_tree_groups_large(int64_t ntot, const int2 *node_range, const 
 // Morton-curve jump -- and open most of the tree -- start first instead of forming the tail.
 __global__ void k_group_cost_keys(const double *tpos, const int2 *groups, int64_t ngroups, uint64_t *keys,
                                   uint32_t *vals) {
+    chain_wait();
+    chain_next();
     int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= ngroups) return;
     int2 gr = groups[g];
@@ -1609,6 +1624,8 @@ __global__ void k_group_cost_keys(const double *tpos, const int2 *groups, int64_
     vals[g] = (uint32_t)g;
 }
 __global__ void k_group_start_keys(const int2 *groups, int64_t ngroups, uint64_t *keys, uint32_t *vals) {
+    chain_wait();
+    chain_next();
     int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= ngroups) return;
     keys[g] = (uint32_t)groups[g].x;
@@ -1616,6 +1633,8 @@ __global__ void k_group_start_keys(const int2 *groups, int64_t ngroups, uint64_t
 }
 __global__ void k_permute_groups(const uint32_t *perm, int64_t ngroups, const int2 *gin, const int *rin, const int *nin,
                                  int2 *gout, int *rout, int *nout) {
+    chain_wait();
+    chain_next();
     int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= ngroups) return;
     gout[g] = gin[perm[g]];
@@ -1626,6 +1645,8 @@ __global__ void k_permute_groups(const uint32_t *perm, int64_t ngroups, const in
 // Targets in walk order split once per walk into hi/lo parts in the walk precision.
 template <typename T>
 __global__ void k_prep_targets(const double *tpos, const double *th, int64_t n, vec4<T> *thi, vec4<T> *tlo) {
+    chain_wait();
+    chain_next();
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     T hx, hy, hz, lx, ly, lz;
@@ -1846,7 +1867,7 @@ static tg_status launch_walk(WalkArgs<T> &a, int warps, cudaStream_t st) {
         blocks = num_sms();
     }
     if (blocks < 1) blocks = 1;
-    { kern<<<(unsigned)blocks, warps * 32, smem, st>>>(a); tg::note_launch(); }
+    TG_CHAIN(kern, blocks, warps * 32, smem, st, a);
     TG_CUDA(cudaGetLastError());
     return TG_OK;
 }
@@ -1861,7 +1882,7 @@ static tg_status launch_team(WalkArgs<float> &a, cudaStream_t st) {
     TG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, TEAM_WARPS * 32, smem));
     int64_t blocks = (int64_t)std::max(per_sm, 1) * num_sms();
     if (!a.ngroups_dev) blocks = std::min(blocks, std::max<int64_t>(a.ngroups, 1));
-    { kern<<<(unsigned)blocks, TEAM_WARPS * 32, smem, st>>>(a); tg::note_launch(); }
+    TG_CHAIN(kern, blocks, TEAM_WARPS * 32, smem, st, a);
     TG_CUDA(cudaGetLastError());
     return TG_OK;
 }
@@ -2239,7 +2260,7 @@ tg_status run_walk(tg_tree_s *t, const double *tpos, const double *th, int64_t n
         vec4<double> *thi = nullptr, *tlo = nullptr;
         TG_CUDA(tg::dev_malloc((void **)&thi, sizeof(vec4<double>) * std::max<int64_t>(ntargets, 1), st));
         TG_CUDA(tg::dev_malloc((void **)&tlo, sizeof(vec4<double>) * std::max<int64_t>(ntargets, 1), st));
-        { k_prep_targets<double><<<div_up(ntargets, 256), 256, 0, st>>>(tpos, th, ntargets, thi, tlo); tg::note_launch(); }
+        TG_CHAIN(k_prep_targets<double>, div_up(ntargets, 256), 256, 0, st, tpos, th, ntargets, thi, tlo);
         a.thi = thi;
         a.tlo = tlo;
         rc = walk_with_fallback<double>(t, a, t->arena64, fields, quadrupole != 0, t->walk_warps, t->walk_stack,
@@ -2269,7 +2290,7 @@ tg_status run_walk(tg_tree_s *t, const double *tpos, const double *th, int64_t n
         } else {
             TG_CUDA(tg::dev_malloc((void **)&thi, sizeof(vec4<float>) * std::max<int64_t>(ntargets, 1), st));
             TG_CUDA(tg::dev_malloc((void **)&tlo, sizeof(vec4<float>) * std::max<int64_t>(ntargets, 1), st));
-            { k_prep_targets<float><<<div_up(ntargets, 256), 256, 0, st>>>(tpos, th, ntargets, thi, tlo); tg::note_launch(); }
+            TG_CHAIN(k_prep_targets<float>, div_up(ntargets, 256), 256, 0, st, tpos, th, ntargets, thi, tlo);
             a.thi = thi;
             a.tlo = tlo;
         }
@@ -2331,10 +2352,10 @@ tg_status tree_groups(tg_tree_s *t, int G, cudaStream_t st) {
     TG_CUDA(tg::dev_malloc((void **)&large, sizeof(LargeNode) * std::max<int64_t>(M, 1), st));
     TG_CUDA(tg::dev_malloc((void **)&nlarge, sizeof(int), st));
     TG_CUDA(cudaMemsetAsync(nlarge, 0, sizeof(int), st));
-    { k_tree_groups_mark<<<div_up(M, 256), 256, 0, st>>>(N, M, t->node_range, t->first, t->next, t->parent, G, d_sys,
-                                                       d_node, t->nsys, g0, r0, n0, cnt, large, nlarge); tg::note_launch(); }
-    { k_tree_groups_large<<<num_sms() * 8, 256, 0, st>>>(N, t->node_range, t->cell_center, t->size, t->coord, G, large,
-                                                       nlarge, g0, r0, n0, cnt); tg::note_launch(); }
+    TG_CHAIN(k_tree_groups_mark, div_up(M, 256), 256, 0, st, N, M, t->node_range, t->first, t->next, t->parent, G,
+             d_sys, d_node, t->nsys, g0, r0, n0, cnt, large, nlarge);
+    TG_CHAIN(k_tree_groups_large, num_sms() * 8, 256, 0, st, N, t->node_range, t->cell_center, t->size, t->coord, G,
+             large, nlarge, g0, r0, n0, cnt);
     TG_CUDA(cudaGetLastError());
     unsigned long long ng = 0;
     TG_CUDA(cudaMemcpyAsync(&ng, cnt, sizeof(ng), cudaMemcpyDeviceToHost, st));
@@ -2348,9 +2369,10 @@ tg_status tree_groups(tg_tree_s *t, int G, cudaStream_t st) {
     TG_CUDA(tg::dev_malloc((void **)&t->groups, sizeof(int2) * ng1, st));
     TG_CUDA(tg::dev_malloc((void **)&t->group_root, sizeof(int) * ng1, st));
     TG_CUDA(tg::dev_malloc((void **)&t->group_node, sizeof(int) * ng1, st));
-    { k_group_start_keys<<<div_up(ng, 256), 256, 0, st>>>(g0, ng, keys, vals); tg::note_launch(); }
+    TG_CHAIN(k_group_start_keys, div_up(ng, 256), 256, 0, st, g0, ng, keys, vals);
     TG_TRY(radix_sort_pairs(keys, vals, ng, 32, st, t->sort_err));
-    { k_permute_groups<<<div_up(ng, 256), 256, 0, st>>>(vals, ng, g0, r0, n0, t->groups, t->group_root, t->group_node); tg::note_launch(); }
+    TG_CHAIN(k_permute_groups, div_up(ng, 256), 256, 0, st, vals, ng, g0, r0, n0, t->groups, t->group_root,
+             t->group_node);
     TG_CUDA(cudaGetLastError());
     TG_CUDA(cudaFreeAsync(keys, st));
     TG_CUDA(cudaFreeAsync(vals, st));
@@ -2398,9 +2420,8 @@ tg_status tree_groups_with_arena(tg_tree_s *t, int G, bool fp64, cudaStream_t st
                 t->own32 = nullptr;
                 r = TG_ERR_CUDA;
             } else {
-                k_prep_targets<float><<<div_up(t->ntot, 256), 256, 0, t->side>>>(t->coord, t->soft, t->ntot, t->own32,
-                                                                                 t->own32 + t->ntot);
-                tg::note_launch();
+                TG_CHAIN(k_prep_targets<float>, div_up(t->ntot, 256), 256, 0, t->side, t->coord, t->soft, t->ntot,
+                         t->own32, t->own32 + t->ntot);
             }
         }
         const cudaError_t ej = cudaEventRecord(t->ev_join, t->side);
@@ -2425,7 +2446,7 @@ tg_status make_cost_order(const double *tpos, const int2 *groups, int64_t ngroup
     uint64_t *keys = nullptr;
     TG_CUDA(tg::dev_malloc((void **)&keys, sizeof(uint64_t) * std::max<int64_t>(ngroups, 1), st));
     TG_CUDA(tg::dev_malloc((void **)order, sizeof(int) * std::max<int64_t>(ngroups, 1), st));
-    { k_group_cost_keys<<<div_up(ngroups, 256), 256, 0, st>>>(tpos, groups, ngroups, keys, (uint32_t *)*order); tg::note_launch(); }
+    TG_CHAIN(k_group_cost_keys, div_up(ngroups, 256), 256, 0, st, tpos, groups, ngroups, keys, (uint32_t *)*order);
     TG_CUDA(cudaGetLastError());
     TG_TRY(radix_sort_pairs(keys, (uint32_t *)*order, ngroups, 16, st, sort_err));
     TG_CUDA(cudaFreeAsync(keys, st));
