@@ -584,6 +584,46 @@ __device__ __forceinline__ void acc_mono_quad(T m, const T *q, T dx, T dy, T dz,
     p.v[3] = fma(-qdz, r5inv, fma(sc, dz, p.v[3]));
 }
 
+// Two sources at a time for the walks whose sums take the sources one after another (the tidal tensor together
+// with another field): everything up to a source's term in paired arithmetic, then the terms added in the sources'
+// order, each operation rounded as point_mass and quad_terms round it, so the sums are theirs bit for bit. Issue
+// slots bound these walks (3.1 of 4 per cycle) before the FMA pipe (66 %): all fields of 1e6 particles, quadrupole
+// 8.57 -> 7.52 ms, monopole 3.85 -> 3.20. (Potential and acceleration alone, mostly traversal, gain nothing:
+// 10 % slower that way.)
+__device__ __forceinline__ void mono_pair(f2 m, f2 dx, f2 dy, f2 dz, f2 rinv, f2 u, f2 &mr, f2 &mr3, f2 &qx, f2 &qy,
+                                          f2 &txx, f2 &tyy, f2 &tzz) {
+    mr = f2_mul(m, rinv);
+    mr3 = f2_mul(mr, u);
+    const f2 mr3n = f2_mul(mr3, f2_pack(-1.f, -1.f));
+    const f2 q3 = f2_mul(f2_mul(f2_pack(3.f, 3.f), mr3), u);
+    qx = f2_mul(q3, dx);
+    qy = f2_mul(q3, dy);
+    txx = f2_fma(qx, dx, mr3n);
+    tyy = f2_fma(qy, dy, mr3n);
+    tzz = f2_fma(f2_mul(q3, dz), dz, mr3n);
+}
+__device__ __forceinline__ float f2_lo(f2 v) { return __uint_as_float((unsigned)v); }
+__device__ __forceinline__ float f2_hi(f2 v) { return __uint_as_float((unsigned)(v >> 32)); }
+template <int H>
+__device__ __forceinline__ float f2_half(f2 v) { return H ? f2_hi(v) : f2_lo(v); }
+
+template <int FIELDS, int H, typename T>
+__device__ __forceinline__ void add_mono(Acc<T> &p, f2 dx, f2 dy, f2 dz, f2 mr, f2 mr3, f2 qx, f2 qy, f2 txx, f2 tyy,
+                                         f2 tzz) {
+    if (FIELDS & F_POT) p.v[0] = __fsub_rn(p.v[0], f2_half<H>(mr));
+    if (FIELDS & F_ACC) {
+        p.v[1] = __fmaf_rn(f2_half<H>(mr3), f2_half<H>(dx), p.v[1]);
+        p.v[2] = __fmaf_rn(f2_half<H>(mr3), f2_half<H>(dy), p.v[2]);
+        p.v[3] = __fmaf_rn(f2_half<H>(mr3), f2_half<H>(dz), p.v[3]);
+    }
+    p.v[4] = __fadd_rn(p.v[4], f2_half<H>(txx));
+    p.v[5] = __fmaf_rn(f2_half<H>(qx), f2_half<H>(dy), p.v[5]);
+    p.v[6] = __fmaf_rn(f2_half<H>(qx), f2_half<H>(dz), p.v[6]);
+    p.v[7] = __fadd_rn(p.v[7], f2_half<H>(tyy));
+    p.v[8] = __fmaf_rn(f2_half<H>(qy), f2_half<H>(dz), p.v[8]);
+    p.v[9] = __fadd_rn(p.v[9], f2_half<H>(tzz));
+}
+
 template <int FIELDS>
 __device__ __forceinline__ constexpr bool comp(int c) {
     return c == 0 ? (FIELDS & F_POT) : (c <= 3 ? (FIELDS & F_ACC) : (FIELDS & F_TID));
@@ -648,13 +688,16 @@ __device__ __forceinline__ void write_fields(double *o, int out_fields, const do
 // Register caps (registers are granted 8 per thread at a time): the FP32 quadrupole acceleration
 // walk with the small stack runs at 72, which with its shared memory lets 7 blocks of 4 warps share
 // an SM (6 at 80); the other small-stack walks at 80 (6 blocks of 4 warps, 3 of 8; 81 would round
-// to 88 and leave 5 or 2); FP64 walks, bound by the FP64 pipe at any occupancy, at 112 (4 blocks of 4
-// warps; 50000 particles 5.67 ms at 80 and 5.28 at 112); large-stack walks uncapped.
+// to 88 and leave 5 or 2), but 128 for the quadrupole walk of the tidal tensor with other fields, whose paired
+// terms gain more from registers than from warps (1e6 particles: 8.03 ms at 80, 7.85 at 96, 7.52 at
+// 128); FP64 walks, bound by the FP64 pipe at any occupancy, at 112 (4 blocks of 4 warps; 50000
+// particles 5.67 ms at 80 and 5.28 at 112); large-stack walks uncapped.
 template <typename T, int FIELDS, bool QUAD, int STACK, bool TEAM = false>
 constexpr int walk_reg_cap() {
     if (TEAM) return 128;  // two blocks of eight warps per SM
     if (STACK != STACK_SMALL) return 255;
     if (sizeof(T) == 8) return 112;
+    if (QUAD && (FIELDS & F_TID) && FIELDS != F_TID) return 128;
     return (sizeof(T) == 4 && FIELDS == F_ACC && QUAD) ? 72 : 80;
 }
 template <typename T, int FIELDS, bool QUAD, int STACK, bool TEAM = false>
@@ -830,6 +873,8 @@ __global__ void __launch_bounds__(MAX_WALK_WARPS * 32) __maxnreg__((walk_reg_cap
             if constexpr (sizeof(T) == 4 && (FIELDS == F_TID || ((FIELDS & F_TID) == 0 &&
                                                                   (QUAD || FIELDS != (F_POT | F_ACC)))))
                 paired = GS >= 2;
+            constexpr bool ORDERED = sizeof(T) == 4 && (FIELDS & F_TID) != 0 && FIELDS != F_TID;  // see mono_pair
+            if (ORDERED && GS >= 2) paired = true;
             if (paired) {
                 float *o = reinterpret_cast<float *>(sm.spos) + 8 * (lane >> 1) + (lane & 1);
                 o[0] = (float)st.x;
@@ -845,7 +890,22 @@ __global__ void __launch_bounds__(MAX_WALK_WARPS * 32) __maxnreg__((walk_reg_cap
 #pragma unroll
             for (int c = 0; c < 10; c++) b.v[c] = T(0);
             const vec4<T> *chunk = sm.spos + slice * GS;
-            if (paired) {
+            if (ORDERED && paired) {
+                if constexpr (ORDERED) {
+                    const f2 TX = f2_pack(tx, tx), TY = f2_pack(ty, ty), TZ = f2_pack(tz, tz);
+                    const ulonglong2 *src = reinterpret_cast<const ulonglong2 *>(sm.spos) + 2 * ((slice * GS) >> 1);
+#pragma unroll 4
+                    for (int i = 0; i < (GS >> 1); i++) {
+                        const ulonglong2 w0 = src[2 * i], w1 = src[2 * i + 1];
+                        const f2 dx = f2_sub(w0.x, TX), dy = f2_sub(w0.y, TY), dz = f2_sub(w1.x, TZ);
+                        const f2 rinv = f2_rsqrt(f2_fma(dz, dz, f2_fma(dx, dx, f2_mul(dy, dy))));
+                        f2 mr, mr3, qx, qy, txx, tyy, tzz;
+                        mono_pair(w1.y, dx, dy, dz, rinv, f2_mul(rinv, rinv), mr, mr3, qx, qy, txx, tyy, tzz);
+                        add_mono<FIELDS, 0>(b, dx, dy, dz, mr, mr3, qx, qy, txx, tyy, tzz);
+                        add_mono<FIELDS, 1>(b, dx, dy, dz, mr, mr3, qx, qy, txx, tyy, tzz);
+                    }
+                }
+            } else if (paired) {
                 const f2 TX = f2_pack((float)tx, (float)tx), TY = f2_pack((float)ty, (float)ty);
                 const f2 TZ = f2_pack((float)tz, (float)tz);
                 // even and odd sources summed apart (bit pattern 0 is +0.0f); ph sums m/r; t0..t5 the
@@ -1023,9 +1083,98 @@ __global__ void __launch_bounds__(MAX_WALK_WARPS * 32) __maxnreg__((walk_reg_cap
             }
             return finish(b, cnt, true);
         };
+        // The same staging, the quadrupole as it is, for walks with the tidal tensor and another field (see mono_pair).
+        auto eval_nodes_ordered = [&](const int *list, int cnt) {
+            Acc<T> b;
+#pragma unroll
+            for (int c = 0; c < 10; c++) b.v[c] = T(0);
+            if constexpr (sizeof(T) == 4) {
+                float *buf = reinterpret_cast<float *>(sm.spos);
+                {
+                    float v[10] = {(float)FAR, (float)FAR, (float)FAR, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+                    if (lane < cnt) {
+                        const int e = list[lane];
+                        const vec4<T> p = a.ar.n_pos[e], q = a.ar.n_lo[e];
+                        const vec4<T> qa = a.ar.n_quad[2 * e], qb = a.ar.n_quad[2 * e + 1];
+                        v[0] = (p.x - gcx) + q.x;
+                        v[1] = (p.y - gcy) + q.y;
+                        v[2] = (p.z - gcz) + q.z;
+                        v[3] = p.w;
+                        v[4] = qa.x; v[5] = qa.y; v[6] = qa.z; v[7] = qa.w; v[8] = qb.x; v[9] = qb.y;
+                    }
+                    float *o = buf + 20 * (lane >> 1) + (lane & 1);
+#pragma unroll
+                    for (int k = 0; k < 10; k++) o[2 * k] = v[k];
+                }
+                __syncwarp();
+                const f2 TX = f2_pack(tx, tx), TY = f2_pack(ty, ty), TZ = f2_pack(tz, tz);
+                auto both = [](float x) { return f2_pack(x, x); };
+                const ulonglong2 *src = reinterpret_cast<const ulonglong2 *>(buf) + 5 * ((slice * GS) >> 1);
+#pragma unroll 1
+                for (int i = 0; i < (GS >> 1); i++) {
+                    const ulonglong2 w0 = src[5 * i], w1 = src[5 * i + 1], w2 = src[5 * i + 2], w3 = src[5 * i + 3],
+                                     w4 = src[5 * i + 4];
+                    const f2 xx = w2.x, xy = w2.y, xz = w3.x, yy = w3.y, yz = w4.x, zz = w4.y;
+                    const f2 dx = f2_sub(w0.x, TX), dy = f2_sub(w0.y, TY), dz = f2_sub(w1.x, TZ);
+                    const f2 rinv = f2_rsqrt(f2_fma(dz, dz, f2_fma(dx, dx, f2_mul(dy, dy))));
+                    const f2 u = f2_mul(rinv, rinv);
+                    f2 mr, mr3, qx, qy, txx, tyy, tzz;
+                    mono_pair(w1.y, dx, dy, dz, rinv, u, mr, mr3, qx, qy, txx, tyy, tzz);
+                    const f2 r5 = f2_mul(f2_mul(u, u), rinv), r5n = f2_mul(r5, both(-1.f));
+                    const f2 r7 = f2_mul(r5, u), r7n = f2_mul(r5n, u);
+                    const f2 nx = f2_fma(xz, dz, f2_fma(xx, dx, f2_mul(xy, dy)));
+                    const f2 ny = f2_fma(yz, dz, f2_fma(xy, dx, f2_mul(yy, dy)));
+                    const f2 nz = f2_fma(zz, dz, f2_fma(xz, dx, f2_mul(yz, dy)));
+                    const f2 A = f2_fma(dz, nz, f2_fma(dx, nx, f2_mul(dy, ny)));
+                    const f2 hA = f2_mul(both(-0.5f), A), A25n = f2_mul(both(-2.5f), A);
+                    const f2 fac = f2_mul(f2_mul(f2_mul(both(17.5f), A), r7), u);
+                    const f2 fx = f2_mul(fac, dx), fy = f2_mul(fac, dy), fz = f2_mul(fac, dz);
+                    auto diag = [&](f2 q, f2 d, f2 n, f2 fd) {
+                        return f2_fma(fd, d, f2_fma(A25n, r7, f2_fma(q, r5, f2_mul(f2_mul(f2_mul(both(10.f), d), n), r7n))));
+                    };
+                    auto off = [&](f2 q, f2 da, f2 db, f2 na, f2 nb, f2 fa) {
+                        const f2 s = f2_fma(db, na, f2_mul(da, nb));
+                        return f2_fma(fa, db, f2_fma(q, r5, f2_mul(f2_mul(both(5.f), s), r7n)));
+                    };
+                    const f2 qxx = diag(xx, dx, nx, fx), qyy = diag(yy, dy, ny, fy), qzz = diag(zz, dz, nz, fz);
+                    const f2 qxy = off(xy, dx, dy, nx, ny, fx), qxz = off(xz, dx, dz, nx, nz, fx);
+                    const f2 qyz = off(yz, dy, dz, ny, nz, fy);
+                    f2 gx = 0, gy = 0, gz = 0;
+                    if constexpr ((FIELDS & F_ACC) != 0) {
+                        const f2 qf = f2_mul(A25n, r7n);
+                        gx = f2_fma(qf, dx, f2_mul(nx, r5n));
+                        gy = f2_fma(qf, dy, f2_mul(ny, r5n));
+                        gz = f2_fma(qf, dz, f2_mul(nz, r5n));
+                    }
+                    auto add = [&](auto half) {
+                        constexpr int H = decltype(half)::value;
+                        add_mono<FIELDS, H>(b, dx, dy, dz, mr, mr3, qx, qy, txx, tyy, tzz);
+                        if (FIELDS & F_POT) b.v[0] = __fmaf_rn(f2_half<H>(hA), f2_half<H>(r5), b.v[0]);
+                        if (FIELDS & F_ACC) {
+                            b.v[1] = __fadd_rn(b.v[1], f2_half<H>(gx));
+                            b.v[2] = __fadd_rn(b.v[2], f2_half<H>(gy));
+                            b.v[3] = __fadd_rn(b.v[3], f2_half<H>(gz));
+                        }
+                        b.v[4] = __fadd_rn(b.v[4], f2_half<H>(qxx));
+                        b.v[5] = __fadd_rn(b.v[5], f2_half<H>(qxy));
+                        b.v[6] = __fadd_rn(b.v[6], f2_half<H>(qxz));
+                        b.v[7] = __fadd_rn(b.v[7], f2_half<H>(qyy));
+                        b.v[8] = __fadd_rn(b.v[8], f2_half<H>(qyz));
+                        b.v[9] = __fadd_rn(b.v[9], f2_half<H>(qzz));
+                    };
+                    add(std::integral_constant<int, 0>());
+                    add(std::integral_constant<int, 1>());
+                }
+                __syncwarp();
+            }
+            return finish(b, cnt, true);
+        };
         auto eval_nodes = [&](const int *list, int cnt) {
             if constexpr (sizeof(T) == 4 && ((FIELDS & F_TID) == 0 || FIELDS == F_TID)) {
                 if (GS >= 2) return eval_nodes_paired(list, cnt);
+            }
+            if constexpr (sizeof(T) == 4 && (FIELDS & F_TID) != 0 && FIELDS != F_TID) {
+                if (GS >= 2) return eval_nodes_ordered(list, cnt);
             }
             vec4<T> st = vec4<T>{FAR, FAR, FAR, T(0)}, q0 = vec4<T>{T(0), T(0), T(0), T(0)}, q1 = q0;
             if (lane < cnt) {
