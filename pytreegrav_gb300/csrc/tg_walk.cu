@@ -685,23 +685,34 @@ __device__ __forceinline__ void write_fields(double *o, int out_fields, const do
     }
 }
 
-// Register caps (registers are granted 8 per thread at a time): the FP32 quadrupole acceleration
-// walk with the small stack runs at 72, which with its shared memory lets 7 blocks of 4 warps share
-// an SM (6 at 80); the other small-stack walks at 80 (6 blocks of 4 warps, 3 of 8; 81 would round
-// to 88 and leave 5 or 2), but 128 for the quadrupole walk of the tidal tensor with other fields, whose paired
-// terms gain more from registers than from warps (1e6 particles: 8.03 ms at 80, 7.85 at 96, 7.52 at
-// 128); FP64 walks, bound by the FP64 pipe at any occupancy, at 112 (4 blocks of 4 warps; 50000
-// particles 5.67 ms at 80 and 5.28 at 112); large-stack walks uncapped.
-template <typename T, int FIELDS, bool QUAD, int STACK, bool TEAM = false>
+// Register caps (registers are granted 8 per thread at a time): small-stack walks at 80 (6 blocks of 4 warps, 3 of
+// 8; 81 would round to 88 and leave 5 or 2; the quadrupole acceleration at 72, 7 blocks of 4 with the
+// largest shared-memory carveout, is 1 % slower with groups of 32 and 2 to 6 % with uniform points in groups of
+// 8), but 128 for the quadrupole walk of the tidal tensor with other fields, whose paired terms gain more from
+// registers than from warps (1e6 particles: 8.03 ms at 80, 7.85 at 96, 7.52 at 128); FP64 walks, bound
+// by the FP64 pipe at any occupancy, at 112 (4 blocks of 4 warps; 50000 particles 5.67 ms at 80 and 5.28 at
+// 112); large-stack walks uncapped. LEAN walks (lean_walk) at 64: a third more warps.
+template <typename T, int FIELDS, bool QUAD, int STACK, bool TEAM = false, bool LEAN = false>
 constexpr int walk_reg_cap() {
     if (TEAM) return 128;  // two blocks of eight warps per SM
     if (STACK != STACK_SMALL) return 255;
     if (sizeof(T) == 8) return 112;
     if (QUAD && (FIELDS & F_TID) && FIELDS != F_TID) return 128;
-    return (sizeof(T) == 4 && FIELDS == F_ACC && QUAD) ? 72 : 80;
+    return LEAN ? 64 : 80;
 }
-template <typename T, int FIELDS, bool QUAD, int STACK, bool TEAM = false>
-__global__ void __launch_bounds__(MAX_WALK_WARPS * 32) __maxnreg__((walk_reg_cap<T, FIELDS, QUAD, STACK, TEAM>()))
+// Monopole walks without the tidal tensor are bound by their traversal's latencies (2.7 of 4 issue slots with 24 warps
+// per SM): 32 warps of 64 registers make them 5 to 11 % faster (1e6 particles in tree groups of 32: Plummer
+// 1.93 -> 1.80 ms, uniform 0.98 -> 0.89, clustered 1.90 -> 1.76; 3e5 single targets 4.87 -> 4.38), but walks with few
+// groups, bound by their longest, are up to 3 % slower (20000 particles in groups of 2: 0.321 ms, lean 0.325),
+// and so are groups of 8 of uniform points (1e6: 2.36 ms, lean 2.48; Plummer 3.89 and 3.61).
+constexpr int64_t LEAN_GROUPS = 16384;
+template <typename T, int FIELDS, bool QUAD, int STACK>
+constexpr bool can_be_lean() {
+    return sizeof(T) == 4 && !QUAD && !(FIELDS & F_TID) && STACK == STACK_SMALL;
+}
+inline bool lean_walk(int gs, int64_t ngroups) { return (gs <= 2 || gs >= 16) && ngroups >= LEAN_GROUPS; }
+template <typename T, int FIELDS, bool QUAD, int STACK, bool TEAM = false, bool LEAN = false>
+__global__ void __launch_bounds__(MAX_WALK_WARPS * 32) __maxnreg__((walk_reg_cap<T, FIELDS, QUAD, STACK, TEAM, LEAN>()))
     k_walk(WalkArgs<T> a) {
     chain_wait();
     chain_next();
@@ -1998,9 +2009,12 @@ template <typename T, int FIELDS, bool QUAD, int STACK>
 static tg_status launch_walk(WalkArgs<T> &a, int warps, cudaStream_t st) {
     size_t smem = sizeof(WarpSmem<T, QUAD, STACK>) * warps;
     auto kern = k_walk<T, FIELDS, QUAD, STACK>;
+    if constexpr (can_be_lean<T, FIELDS, QUAD, STACK>()) {
+        if (!a.ngroups_dev && lean_walk(a.gs, a.ngroups)) kern = k_walk<T, FIELDS, QUAD, STACK, false, true>;
+    }
     TG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    // the 72-register walk reaches 7 blocks per SM only with the largest shared-memory carveout; the
-    // others keep the driver's choice, which leaves them more L1
+    // the largest shared-memory carveout for the quadrupole acceleration (the others keep the driver's choice, which
+    // leaves them more L1)
     if (sizeof(T) == 4 && FIELDS == F_ACC && QUAD && STACK == STACK_SMALL)
         TG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
                                      cudaSharedmemCarveoutMaxShared));

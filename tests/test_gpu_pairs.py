@@ -36,3 +36,18 @@ def test_fields_together(n, gs, quadrupole):
     for k in one:
         assert rel_rms(got[k], one[k]) < 2e-5, k
         assert rel_rms(got[k], ref[k]) < 2e-5, k
+
+
+@pytest.mark.parametrize("fields", [("accel",), ("potential",), ("potential", "accel")])
+@pytest.mark.parametrize("n,gs", [(16383, 1), (16384, 1), (32768, 2), (40001, 2)])
+def test_walks_on_both_sides_of_the_lean_line(n, gs, fields):
+    """Monopole walks take the 64-register kernel from 16384 groups on (groups of 1, 2, 16 or 32 targets)."""
+    import pytreegrav_gb300 as tg
+    from pytreegrav_gb300 import synthetic
+
+    x, m, h = synthetic.plummer(n, 5), np.full(n, 1.0 / n), np.full(n, 0.01)
+    kw = dict({k: True for k in fields}, group_size=gs, theta=0.7)
+    got = tg.ConstructTree(x, m, h).fields(**kw)
+    ref, _ = O.self_fields(x, m, h, nthreads=O.num_threads(), **kw)
+    for k in fields:
+        assert rel_rms(got[k], ref[k]) < 2e-5, k
