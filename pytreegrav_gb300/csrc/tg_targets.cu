@@ -33,10 +33,12 @@ bool valid_gs(int gs) { return gs == 1 || gs == 2 || gs == 4 || gs == 8 || gs ==
 
 int width_of(int fields) { return ((fields & 1) ? 1 : 0) + ((fields & 2) ? 3 : 0) + ((fields & 4) ? 9 : 0); }
 
-// One thread per group: the group's FP64 bounding box, then a descent from the source root (node 0)
-// through the node child whose cell (cell centre +- size / 2) holds the whole box, as long as one
-// does. Children come from the walk arena's traversal records (first node child << 4 | count). The
-// descent goes one level deeper per step; it is bounded by the node count in any case.
+// Eight lanes per group: the group's FP64 bounding box, then a descent from the source root (node 0)
+// through the first node child whose cell (cell centre +- size / 2) holds the whole box, as long as one
+// does, a lane testing each child. Children come from the walk arena's traversal records (first node child << 4 |
+// count). The descent goes one level deeper per step; it is bounded by the node count in any case. Bound by the
+// chain of dependent loads down the tree (a thread per group tried the children one after another: 22000
+// groups of 5e5 targets in 8e6 sources 192 us, 267 with the cut; now 81 and 159).
 // With nsub non-null, also the number of pieces the group is cut into (see k_split_groups). The
 // local source density comes from the smallest source cell that holds the box's centre and is at
 // least as large as the box (found by continuing the descent through the children holding the
@@ -50,67 +52,65 @@ __global__ void k_target_src_nodes(int64_t ntot, int64_t mtot, const double *cel
                                    int *node, int *nsub, int *sublen) {
     chain_wait();
     chain_next();
-    const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= ng) return;
-    const int2 gr = groups[g];
-    double lo[3], hi[3];
-    for (int k = 0; k < 3; k++) lo[k] = hi[k] = tpos[3 * (int64_t)gr.x + k];
-    for (int i = 1; i < gr.y; i++)
+    const int lane = lane_id(), sub = lane & 7;
+    const int64_t g = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 3;
+    const bool valid = g < ng;
+    const int2 gr = valid ? groups[g] : make_int2(0, 1);
+    unsigned long long ulo[3], uhi[3];  // as ordered integers: FP64 minima cost the FP64 pipe
+    for (int i = sub < gr.y ? sub : 0, first = 1; i < gr.y; i += 8, first = 0)
+#pragma unroll
         for (int k = 0; k < 3; k++) {
-            const double v = tpos[3 * ((int64_t)gr.x + i) + k];
-            lo[k] = fmin(lo[k], v);
-            hi[k] = fmax(hi[k], v);
+            const unsigned long long u = dbl_to_ordered(tpos[3 * ((int64_t)gr.x + i) + k]);
+            ulo[k] = first ? u : min(ulo[k], u);
+            uhi[k] = first ? u : max(uhi[k], u);
         }
-    int j = 0;
-    if (!(ar.bad && *ar.bad)) {
-        for (int64_t steps = 0; steps < mtot; steps++) {
-            const int cb = __float_as_int(ar.n_trav[2 * j + 1].z);
-            const int fc = cb >> 4, nc = cb & 15;
-            int nxt = -1;
-            for (int c = fc; c < fc + nc; c++) {
-                if (c < 0 || c >= mtot) break;
-                const double hs = 0.5 * size[ntot + c];
-                bool inside = true;
-                for (int k = 0; k < 3; k++)
-                    inside = inside && lo[k] >= cell[3 * (int64_t)c + k] - hs && hi[k] <= cell[3 * (int64_t)c + k] + hs;
-                if (inside) {
-                    nxt = c;
-                    break;
-                }
-            }
-            if (nxt < 0) break;
-            j = nxt;
+    double lo[3], hi[3];
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        for (int o = 4; o; o >>= 1) {
+            ulo[k] = min(ulo[k], __shfl_xor_sync(FULL, ulo[k], o));
+            uhi[k] = max(uhi[k], __shfl_xor_sync(FULL, uhi[k], o));
         }
+        lo[k] = ordered_to_dbl(ulo[k]);
+        hi[k] = ordered_to_dbl(uhi[k]);
     }
-    node[g] = j;
+    const bool ok = valid && !(ar.bad && *ar.bad);
+    // the node reached from j through the first child at a time that passes the test
+    auto descend = [&](int j, auto holds) {
+        bool active = ok;
+        for (int64_t steps = 0; steps < mtot && __any_sync(FULL, active); steps++) {
+            const int cb = active ? __float_as_int(ar.n_trav[2 * j + 1].z) : 0;
+            const int fc = cb >> 4, nc = cb & 15, c = fc + sub;
+            const bool in = active && sub < nc && c >= 0 && c < mtot && holds(c);
+            const unsigned b = (__ballot_sync(FULL, in) >> (lane & 24)) & 0xff;
+            if (b) j = fc + __ffs(b) - 1;
+            else active = false;
+        }
+        return j;
+    };
+    const int j = descend(0, [&](int c) {
+        const double hs = 0.5 * size[ntot + c];
+        bool inside = true;
+        for (int k = 0; k < 3; k++)
+            inside = inside && lo[k] >= cell[3 * (int64_t)c + k] - hs && hi[k] <= cell[3 * (int64_t)c + k] + hs;
+        return inside;
+    });
+    if (valid && sub == 0) node[g] = j;
     if (nsub) {
         int k = gr.y;
         const double e = fmax(fmax(hi[0] - lo[0], hi[1] - lo[1]), hi[2] - lo[2]);
         const double ctr[3] = {0.5 * (lo[0] + hi[0]), 0.5 * (lo[1] + hi[1]), 0.5 * (lo[2] + hi[2])};
-        int d = j;  // the density cell: from j down through the children holding the centre
-        if (!(ar.bad && *ar.bad)) {
-            for (int64_t steps = 0; steps < mtot; steps++) {
-                const int cb = __float_as_int(ar.n_trav[2 * d + 1].z);
-                const int fc = cb >> 4, nc = cb & 15;
-                int nxt = -1;
-                for (int c = fc; c < fc + nc; c++) {
-                    if (c < 0 || c >= mtot) break;
-                    const double sc = size[ntot + c], hs = 0.5 * sc;
-                    if (sc < e) continue;
-                    bool inside = true;
-                    for (int q = 0; q < 3; q++)
-                        inside = inside && ctr[q] >= cell[3 * (int64_t)c + q] - hs && ctr[q] <= cell[3 * (int64_t)c + q] + hs;
-                    if (inside) {
-                        nxt = c;
-                        break;
-                    }
-                }
-                if (nxt < 0) break;
-                d = nxt;
-            }
-        }
+        // the density cell: from j down through the children holding the centre
+        const int d = descend(j, [&](int c) {
+            const double sc = size[ntot + c], hs = 0.5 * sc;
+            bool inside = !(sc < e);
+            for (int q = 0; q < 3; q++)
+                inside = inside && ctr[q] >= cell[3 * (int64_t)c + q] - hs && ctr[q] <= cell[3 * (int64_t)c + q] + hs;
+            return inside;
+        });
+        if (!valid || sub != 0) return;
         const double sd = size[ntot + d];
-        if (!(ar.bad && *ar.bad) && sd > 0.0 && gr.y > 1) {
+        if (ok && sd > 0.0 && gr.y > 1) {
             const double q = e / sd;
             const double n_in = (double)(node_range[d].y - node_range[d].x) * q * q * q;
             k = 1;  // the largest power of two (at most the count) with k n_in <= 2 G count
@@ -149,7 +149,7 @@ tg_status targets_src_nodes(tg_targets_s *ts, cudaStream_t st) {
     const int64_t ng = tt->ngroups;
     TG_CUDA(dev_malloc((void **)&ts->src_node, sizeof(int) * std::max<int64_t>(ng, 1), st));
     if (ng > 0) {
-        TG_CHAIN(k_target_src_nodes, div_up(ng, 128), 128, 0, st, src->ntot, src->mtot, src->cell_center, src->size,
+        TG_CHAIN(k_target_src_nodes, div_up(8 * ng, 128), 128, 0, st, src->ntot, src->mtot, src->cell_center, src->size,
                  src->arena32, src->node_range, tt->coord, tt->groups, ng, ts->group_size, ts->src_node, nullptr,
                  nullptr);
         TG_CUDA(cudaGetLastError());
@@ -171,7 +171,7 @@ tg_status targets_refine_groups(tg_targets_s *ts, cudaStream_t st) {
     TG_CUDA(sublen.alloc(ng));
     TG_CUDA(off.alloc(ng + 1));
     TG_CUDA(cudaMemsetAsync(nsub.p + ng, 0, sizeof(int), st));
-    TG_CHAIN(k_target_src_nodes, div_up(ng, 128), 128, 0, st, src->ntot, src->mtot, src->cell_center, src->size,
+    TG_CHAIN(k_target_src_nodes, div_up(8 * ng, 128), 128, 0, st, src->ntot, src->mtot, src->cell_center, src->size,
              src->arena32, src->node_range, tt->coord, tt->groups, ng, ts->group_size, node.p, nsub.p, sublen.p);
     TG_CUDA(cudaGetLastError());
     TG_TRY(exclusive_scan_i32(nsub.p, off.p, ng + 1, st));
