@@ -9,7 +9,10 @@
  *
  * `mem` says where the caller's arrays live: TG_MEM_HOST (pageable or pinned host memory; the
  * library copies in and out on `stream` and synchronises before returning) or TG_MEM_DEVICE
- * (device pointers; the call is asynchronous on `stream` except where noted).
+ * (device pointers; the call is asynchronous on `stream` except where noted). tg_tree_fields,
+ * tg_tree_fields_learned, tg_targets_fields, tg_targets_fields_learned and tg_bruteforce also take
+ * TG_MEM_HOST_FIELDS: host memory with every requested field in an array of its own, `out` then
+ * pointing to the arrays' addresses (double *const *) in the order potential, accel, tidal.
  *
  * Citations name the pytreegrav interface each entry replaces (paths relative to the pytreegrav
  * project).
@@ -35,7 +38,7 @@ typedef enum {
     TG_ERR_NO_QUADRUPOLES = 8  /* quadrupole walk on a monopole tree (frontend.py:28-37) */
 } tg_status;
 
-enum { TG_MEM_HOST = 0, TG_MEM_DEVICE = 1 };
+enum { TG_MEM_HOST = 0, TG_MEM_DEVICE = 1, TG_MEM_HOST_FIELDS = 2 };
 
 /* Field bits for tg_tree_fields / tg_bruteforce. */
 enum { TG_FIELD_POTENTIAL = 1, TG_FIELD_ACCEL = 2, TG_FIELD_TIDAL = 4 };

@@ -24,6 +24,7 @@ TG_ERR_CUDA = 7
 TG_ERR_NO_QUADRUPOLES = 8
 
 TG_MEM_HOST = 0
+TG_MEM_HOST_FIELDS = 2
 TG_MEM_DEVICE = 1
 TG_FIELD_POTENTIAL = 1
 TG_FIELD_ACCEL = 2

@@ -58,6 +58,26 @@ __global__ void k_gather_targets(const uint32_t *perm, int64_t n, const double *
     scatter[i] = o;
 }
 
+// Rows of W components (potential, np = 0 or 1; acceleration, na = 0 or 3; tidal tensor) into one array per field.
+__global__ void k_field_planes(const double *rows, int64_t n, int W, int np, int na, double *planes) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n * W) return;
+    int64_t e = i;
+    int w = 1, c0 = 0;  // the field's width and first component
+    if (e >= np * n) {
+        e -= np * n;
+        w = 3;
+        c0 = np;
+        if (e >= na * n) {
+            e -= na * n;
+            w = 9;
+            c0 = np + na;
+        }
+    }
+    const int64_t row = e / w;
+    planes[i] = rows[row * W + c0 + (int)(e - row * w)];
+}
+
 // Device copies of caller arrays (or the caller's own device pointers), freed on scope exit.
 struct DevBuf {
     const double *ptr = nullptr;
@@ -123,6 +143,32 @@ int field_width(int fields) {
 bool valid_group_size(int gs) { return gs == 1 || gs == 2 || gs == 4 || gs == 8 || gs == 16 || gs == 32; }
 
 }  // namespace
+
+// TG_MEM_HOST_FIELDS: the fields are taken apart on the GPU, so that the caller has no strided copies to make
+// (numpy took 430 us for the potential and acceleration of 100000 targets, more than their walk's share
+// of that call on the GPU; the kernel takes 4).
+tg_status copy_results(const double *rows, int64_t n, int fields, int mem, double *out, cudaStream_t st) {
+    const int W = field_width(fields);
+    if (mem == TG_MEM_HOST) {
+        TG_CUDA(cudaMemcpyAsync(out, rows, sizeof(double) * n * W, cudaMemcpyDeviceToHost, st));
+        return TG_OK;
+    }
+    DevArray<double> planes(st);
+    TG_CUDA(planes.alloc(n * W));
+    const int np = (fields & 1) ? 1 : 0, na = (fields & 2) ? 3 : 0;
+    { k_field_planes<<<div_up(n * W, 256), 256, 0, st>>>(rows, n, W, np, na, planes.p); tg::note_launch(); }
+    TG_CUDA(cudaGetLastError());
+    double *const *dst = reinterpret_cast<double *const *>(out);
+    const double *src = planes.p;
+    const int width[3] = {1, 3, 9};
+    for (int f = 0; f < 3; f++) {
+        if (!(fields & (1 << f))) continue;
+        TG_CUDA(cudaMemcpyAsync(*dst++, src, sizeof(double) * n * width[f], cudaMemcpyDeviceToHost, st));
+        src += n * width[f];
+    }
+    return TG_OK;
+}
+
 }  // namespace tg
 
 using namespace tg;
@@ -327,7 +373,7 @@ tg_status tg_tree_fields(tg_tree t, const double *pos, const double *h, int64_t 
             wg = groups;
             wr = groot;
         }
-        if (mem == TG_MEM_HOST) TG_CUDA(tg::dev_malloc((void **)&dout, sizeof(double) * nt * W, st));
+        if (results_to_host(mem)) TG_CUDA(tg::dev_malloc((void **)&dout, sizeof(double) * nt * W, st));
         else dout = out;
         rc = run_walk(t, t->coord, t->soft, nt, wg, wr, gorder, ngroups, t->walk_idx, fields, quadrupole, theta,
                       G, group_size, precision, theta_per_group, nullptr, dout, st);
@@ -360,7 +406,7 @@ tg_status tg_tree_fields(tg_tree t, const double *pos, const double *h, int64_t 
         std::vector<int64_t> toff = {0, n};
         TG_TRY(make_groups(t, toff, group_size, &groups, &groot, &ngroups, st));
         if (group_size > 1) TG_TRY(make_cost_order(sp ? sp : dp.ptr, groups, ngroups, &gorder, st, t->sort_err));
-        if (mem == TG_MEM_HOST) TG_CUDA(tg::dev_malloc((void **)&dout, sizeof(double) * nt * W, st));
+        if (results_to_host(mem)) TG_CUDA(tg::dev_malloc((void **)&dout, sizeof(double) * nt * W, st));
         else dout = out;
         rc = run_walk(t, sp ? sp : dp.ptr, sh, nt, groups, groot, gorder, ngroups, scatter, fields, quadrupole, theta, G,
                       group_size, precision, theta_per_group, nullptr, dout, st);
@@ -373,9 +419,8 @@ tg_status tg_tree_fields(tg_tree t, const double *pos, const double *h, int64_t 
     if (groups) cudaFreeAsync(groups, st);
     if (groot) cudaFreeAsync(groot, st);
     if (gorder) cudaFreeAsync(gorder, st);
-    if (rc == TG_OK && mem == TG_MEM_HOST)
-        TG_CUDA(cudaMemcpyAsync(out, dout, sizeof(double) * nt * W, cudaMemcpyDeviceToHost, st));
-    if (mem == TG_MEM_HOST && dout) cudaFreeAsync(dout, st);
+    if (rc == TG_OK && results_to_host(mem)) rc = copy_results(dout, nt, fields, mem, out, st);
+    if (results_to_host(mem) && dout) cudaFreeAsync(dout, st);
     TG_CUDA(cudaStreamSynchronize(st));
     return rc;
 }
@@ -465,12 +510,11 @@ tg_status tg_bruteforce(const double *pos_t, const double *h_t, int64_t nt, cons
         if (mutual) dht.ptr = zs;
     }
     double *dout = out;
-    if (mem == TG_MEM_HOST) TG_CUDA(tg::dev_malloc((void **)&dout, sizeof(double) * nt * W, st));
+    if (results_to_host(mem)) TG_CUDA(tg::dev_malloc((void **)&dout, sizeof(double) * nt * W, st));
     tg_status rc = run_bruteforce(dpt.ptr, dht.ptr, nt, dps.ptr, dms.ptr, dhs.ptr, ns, fields, mutual, G, precision,
                                   dout, st);
-    if (rc == TG_OK && mem == TG_MEM_HOST)
-        TG_CUDA(cudaMemcpyAsync(out, dout, sizeof(double) * nt * W, cudaMemcpyDeviceToHost, st));
-    if (mem == TG_MEM_HOST) cudaFreeAsync(dout, st);
+    if (rc == TG_OK && results_to_host(mem)) rc = copy_results(dout, nt, fields, mem, out, st);
+    if (results_to_host(mem)) cudaFreeAsync(dout, st);
     if (zt) cudaFreeAsync(zt, st);
     if (zs) cudaFreeAsync(zs, st);
     TG_CUDA(cudaStreamSynchronize(st));

@@ -361,6 +361,10 @@ struct SortedPairs {
     explicit SortedPairs(cudaStream_t s) : mem(s) {}
 };
 
+// A walk's or direct sum's rows (n, W) of the requested fields to the caller's host memory, as mem says.
+inline bool results_to_host(int mem) { return mem == TG_MEM_HOST || mem == TG_MEM_HOST_FIELDS; }
+tg_status copy_results(const double *rows, int64_t n, int fields, int mem, double *out, cudaStream_t st);
+
 // Counts kernel launches (every launch site calls it; read through tg_launch_count()).
 void note_launch();
 // Adjusts the count by delta: + the kernels of a replayed CUDA graph, - the launches recorded (not

@@ -283,7 +283,7 @@ tg_status tg_targets_groups_copy(tg_targets ts, int32_t *first, int32_t *count, 
 tg_status tg_targets_fields(tg_targets ts, int fields, int quadrupole, double theta, double G, int precision,
                             const float *tol_per_group, int mem, double *out, void *stream) {
     if (!ts || !out || (fields & 7) == 0 || (fields & ~7) || !(theta > 0) ||
-        (precision != TG_FP32 && precision != TG_FP64) || (mem != TG_MEM_HOST && mem != TG_MEM_DEVICE))
+        (precision != TG_FP32 && precision != TG_FP64) || (!results_to_host(mem) && mem != TG_MEM_DEVICE))
         return TG_ERR_BAD_ARG;
     if (tol_per_group && precision != TG_FP32) return TG_ERR_BAD_ARG;
     tg_tree_s *src = ts->src, *tt = ts->tt;
@@ -294,13 +294,12 @@ tg_status tg_targets_fields(tg_targets ts, int fields, int quadrupole, double th
     const int64_t n = ts->n;
     const int W = width_of(fields);
     double *dout = out;
-    if (mem == TG_MEM_HOST) TG_CUDA(dev_malloc((void **)&dout, sizeof(double) * n * W, st));
+    if (results_to_host(mem)) TG_CUDA(dev_malloc((void **)&dout, sizeof(double) * n * W, st));
     tg_status rc = run_walk(src, tt->coord, tt->soft, n, tt->groups, tt->group_root, nullptr, tt->ngroups,
                             tt->walk_idx, fields, quadrupole, theta, G, ts->group_size, precision, nullptr,
                             tol_per_group, dout, st);
-    if (rc == TG_OK && mem == TG_MEM_HOST)
-        TG_CUDA(cudaMemcpyAsync(out, dout, sizeof(double) * n * W, cudaMemcpyDeviceToHost, st));
-    if (mem == TG_MEM_HOST) cudaFreeAsync(dout, st);
+    if (rc == TG_OK && results_to_host(mem)) rc = copy_results(dout, n, fields, mem, out, st);
+    if (results_to_host(mem)) cudaFreeAsync(dout, st);
     TG_CUDA(cudaStreamSynchronize(st));
     return rc;
 }

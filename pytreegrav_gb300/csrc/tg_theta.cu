@@ -697,15 +697,14 @@ tg_status learned_walk(tg_tree_s *t, FeatFn feats, const double *tpos, const dou
     }
     const int W = field_width_of(fields);
     double *dout = out;
-    if (mem == TG_MEM_HOST) TG_CUDA(dev_malloc((void **)&dout, sizeof(double) * nt * W, st));
+    if (results_to_host(mem)) TG_CUDA(dev_malloc((void **)&dout, sizeof(double) * nt * W, st));
     t->err_budget = (m && tol) ? m->err_budget : 0.f;
     t->rewalk_theta = theta_fallback;
     tg_status rc = run_walk(t, tpos, tsoft, nt, groups, groot, nullptr, ng, scatter, fields, quadrupole, theta, G,
                             group_size, TG_FP32, tg_theta, tol, dout, st);
     t->err_budget = 0.f;
-    if (rc == TG_OK && mem == TG_MEM_HOST)
-        TG_CUDA(cudaMemcpyAsync(out, dout, sizeof(double) * nt * W, cudaMemcpyDeviceToHost, st));
-    if (mem == TG_MEM_HOST) cudaFreeAsync(dout, st);
+    if (rc == TG_OK && results_to_host(mem)) rc = copy_results(dout, nt, fields, mem, out, st);
+    if (results_to_host(mem)) cudaFreeAsync(dout, st);
     TG_CUDA(cudaStreamSynchronize(st));
     return rc;
 }

@@ -177,7 +177,6 @@ class Octree:
             raise ValueError("request at least one of potential=True, accel=True, tidal=True")
         if quadrupole and not self.HasQuads:
             _lib.check(_lib.TG_ERR_NO_QUADRUPOLES)
-        W = int(bool(potential)) + 3 * int(bool(accel)) + 9 * int(bool(tidal))
         ord_code = {"tree": _lib.TG_ORDER_TREE, "morton": _lib.TG_ORDER_MORTON, "given": _lib.TG_ORDER_GIVEN}[order]
         prec = {"fp32": _lib.TG_FP32, "fp64": _lib.TG_FP64}[precision]
         if ord_code == _lib.TG_ORDER_TREE:
@@ -188,18 +187,17 @@ class Octree:
             n = len(pos)
             soft = None if soft is None else _as_f64(soft, (n,))
             pos_p, soft_p = _lib.ptr(pos), _lib.ptr(soft)
-        out = np.empty((n, W))
+        res, out, mem = _results(n, potential, accel, tidal)
         if n == 0:
-            return _split(out, potential, accel, tidal)
+            return res
         tpg = None
         if theta_per_group is not None:
             tpg = ctypes.c_void_p(int(theta_per_group))  # a device pointer (float32, one per group)
         grp = {"blocks": _lib.TG_GROUP_BLOCKS, "tree": _lib.TG_GROUP_TREE}[grouping]
         rc = _lib.load().tg_tree_fields(self._h, pos_p, soft_p, n, fields, int(bool(quadrupole)), float(theta),
-                                        float(G), int(group_size), grp, ord_code, prec, tpg, _lib.TG_MEM_HOST,
-                                        _lib.ptr(out), None)
+                                        float(G), int(group_size), grp, ord_code, prec, tpg, mem, out, None)
         _lib.check(rc, "tree walk")
-        return _split(out, potential, accel, tidal)
+        return res
 
     def _fields_learned(self, potential, accel, tidal, quadrupole, theta, G, order, precision, learned, error_ratio):
         from . import theta as th
@@ -215,13 +213,11 @@ class Octree:
         if quadrupole and not self.HasQuads:
             _lib.check(_lib.TG_ERR_NO_QUADRUPOLES)
         model, l10 = _model_and_lambda(learned, error_ratio, quadrupole)
-        W = int(bool(potential)) + 3 * int(bool(accel)) + 9 * int(bool(tidal))
-        out = np.empty((self.NumParticles, W))
+        res, out, mem = _results(self.NumParticles, potential, accel, tidal)
         rc = _lib.load().tg_tree_fields_learned(self._h, fields, int(bool(quadrupole)), float(G), th.GROUP_SIZE,
-                                                model.handle(), float(l10), float(theta), _lib.TG_MEM_HOST,
-                                                _lib.ptr(out), None)
+                                                model.handle(), float(l10), float(theta), mem, out, None)
         _lib.check(rc, "learned tree walk")
-        return _split(out, potential, accel, tidal)
+        return res
 
     def column_density(self, pos, rays=None, theta=0.5, group_size=0):
         """Column density of this tree's particles (uniform spheres, radius = softening) from each
@@ -413,14 +409,12 @@ class TargetSet:
             raise ValueError("request at least one of potential=True, accel=True, tidal=True")
         if quadrupole and not self.tree.HasQuads:
             _lib.check(_lib.TG_ERR_NO_QUADRUPOLES)
-        W = int(bool(potential)) + 3 * int(bool(accel)) + 9 * int(bool(tidal))
-        out = np.empty((self.n, W))
+        res, out, mem = _results(self.n, potential, accel, tidal)
         if self.n:
             prec = {"fp32": _lib.TG_FP32, "fp64": _lib.TG_FP64}[precision]
             _lib.check(_lib.load().tg_targets_fields(self._h, fields, int(bool(quadrupole)), float(theta), float(G),
-                                                     prec, None, _lib.TG_MEM_HOST, _lib.ptr(out), None),
-                       "target walk")
-        return _split(out, potential, accel, tidal)
+                                                     prec, None, mem, out, None), "target walk")
+        return res
 
     def fields_learned(self, potential=False, accel=False, tidal=False, quadrupole=False, theta=0.7, G=1.0,
                        precision="fp32", learned=True, error_ratio=None):
@@ -435,14 +429,12 @@ class TargetSet:
         if quadrupole and not self.tree.HasQuads:
             _lib.check(_lib.TG_ERR_NO_QUADRUPOLES)
         model, l10 = _model_and_lambda(learned, error_ratio, quadrupole, targets=True)
-        W = int(bool(potential)) + 3 * int(bool(accel)) + 9 * int(bool(tidal))
-        out = np.empty((self.n, W))
+        res, out, mem = _results(self.n, potential, accel, tidal)
         if self.n:
             _lib.check(_lib.load().tg_targets_fields_learned(self._h, fields, int(bool(quadrupole)), float(G),
-                                                             model.handle(), float(l10), float(theta),
-                                                             _lib.TG_MEM_HOST, _lib.ptr(out), None),
-                       "learned target walk")
-        return _split(out, potential, accel, tidal)
+                                                             model.handle(), float(l10), float(theta), mem, out,
+                                                             None), "learned target walk")
+        return res
 
     def close(self):
         h = getattr(self, "_h", None)
@@ -494,17 +486,19 @@ class WalkGraph:
             pass
 
 
-def _split(out, potential, accel, tidal):
-    res, o = {}, 0
+def _results(n, potential, accel, tidal):
+    """The requested fields' arrays for n targets, with the `out` and `mem` that have the library fill them."""
+    res = {}
     if potential:
-        res["potential"] = out[:, 0].copy()
-        o = 1
+        res["potential"] = np.empty(n)
     if accel:
-        res["accel"] = np.ascontiguousarray(out[:, o:o + 3])
-        o += 3
+        res["accel"] = np.empty((n, 3))
     if tidal:
-        res["tidal"] = np.ascontiguousarray(out[:, o:o + 9]).reshape(-1, 3, 3)
-    return res
+        res["tidal"] = np.empty((n, 3, 3))
+    addr = [a.ctypes.data for a in res.values()]
+    if len(addr) == 1:
+        return res, ctypes.c_void_p(addr[0]), _lib.TG_MEM_HOST
+    return res, (ctypes.c_void_p * len(addr))(*addr), _lib.TG_MEM_HOST_FIELDS
 
 
 def morton_order(pos):
@@ -542,12 +536,11 @@ def bruteforce(pos_t, h_t, pos_s, m_s, h_s, potential=False, accel=False, tidal=
         pos_t = _as_f64(pos_t, (-1, 3))
         h_t = None if h_t is None else _as_f64(h_t, (len(pos_t),))
     nt = len(pos_t)
-    W = int(bool(potential)) + 3 * int(bool(accel)) + 9 * int(bool(tidal))
-    out = np.empty((nt, W))
+    res, out, mem = _results(nt, potential, accel, tidal)
     if nt:
         prec = {"fp32": _lib.TG_FP32, "fp64": _lib.TG_FP64}[precision]
         rc = _lib.load().tg_bruteforce(_lib.ptr(pos_t), _lib.ptr(h_t), nt, _lib.ptr(pos_s), _lib.ptr(m_s),
                                        _lib.ptr(h_s), ns, fields, int(bool(mutual)), float(G), prec,
-                                       _lib.TG_MEM_HOST, _lib.ptr(out), None)
+                                       mem, out, None)
         _lib.check(rc, "bruteforce")
-    return _split(out, potential, accel, tidal)
+    return res

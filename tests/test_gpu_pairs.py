@@ -51,3 +51,30 @@ def test_walks_on_both_sides_of_the_lean_line(n, gs, fields):
     ref, _ = O.self_fields(x, m, h, nthreads=O.num_threads(), **kw)
     for k in fields:
         assert rel_rms(got[k], ref[k]) < 2e-5, k
+
+
+@pytest.mark.parametrize("n", [1, 2, 85, 86, 1000])
+def test_results_in_arrays_of_their_own(n):
+    """Every combination of fields, taken apart on the GPU, against each field asked for alone through the FP64
+    direct sum (the same sums) and the FP64 walk with one target per group."""
+    import itertools
+
+    import pytreegrav_gb300 as tg
+    from pytreegrav_gb300.tree import bruteforce
+
+    rng = np.random.default_rng(n)
+    x, m = rng.random((n, 3)), rng.random(n)
+    names = ("potential", "accel", "tidal")
+    shape = {"potential": (n,), "accel": (n, 3), "tidal": (n, 3, 3)}
+    tree = tg.ConstructTree(x, m)
+    for k in (1, 2, 3):
+        for some in itertools.combinations(names, k):
+            kw = {f: True for f in some}
+            got = bruteforce(None, None, x, m, None, mutual=True, **kw)
+            walked = tree.fields(precision="fp64", group_size=1, theta=1e-3, **kw)
+            assert list(got) == list(walked) == list(some)
+            for f in some:
+                alone = bruteforce(None, None, x, m, None, mutual=True, **{f: True})[f]
+                assert got[f].shape == walked[f].shape == shape[f] and got[f].flags.c_contiguous and got[f].base is None
+                assert np.allclose(got[f], alone, rtol=1e-12, atol=1e-12 * np.abs(alone).max())
+                assert np.allclose(walked[f], alone, rtol=1e-10, atol=1e-10 * np.abs(alone).max())
