@@ -1210,9 +1210,11 @@ __device__ __forceinline__ void node_moments_kids(const MomentArgs &a, int64_t j
 // Large levels (FP64-throughput-bound): one thread per node, the block's nodes first ordered by
 // child count (a counting sort in shared memory, most children first) so that a warp's lanes run
 // the same number of child steps. Which thread takes which node does not change any result.
-// MOM_BLOCK: 64, 128 or 256 threads.
+// MOM_BLOCK: 64, 128 or 256 threads. Blocks of 256 (levels of ~1e5 nodes and more) keep to the registers that let six share
+// an SM: their warps wait for the children's scattered loads (build of 8e6 particles: four blocks 3.69 ms, five
+// 3.63, six 3.46, seven and eight, which spill, 3.73); for the smaller ones, on smaller levels, that was slower.
 template <int MOM_BLOCK>
-__global__ void __launch_bounds__(MOM_BLOCK) k_moments_sorted(MomentArgs a, const int32_t *list, int count,
+__global__ void __launch_bounds__(MOM_BLOCK, MOM_BLOCK == 256 ? 6 : 1) k_moments_sorted(MomentArgs a, const int32_t *list, int count,
                                                               const int32_t *kids, const int8_t *nk) {
     chain_wait();
     chain_next();
@@ -1256,8 +1258,6 @@ constexpr int WIDE_MAX_LEVEL = 12288;  // levels up to this many nodes use k_mom
 
 __global__ void __launch_bounds__(WIDE_THREADS) k_moments_wide(MomentArgs a, const int32_t *list, int count,
                                                               const int32_t *kids, const int8_t *nk) {
-    chain_wait();
-    chain_next();
     __shared__ double s_m[8][WIDE_NODES], s_t[3][8][WIDE_NODES], s_h[8][WIDE_NODES];  // child terms
     __shared__ double s_sum[5][WIDE_NODES], s_com[3][WIDE_NODES];
     __shared__ float s_q[6][8][WIDE_NODES];  // the children's FP32 quadrupole terms
