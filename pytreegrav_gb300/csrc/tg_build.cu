@@ -232,13 +232,17 @@ __device__ __forceinline__ bool nonfinite_bits(double x) {  // the all-ones expo
 }
 __global__ void k_gather(const uint32_t *perm, int64_t n, const double *pos, const double *m, const double *h,
                          const uint64_t *keys_in, double *coord, double *mass, double *soft, uint64_t *keys_sorted,
-                         int64_t *walk_idx, const int *sort_err, int *nonfinite) {
+                         int64_t *walk_idx, int *sort_err, int *nonfinite) {
     chain_wait();
     chain_next();
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const bool bad = *sort_err != 0;
     int64_t o = bad ? i : (int64_t)perm[i];
+    if (o >= n) {  // no permutation: the sort is reported as failed, and nothing is read out of range
+        atomicExch(sort_err, 1);
+        o = i;
+    }
     const double x = pos[3 * o], y = pos[3 * o + 1], z = pos[3 * o + 2];
     const double mi = m ? m[o] : 0.0, hi = h ? h[o] : 0.0;
     coord[3 * i] = x;
@@ -877,6 +881,7 @@ __global__ void k_final_index(const uint64_t *sorted_keys, const uint32_t *vals,
     }
     if (q < count) {
         int64_t c = vals[q];
+        if (c >= count) c = q;  // no permutation: k_write finds the slots left out
         int s = nd_sys[c];
         if (q < count - nsys) final_of_slot[c] = ntot + q + s + 1;
     }
@@ -940,6 +945,10 @@ __global__ void k_write(Nodes nd, int64_t count, int64_t ntot, int node_blocks, 
     int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= count) return;
     int64_t f = final_of_slot[c];
+    if (f < ntot || f >= NE) {  // the numbering left the slot out: nothing is written out of range
+        atomicOr(bad, 4);
+        f = ntot + c;
+    }
     o.mass[f] = 0.0;  // the moment pass fills these
     o.soft[f] = 0.0;
     o.delta[f] = 0.0;

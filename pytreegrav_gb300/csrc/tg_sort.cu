@@ -532,8 +532,8 @@ __global__ void __launch_bounds__(OS_THREADS, 2)
 #pragma unroll
     for (int r = 0; r < ROUNDS; r++) {
         const int i = wofs + r * 32;
-        kv[r] = i < cnt ? __ldg(kp + i) : 0ull;
-        vv[r] = i < cnt ? __ldg(vp + i) : 0u;
+        kv[r] = i < cnt ? kp[i] : 0ull;  // coherent loads: the pass before may still write when this kernel starts
+        vv[r] = i < cnt ? vp[i] : 0u;
     }
     // ranks round by round: the lanes of one digit find one another through a word per digit
 #pragma unroll

@@ -1796,9 +1796,11 @@ __global__ void k_permute_groups(const uint32_t *perm, int64_t ngroups, const in
     chain_next();
     int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= ngroups) return;
-    gout[g] = gin[perm[g]];
-    rout[g] = rin[perm[g]];
-    if (nin) nout[g] = nin[perm[g]];
+    int64_t o = perm[g];
+    if (o >= ngroups) o = g;  // a sort that failed: nothing is read out of range
+    gout[g] = gin[o];
+    rout[g] = rin[o];
+    if (nin) nout[g] = nin[o];
 }
 
 // Targets in walk order split once per walk into hi/lo parts in the walk precision.
