@@ -822,7 +822,9 @@ __global__ void __launch_bounds__(MAX_WALK_WARPS * 32) __maxnreg__((walk_reg_cap
         float err_est = 0.f;  // this lane's share of the group's truncation estimate
         // a node's mass-aware radius is its stored factor times tol^(-1/(p+2))
         const float tol_k = mass_aware ? exp2f(-log2f(tolg) * (QUAD ? 0.2f : 0.25f)) : 0.f;
-        const float rel_eps = 1e-5f, abs_eps = 1e-6f;
+        // the absolute part of the node test's margin: the box's rounding, and distances whose FP32 squares are
+        // subnormal and round by more than the relative part (2^-63: below it nothing is certain)
+        const float rel_eps = 1e-5f, abs_tol = 1e-6f * gscale + 1.2e-19f;
         // softening-path threshold: a source whose squared distance to the box exceeds this cannot
         // be within any target's softening length, nor coincide with a target
         const T near_eps = (sizeof(T) == 4 ? T(4e-7) : T(1e-15)) * ((T)gscale + T(1e-30));
@@ -1329,7 +1331,7 @@ __global__ void __launch_bounds__(MAX_WALK_WARPS * 32) __maxnreg__((walk_reg_cap
                     float crit = c1 > c2 ? c1 : c2;
                     // FP32 error bound: node positions near the boundary are within gscale + 2 crit of
                     // the origin, so the relative term covers their rounding
-                    float tol = rel_eps * crit + abs_eps * gscale;
+                    float tol = rel_eps * crit + abs_tol;
                     float hiq = crit + tol, loq = crit - tol;
                     if (mass_aware) {  // no pytreegrav decision to reproduce
                         acc = r2 > crit * crit;
