@@ -33,6 +33,10 @@ int tg_measure_fp32_fma(double *tflops, double *ms, void *stream);
  * for bit (NaN results: NaN on both sides). *mismatches receives the count of differing values. */
 int tg_check_f32_conversion(const double *x, int64_t n, int64_t *mismatches, void *stream);
 
+/* The FP64 walk's reciprocal square root of each of the n doubles at x (device memory, any values), written
+ * to out (device memory), for a test of its error. Asynchronous on `stream`. */
+int tg_check_rsqrt64(const double *x, int64_t n, double *out, void *stream);
+
 /* Bounds of the library's bounded device loops, for tests that make each one run out (0 or less:
  * the built-in bound): polls of one look-back word in a radix pass (built in: 2^22; running out
  * gives TG_ERR_QUEUE_TIMEOUT), traversal steps of one group of a tree walk (the node count, which

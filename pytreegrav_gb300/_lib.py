@@ -106,6 +106,7 @@ MEASURE_EXPORTS = [
     "tg_launch_count",
     "tg_measure_fp32_fma",
     "tg_check_f32_conversion",
+    "tg_check_rsqrt64",
     "tg_set_loop_limits",
 ]
 TG_THETA_NFEAT = 16

@@ -82,10 +82,12 @@ __device__ __forceinline__ float rsqrt_t(float x) {
     asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
-// 1 / sqrt(x) to about an ulp in five FP64 operations (GB300 issues one per sub-partition every ~76 cycles):
-// the FP32 approximation y of the significand's, taken with an even exponent on the integer units, and one
-// step of Householder's third-order iteration, y + y e (1/2 + 3/8 e) with e = 1 - x y^2 (|e| < 2^-20: the next term is
-// 5/16 e^3). Zeros, subnormals, negative values, infinities and NaN take the library's.
+// 1 / sqrt(x), all but correctly rounded, in five FP64 operations (GB300 issues one per sub-partition every ~76
+// cycles): the FP32 approximation y of the significand's, taken with an even exponent on the integer units, and one
+// step of Householder's third-order iteration, y + y e (1/2 + 3/8 e) with e = 1 - x y^2. y has 24 bits, so y^2 is
+// exact (subnormal ones too) and e rounds once; |e| < 2^-21, the next term is 5/16 e^3. Largest error 0.500 units in
+// the last place (0.97 with e from x y, rounded, times y). Zeros, subnormals, negative values, infinities and NaN
+// take the library's.
 __device__ __forceinline__ double rsqrt_t(double x) {
     const uint64_t u = (uint64_t)__double_as_longlong(x);
     const uint32_t hi = (uint32_t)(u >> 32), E = hi >> 20;  // sign and exponent
@@ -97,7 +99,7 @@ __device__ __forceinline__ double rsqrt_t(double x) {
     const uint32_t yb = __float_as_uint(rsqrt_t(m));  // 1/2 < y <= 1
     const double y = __longlong_as_double((long long)(((uint64_t)((yb >> 3) + ((896u - (uint32_t)half) << 20)) << 32) |
                                                       (uint64_t)(yb << 29)));
-    const double e = fma(-(x * y), y, 1.0);
+    const double e = fma(-x, y * y, 1.0);
     return fma(y * e, fma(0.375, e, 0.5), y);
 }
 __device__ __forceinline__ float sqrt_t(float x) { return sqrtf(x); }
@@ -1805,6 +1807,11 @@ __global__ void k_permute_groups(const uint32_t *perm, int64_t ngroups, const in
     if (nin) nout[g] = nin[o];
 }
 
+__global__ void k_rsqrt64(const double *x, int64_t n, double *out) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) out[i] = rsqrt_t(x[i]);
+}
+
 // Targets in walk order split once per walk into hi/lo parts in the walk precision.
 template <typename T>
 __global__ void k_prep_targets(const double *tpos, const double *th, int64_t n, vec4<T> *thi, vec4<T> *tlo) {
@@ -2808,6 +2815,14 @@ tg_status tg_walk_graph_status(tg_walk_graph g, void *stream) {
 
 tg_status tg_walk_graph_free(tg_walk_graph g) {
     graph_release(g);
+    return TG_OK;
+}
+
+int tg_check_rsqrt64(const double *x, int64_t n, double *out, void *stream) {
+    if (n < 0 || (n > 0 && (!x || !out))) return TG_ERR_BAD_ARG;
+    if (n == 0) return TG_OK;
+    { tg::k_rsqrt64<<<tg::div_up(n, 256), 256, 0, (cudaStream_t)stream>>>(x, n, out); tg::note_launch(); }
+    TG_CUDA(cudaGetLastError());
     return TG_OK;
 }
 
