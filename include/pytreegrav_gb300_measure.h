@@ -37,6 +37,11 @@ int tg_check_f32_conversion(const double *x, int64_t n, int64_t *mismatches, voi
  * to out (device memory), for a test of its error. Asynchronous on `stream`. */
 int tg_check_rsqrt64(const double *x, int64_t n, double *out, void *stream);
 
+/* Device addresses of the grouping that a tree (tg_tree_groups) or, with targets non-null, a target set keeps:
+ * (first target, count) pairs of int32 and each group's root node (int32), ngroups of both. For tests that
+ * damage them: a walk skips a group whose record is out of range and returns an error. */
+int tg_group_arrays(void *tree, void *targets, void **groups, void **roots, int64_t *ngroups);
+
 /* Bounds of the library's bounded device loops, for tests that make each one run out (0 or less:
  * the built-in bound): polls of one look-back word in a radix pass (built in: 2^22; running out
  * gives TG_ERR_QUEUE_TIMEOUT), traversal steps of one group of a tree walk (the node count, which

@@ -107,6 +107,7 @@ MEASURE_EXPORTS = [
     "tg_measure_fp32_fma",
     "tg_check_f32_conversion",
     "tg_check_rsqrt64",
+    "tg_group_arrays",
     "tg_set_loop_limits",
 ]
 TG_THETA_NFEAT = 16

@@ -48,14 +48,18 @@ int width_of(int fields) { return ((fields & 1) ? 1 : 0) + ((fields & 2) ? 3 : 0
 // so it is cut into runs of k consecutive targets, k the largest power of two with
 // k n_in / count <= 2G.
 __global__ void k_target_src_nodes(int64_t ntot, int64_t mtot, const double *cell, const double *size, Arena<float> ar,
-                                   const int2 *node_range, const double *tpos, const int2 *groups, int64_t ng, int G,
-                                   int *node, int *nsub, int *sublen) {
+                                   const int2 *node_range, const double *tpos, int64_t nt, const int2 *groups, int64_t ng,
+                                   int G, int *node, int *nsub, int *sublen) {
     chain_wait();
     chain_next();
     const int lane = lane_id(), sub = lane & 7;
     const int64_t g = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 3;
     const bool valid = g < ng;
-    const int2 gr = valid ? groups[g] : make_int2(0, 1);
+    int2 gr = valid ? groups[g] : make_int2(0, 1);
+    // a record out of range is kept as it is, uncut, and not followed here: the walk reports it
+    const int whole = gr.y;
+    const bool sound = gr.x >= 0 && gr.y >= 1 && gr.y <= G && (int64_t)gr.x + gr.y <= nt;
+    if (!sound) gr = make_int2(0, 1);
     unsigned long long ulo[3], uhi[3];  // as ordered integers: FP64 minima cost the FP64 pipe
     for (int i = sub < gr.y ? sub : 0, first = 1; i < gr.y; i += 8, first = 0)
 #pragma unroll
@@ -118,21 +122,21 @@ __global__ void k_target_src_nodes(int64_t ntot, int64_t mtot, const double *cel
             if (n_in <= 2.0 * G) k = gr.y;
         }
         nsub[g] = (gr.y + k - 1) / k;
-        sublen[g] = k;
+        sublen[g] = sound ? k : whole;
     }
 }
 
 // The refined groups: group g's targets cut into nsub[g] runs of sublen[g] (the last shorter), at
-// offset off[g], in start order.
+// offset off[g], in start order; total of them.
 __global__ void k_split_groups(const int2 *groups, const int *gnode, int64_t ng, const int *nsub, const int *sublen,
-                               const int *off, int2 *out, int *out_root, int *out_node) {
+                               const int *off, int total, int2 *out, int *out_root, int *out_node) {
     chain_wait();
     chain_next();
     const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= ng) return;
     const int2 gr = groups[g];
     const int k = sublen[g], o = off[g];
-    for (int i = 0; i < nsub[g]; i++) {
+    for (int i = 0; i < nsub[g] && o + i < total; i++) {
         const int first = gr.x + i * k;
         out[o + i] = make_int2(first, min(k, gr.x + gr.y - first));
         out_root[o + i] = 0;
@@ -150,7 +154,7 @@ tg_status targets_src_nodes(tg_targets_s *ts, cudaStream_t st) {
     TG_CUDA(dev_malloc((void **)&ts->src_node, sizeof(int) * std::max<int64_t>(ng, 1), st));
     if (ng > 0) {
         TG_CHAIN(k_target_src_nodes, div_up(8 * ng, 128), 128, 0, st, src->ntot, src->mtot, src->cell_center, src->size,
-                 src->arena32, src->node_range, tt->coord, tt->groups, ng, ts->group_size, ts->src_node, nullptr,
+                 src->arena32, src->node_range, tt->coord, ts->n, tt->groups, ng, ts->group_size, ts->src_node, nullptr,
                  nullptr);
         TG_CUDA(cudaGetLastError());
     }
@@ -172,7 +176,7 @@ tg_status targets_refine_groups(tg_targets_s *ts, cudaStream_t st) {
     TG_CUDA(off.alloc(ng + 1));
     TG_CUDA(cudaMemsetAsync(nsub.p + ng, 0, sizeof(int), st));
     TG_CHAIN(k_target_src_nodes, div_up(8 * ng, 128), 128, 0, st, src->ntot, src->mtot, src->cell_center, src->size,
-             src->arena32, src->node_range, tt->coord, tt->groups, ng, ts->group_size, node.p, nsub.p, sublen.p);
+             src->arena32, src->node_range, tt->coord, ts->n, tt->groups, ng, ts->group_size, node.p, nsub.p, sublen.p);
     TG_CUDA(cudaGetLastError());
     TG_TRY(exclusive_scan_i32(nsub.p, off.p, ng + 1, st));
     int total = 0;
@@ -185,7 +189,7 @@ tg_status targets_refine_groups(tg_targets_s *ts, cudaStream_t st) {
     TG_CUDA(dev_malloc((void **)&root, sizeof(int) * total, st));
     TG_CUDA(dev_malloc((void **)&gnode, sizeof(int) * total, st));
     TG_CHAIN(k_split_groups, div_up(ng, 128), 128, 0, st, tt->groups, tt->group_node, ng, nsub.p, sublen.p, off.p,
-             groups, root, gnode);
+             total, groups, root, gnode);
     TG_CUDA(cudaGetLastError());
     cudaFreeAsync(tt->groups, st);
     cudaFreeAsync(tt->group_root, st);
@@ -247,6 +251,15 @@ tg_status tg_targets_info(tg_targets ts, int64_t *n, int64_t *ngroups) {
     if (!ts) return TG_ERR_BAD_ARG;
     if (n) *n = ts->n;
     if (ngroups) *ngroups = ts->tt->ngroups;
+    return TG_OK;
+}
+
+int tg_group_arrays(tg_tree t, tg_targets ts, void **groups, void **roots, int64_t *ngroups) {
+    if (ts) t = ts->tt;
+    if (!t || !t->groups || !groups || !roots || !ngroups) return TG_ERR_BAD_ARG;
+    *groups = t->groups;
+    *roots = t->group_root;
+    *ngroups = t->ngroups;
     return TG_OK;
 }
 

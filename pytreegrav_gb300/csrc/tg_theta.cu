@@ -133,7 +133,8 @@ __global__ void k_features(int64_t ntot, const double *coord, const double *mass
                            const double *tcoord, const double *tsoft, const int2 *groups, const int *group_node,
                            int64_t ngroups,
                            const float4 *rec, const float *hs2, const int *ntop_p, const float4 *origin, int quad,
-                           float log10n, float *feat, unsigned long long *field_sums) {
+                           float log10n, int64_t mtot, int64_t ntargets, float *feat,
+                           unsigned long long *field_sums) {
     chain_wait();
     chain_next();
     // the tolerance unit's sums, added per block and then once to field_sums
@@ -143,7 +144,12 @@ __global__ void k_features(int64_t ntot, const double *coord, const double *mass
     const int64_t g = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (g < ngroups) {  // warp-uniform
-        const int2 gr = groups[g];
+        int2 gr = groups[g];
+        int gnode = group_node[g];
+        if (gr.x < 0 || gr.y < 1 || gr.y > 32 || (int64_t)gr.x + gr.y > ntargets || gnode < 0 || gnode >= mtot) {
+            gr = make_int2(0, 1);  // the walk reports it
+            gnode = 0;
+        }
         const float4 o4 = *origin;
         // targets: box and softening
         float lo[3], hi[3], hm;
@@ -198,7 +204,7 @@ __global__ void k_features(int64_t ntot, const double *coord, const double *mass
             vz += __shfl_xor_sync(FULL, vz, s);
         }
         // the features, one per lane (the sums above are on every lane after the butterfly)
-        const int64_t R = ntot, P = ntot + group_node[g];  // system root (node 0) and the group's node
+        const int64_t R = ntot, P = ntot + gnode;  // system root (node 0) and the group's node
         // FP64 compares and conversions as integer work (finite inputs: x > 0 iff its bits are a
         // positive int64)
         auto pos = [](double x) { return __double_as_longlong(x) > 0; };
@@ -581,7 +587,7 @@ using namespace tg;
 // Features of ng groups of targets (tcoord/tsoft in walk order; group_node: the source tree's node
 // holding each group) into feat (ng x NF); field_sums (2 x uint64, device, may be NULL) receives the
 // sums behind the tolerance unit.
-tg_status features_of_groups(tg_tree_s *t, const double *tcoord, const double *tsoft, const int2 *groups,
+tg_status features_of_groups(tg_tree_s *t, const double *tcoord, const double *tsoft, int64_t nt, const int2 *groups,
                              const int *group_node, int64_t ng, int quadrupole, float *feat, cudaStream_t st,
                              unsigned long long *field_sums) {
     if (t->nsys != 1) {
@@ -603,8 +609,8 @@ tg_status features_of_groups(tg_tree_s *t, const double *tcoord, const double *t
              origin);
     if (ng > 0) {
         TG_CHAIN(k_features, div_up(ng * 32, 256), 256, 0, st, t->ntot, t->coord, t->mass, t->size, tcoord, tsoft,
-                 groups, group_node, ng, rec, hs2, top, origin, quadrupole, (float)log10((double)t->ntot), feat,
-                 sums);
+                 groups, group_node, ng, rec, hs2, top, origin, quadrupole, (float)log10((double)t->ntot),
+                 t->mtot, nt, feat, sums);
     }
     TG_CUDA(cudaGetLastError());
     TG_CUDA(cudaFreeAsync(scr, st));
@@ -619,7 +625,7 @@ tg_status features_device(tg_tree_s *t, int group_size, int quadrupole, float *f
         return TG_ERR_BAD_ARG;
     }
     TG_TRY(tree_groups(t, group_size, st));
-    return features_of_groups(t, t->coord, t->soft, t->groups, t->group_node, t->ngroups, quadrupole, feat, st,
+    return features_of_groups(t, t->coord, t->soft, t->ntot, t->groups, t->group_node, t->ngroups, quadrupole, feat, st,
                               field_sums);
 }
 
@@ -627,7 +633,7 @@ tg_status features_device(tg_tree_s *t, int group_size, int quadrupole, float *f
 tg_status features_targets(tg_targets_s *ts, int quadrupole, float *feat, cudaStream_t st,
                            unsigned long long *field_sums = nullptr) {
     TG_TRY(targets_src_nodes(ts, st));
-    return features_of_groups(ts->src, ts->tt->coord, ts->tt->soft, ts->tt->groups, ts->src_node, ts->tt->ngroups,
+    return features_of_groups(ts->src, ts->tt->coord, ts->tt->soft, ts->n, ts->tt->groups, ts->src_node, ts->tt->ngroups,
                               quadrupole, feat, st, field_sums);
 }
 

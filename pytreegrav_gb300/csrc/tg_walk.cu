@@ -382,7 +382,11 @@ struct WalkArgs {
     const int2 *groups;                        // (first target, count)
     const int *group_root;                     // arena node index of each group's tree root
     const int *group_order;                    // queue position -> group (null: identity)
-    int64_t ngroups;
+    int64_t ngroups;                           // units of this pass (with ngroups_dev: at most)
+    // Bounds of what the walk reads from device memory and indexes with: the groups, the targets (and rows of
+    // out). A record beyond them (lists, groups, roots, rows) is not followed: its group is skipped and the
+    // status says so.
+    int64_t all_groups, ntargets;
     double theta;
     const float *theta_group;
     // per group error tolerance (null or <= 0: pytreegrav's geometric criterion). A group with a
@@ -727,7 +731,7 @@ __global__ void __launch_bounds__(MAX_WALK_WARPS * 32) __maxnreg__((walk_reg_cap
     const unsigned lt = lanemask_lt();
     unsigned long long n_int = 0, n_tests = 0, n_steps = 0, n_qint = 0;
     int max_sp = 0;
-    const int64_t ngroups = a.ngroups_dev ? (int64_t)*a.ngroups_dev : a.ngroups;
+    const int64_t ngroups = a.ngroups_dev ? min((int64_t)*a.ngroups_dev, a.ngroups) : a.ngroups;
     if (a.ar.bad && *a.ar.bad) {  // the tree's links did not make a valid arena: read nothing
         if (threadIdx.x == 0 && blockIdx.x == 0) atomicOr(a.status, 1 << TG_ERR_CUDA);
         return;
@@ -746,14 +750,18 @@ __global__ void __launch_bounds__(MAX_WALK_WARPS * 32) __maxnreg__((walk_reg_cap
         if (g >= ngroups) break;
         const int unit = g;
         int start;  // the node the traversal starts from (an item may be a particle: ~leaf)
-        if (a.item_group) {
-            start = a.item_node[unit];
-            g = a.item_group[unit];
-        } else {
-            if (a.group_order) g = a.group_order[g];
-            start = a.group_root[g];
+        if (a.item_group) g = a.item_group[unit];
+        else if (a.group_order) g = a.group_order[g];
+        const bool known = g >= 0 && g < a.all_groups;
+        const int2 gr = known ? a.groups[g] : make_int2(0, 0);
+        start = !known ? 0 : (a.item_group ? a.item_node[unit] : a.group_root[g]);
+        if (gr.x < 0 || gr.y < 1 || gr.y > a.gs || (int64_t)gr.x + gr.y > a.ntargets ||
+            !(start >= 0 ? start < a.ar.n_nodes : a.item_group && ~start < a.ar.n_leaves)) {
+            if (lane == 0) atomicOr(a.status, 1 << TG_ERR_CUDA);
+            if (TEAM) __syncthreads();  // every warp has read the unit before the next one is drawn
+            else __syncwarp();
+            continue;
         }
-        const int2 gr = a.groups[g];
         // lanes per target slot: the smallest power of two holding the group (at most a.gs); the
         // other lanes of the warp take interleaved shares of every source batch
         int GS = a.gs;
@@ -1507,7 +1515,8 @@ __global__ void __launch_bounds__(MAX_WALK_WARPS * 32) __maxnreg__((walk_reg_cap
                 for (int c = 0; c < 10; c++) o[c] = v[c];
             } else {
                 const int64_t row = a.scatter ? a.scatter[t] : t;
-                write_fields(a.out + row * a.out_w, a.out_fields, v, a.G);
+                if (row >= 0 && row < a.ntargets) write_fields(a.out + row * a.out_w, a.out_fields, v, a.G);
+                else atomicOr(a.status, 1 << TG_ERR_CUDA);
             }
         }
         __syncwarp();
@@ -1590,9 +1599,11 @@ __global__ void k_tree_groups_mark(int64_t ntot, int64_t mtot, const int2 *node_
         root = (int)sys_node_off[s];
         if (r.y - r.x <= G && parent[ntot + j] < 0) {
             unsigned long long q = atomicAdd(count, 1ull);
-            groups[q] = make_int2(r.x, r.y - r.x);
-            group_root[q] = root;
-            group_node[q] = (int)j;
+            if (q < ntot) {  // (groups hold particles of their own, so there are at most ntot)
+                groups[q] = make_int2(r.x, r.y - r.x);
+                group_root[q] = root;
+                group_node[q] = (int)j;
+            }
         }
     }
     const bool big = valid && r.y - r.x > G;
@@ -1754,7 +1765,7 @@ __global__ void k_tree_groups_large(int64_t ntot, const int2 *node_range, const 
             unsigned long long base = 0;
             if (lane == 0) base = atomicAdd(count, (unsigned long long)nemit);
             base = __shfl_sync(FULL, base, 0);
-            if (lane < nemit) {
+            if (lane < nemit && base + lane < ntot) {
                 groups[base + lane] = make_int2(my_glo, my_gcnt);
                 group_root[base + lane] = root;
                 group_node[base + lane] = (int)j;
@@ -1862,6 +1873,7 @@ struct TopArgs {
     int *item_count;  // per unit
     int item_cap;
     int *status;
+    int64_t all_groups, ntargets;  // as in WalkArgs
 };
 
 template <typename T>
@@ -1877,7 +1889,15 @@ __global__ void __launch_bounds__(TOP_WARPS * 32) k_walk_top(TopArgs<T> a) {
         return;
     }
     const int g = a.heavy[u];
-    const int2 gr = a.groups[g];
+    const bool known = g >= 0 && g < a.all_groups;
+    const int2 gr = known ? a.groups[g] : make_int2(0, 0);
+    if (gr.x < 0 || gr.y < 1 || gr.y > 32 || (int64_t)gr.x + gr.y > a.ntargets) {
+        if (lane == 0) {
+            atomicOr(a.status, 1 << TG_ERR_CUDA);
+            a.item_count[u] = 0;
+        }
+        return;
+    }
     const int64_t t = gr.x + (lane < gr.y ? lane : 0);
     double bmin[3], bmax[3], hmax = a.th[t];
     for (int k = 0; k < 3; k++) bmin[k] = bmax[k] = a.tpos[3 * t + k];
@@ -1980,11 +2000,14 @@ constexpr int RED_THREADS = 256;
 __global__ void __launch_bounds__(RED_THREADS) k_reduce_items(const int *heavy, int nheavy, const int64_t *off,
                                                               const int *count, const int2 *groups, int gs,
                                                               const double *partial, const int64_t *scatter,
+                                                              int64_t ngroups, int64_t ntargets, int *status,
                                                               int out_fields, int out_w, double G, double *out) {
     __shared__ double sh[10][RED_THREADS];
     const int u = blockIdx.x / gs, slot = blockIdx.x % gs;
     if (u >= nheavy || count[u] < 0) return;  // block-uniform: walked whole
-    const int2 gr = groups[heavy[u]];
+    const int g = heavy[u];
+    if (g < 0 || g >= ngroups) return;  // reported by k_walk_top
+    const int2 gr = groups[g];
     if (slot >= gr.y) return;  // block-uniform
     const int t = threadIdx.x;
     double v[10];
@@ -2010,8 +2033,9 @@ __global__ void __launch_bounds__(RED_THREADS) k_reduce_items(const int *heavy, 
 #pragma unroll
         for (int c = 0; c < 10; c++) tot[c] = sh[c][0];
         const int64_t tg_ = gr.x + slot;
-        const int64_t row = scatter ? scatter[tg_] : tg_;
-        write_fields(out + row * out_w, out_fields, tot, G);
+        const int64_t row = tg_ < 0 || tg_ >= ntargets ? -1 : (scatter ? scatter[tg_] : tg_);
+        if (row >= 0 && row < ntargets) write_fields(out + row * out_w, out_fields, tot, G);
+        else atomicOr(status, 1 << TG_ERR_CUDA);
     }
 }
 
@@ -2265,6 +2289,8 @@ static tg_status walk_heavy(tg_tree_s *t, const WalkArgs<T> &a, Arena<T> &ar, in
     ta.item_count = counts.p;
     ta.item_cap = cap;
     ta.status = a.status;
+    ta.all_groups = a.all_groups;
+    ta.ntargets = a.ntargets;
     { k_walk_top<T><<<div_up(nheavy, TOP_WARPS), TOP_WARPS * 32, 0, st>>>(ta); note_launch(); }
     TG_CUDA(cudaGetLastError());
     std::vector<int> hc(nheavy), hg(nheavy);
@@ -2307,6 +2333,7 @@ static tg_status walk_heavy(tg_tree_s *t, const WalkArgs<T> &a, Arena<T> &ar, in
         TG_TRY((dispatch_walk<T, STACK_LARGE>(b, fields, quad, warps, st)));
         { k_reduce_items<<<(unsigned)((int64_t)nheavy * a.gs), RED_THREADS, 0, st>>>(heavy, nheavy, doff.p, counts.p,
                                                                                      a.groups, a.gs, partial.p, a.scatter,
+                                                                                     a.all_groups, a.ntargets, a.status,
                                                                                      a.out_fields, a.out_w, a.G, a.out); note_launch(); }
         TG_CUDA(cudaGetLastError());
     }
@@ -2423,7 +2450,7 @@ tg_status run_walk(tg_tree_s *t, const double *tpos, const double *th, int64_t n
         a.tc = t->coord; a.ts = t->soft; a.tsize = t->size; a.tdelta = t->delta;
         a.tpos = tpos; a.th = th; a.scatter = scatter; a.groups = groups; a.group_root = group_root;
         a.group_order = group_order;
-        a.ngroups = ngroups; a.theta = theta; a.theta_group = theta_group; a.tol_group = tol_group; a.G = G;
+        a.ngroups = a.all_groups = ngroups; a.ntargets = ntargets; a.theta = theta; a.theta_group = theta_group; a.tol_group = tol_group; a.G = G;
         a.err_budget = tol_group ? t->err_budget : 0.f;
         a.gerr = gerr;
         a.rewalk_theta = t->rewalk_theta;
@@ -2448,7 +2475,7 @@ tg_status run_walk(tg_tree_s *t, const double *tpos, const double *th, int64_t n
         a.tc = t->coord; a.ts = t->soft; a.tsize = t->size; a.tdelta = t->delta;
         a.tpos = tpos; a.th = th; a.scatter = scatter; a.groups = groups; a.group_root = group_root;
         a.group_order = group_order;
-        a.ngroups = ngroups; a.theta = theta; a.theta_group = theta_group; a.tol_group = tol_group; a.G = G;
+        a.ngroups = a.all_groups = ngroups; a.ntargets = ntargets; a.theta = theta; a.theta_group = theta_group; a.tol_group = tol_group; a.G = G;
         a.err_budget = tol_group ? t->err_budget : 0.f;
         a.gerr = gerr;
         a.rewalk_theta = t->rewalk_theta;
@@ -2490,7 +2517,8 @@ tg_status run_walk(tg_tree_s *t, const double *tpos, const double *th, int64_t n
         return TG_ERR_QUEUE_TIMEOUT;
     }
     if (status & (1 << TG_ERR_CUDA)) {
-        set_last_error_msg("internal error: tree links do not form a valid octree for the walk arena");
+        set_last_error_msg("internal error: tree links do not form a valid octree for the walk arena, or a walk record "
+                           "is out of range");
         return TG_ERR_CUDA;
     }
     if (status & (1 << TG_ERR_STACK_OVERFLOW)) return TG_ERR_STACK_OVERFLOW;
@@ -2533,6 +2561,10 @@ tg_status tree_groups(tg_tree_s *t, int G, cudaStream_t st) {
     unsigned long long ng = 0;
     TG_CUDA(cudaMemcpyAsync(&ng, cnt, sizeof(ng), cudaMemcpyDeviceToHost, st));
     TG_CUDA(cudaStreamSynchronize(st));
+    if (ng > (unsigned long long)N) {
+        set_last_error_msg("internal error: the tree grouping made more groups than there are particles");
+        return TG_ERR_CUDA;
+    }
     // deterministic Morton order of the groups (their emission order depends on thread timing)
     uint64_t *keys = nullptr;
     uint32_t *vals = nullptr;
@@ -2756,7 +2788,7 @@ tg_status tg_walk_graph_create(tg_tree t, int fields, int quadrupole, double the
     a.tc = t->coord; a.ts = t->soft; a.tsize = t->size; a.tdelta = t->delta;
     a.tpos = t->coord; a.th = t->soft; a.scatter = t->walk_idx; a.groups = wg; a.group_root = wr;
     a.group_order = g->gorder;
-    a.ngroups = ng; a.theta = theta; a.theta_group = nullptr; a.tol_group = nullptr; a.G = G;
+    a.ngroups = a.all_groups = ng; a.ntargets = n; a.theta = theta; a.theta_group = nullptr; a.tol_group = nullptr; a.G = G;
     a.out_fields = fields;
     a.out_w = ((fields & F_POT) ? 1 : 0) + ((fields & F_ACC) ? 3 : 0) + ((fields & F_TID) ? 9 : 0);
     a.out = out; a.gs = group_size;
@@ -2805,7 +2837,8 @@ tg_status tg_walk_graph_status(tg_walk_graph g, void *stream) {
     TG_CUDA(cudaMemcpyAsync(&status, g->scratch + tg::WS_STATUS, sizeof(int), cudaMemcpyDeviceToHost, st));
     TG_CUDA(cudaStreamSynchronize(st));
     if (status & (1 << TG_ERR_CUDA)) {
-        tg::set_last_error_msg("internal error: tree links do not form a valid octree for the walk arena");
+        tg::set_last_error_msg("internal error: tree links do not form a valid octree for the walk arena, or a walk "
+                               "record is out of range");
         return TG_ERR_CUDA;
     }
     if (status & (1 << TG_ERR_STACK_OVERFLOW)) return TG_ERR_STACK_OVERFLOW;
