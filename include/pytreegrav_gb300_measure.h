@@ -42,6 +42,11 @@ int tg_check_rsqrt64(const double *x, int64_t n, double *out, void *stream);
  * damage them: a walk skips a group whose record is out of range and returns an error. */
 int tg_group_arrays(void *tree, void *targets, void **groups, void **roots, int64_t *ngroups);
 
+/* The check behind a tree's grouping, on the caller's arrays (device memory): ngroups (first, count) pairs taken in
+ * the order perm must be a partition of n particles. *err (host) receives 0, or 2 if they are not. */
+int tg_check_group_order(const uint32_t *perm, const int32_t *groups, int64_t ngroups, int64_t n, int *err,
+                         void *stream);
+
 /* Bounds of the library's bounded device loops, for tests that make each one run out (0 or less:
  * the built-in bound): polls of one look-back word in a radix pass (built in: 2^22; running out
  * gives TG_ERR_QUEUE_TIMEOUT), traversal steps of one group of a tree walk (the node count, which

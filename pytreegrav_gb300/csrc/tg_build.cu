@@ -240,7 +240,7 @@ __global__ void k_gather(const uint32_t *perm, int64_t n, const double *pos, con
     const bool bad = *sort_err != 0;
     int64_t o = bad ? i : (int64_t)perm[i];
     if (o >= n) {  // no permutation: the sort is reported as failed, and nothing is read out of range
-        atomicExch(sort_err, 1);
+        atomicExch(sort_err, SORT_ERR_SORT);
         o = i;
     }
     const double x = pos[3 * o], y = pos[3 * o + 1], z = pos[3 * o + 2];
@@ -719,10 +719,14 @@ __global__ void k_rekey_segkeys(RoundView v, const uint32_t *vals, int64_t E, ui
 // sort_err set: the segments' keys become their element indices (sorted within every segment).
 __global__ void k_rekey_gather(RoundView v, int64_t E, const uint32_t *vals, const double *coord, const double *mass,
                                const double *soft, const int64_t *widx, const uint64_t *newkeys_by_elem, double *tc,
-                               double *tm, double *ts, int64_t *tw, uint64_t *tk, const int *sort_err) {
+                               double *tm, double *ts, int64_t *tw, uint64_t *tk, int *sort_err) {
     int64_t a = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (a >= E) return;
     int64_t esrc = vals[a];
+    if (esrc >= E) {  // no permutation, as in k_gather
+        atomicExch(sort_err, SORT_ERR_SORT);
+        esrc = a;
+    }
     int s;
     int64_t isrc;
     elem_loc(v, esrc, s, isrc);
@@ -871,7 +875,7 @@ __global__ void k_number_keys(Nodes nd, int64_t count, const int64_t *sys_off, N
 // 3900 particles.)
 __global__ void k_final_index(const uint64_t *sorted_keys, const uint32_t *vals, int64_t count, const int32_t *nd_sys,
                               int64_t ntot, int sys_shift, int64_t *sys_node_off, int64_t *final_of_slot,
-                              const int64_t *root_slot_of_sys, int nsys, const int *sort_err) {
+                              const int64_t *root_slot_of_sys, int nsys, int *sort_err) {
     chain_wait();
     chain_next();
     int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -881,7 +885,10 @@ __global__ void k_final_index(const uint64_t *sorted_keys, const uint32_t *vals,
     }
     if (q < count) {
         int64_t c = vals[q];
-        if (c >= count) c = q;  // no permutation: k_write finds the slots left out
+        if (c >= count) {  // no permutation: reported as a failed sort (and k_write checks every slot's index)
+            atomicExch(sort_err, SORT_ERR_SORT);
+            c = q;
+        }
         int s = nd_sys[c];
         if (q < count - nsys) final_of_slot[c] = ntot + q + s + 1;
     }

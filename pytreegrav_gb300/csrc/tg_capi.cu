@@ -47,10 +47,14 @@ __global__ void k_u32_to_i64(const uint32_t *a, int64_t n, int64_t *b) {
 }
 
 __global__ void k_gather_targets(const uint32_t *perm, int64_t n, const double *pos, const double *h, double *pos_s,
-                                 double *h_s, int64_t *scatter) {
+                                 double *h_s, int64_t *scatter, int *sort_err) {
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     int64_t o = perm[i];
+    if (o >= n) {  // no permutation: reported as a failed sort with the walk's results
+        atomicExch(sort_err, SORT_ERR_SORT);
+        o = i;
+    }
     pos_s[3 * i] = pos[3 * o];
     pos_s[3 * i + 1] = pos[3 * o + 1];
     pos_s[3 * i + 2] = pos[3 * o + 2];
@@ -395,7 +399,7 @@ tg_status tg_tree_fields(tg_tree t, const double *pos, const double *h, int64_t 
             TG_CUDA(tg::dev_malloc((void **)&sp, sizeof(double) * 3 * n, st));
             TG_CUDA(tg::dev_malloc((void **)&sh, sizeof(double) * n, st));
             TG_CUDA(tg::dev_malloc((void **)&scatter, sizeof(int64_t) * n, st));
-            { k_gather_targets<<<div_up(n, 256), 256, 0, st>>>(perm, n, dp.ptr, dh.ptr, sp, sh, scatter); tg::note_launch(); }
+            { k_gather_targets<<<div_up(n, 256), 256, 0, st>>>(perm, n, dp.ptr, dh.ptr, sp, sh, scatter, t->sort_err); tg::note_launch(); }
             TG_CUDA(cudaGetLastError());
             TG_CUDA(cudaFreeAsync(perm, st));
         } else {

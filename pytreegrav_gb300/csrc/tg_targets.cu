@@ -179,9 +179,11 @@ tg_status targets_refine_groups(tg_targets_s *ts, cudaStream_t st) {
              src->arena32, src->node_range, tt->coord, ts->n, tt->groups, ng, ts->group_size, node.p, nsub.p, sublen.p);
     TG_CUDA(cudaGetLastError());
     TG_TRY(exclusive_scan_i32(nsub.p, off.p, ng + 1, st));
-    int total = 0;
+    int total = 0, bad = 0;
     TG_CUDA(cudaMemcpyAsync(&total, off.p + ng, sizeof(int), cudaMemcpyDeviceToHost, st));
+    TG_CUDA(cudaMemcpyAsync(&bad, tt->sort_err, sizeof(int), cudaMemcpyDeviceToHost, st));  // of the grouping
     TG_CUDA(cudaStreamSynchronize(st));
+    if (bad) return sort_status(tt, bad);
     if (total == ng) return TG_OK;  // nothing to cut
     int2 *groups = nullptr;
     int *root = nullptr, *gnode = nullptr;

@@ -88,8 +88,8 @@ struct tg_tree_s {
     int2 *node_range = nullptr;   // per node: particle range [lo, hi) of its subtree
     double *cell_center = nullptr;  // per node: geometric centre of its cell (3)
 
-    // The look-back error word of every radix sort made for this tree (build, grouping, queue
-    // order), read back by the build and by each walk (nonzero: a sort failed).
+    // The error word (SORT_ERR_*) of every radix sort made for this tree (build, grouping, queue order) and
+    // of what is indexed with a sort's result, read back by the build and by each walk (nonzero: failed).
     int *sort_err = nullptr;
 
     // Velocities (tg_tree_set_velocities): per element, particles' own and nodes' mass-weighted mean
@@ -143,6 +143,10 @@ namespace tg {
 inline void tree_wait_built(const tg_tree_s *t, cudaStream_t s) {
     if (t && t->ev_built) cudaStreamWaitEvent(s, t->ev_built, 0);
 }
+// Bits of a tree's sort error word: a sort's look-back ran out (its result is the identity permutation); the
+// grouping is not a partition of the particles.
+constexpr int SORT_ERR_SORT = 1, SORT_ERR_GROUPS = 2;
+tg_status sort_status(tg_tree_s *t, int word);
 // The FP64 quadrupoles (t->quad) of a quadrupole tree, computed on s the first time they are needed.
 tg_status ensure_quad64(tg_tree_s *t, cudaStream_t s);
 }  // namespace tg

@@ -1805,15 +1805,27 @@ __global__ void k_group_start_keys(const int2 *groups, int64_t ngroups, uint64_t
     keys[g] = (uint32_t)groups[g].x;
     vals[g] = (uint32_t)g;
 }
-__global__ void k_permute_groups(const uint32_t *perm, int64_t ngroups, const int2 *gin, const int *rin, const int *nin,
-                                 int2 *gout, int *rout, int *nout) {
+// The groups in start order, which must be a partition of the n particles: each starts where the one before ends. A
+// permutation that is none, or a grouping that leaves a particle out or takes one twice, sets SORT_ERR_GROUPS in
+// *sort_err (after a sort that failed, which has set its own flag, the groups are merely in another order).
+__global__ void k_permute_groups(const uint32_t *perm, int64_t ngroups, int64_t n, const int2 *gin, const int *rin,
+                                 const int *nin, int2 *gout, int *rout, int *nout, int *sort_err) {
     chain_wait();
     chain_next();
     int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= ngroups) return;
-    int64_t o = perm[g];
-    if (o >= ngroups) o = g;  // a sort that failed: nothing is read out of range
-    gout[g] = gin[o];
+    int64_t o = perm[g], before = g > 0 ? (int64_t)perm[g - 1] : 0;
+    bool ok = o < ngroups && before < ngroups;
+    if (!ok) o = before = g;  // nothing is read out of range
+    const int2 gr = gin[o];
+    int64_t start = 0;
+    if (g > 0) {
+        const int2 b = gin[before];
+        start = (int64_t)b.x + b.y;
+    }
+    ok = ok && gr.y >= 1 && gr.x == start && (g < ngroups - 1 || (int64_t)gr.x + gr.y == n);
+    if (!ok && !(*(volatile int *)sort_err & SORT_ERR_SORT)) atomicOr(sort_err, SORT_ERR_GROUPS);
+    gout[g] = gr;
     rout[g] = rin[o];
     if (nin) nout[g] = nin[o];
 }
@@ -2407,6 +2419,17 @@ static int arena_exceeds_l2(const Arena<T> &ar) {
     return bytes > (int64_t)l2;
 }
 
+// The status of a tree whose sort error word was found set.
+tg_status sort_status(tg_tree_s *t, int word) {
+    if (word & SORT_ERR_GROUPS) {
+        t->groups_G = 0;  // made again by the next call
+        set_last_error_msg("internal error: the tree grouping is not a partition of the particles");
+        return TG_ERR_CUDA;
+    }
+    set_last_error_msg("radix sort: a tile's look-back did not complete within its bound");
+    return TG_ERR_QUEUE_TIMEOUT;
+}
+
 // Walk targets already in walk order (tpos/th on the device). groups/group_root describe the
 // grouping; scatter maps walk order to output rows.
 tg_status run_walk(tg_tree_s *t, const double *tpos, const double *th, int64_t ntargets, const int2 *groups,
@@ -2511,10 +2534,9 @@ tg_status run_walk(tg_tree_s *t, const double *tpos, const double *th, int64_t n
     t->last_stats.steps = (int64_t)stats[3];
     t->last_stats.quad_interactions = (int64_t)stats[4];
     t->last_stats.kernel_ms = kms;
-    if (sort_bad) {  // the grouping's or the queue order's sort (reported once; the groups are valid)
+    if (sort_bad) {  // the grouping's or the queue order's (reported once)
         cudaMemsetAsync(t->sort_err, 0, sizeof(int), st);
-        set_last_error_msg("radix sort: a tile's look-back did not complete within its bound");
-        return TG_ERR_QUEUE_TIMEOUT;
+        return sort_status(t, sort_bad);
     }
     if (status & (1 << TG_ERR_CUDA)) {
         set_last_error_msg("internal error: tree links do not form a valid octree for the walk arena, or a walk record "
@@ -2576,8 +2598,8 @@ tg_status tree_groups(tg_tree_s *t, int G, cudaStream_t st) {
     TG_CUDA(tg::dev_malloc((void **)&t->group_node, sizeof(int) * ng1, st));
     TG_CHAIN(k_group_start_keys, div_up(ng, 256), 256, 0, st, g0, ng, keys, vals);
     TG_TRY(radix_sort_pairs(keys, vals, ng, 32, st, t->sort_err));
-    TG_CHAIN(k_permute_groups, div_up(ng, 256), 256, 0, st, vals, ng, g0, r0, n0, t->groups, t->group_root,
-             t->group_node);
+    TG_CHAIN(k_permute_groups, div_up(ng, 256), 256, 0, st, vals, ng, N, g0, r0, n0, t->groups, t->group_root,
+             t->group_node, t->sort_err);
     TG_CUDA(cudaGetLastError());
     TG_CUDA(cudaFreeAsync(keys, st));
     TG_CUDA(cudaFreeAsync(vals, st));
@@ -2777,9 +2799,10 @@ tg_status tg_walk_graph_create(tg_tree t, int fields, int quadrupole, double the
     if (t->sort_err && cudaMemcpyAsync(&sort_bad, t->sort_err, sizeof(int), cudaMemcpyDeviceToHost, cs) != cudaSuccess)
         return fail(TG_ERR_CUDA);
     if (cudaStreamSynchronize(cs) != cudaSuccess) return fail(TG_ERR_CUDA);
-    if (sort_bad) {  // the grouping's or the queue order's sort
-        set_last_error_msg("radix sort: a tile's look-back did not complete within its bound");
-        return fail(TG_ERR_QUEUE_TIMEOUT);
+    if (sort_bad) {  // the grouping's or the queue order's (reported once)
+        cudaMemsetAsync(t->sort_err, 0, sizeof(int), cs);
+        cudaStreamSynchronize(cs);
+        return fail(sort_status(t, sort_bad));
     }
 
     WalkArgs<float> a;
@@ -2848,6 +2871,24 @@ tg_status tg_walk_graph_status(tg_walk_graph g, void *stream) {
 
 tg_status tg_walk_graph_free(tg_walk_graph g) {
     graph_release(g);
+    return TG_OK;
+}
+
+int tg_check_group_order(const uint32_t *perm, const int32_t *groups, int64_t ngroups, int64_t n, int *err, void *stream) {
+    using namespace tg;
+    if (!perm || !groups || !err || ngroups < 1) return TG_ERR_BAD_ARG;
+    cudaStream_t st = (cudaStream_t)stream;
+    DevArray<int2> out(st);
+    DevArray<int> root(st), flag(st);
+    TG_CUDA(out.alloc(ngroups));
+    TG_CUDA(root.alloc(2 * ngroups));
+    TG_CUDA(flag.alloc(1));
+    TG_CUDA(cudaMemsetAsync(root.p, 0, sizeof(int) * 2 * ngroups, st));
+    TG_CUDA(cudaMemsetAsync(flag.p, 0, sizeof(int), st));
+    TG_CHAIN(k_permute_groups, div_up(ngroups, 256), 256, 0, st, perm, ngroups, n, (const int2 *)groups, root.p, nullptr,
+             out.p, root.p + ngroups, nullptr, flag.p);
+    TG_CUDA(cudaMemcpyAsync(err, flag.p, sizeof(int), cudaMemcpyDeviceToHost, st));
+    TG_CUDA(cudaStreamSynchronize(st));
     return TG_OK;
 }
 
