@@ -189,7 +189,7 @@ const char *tg_last_error(void) { return tg::last_error(); }
 
 static tg_status build_common(const double *pos, const double *m, const double *h, std::vector<int64_t> off,
                               int quadrupole, int compute_moments, int mem, void *stream, tg_tree *out) {
-    if (!out || !pos) return TG_ERR_BAD_ARG;
+    if (!out || !pos || !valid_mem(mem)) return TG_ERR_BAD_ARG;
     *out = nullptr;
     cudaStream_t st = (cudaStream_t)stream;
     const int64_t n = off.back();
@@ -346,7 +346,7 @@ tg_status tg_tree_free(tg_tree t) {
 tg_status tg_tree_fields(tg_tree t, const double *pos, const double *h, int64_t n, int fields, int quadrupole,
                          double theta, double G, int group_size, int grouping, int order, int precision,
                          const float *theta_per_group, int mem, double *out, void *stream) {
-    if (!t || !out) return TG_ERR_BAD_ARG;
+    if (!t || !out || !valid_fields_mem(mem)) return TG_ERR_BAD_ARG;
     if (grouping != TG_GROUP_BLOCKS && grouping != TG_GROUP_TREE) return TG_ERR_BAD_ARG;
     if (grouping == TG_GROUP_TREE && order != TG_ORDER_TREE) return TG_ERR_BAD_ARG;
     if ((fields & 7) == 0 || (fields & ~7)) return TG_ERR_BAD_ARG;
@@ -452,7 +452,7 @@ double tg_tree_last_walk_kernel_ms(tg_tree t) {
 }
 
 tg_status tg_morton_order(const double *pos, int64_t n, int mem, int64_t *perm, void *stream) {
-    if (!perm || (!pos && n > 0) || n < 0) return TG_ERR_BAD_ARG;
+    if (!perm || (!pos && n > 0) || n < 0 || !valid_mem(mem)) return TG_ERR_BAD_ARG;
     if (n == 0) return TG_OK;
     cudaStream_t st = (cudaStream_t)stream;
     DevBuf dp;
@@ -480,7 +480,7 @@ tg_status tg_bruteforce(const double *pos_t, const double *h_t, int64_t nt, cons
                         const double *h_s, int64_t ns, int fields, int mutual, double G, int precision, int mem,
                         double *out, void *stream) {
     if ((fields & 7) == 0 || (fields & ~7) || !out || !pos_s || !m_s || ns < 0) return TG_ERR_BAD_ARG;
-    if (precision != TG_FP32 && precision != TG_FP64) return TG_ERR_BAD_ARG;
+    if ((precision != TG_FP32 && precision != TG_FP64) || !valid_fields_mem(mem)) return TG_ERR_BAD_ARG;
     if (mutual) {
         pos_t = pos_s;
         h_t = h_s;

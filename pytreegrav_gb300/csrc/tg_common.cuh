@@ -363,6 +363,9 @@ struct SortedPairs {
 
 // A walk's or direct sum's rows (n, W) of the requested fields to the caller's host memory, as mem says.
 inline bool results_to_host(int mem) { return mem == TG_MEM_HOST || mem == TG_MEM_HOST_FIELDS; }
+// What an entry point takes for `mem`: arrays, or (results in arrays of their own) the fields' addresses too.
+inline bool valid_mem(int mem) { return mem == TG_MEM_HOST || mem == TG_MEM_DEVICE; }
+inline bool valid_fields_mem(int mem) { return valid_mem(mem) || mem == TG_MEM_HOST_FIELDS; }
 tg_status copy_results(const double *rows, int64_t n, int fields, int mem, double *out, cudaStream_t st);
 
 // Counts kernel launches (every launch site calls it; read through tg_launch_count()).

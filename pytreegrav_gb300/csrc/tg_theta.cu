@@ -736,7 +736,7 @@ tg_status tg_tree_groups(tg_tree t, int group_size, int64_t *ngroups, void *stre
 
 tg_status tg_tree_groups_copy(tg_tree t, int group_size, int32_t *first, int32_t *count, int32_t *node, int mem,
                               void *stream) {
-    if (!t || !valid_gs(group_size)) return TG_ERR_BAD_ARG;
+    if (!t || !valid_gs(group_size) || !valid_mem(mem)) return TG_ERR_BAD_ARG;
     cudaStream_t st = (cudaStream_t)stream;
     tree_wait_built(t, st);
     TG_TRY(tree_groups(t, group_size, st));
@@ -773,7 +773,7 @@ tg_status tg_theta_model_set_error_budget(tg_theta_model m, float budget) {
 }
 
 tg_status tg_tree_last_group_error(tg_tree t, float *out, int mem, void *stream) {
-    if (!t || !out || !t->gerr) return TG_ERR_BAD_ARG;
+    if (!t || !out || !valid_mem(mem) || !t->gerr) return TG_ERR_BAD_ARG;
     cudaStream_t st = (cudaStream_t)stream;
     TG_CUDA(cudaMemcpyAsync(out, t->gerr, sizeof(float) * t->last_stats.groups,
                             mem == TG_MEM_HOST ? cudaMemcpyDeviceToHost : cudaMemcpyDeviceToDevice, st));
@@ -782,7 +782,7 @@ tg_status tg_tree_last_group_error(tg_tree t, float *out, int mem, void *stream)
 }
 
 tg_status tg_tree_last_group_stats(tg_tree t, uint32_t *out, int mem, void *stream) {
-    if (!t || !out || !t->gstats) return TG_ERR_BAD_ARG;
+    if (!t || !out || !valid_mem(mem) || !t->gstats) return TG_ERR_BAD_ARG;
     cudaStream_t st = (cudaStream_t)stream;
     const int64_t ng = t->last_stats.groups;  // the groups of the last walk (tree grouping or a target set)
     TG_CUDA(cudaMemcpyAsync(out, t->gstats, sizeof(uint32_t) * 3 * ng,
@@ -847,7 +847,7 @@ tg_status tg_theta_loss(const float *y, const float *log_cost, const float *log_
 
 tg_status tg_theta_model_create(const float *params, const float *feat_mean, const float *feat_std, int kind,
                                 float out_min, float out_max, float theta_max, int mem, tg_theta_model *out) {
-    if (!params || !feat_mean || !feat_std || !out || !(out_max > out_min)) return TG_ERR_BAD_ARG;
+    if (!params || !feat_mean || !feat_std || !out || !(out_max > out_min) || !valid_mem(mem)) return TG_ERR_BAD_ARG;
     if (kind == TG_THETA_KIND_ANGLE ? !(out_min > 0) : (kind != TG_THETA_KIND_TOLERANCE || !(theta_max > 0)))
         return TG_ERR_BAD_ARG;
     std::vector<float> P, mu, sd;
@@ -946,7 +946,7 @@ tg_status tg_theta_tolerances(tg_tree t, int group_size, int quadrupole, const f
 tg_status tg_tree_fields_grouped(tg_tree t, int fields, int quadrupole, double G, int group_size, double theta,
                                  const float *theta_per_group, const float *tol_per_group, int mem, double *out,
                                  void *stream) {
-    if (!t || !out || (fields & 7) == 0 || (fields & ~7) || !valid_gs(group_size) || !(theta > 0))
+    if (!t || !out || (fields & 7) == 0 || (fields & ~7) || !valid_gs(group_size) || !(theta > 0) || !valid_mem(mem))
         return TG_ERR_BAD_ARG;
     if (quadrupole && !t->has_quads) return TG_ERR_NO_QUADRUPOLES;
     cudaStream_t st = (cudaStream_t)stream;
@@ -968,7 +968,8 @@ tg_status tg_tree_fields_grouped(tg_tree t, int fields, int quadrupole, double G
 
 tg_status tg_tree_fields_learned(tg_tree t, int fields, int quadrupole, double G, int group_size, tg_theta_model m,
                                  float log10_lambda, double theta_fallback, int mem, double *out, void *stream) {
-    if (!t || !out || (fields & 7) == 0 || (fields & ~7) || !valid_gs(group_size) || !(theta_fallback > 0))
+    if (!t || !out || (fields & 7) == 0 || (fields & ~7) || !valid_gs(group_size) || !(theta_fallback > 0) ||
+        !valid_fields_mem(mem))
         return TG_ERR_BAD_ARG;
     if (quadrupole && !t->has_quads) return TG_ERR_NO_QUADRUPOLES;
     cudaStream_t st = (cudaStream_t)stream;
@@ -983,7 +984,8 @@ tg_status tg_tree_fields_learned(tg_tree t, int fields, int quadrupole, double G
 
 tg_status tg_targets_fields_learned(tg_targets ts, int fields, int quadrupole, double G, tg_theta_model m,
                                     float log10_lambda, double theta_fallback, int mem, double *out, void *stream) {
-    if (!ts || !out || (fields & 7) == 0 || (fields & ~7) || !(theta_fallback > 0)) return TG_ERR_BAD_ARG;
+    if (!ts || !out || (fields & 7) == 0 || (fields & ~7) || !(theta_fallback > 0) || !valid_fields_mem(mem))
+        return TG_ERR_BAD_ARG;
     tg_tree_s *t = ts->src, *tt = ts->tt;
     if (quadrupole && !t->has_quads) return TG_ERR_NO_QUADRUPOLES;
     cudaStream_t st = (cudaStream_t)stream;
