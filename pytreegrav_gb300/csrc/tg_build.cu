@@ -1510,33 +1510,24 @@ __global__ void k_fold_only(MomentArgs a) {
 }
 
 // ---------------------------------------------------------------------------------------------
-// A non-blocking stream per host thread (and device) for build work that can run beside the
-// build's own stream, with its fork and join events; created once.
+// A non-blocking stream for build work that can run beside the build's own stream, with its fork and join events:
+// the build's from open() to its end, then back in the device's pools (work still queued on the stream runs on).
 struct BuildSide {
-    int dev = -1;
-    unsigned long long ctx = 0;  // id of the CUDA context the stream and events belong to
     cudaStream_t s = nullptr;
     cudaEvent_t fork = nullptr, join = nullptr;
-};
-static tg_status build_side(BuildSide *&out) {
-    static thread_local BuildSide side;
-    int dev = 0;
-    TG_CUDA(cudaGetDevice(&dev));
-    // another device (this thread's old one is kept alive), or a new context after a device reset
-    // (the old handles died with it)
-    const unsigned long long ctx = tg::current_cuda_context_id();
-    if (side.s && (side.dev != dev || (ctx && side.ctx && side.ctx != ctx))) side = BuildSide();
-    if (!side.s) {
-        TG_CUDA(cudaStreamCreateWithFlags(&side.s, cudaStreamNonBlocking));
-        TG_CUDA(cudaEventCreateWithFlags(&side.fork, cudaEventDisableTiming));
-        TG_CUDA(cudaEventCreateWithFlags(&side.join, cudaEventDisableTiming));
-        side.dev = dev;
-        side.ctx = tg::current_cuda_context_id();
+    bool forked = false;  // work is queued that the build's stream has to wait for
+    tg_status open() {
+        if (!s) TG_CUDA(pool_stream(&s));
+        if (!fork) TG_CUDA(pool_event(&fork, false));
+        if (!join) TG_CUDA(pool_event(&join, false));
+        return TG_OK;
     }
-    if (!side.ctx) side.ctx = ctx;
-    out = &side;
-    return TG_OK;
-}
+    ~BuildSide() {
+        release_stream(s);
+        release_event(fork, false);
+        release_event(join, false);
+    }
+};
 
 template <typename T>
 static tg_status dalloc(T **p, int64_t n, cudaStream_t s) {
@@ -1713,8 +1704,9 @@ tg_status build_tree(tg_tree_s *T, const double *pos, const StageMH &stage_mh,
     T->has_quads = quadrupole;
     T->compute_moments = compute_moments;
     T->stream = st;
-    void *host = nullptr;  // read-backs
-    TG_TRY(host_words(&host));
+    HostWords words;  // read-backs
+    TG_TRY(words.take());
+    void *const host = words.p;
 
     // zeroed together: the summary, the depth lists' cursors, the input check's flag, the level scan's status words and counter, the
     // cubes' maxima and (kept with the tree) the sorts' error word
@@ -1814,17 +1806,15 @@ tg_status build_tree(tg_tree_s *T, const double *pos, const StageMH &stage_mh,
         return TG_OK;
     };
     bool summary_final = false;
-    BuildSide *side = nullptr;  // k_node_centers of the last round runs there when set
-    bool centers_forked = false;
+    BuildSide side;  // k_node_centers of the last round runs there
     // work that reads the temporaries on the side stream is waited for before they are freed, also on errors
     struct Join {
-        BuildSide *&side;
-        const bool &forked;
+        const BuildSide &side;
         cudaStream_t st;
         ~Join() {
-            if (forked) cudaStreamWaitEvent(st, side->join, 0);
+            if (side.forked) cudaStreamWaitEvent(st, side.join, 0);
         }
-    } join{side, centers_forked, st};
+    } join{side, st};
     // Non-finite input is reported once the build has run to its end: every kernel stays in bounds on
     // such input (keys of NaN quantize to 0, every link is checked).
     bool nonfinite_seen = false;
@@ -1918,15 +1908,19 @@ tg_status build_tree(tg_tree_s *T, const double *pos, const StageMH &stage_mh,
             // node numbering, which does not read them; k_write joins them
             cudaStream_t cs = st;
             if (hs.n_exh == 0) {
-                TG_TRY(build_side(side));
-                TG_CUDA(cudaEventRecord(side->fork, st));
-                TG_CUDA(cudaStreamWaitEvent(side->s, side->fork, 0));
-                cs = side->s;
+                TG_TRY(side.open());
+                TG_CUDA(cudaEventRecord(side.fork, st));
+                TG_CUDA(cudaStreamWaitEvent(side.s, side.fork, 0));
+                cs = side.s;
             }
             { k_node_centers<<<div_up(Mr, CENTER_BLOCK), CENTER_BLOCK, 0, cs>>>(v, nd, slot_base, Mr, keys); tg::note_launch(); }
             if (cs != st) {
-                TG_CUDA(cudaEventRecord(side->join, cs));
-                centers_forked = true;
+                const cudaError_t ej = cudaEventRecord(side.join, cs);
+                if (ej != cudaSuccess) {  // no event to wait for: the temporaries must outlive the kernel all the same
+                    cudaStreamSynchronize(cs);
+                    TG_CUDA(ej);
+                }
+                side.forked = true;
             }
         }
         n_exh = (int)hs.n_exh;
@@ -2055,7 +2049,7 @@ tg_status build_tree(tg_tree_s *T, const double *pos, const StageMH &stage_mh,
         lo.at[d] = T->lvl_off[d];
         T->lvl_off[d + 1] = T->lvl_off[d] + hs.depth_hist[d];
     }
-    if (centers_forked) TG_CUDA(cudaStreamWaitEvent(st, side->join, 0));
+    if (side.forked) TG_CUDA(cudaStreamWaitEvent(st, side.join, 0));
     FinalArrays fa{T->coord, T->mass, T->soft, T->size, T->delta, T->first, T->next, T->parent, T->node_range,
                    T->cell_center};
     const int node_blocks = div_up(M, 256);
@@ -2248,8 +2242,9 @@ tg_status morton_order_device(const double *pos, int64_t n, uint32_t *perm, cuda
     if (sorted.vals != perm)
         TG_CUDA(cudaMemcpyAsync(perm, sorted.vals, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, st));
     if (err_dev) return TG_OK;
-    void *host = nullptr;
-    TG_TRY(host_words(&host));
+    HostWords words;
+    TG_TRY(words.take());
+    void *const host = words.p;
     TG_CUDA(cudaMemcpyAsync(host, err, sizeof(int), cudaMemcpyDeviceToHost, st));
     TG_CUDA(cudaStreamSynchronize(st));
     if (*(const int *)host) {

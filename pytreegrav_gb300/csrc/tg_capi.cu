@@ -114,12 +114,12 @@ tg_status check_finite(const double *const *arrs, const int64_t *counts, int k, 
     TG_CUDA(cudaMemsetAsync(flag, 0, sizeof(int), st));
     for (int q = 0; q < k; q++)
         if (arrs[q] && counts[q] > 0) { k_nonfinite<<<div_up(counts[q], 256), 256, 0, st>>>(arrs[q], counts[q], flag); tg::note_launch(); }
-    void *host = nullptr;
-    TG_TRY(host_words(&host));
-    TG_CUDA(cudaMemcpyAsync(host, flag, sizeof(int), cudaMemcpyDeviceToHost, st));
+    HostWords words;
+    TG_TRY(words.take());
+    TG_CUDA(cudaMemcpyAsync(words.p, flag, sizeof(int), cudaMemcpyDeviceToHost, st));
     TG_CUDA(cudaFreeAsync(flag, st));
     TG_CUDA(cudaStreamSynchronize(st));
-    return *(const int *)host ? TG_ERR_NONFINITE : TG_OK;
+    return *(const int *)words.p ? TG_ERR_NONFINITE : TG_OK;
 }
 
 void destroy(tg_tree_s *t) {

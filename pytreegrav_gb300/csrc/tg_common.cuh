@@ -294,11 +294,21 @@ LoopLimits &loop_limits();
 
 int num_sms();
 
-// A few words of page-locked host memory per thread (HOST_WORDS_BYTES), for reading results back without the
-// driver's staging: copies into it are asynchronous, so several share one synchronisation. A call has the
-// words from its copies to its last read; nothing is kept in them between calls.
+// A few words of page-locked host memory (HOST_WORDS_BYTES), for reading results back without the driver's
+// staging: copies into it are asynchronous, so several share one synchronisation. A call has words of its own from
+// take() to its end, when they go back to the device's pool (as streams and events do: a pool holds as many as
+// were ever in use at a time). (They were kept per thread, and a thread that went back and forth between two devices
+// left a block behind at every change.)
 constexpr size_t HOST_WORDS_BYTES = 4096;
-tg_status host_words(void **p);
+struct HostWords {
+    void *p = nullptr;
+    int dev = -1;
+    HostWords() = default;
+    ~HostWords();
+    HostWords(const HostWords &) = delete;
+    HostWords &operator=(const HostWords &) = delete;
+    tg_status take();
+};
 // Polls of one look-back word in a one-pass scan.
 long long scan_spins();
 

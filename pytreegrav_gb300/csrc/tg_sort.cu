@@ -64,12 +64,13 @@ unsigned long long current_cuda_context_id() {
 namespace {
 constexpr int POOL_DEVICES = 64;
 std::mutex g_res_mu;
-// Per device: the context the pooled streams and events belong to, and the pools. After a device
-// reset (a new context) the old handles are dropped, not reused.
+// Per device: the context the pooled streams, events and page-locked words belong to, and the pools. After a
+// device reset (a new context) the old handles are dropped, not reused.
 struct ResPool {
     unsigned long long ctx = 0;  // context id
     std::vector<cudaStream_t> streams;
     std::vector<cudaEvent_t> events[2];  // [timing]
+    std::vector<void *> words;           // HOST_WORDS_BYTES each
 };
 ResPool g_res[POOL_DEVICES];
 int current_device() {
@@ -86,6 +87,7 @@ ResPool &res_pool(int dev) {
         r.streams.clear();
         r.events[0].clear();
         r.events[1].clear();
+        r.words.clear();
         r.ctx = ctx;
     }
     return r;
@@ -149,26 +151,30 @@ void release_event(cudaEvent_t e, bool timing, int dev) {
     res_pool(dev).events[timing ? 1 : 0].push_back(e);
 }
 
-namespace {
-struct HostWords {
-    void *p = nullptr;
-    unsigned long long ctx = 0;
-    ~HostWords() {  // the thread ends: given back, unless its context has gone (and the memory with it)
-        if (p && current_cuda_context_id() == ctx) cudaFreeHost(p);
+tg_status HostWords::take() {
+    if (p) return TG_OK;
+    dev = current_device();
+    if (dev >= 0) {
+        std::lock_guard<std::mutex> lock(g_res_mu);
+        auto &v = res_pool(dev).words;
+        if (!v.empty()) {
+            p = v.back();
+            v.pop_back();
+            return TG_OK;
+        }
     }
-};
-}  // namespace
-
-tg_status host_words(void **p) {
-    static thread_local HostWords w;
-    const unsigned long long ctx = current_cuda_context_id();
-    if (w.p && w.ctx != ctx) w.p = nullptr;  // a new context: the old memory died with the old one
-    if (!w.p) {
-        TG_CUDA(cudaHostAlloc(&w.p, HOST_WORDS_BYTES, cudaHostAllocPortable));
-        w.ctx = current_cuda_context_id();
-    }
-    *p = w.p;
+    TG_CUDA(cudaHostAlloc(&p, HOST_WORDS_BYTES, cudaHostAllocDefault));
     return TG_OK;
+}
+
+HostWords::~HostWords() {
+    if (!p) return;
+    if (dev < 0 || dev != current_device()) {  // pooled only on the current device (as streams)
+        cudaFreeHost(p);
+        return;
+    }
+    std::lock_guard<std::mutex> lock(g_res_mu);
+    res_pool(dev).words.push_back(p);
 }
 
 cudaError_t dev_malloc(void **p, size_t bytes, cudaStream_t s) {

@@ -2378,10 +2378,10 @@ static tg_status walk_with_fallback(tg_tree_s *t, WalkArgs<T> &a, Arena<T> &ar, 
     } evs{&e0, &e1};
     TG_CUDA(pool_event(&e0, true));
     TG_CUDA(pool_event(&e1, true));
-    void *words = nullptr;
-    TG_TRY(host_words(&words));
+    HostWords words;
+    TG_TRY(words.take());
     static_assert(sizeof(WalkReadback) <= HOST_WORDS_BYTES, "a walk's read-back must fit the host words");
-    WalkReadback *host = static_cast<WalkReadback *>(words);
+    WalkReadback *host = static_cast<WalkReadback *>(words.p);
     auto read_back = [&]() -> tg_status {
         TG_CUDA(cudaEventRecord(e1, st));
         host->sort_bad = 0;

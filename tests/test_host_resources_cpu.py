@@ -1,0 +1,105 @@
+"""What the library holds on the host between calls, and what it does when a launch fails, against a stand-in for
+the CUDA runtime (fake_cudart.c: several devices, counted resources, launches that can be made to fail; kernels do
+nothing). No GPU. Every test runs in a process of its own, in which the stand-in is loaded under the runtime's name."""
+
+import os
+import shutil
+import subprocess
+import sys
+import textwrap
+
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+ROOT = os.path.dirname(HERE)
+SONAME = "libcudart.so.13"
+
+PRELUDE = textwrap.dedent("""
+    import ctypes, sys
+    import numpy as np
+    sys.path.insert(0, %r)
+    F = ctypes.CDLL(%%r, mode=ctypes.RTLD_GLOBAL)
+    F.fake_log.restype = ctypes.c_char_p
+    F.fake_host_blocks.restype = F.fake_streams.restype = F.fake_events.restype = ctypes.c_long
+    F.fake_device_blocks.restype = ctypes.c_long
+    F.fake_patch.argtypes = [ctypes.c_size_t, ctypes.c_void_p, ctypes.c_size_t]
+    from pytreegrav_gb300 import _lib
+    L = _lib.load()
+    n = 64
+    x = np.random.default_rng(0).random((n, 3)); m = np.ones(n); h = np.full(n, 0.01)
+
+    def build():
+        t = ctypes.c_void_p()
+        rc = L.tg_tree_build(_lib.ptr(x), _lib.ptr(m), _lib.ptr(h), n, 1, 1, _lib.TG_MEM_HOST, None, ctypes.byref(t))
+        return rc, t
+""") % ROOT
+
+
+@pytest.fixture(scope="module")
+def fake(tmp_path_factory):
+    cc = shutil.which("gcc") or shutil.which("cc")
+    if not cc:
+        pytest.skip("no C compiler")
+    from pytreegrav_gb300 import build
+
+    build.build()
+    d = tmp_path_factory.mktemp("fake")
+    ver = d / "v.map"
+    ver.write_text(SONAME + " { global: *; };\n")
+    lib = d / SONAME
+    subprocess.check_call([cc, "-O1", "-shared", "-fPIC", "-Wall", "-Werror", "-o", str(lib),
+                           os.path.join(HERE, "fake_cudart.c"), "-Wl,-soname," + SONAME,
+                           "-Wl,--version-script," + str(ver)])
+
+    def run(code):
+        env = dict(os.environ, LD_LIBRARY_PATH=str(d), PYTHONPATH=ROOT)
+        r = subprocess.run([sys.executable, "-c", PRELUDE % str(lib) + textwrap.dedent(code)], capture_output=True,
+                           text=True, timeout=300, env=env)
+        assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-4000:]
+
+    return run
+
+
+def test_page_locked_words_do_not_grow_with_device_changes(fake):
+    """A thread that goes back and forth between two devices: one block per device."""
+    fake("""
+        perm = np.empty(n, np.int64)
+        for i in range(50):
+            F.fake_set_device(i % 2)
+            assert L.tg_morton_order(_lib.ptr(x), n, _lib.TG_MEM_HOST, _lib.ptr(perm), None) == 0
+        assert F.fake_host_blocks() <= 2, F.fake_host_blocks()
+        F.fake_new_context(0)  # a device reset: its block died with the old context, another is made
+        F.fake_set_device(0)
+        for i in range(10):
+            assert L.tg_morton_order(_lib.ptr(x), n, _lib.TG_MEM_HOST, _lib.ptr(perm), None) == 0
+        assert F.fake_host_blocks() <= 3, F.fake_host_blocks()
+    """)
+
+
+def test_build_streams_do_not_grow_with_device_changes(fake):
+    """Builds with node centres on a side stream (the stand-in reports five nodes): each device's streams and events
+    are reused, from one thread and from several that end."""
+    fake("""
+        import threading
+        five = (ctypes.c_uint64 * 1)(5)
+        F.fake_patch(224, five, 8)  # the round's summary: five nodes made
+
+        def once():
+            rc, t = build()
+            assert rc == 0, (rc, L.tg_last_error())
+            L.tg_tree_free(t)
+
+        for d in (0, 1):
+            F.fake_set_device(d)
+            once()
+        assert b"k_node_centers" in F.fake_log()
+        s, e, b = F.fake_streams(), F.fake_events(), F.fake_host_blocks()
+        for i in range(50):
+            F.fake_set_device(i % 2)
+            once()
+        for i in range(10):
+            t = threading.Thread(target=once)
+            t.start()
+            t.join()
+        assert (F.fake_streams(), F.fake_events(), F.fake_host_blocks()) == (s, e, b)
+    """)
