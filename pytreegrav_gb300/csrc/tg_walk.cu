@@ -2647,8 +2647,16 @@ tg_status tree_groups_with_arena(tg_tree_s *t, int G, bool fp64, cudaStream_t st
                 t->own32 = nullptr;
                 r = TG_ERR_CUDA;
             } else {
-                TG_CHAIN(k_prep_targets<float>, div_up(t->ntot, 256), 256, 0, t->side, t->coord, t->soft, t->ntot,
-                         t->own32, t->own32 + t->ntot);
+                auto prep = [&]() -> tg_status {
+                    TG_CHAIN(k_prep_targets<float>, div_up(t->ntot, 256), 256, 0, t->side, t->coord, t->soft, t->ntot,
+                             t->own32, t->own32 + t->ntot);
+                    return TG_OK;
+                };
+                r = prep();
+                if (r != TG_OK) {  // not filled: a later walk prepares its own
+                    cudaFreeAsync(t->own32, t->side);
+                    t->own32 = nullptr;
+                }
             }
         }
         const cudaError_t ej = cudaEventRecord(t->ev_join, t->side);

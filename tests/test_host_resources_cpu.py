@@ -103,3 +103,32 @@ def test_build_streams_do_not_grow_with_device_changes(fake):
             t.join()
         assert (F.fake_streams(), F.fake_events(), F.fake_host_blocks()) == (s, e, b)
     """)
+
+
+def test_side_stream_is_joined_when_a_launch_on_it_fails(fake):
+    """A first tree-grouped walk whose targets' preparation fails to launch on the tree's side stream: the caller's
+    stream waits for the side stream all the same, and a later walk prepares the targets instead of reading the
+    buffer that was never filled."""
+    fake("""
+        rc, t = build()
+        assert rc == 0
+        acc = np.empty((n, 3))
+
+        def walk():
+            F.fake_clear_log()
+            rc = L.tg_tree_fields(t, None, None, n, _lib.TG_FIELD_ACCEL, 1, 0.7, 1.0, 32, _lib.TG_GROUP_TREE,
+                                  _lib.TG_ORDER_TREE, _lib.TG_FP32, None, _lib.TG_MEM_HOST, _lib.ptr(acc), None)
+            return rc, [l.split() for l in F.fake_log().decode().splitlines()]
+
+        F.fake_fail_launch(b"k_prep_targets")
+        rc, log = walk()
+        assert rc == _lib.TG_ERR_CUDA, rc
+        at = [k for k, l in enumerate(log) if l[0] == "failed-launch"]
+        assert len(at) == 1
+        side = log[at[0]][2]
+        joins = [l[1] for l in log[at[0]:] if l[0] == "record" and l[2] == side]
+        assert joins and any(l[0] == "wait" and l[1] in joins and l[2] != side for l in log[at[0]:]), log
+        rc, log = walk()
+        assert rc == 0, (rc, L.tg_last_error())
+        assert any("k_prep_targets" in l[0] for l in log)
+    """)
