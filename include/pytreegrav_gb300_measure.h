@@ -47,6 +47,10 @@ int tg_group_arrays(void *tree, void *targets, void **groups, void **roots, int6
 int tg_check_group_order(const uint32_t *perm, const int32_t *groups, int64_t ngroups, int64_t n, int *err,
                          void *stream);
 
+/* Device memory of the library's pool on the current device: the bytes it has mapped, and the most that were in use
+ * at a time since the last call with reset nonzero (or since the pool was made). */
+int tg_memory_use(int64_t *reserved, int64_t *used_high, int reset);
+
 /* Bounds of the library's bounded device loops, for tests that make each one run out (0 or less:
  * the built-in bound): polls of one look-back word in a radix pass (built in: 2^22; running out
  * gives TG_ERR_QUEUE_TIMEOUT), traversal steps of one group of a tree walk (the node count, which

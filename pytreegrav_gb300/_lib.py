@@ -109,6 +109,7 @@ MEASURE_EXPORTS = [
     "tg_check_rsqrt64",
     "tg_group_arrays",
     "tg_check_group_order",
+    "tg_memory_use",
     "tg_set_loop_limits",
 ]
 TG_THETA_NFEAT = 16

@@ -2091,6 +2091,12 @@ tg_status build_tree(tg_tree_s *T, const double *pos, const StageMH &stage_mh,
         int64_t node_hi = np + (T->sys_node_off[s + 1] - T->sys_node_off[s]);
         T->sys_capacity[s] = reference_capacity(np, std::max<int64_t>(node_hi, (int64_t)rq[s]));
     }
+    // everything but the tree's arrays and the depth lists has been read (the side stream was joined ahead of k_write);
+    // the moment pass's lists and sums take its place. Peak: 409 bytes per particle at 2e6 (452 when the temporaries
+    // stayed to the end)
+    for (DevArray<unsigned char> *mem : {&temps, &slots, &elem_mem, &round_mem, &numbering, &by_key.mem, &by_sys.mem,
+                                         &numbered.mem})
+        mem->reset();
     // 9. moments: nodes deeper than DEPTH_CAP by climbing, then one launch per depth, deepest first
     // (the moment kernels bound every link they follow). With quadrupoles the pass sums them in FP32
     // for the FP32 walk; the FP64 quadrupoles come from ensure_quad64 when first needed, which the

@@ -330,6 +330,8 @@ unsigned long long current_cuda_context_id();
 #define TG_POOL_KEEP_BYTES (4ull << 30)
 #endif
 cudaError_t dev_malloc(void **p, size_t bytes, cudaStream_t s);
+// The pool's mapped bytes and the most that were in use since the last reset (zeros without a pool).
+cudaError_t pool_bytes(int64_t *reserved, int64_t *used_high, bool reset);
 
 // Streams (non-blocking) and events (timing or not) of the current device from a library-owned pool:
 // a tree takes a side stream and up to four events and a walk two timing events on every call, and

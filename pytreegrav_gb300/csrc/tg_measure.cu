@@ -99,6 +99,12 @@ int tg_check_f32_conversion(const double *x, int64_t n, int64_t *mismatches, voi
 
 }  // extern "C"
 
+extern "C" int tg_memory_use(int64_t *reserved, int64_t *used_high, int reset) {
+    if (!reserved || !used_high) return TG_ERR_BAD_ARG;
+    TG_CUDA(tg::pool_bytes(reserved, used_high, reset != 0));
+    return TG_OK;
+}
+
 extern "C" int tg_set_loop_limits(int64_t sort_spin, int64_t walk_steps, int64_t column_visits,
                                   int64_t heavy_entries) {
     tg::LoopLimits &l = tg::loop_limits();

@@ -177,41 +177,59 @@ HostWords::~HostWords() {
     res_pool(dev).words.push_back(p);
 }
 
-cudaError_t dev_malloc(void **p, size_t bytes, cudaStream_t s) {
+// The library's memory pool of the current device, made on first use.
+static cudaError_t current_pool(cudaMemPool_t *pool) {
     constexpr int MAX_DEVICES = 64;
     static std::mutex mu;
     static cudaMemPool_t pools[MAX_DEVICES] = {};
     static unsigned long long pool_ctx[MAX_DEVICES] = {};  // context ids: a device reset makes a new context
+    *pool = nullptr;
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return e;
-    if (dev < 0 || dev >= MAX_DEVICES) return cudaMallocAsync(p, bytes, s);
-    cudaMemPool_t pool;
-    {
-        std::lock_guard<std::mutex> lock(mu);
-        const unsigned long long ctx = current_cuda_context_id();
-        if (pools[dev] && ctx && !pool_ctx[dev]) pool_ctx[dev] = ctx;          // made before a context was bound
-        if (pools[dev] && ctx && pool_ctx[dev] != ctx) pools[dev] = nullptr;  // the old pool died with its context
-        if (!pools[dev]) {
-            cudaMemPoolProps props = {};
-            props.allocType = cudaMemAllocationTypePinned;
-            props.location.type = cudaMemLocationTypeDevice;
-            props.location.id = dev;
-            e = cudaMemPoolCreate(&pools[dev], &props);
-            if (e != cudaSuccess) {
-                pools[dev] = nullptr;
-                return e;
-            }
-            pool_ctx[dev] = current_cuda_context_id();
-            size_t free_b = 0, total_b = 0;
-            unsigned long long keep = TG_POOL_KEEP_BYTES;
-            if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && total_b / 4 > keep) keep = total_b / 4;
-            e = cudaMemPoolSetAttribute(pools[dev], cudaMemPoolAttrReleaseThreshold, &keep);
-            if (e != cudaSuccess) return e;
+    if (e != cudaSuccess || dev < 0 || dev >= MAX_DEVICES) return e;
+    std::lock_guard<std::mutex> lock(mu);
+    const unsigned long long ctx = current_cuda_context_id();
+    if (pools[dev] && ctx && !pool_ctx[dev]) pool_ctx[dev] = ctx;          // made before a context was bound
+    if (pools[dev] && ctx && pool_ctx[dev] != ctx) pools[dev] = nullptr;  // the old pool died with its context
+    if (!pools[dev]) {
+        cudaMemPoolProps props = {};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = dev;
+        e = cudaMemPoolCreate(&pools[dev], &props);
+        if (e != cudaSuccess) {
+            pools[dev] = nullptr;
+            return e;
         }
-        pool = pools[dev];
+        pool_ctx[dev] = current_cuda_context_id();
+        size_t free_b = 0, total_b = 0;
+        unsigned long long keep = TG_POOL_KEEP_BYTES;
+        if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && total_b / 4 > keep) keep = total_b / 4;
+        e = cudaMemPoolSetAttribute(pools[dev], cudaMemPoolAttrReleaseThreshold, &keep);
+        if (e != cudaSuccess) return e;
     }
-    return cudaMallocFromPoolAsync(p, bytes, pool, s);
+    *pool = pools[dev];
+    return cudaSuccess;
+}
+
+cudaError_t dev_malloc(void **p, size_t bytes, cudaStream_t s) {
+    cudaMemPool_t pool;
+    const cudaError_t e = current_pool(&pool);
+    if (e != cudaSuccess) return e;
+    return pool ? cudaMallocFromPoolAsync(p, bytes, pool, s) : cudaMallocAsync(p, bytes, s);
+}
+
+cudaError_t pool_bytes(int64_t *reserved, int64_t *used_high, bool reset) {
+    *reserved = *used_high = 0;
+    cudaMemPool_t pool;
+    cudaError_t e = current_pool(&pool);
+    if (e != cudaSuccess || !pool) return e;
+    unsigned long long r = 0, h = 0, zero = 0;
+    if ((e = cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &r)) != cudaSuccess) return e;
+    if ((e = cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemHigh, &h)) != cudaSuccess) return e;
+    *reserved = (int64_t)r;
+    *used_high = (int64_t)h;
+    return reset ? cudaMemPoolSetAttribute(pool, cudaMemPoolAttrUsedMemHigh, &zero) : cudaSuccess;
 }
 
 // ---------------------------------------------------------------------------------------------
