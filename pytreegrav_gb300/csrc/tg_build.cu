@@ -1815,9 +1815,6 @@ tg_status build_tree(tg_tree_s *T, const double *pos, const StageMH &stage_mh,
             if (side.forked) cudaStreamWaitEvent(st, side.join, 0);
         }
     } join{side, st};
-    // Non-finite input is reported once the build has run to its end: every kernel stays in bounds on
-    // such input (keys of NaN quantize to 0, every link is checked).
-    bool nonfinite_seen = false;
 
     for (int round = 0; round <= MORTON_MAX_ROUNDS; round++) {
         // element offsets of the segments; round 0's segments are the systems
@@ -1888,8 +1885,10 @@ tg_status build_tree(tg_tree_s *T, const double *pos, const StageMH &stage_mh,
             }
             TG_CUDA(cudaGetLastError());
             TG_TRY(read_summary());
-            if (hs.nonfinite) nonfinite_seen = true;
-            return TG_OK;
+            // Non-finite input, found by the gather, is reported here: the kernels so far stay in bounds on it (keys of
+            // NaN quantize to 0, every link is checked). Going on sent all particles, which one NaN in the bounding
+            // cube gives the same key, through three re-key rounds and one thread's bucket.
+            return hs.nonfinite ? TG_ERR_NONFINITE : TG_OK;
         };
         TG_TRY(run_round());
         const int64_t Mr = (int64_t)hs.nodes;
@@ -1975,7 +1974,6 @@ tg_status build_tree(tg_tree_s *T, const double *pos, const StageMH &stage_mh,
         TG_TRY(read_summary());
     }
     if (hs.bad) {
-        if (nonfinite_seen) return TG_ERR_NONFINITE;
         set_last_error_msg("internal error: octree build produced an invalid node reference");
         return TG_ERR_CUDA;
     }
@@ -2076,8 +2074,7 @@ tg_status build_tree(tg_tree_s *T, const double *pos, const StageMH &stage_mh,
     if (req) TG_CUDA(cudaMemcpyAsync(rq.data(), req, sizeof(unsigned long long) * nsys, cudaMemcpyDeviceToHost, st));
     TG_CUDA(cudaStreamSynchronize(st));
     const int sort_bad = flags[0], links_bad = flags[1];
-    if (nonfinite_seen || sort_bad || links_bad) {
-        if (nonfinite_seen) return TG_ERR_NONFINITE;
+    if (sort_bad || links_bad) {
         if (sort_bad) {
             set_last_error_msg("radix sort: a tile's look-back did not complete within its bound");
             return TG_ERR_QUEUE_TIMEOUT;
