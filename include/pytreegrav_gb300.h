@@ -140,7 +140,8 @@ tg_status tg_tree_set_walk_config(tg_tree tree, int warps_per_block, int first_s
  * launch replays the graph on `stream` (zeroing the counters, the walk, and the large-stack pass
  * over the groups that overflowed the first stack) with no host synchronisation and writes `out`
  * (device, ntot x W, the caller's order); status waits for `stream` and returns the last replay's
- * status. The tree and `out` must outlive the graph; replays on one graph must not overlap. */
+ * status. The tree and `out` must outlive the graph; replays on one graph must not overlap. A graph may be
+ * freed while its last replay is running: its memory is used again after that. */
 typedef struct tg_walk_graph_s *tg_walk_graph;
 tg_status tg_walk_graph_create(tg_tree tree, int fields, int quadrupole, double theta, double G,
                                int group_size, int grouping, double *out, tg_walk_graph *graph);

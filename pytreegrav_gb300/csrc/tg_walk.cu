@@ -2743,6 +2743,7 @@ struct tg_walk_graph_s {
     int2 *groups = nullptr;  // owned when the grouping is not the tree's cached one
     int *groot = nullptr, *gorder = nullptr;
     int64_t kernels = 0;     // kernel nodes per replay
+    cudaEvent_t replayed = nullptr;  // recorded after each replay, on its stream
 };
 
 namespace {
@@ -2751,6 +2752,11 @@ void graph_release(tg_walk_graph_s *g) {
     if (!g) return;
     if (g->exec) cudaGraphExecDestroy(g->exec);
     if (g->graph) cudaGraphDestroy(g->graph);
+    // the buffers may be used again once the last replay, whatever its stream, is done with them
+    if (g->replayed) {
+        if (cudaStreamWaitEvent(0, g->replayed, 0) != cudaSuccess) cudaGetLastError();
+        tg::release_event(g->replayed, false);
+    }
     void *bufs[] = {g->scratch, g->thi, g->tlo, g->groups, g->groot, g->gorder};
     for (void *b : bufs)
         if (b) cudaFreeAsync(b, 0);
@@ -2856,8 +2862,10 @@ tg_status tg_walk_graph_create(tg_tree t, int fields, int quadrupole, double the
 
 tg_status tg_walk_graph_launch(tg_walk_graph g, void *stream) {
     if (!g) return TG_ERR_BAD_ARG;
+    if (!g->replayed) TG_CUDA(tg::pool_event(&g->replayed, false));
     TG_CUDA(cudaGraphLaunch(g->exec, (cudaStream_t)stream));
     tg::note_launches(g->kernels);
+    TG_CUDA(cudaEventRecord(g->replayed, (cudaStream_t)stream));
     return TG_OK;
 }
 

@@ -132,3 +132,31 @@ def test_side_stream_is_joined_when_a_launch_on_it_fails(fake):
         assert rc == 0, (rc, L.tg_last_error())
         assert any("k_prep_targets" in l[0] for l in log)
     """)
+
+
+def test_graph_memory_waits_for_the_last_replay(fake):
+    """A walk graph replayed on a stream of the caller's and freed: its buffers are given back on a stream that waits for
+    that replay first."""
+    fake("""
+        rc, t = build()
+        assert rc == 0
+        out, g = np.empty((n, 3)), ctypes.c_void_p()
+        assert L.tg_walk_graph_create(t, _lib.TG_FIELD_ACCEL, 0, 0.7, 1.0, 32, _lib.TG_GROUP_TREE, _lib.ptr(out),
+                                      ctypes.byref(g)) == 0
+        stream = ctypes.c_void_p()
+        F.cudaStreamCreateWithFlags(ctypes.byref(stream), 1)
+        events = F.fake_events()
+        F.fake_clear_log()
+        for _ in range(3):
+            assert L.tg_walk_graph_launch(g, stream) == 0
+        assert L.tg_walk_graph_free(g) == 0
+        log = [l.split() for l in F.fake_log().decode().splitlines()]
+        replays = [k for k, l in enumerate(log) if l[0] == "graph-launch"]
+        assert len(replays) == 3
+        frees = [k for k, l in enumerate(log) if l[0] == "free"]
+        assert frees
+        after = [l[1] for l in log[replays[-1]:] if l[0] == "record" and l[2] == hex(stream.value)]
+        waits = [k for k, l in enumerate(log) if l[0] == "wait" and l[1] in after and l[2] == log[frees[0]][2]]
+        assert waits and waits[0] < frees[0], log
+        assert F.fake_events() <= events + 1  # one event, back in the pool
+    """)
