@@ -125,6 +125,7 @@ tg_status check_finite(const double *const *arrs, const int64_t *counts, int k, 
 void destroy(tg_tree_s *t) {
     if (!t) return;
     cudaStream_t st = t->stream;
+    if (t->ev_used) cudaStreamWaitEvent(st, t->ev_used, 0);
     auto f = [&](void *p) {
         if (p) cudaFreeAsync(p, st);
     };
@@ -137,6 +138,7 @@ void destroy(tg_tree_s *t) {
     release_event(t->ev_join, false, t->dev);
     release_event(t->ev_topo, false, t->dev);
     release_event(t->ev_built, false, t->dev);
+    release_event(t->ev_used, false, t->dev);
     delete t;
 }
 
@@ -283,6 +285,8 @@ tg_status tg_tree_quadrupoles(tg_tree t, const double **quad, void *stream) {
     if (!t || !quad) return TG_ERR_BAD_ARG;
     *quad = nullptr;
     if (!t->has_quads) return TG_OK;
+    tree_wait_built(t, (cudaStream_t)stream);
+    const TreeUse use{t, nullptr, (cudaStream_t)stream};
     TG_TRY(ensure_quad64(t, (cudaStream_t)stream));
     *quad = t->quad;
     return TG_OK;

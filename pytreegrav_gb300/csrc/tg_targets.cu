@@ -233,6 +233,8 @@ tg_status tg_targets_create(tg_tree src, const double *pos, const double *h, int
         rc = tree_groups(ts->tt, group_size, st);
     }
     if (rc == TG_OK) rc = targets_refine_groups(ts, st);
+    tree_mark_used(src, st);  // its arena; the set's groups
+    tree_mark_used(ts->tt, st);
     if (rc != TG_OK) {
         tg_targets_free(ts);
         return rc;
@@ -243,6 +245,7 @@ tg_status tg_targets_create(tg_tree src, const double *pos, const double *h, int
 
 tg_status tg_targets_free(tg_targets ts) {
     if (!ts) return TG_OK;
+    if (ts->tt && ts->tt->ev_used) cudaStreamWaitEvent(ts->stream, ts->tt->ev_used, 0);
     if (ts->src_node) cudaFreeAsync(ts->src_node, ts->stream);
     if (ts->tt) tg_tree_free(ts->tt);
     delete ts;
@@ -272,6 +275,7 @@ tg_status tg_targets_groups_copy(tg_targets ts, int32_t *first, int32_t *count, 
     tg_tree_s *tt = ts->tt;
     const int64_t ng = tt->ngroups;
     tree_wait_built(ts->src, st);
+    tree_wait_built(tt, st);
     if (src_node) TG_TRY(targets_src_nodes(ts, st));
     const cudaMemcpyKind kind = mem == TG_MEM_HOST ? cudaMemcpyDeviceToHost : cudaMemcpyDeviceToDevice;
     if (first || count) {

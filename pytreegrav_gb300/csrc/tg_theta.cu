@@ -729,6 +729,7 @@ extern "C" {
 tg_status tg_tree_groups(tg_tree t, int group_size, int64_t *ngroups, void *stream) {
     if (!t || !ngroups || !valid_gs(group_size)) return TG_ERR_BAD_ARG;
     tree_wait_built(t, (cudaStream_t)stream);
+    const TreeUse use{t, nullptr, (cudaStream_t)stream};
     TG_TRY(tree_groups(t, group_size, (cudaStream_t)stream));
     *ngroups = t->ngroups;
     return TG_OK;
@@ -794,6 +795,7 @@ tg_status tg_tree_last_group_stats(tg_tree t, uint32_t *out, int mem, void *stre
 tg_status tg_theta_features(tg_tree t, int group_size, int quadrupole, float *features, void *stream) {
     if (!t || !features || !valid_gs(group_size)) return TG_ERR_BAD_ARG;
     tree_wait_built(t, (cudaStream_t)stream);
+    const TreeUse use{t, nullptr, (cudaStream_t)stream};
     return features_device(t, group_size, quadrupole, features, (cudaStream_t)stream);
 }
 
@@ -932,6 +934,7 @@ tg_status tg_theta_tolerances(tg_tree t, int group_size, int quadrupole, const f
     if (!t || !u || !tol || !valid_gs(group_size)) return TG_ERR_BAD_ARG;
     cudaStream_t st = (cudaStream_t)stream;
     tree_wait_built(t, st);
+    const TreeUse use{t, nullptr, st};
     TG_TRY(tree_groups(t, group_size, st));
     float *feat = nullptr;
     const int64_t nfeat = NF * std::max<int64_t>(t->ngroups, 1);
@@ -1001,6 +1004,7 @@ tg_status tg_targets_features(tg_targets ts, int quadrupole, float *features, vo
     cudaStream_t st = (cudaStream_t)stream;
     tree_wait_built(ts->src, st);
     tree_wait_built(ts->tt, st);
+    const TreeUse use{ts->src, ts->tt, st};
     return features_targets(ts, quadrupole, features, st);
 }
 
@@ -1009,6 +1013,7 @@ tg_status tg_targets_tolerances(tg_targets ts, int quadrupole, const float *u, f
     cudaStream_t st = (cudaStream_t)stream;
     tree_wait_built(ts->src, st);
     tree_wait_built(ts->tt, st);
+    const TreeUse use{ts->src, ts->tt, st};
     const int64_t ng = ts->tt->ngroups;
     float *feat = nullptr;
     const int64_t nfeat = NF * std::max<int64_t>(ng, 1);

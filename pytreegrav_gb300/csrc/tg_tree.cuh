@@ -136,13 +136,35 @@ struct tg_tree_s {
     // point orders its own stream after ev_built, and tree grouping, which needs no moments, starts
     // from ev_topo on the side stream.
     cudaEvent_t ev_topo = nullptr, ev_built = nullptr;
+    // Recorded at the end of each call that returns with work on the tree still queued (a target set's groups,
+    // features, the FP64 quadrupoles, a grouping): what it made on the tree may be read on another stream, and
+    // the tree freed, only after it. Every call waits for it and records it anew, so the last record covers all.
+    cudaEvent_t ev_used = nullptr;
 };
 
 namespace tg {
-// Orders work on s after the tree's build (a no-op when s is the build's stream).
+// Orders work on s after the tree's build and after the last call that left work queued on it (a no-op on the
+// streams of both).
 inline void tree_wait_built(const tg_tree_s *t, cudaStream_t s) {
     if (t && t->ev_built) cudaStreamWaitEvent(s, t->ev_built, 0);
+    if (t && t->ev_used) cudaStreamWaitEvent(s, t->ev_used, 0);
 }
+// At the end of a call that leaves work on the tree queued on s (see ev_used); where it cannot be recorded, the host
+// waits for it.
+inline void tree_mark_used(tg_tree_s *t, cudaStream_t s) {
+    if (!t) return;
+    if ((!t->ev_used && pool_event(&t->ev_used, false) != cudaSuccess) || cudaEventRecord(t->ev_used, s) != cudaSuccess)
+        cudaStreamSynchronize(s);
+}
+// The same when a scope ends, whatever it returns.
+struct TreeUse {
+    tg_tree_s *a, *b;
+    cudaStream_t s;
+    ~TreeUse() {
+        tree_mark_used(a, s);
+        tree_mark_used(b, s);
+    }
+};
 // Bits of a tree's sort error word: a sort's look-back ran out (its result is the identity permutation); the
 // grouping is not a partition of the particles.
 constexpr int SORT_ERR_SORT = 1, SORT_ERR_GROUPS = 2;

@@ -160,3 +160,65 @@ def test_graph_memory_waits_for_the_last_replay(fake):
         assert waits and waits[0] < frees[0], log
         assert F.fake_events() <= events + 1  # one event, back in the pool
     """)
+
+
+def test_work_left_queued_orders_other_streams(fake):
+    """What a call leaves queued on its stream -- a target set's groups, features, a grouping, FP64 quadrupoles -- comes
+    before the next call's work on another stream, and before the memory is given back on the build's."""
+    fake("""
+        from pytreegrav_gb300 import theta as th
+        A, B = ctypes.c_void_p(), ctypes.c_void_p()
+        for s in (A, B):
+            F.cudaStreamCreateWithFlags(ctypes.byref(s), 1)
+        a, b = hex(A.value), hex(B.value)
+        out, feat, ng, quad = np.empty((n, 3)), np.empty((n, 16), np.float32), ctypes.c_int64(), ctypes.c_void_p()
+
+        def log_of(f):
+            F.fake_clear_log()
+            assert f() == 0, L.tg_last_error()
+            return [l.split() for l in F.fake_log().decode().splitlines()]
+
+        def left_behind(log):  # the events recorded on A after its last launch
+            last = max(k for k, l in enumerate(log) if l[0].startswith("launch") and l[2] == a)
+            events = [l[1] for l in log[last:] if l[0] == "record" and l[2] == a]
+            assert events or any(l[0] == "synchronize" and l[2] == a for l in log[last:]), log
+            return events
+
+        def waits_first(log, events, stream, what):
+            at = [k for k, l in enumerate(log) if l[0].startswith(what) and l[2] == stream]
+            assert at, log
+            assert not events or any(l[0] == "wait" and l[1] in events and l[2] == stream for l in log[:at[0]]), log
+
+        def fields(stream):
+            return L.tg_tree_fields(t, None, None, n, 2, 0, 0.7, 1.0, 32, _lib.TG_GROUP_TREE, _lib.TG_ORDER_TREE, _lib.TG_FP32,
+                                    None, _lib.TG_MEM_HOST, _lib.ptr(out), stream)
+
+        first = [lambda: L.tg_tree_groups(t, 32, ctypes.byref(ng), A),
+                 lambda: L.tg_theta_features(t, 32, 0, _lib.ptr(feat), A),
+                 lambda: L.tg_tree_quadrupoles(t, ctypes.byref(quad), A)]
+        for call in first:
+            for then in ("other stream", "free"):
+                rc, t = build()
+                assert rc == 0
+                ev = left_behind(log_of(call))
+                if then == "free":
+                    waits_first(log_of(lambda: L.tg_tree_free(t)), ev, "(nil)", "free")
+                else:
+                    waits_first(log_of(lambda: fields(B)), ev, b, "launch")
+                    L.tg_tree_free(t)
+        for then in ("other stream", "features", "free"):
+            rc, t = build()
+            ts = ctypes.c_void_p()
+            ev = left_behind(log_of(lambda: L.tg_targets_create(t, _lib.ptr(x), _lib.ptr(h), n, 32, _lib.TG_MEM_HOST, A,
+                                                                ctypes.byref(ts))))
+            if then == "other stream":
+                log = log_of(lambda: L.tg_targets_fields(ts, 2, 0, 0.7, 1.0, _lib.TG_FP32, None, _lib.TG_MEM_HOST,
+                                                         _lib.ptr(out), B))
+                waits_first(log, ev, b, "launch")
+            elif then == "features":
+                ev2 = ev
+                log = log_of(lambda: L.tg_targets_features(ts, 0, _lib.ptr(feat), B))
+                waits_first(log, ev2, b, "launch")
+            L.tg_targets_free(ts)
+            waits_first(log_of(lambda: L.tg_tree_free(t)), ev if then == "free" else [], "(nil)", "free")
+    """)
