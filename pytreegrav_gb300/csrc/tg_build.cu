@@ -2090,10 +2090,13 @@ tg_status build_tree(tg_tree_s *T, const double *pos, const StageMH &stage_mh,
     }
     // everything but the tree's arrays and the depth lists has been read (the side stream was joined ahead of k_write);
     // the moment pass's lists and sums take its place. Peak: 409 bytes per particle at 2e6 (452 when the temporaries
-    // stayed to the end)
-    for (DevArray<unsigned char> *mem : {&temps, &slots, &elem_mem, &round_mem, &numbering, &by_key.mem, &by_sys.mem,
-                                         &numbered.mem})
-        mem->reset();
+    // stayed to the end). Small builds keep them: the frees' ~4 us would come before the moment pass, with the GPU
+    // idle, and they hold less than EARLY_FREE times 452 bytes, 0.24 GB.
+    constexpr int64_t EARLY_FREE = 1 << 19;
+    if (N >= EARLY_FREE)
+        for (DevArray<unsigned char> *mem : {&temps, &slots, &elem_mem, &round_mem, &numbering, &by_key.mem, &by_sys.mem,
+                                             &numbered.mem})
+            mem->reset();
     // 9. moments: nodes deeper than DEPTH_CAP by climbing, then one launch per depth, deepest first
     // (the moment kernels bound every link they follow). With quadrupoles the pass sums them in FP32
     // for the FP32 walk; the FP64 quadrupoles come from ensure_quad64 when first needed, which the
