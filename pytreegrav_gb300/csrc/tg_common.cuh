@@ -236,8 +236,8 @@ __device__ __forceinline__ long long scan_look_back(long long sum, int tile, uns
 // the one before is still finishing; chain_wait (first, in every block, before any memory is touched) then waits
 // for that kernel's completion, which includes that of all before it, and chain_next lets the following kernel come
 // up in its turn, once every block here has got past its wait. A kernel without chain_wait must not be
-// launched this way. Saves most of the ~2 us and of the ramp between two dependent kernels: build of 12345 particles (49
-// launches) 322 -> 244 us, with its walk 673 -> 574; build of 1e6 688 -> 636.
+// launched this way. Saves most of the ~2 us and of the ramp between two dependent kernels: build of 12345 particles 322
+// -> 244 us, with its walk (50 launches in all) 673 -> 574; build of 1e6 688 -> 636.
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 template <class... P, class... A>
@@ -264,7 +264,7 @@ inline cudaError_t launch_after(void (*kernel)(P...), int64_t grid, int block, s
 
 inline int div_up(int64_t a, int64_t b) { return (int)((a + b - 1) / b); }
 
-// Device-wide helpers implemented in tg_scan.cu / tg_sort.cu.
+// Device-wide helpers implemented in tg_sort.cu.
 tg_status exclusive_scan_i64(const int64_t *in, int64_t *out, int64_t n, int64_t *total_dev,
                              cudaStream_t s);
 tg_status exclusive_scan_i32(const int32_t *in, int32_t *out, int64_t n, cudaStream_t s);

@@ -328,7 +328,7 @@ __device__ __forceinline__ int bin_screen(const CorrArgs &a, float r, float er) 
 // A visit reads one 48-byte record, links included; the jitter, the whole-node test and the bin come from
 // integer and FP32 arithmetic; a contribution takes 11 FP64 instructions (16 before).
 // VelocityStructFunc's walk, 200000 Plummer particles, 57 bins: 11.1 ms with the additions in the step (FP64
-// pipe 79 % busy), 5.17 ms now; 1e6 particles 51.9 -> 23.8 ms. Bound by the FP64 pipe (70 % busy) and the rows'
+// pipe 79 % busy), 5.0 ms now; 1e6 particles 51.9 -> 23.8 ms. Bound by the FP64 pipe (70 % busy) and the rows'
 // read-add-write latency.
 constexpr int CORR_QUEUE = 16;  // entries per lane (8 to 32: within 4 %)
 

@@ -1,9 +1,11 @@
 // Device-wide exclusive scans and a stable LSD radix sort of (uint64 key, uint32 value) pairs.
 //
 // The sort replaces pytreegrav's _radix_argsort (octree.py:101-132). Any stable sort of the keys
-// yields the same permutation, which is what makes the GPU order bit-identical to the reference:
-// 8-bit digits, one tile of 4096 keys per CTA, ranks made stable by processing each warp's slice
-// in order with __match_any_sync, and per-(digit, tile) offsets from a digit-major scan.
+// yields the same permutation, which is what makes the GPU order bit-identical to the reference.
+// radix_sort_pairs is a one-sweep sort: digits of up to nine bits, one kernel per digit over tiles of 4096 or
+// 6144 pairs, each tile's offsets by decoupled look-back (k_onesweep). The two-kernel passes with 8-bit digits and
+// tiles of 4096 keys (radix_hist, radix_scatter; lanes of equal digits found by ballots, offsets from a digit-major
+// scan) remain for the Morton order that allocates nothing (tg_noalloc.cu).
 #include <algorithm>
 #include <cstdio>
 #include <mutex>
@@ -440,6 +442,9 @@ __global__ void __launch_bounds__(RS_THREADS) radix_scatter(const uint64_t *keys
 // its exclusive prefix, and writes the tile out. A look-back spin is bounded; running out sets the sort's own
 // error word instead of hanging, and the sort then leaves the identity permutation (k_sort_fallback).
 // Digits have up to nine bits (63 key bits: seven passes; a sort's bits are shared out evenly over its passes).
+// The passes follow the published one-sweep method (Adinets and Merrill, "Onesweep: A Faster Least Significant Digit
+// Radix Sort for GPUs", 2022); that a warp finds its lanes of equal digits by an OR of lane masks into a word per digit
+// is likewise a known way of GPU radix ranking, in place of a match instruction.
 // A pass is bound by the chain of one tile (load, rank, publish, look back, write) with the ~300 tiles that fit the
 // SMs, a third of the copy bandwidth: hence few instructions per key (lanes of equal digits find one another by
 // an OR into a word per digit, ~12 instructions where ballots over the digit's bits took ~45) and the tile's own
